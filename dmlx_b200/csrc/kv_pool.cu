@@ -21,6 +21,7 @@
 
 #include <vector>
 
+#include "attn_prompt.cuh"
 #include "common.h"
 #include "kv_pool.cuh"
 #include "tma.cuh"
@@ -668,7 +669,10 @@ static b200_status kv_create(const b200_kv_config* c_in, const b200_kv_layer* la
   // split-K scratch for the attention kernel
   kv->max_chunks = c->attn_scratch_chunks > 0 ? c->attn_scratch_chunks : c->n_pages / 4 + c->max_rows + 8;
   KV_ALLOC(kv->d_chunk_start, sizeof(int) * (c->max_rows + 2));
-  KV_ALLOC(kv->d_groups, sizeof(int) * 3 * (c->max_rows + 2));
+  const size_t group_ints = ((size_t)3 * (c->max_rows + 2) + 1) / 2 * 2;  // (the work list behind them is read in pairs)
+  KV_ALLOC(kv->d_groups, sizeof(int) * (group_ints + b200_attn_prompt_plan_ints(c->max_rows)));
+  kv->d_prompt = kv->d_groups + group_ints;
+  cudaMemset(kv->d_prompt, 0, sizeof(int) * 8);
   KV_ALLOC(kv->d_part_o, sizeof(float) * (size_t)kv->max_chunks * c->n_q_heads * std::max(kv->max_vd, 1));
   KV_ALLOC(kv->d_part_ml, sizeof(float) * (size_t)kv->max_chunks * c->n_q_heads * 2);
 #undef KV_ALLOC

@@ -73,6 +73,7 @@ struct b200_kv {
   int max_chunks = 0;
   // row-group plan of the prefill attention path: [3][max_rows + 2] = group_first | part_base | row_group
   int* d_groups = nullptr;
+  int* d_prompt = nullptr;  // work list of attn_prompt.cu, behind d_groups: counters, then {group, chunk} per item
   // 3-D tensor maps over the bf16 pools: [layer][page*kv_head*32 rows][head_dim], box 64 x 32 x 1
   CUtensorMap kmap, vmap;
 };

@@ -19,6 +19,7 @@
 
 #include <algorithm>
 
+#include "attn_prompt.cuh"
 #include "common.h"
 #include "kv_pool.cuh"
 #include "ptx.cuh"
@@ -1674,6 +1675,10 @@ b200_status b200_paged_attn_prefill_strided(b200_kv* kv, int32_t layer, const vo
   // Prefill batches of 1024 rows and more have rows to spare for parallelism (256 groups x kv heads and up): one chunk
   // per group, as long as its context, and the kernel writes the normalised rows itself: no f32 partials, no combine
   // pass (at 8192 rows of config 5 the partials were 400 MB per layer and the combine pass 7 % of the scenario).
+  // bf16 pages go through tcgen05 (attn_prompt.cu), 4 to 6 times as fast at 512 rows and more and level with the groups below at 17 rows.
+  // What stays here: FP8 pages, rows that TMA cannot address, and the hooks that force a chunk length or the chunked form.
+  if (b200_attn_prefill_direct && b200_attn_pages_per_chunk <= 0 && b200_attn_prompt_takes(kv, d_q, q_stride, d_out))
+    return b200_attn_prompt(kv, layer, d_q, q_stride, d_row_seq, d_row_ctx, total_rows, d_out, stream, total_rows < 1024, reuse_plan != 0);
   const bool single_chunk = total_rows >= 1024 && b200_attn_prefill_direct;
   const int ppc = single_chunk ? std::max(c.max_pages_per_seq, 1)
                                : (b200_attn_pages_per_chunk <= 0 ? 8 : std::min(std::max(b200_attn_pages_per_chunk, 4), kMaxChunkPages));

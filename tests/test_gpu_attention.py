@@ -260,3 +260,52 @@ def test_long_contexts_of_the_attention_microbench(kv_dtype):
     for s in range(len(ctxs)):
         r, c = _close(got[s], want[s])
         assert r <= REL_TOL and c >= COS_TOL, (s, ctxs[s], r, c)
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(32, 8, 128), (8, 1, 128), (4, 4, 64), (8, 4, 64)])
+@pytest.mark.parametrize("scratch", [0, 100000])   # partial sums that hardly fit (key ranges stay whole), and room to split them
+@pytest.mark.parametrize("rows", [(31, 32, 33), (63, 64, 65, 1, 1), (127, 128, 129, 2), (255, 256, 257, 1), (1, 1, 1), (700, 330, 1, 1)])
+def test_portions_at_the_edges_of_the_row_tiles(hq, hkv, d, scratch, rows):
+    """Portions of one token less and more than a tile of 128 rows or a pair of them holds (for each size of the GQA group), contexts at the
+    borders of a page and of a block of 128 keys, decoding rows among them: every row against the row-by-row kernel on the same pool, some
+    against the oracle.  One key is no number in one dimension: it weighs nothing, as in the row-by-row kernel."""
+    from dmlx_b200 import device as dev
+
+    rng = np.random.default_rng(sum(rows) + hq + d)
+    before = [0, 1, 95, 127, 128, 1500]
+    reqs = [(before[(i + len(rows)) % len(before)], n) for i, n in enumerate(rows)]
+    totals = [c + n for c, n in reqs]
+    n_pages, n_rows = sum(-(-t // 32) for t in totals) + 4, sum(rows)
+    if scratch == 0:
+        # the smallest scratch that the row-by-row kernel, and the limit of batches below 1024 rows, accept
+        scratch = sum(n * -(-t // 256) for (_, n), t in zip(reqs, totals)) + n_rows + 8
+    kv = dev.PagedKVCache(1, hkv, d, n_pages, len(reqs), -(-max(totals) // 32), hq, max_rows=max(totals) + n_rows, attn_scratch_chunks=scratch)
+    kv.set_free_order(rng.permutation(n_pages).tolist())
+    k = ref_math.bf16_round(rng.normal(0, 1, (sum(totals), hkv, d)).astype(np.float32))
+    v = ref_math.bf16_round(rng.normal(0, 1, (sum(totals), hkv, d)).astype(np.float32))
+    q = ref_math.bf16_round(rng.normal(0, 1, (n_rows, hq, d)).astype(np.float32))
+    nowhere = totals[0] // 2   # of the first request
+    kd = torch.tensor(k, device="cuda").bfloat16()
+    kd[nowhere, :, 3] = float("nan")
+    kv.reserve(dev.pack_desc_array([(s, t, 0, -1) for s, t in enumerate(totals)]).cuda())
+    kv.append(0, kd, torch.tensor(v, device="cuda").bfloat16())
+    row_seq = np.concatenate([np.full(n, s, np.int32) for s, (_, n) in enumerate(reqs)])
+    row_ctx = np.concatenate([np.arange(c + 1, c + n + 1, dtype=np.int32) for c, n in reqs])
+    qd, rs, rc = torch.tensor(q, device="cuda").bfloat16(), torch.tensor(row_seq, device="cuda"), torch.tensor(row_ctx, device="cuda")
+    got = kv.attention(0, qd, rs, rc, prefill=True).float().cpu().numpy()
+    again = kv.attention(0, qd, rs, rc, prefill=True).float().cpu().numpy()
+    per_row = kv.attention(0, qd, rs, rc).float().cpu().numpy()
+    assert kv.error_word() == 0
+    assert np.array_equal(got, again)
+    # both round P and the result to bf16: 2^-8 of the largest weight and of the value, twice
+    assert np.abs(got - per_row).max() <= 1.6e-2 * np.abs(per_row).max()
+    first = np.concatenate([[0], np.cumsum(totals)])
+    for r in sorted({0, 1, 2, 30, 31, 32, 33, 63, 64, 65, 126, 127, 128, 255, 256, n_rows - 2, n_rows - 1} & set(range(n_rows))):
+        s, c = int(row_seq[r]), int(row_ctx[r])
+        keep = np.arange(first[s], first[s] + c)
+        want = ref_math.gqa_attention_decode(q[r], *(x[keep[keep != nowhere] if c > 1 or s > 0 else keep] for x in (k, v)))
+        if s == 0 and c == 1 and nowhere == 0:
+            want = np.zeros_like(want)
+        rel, cos = _close(got[r], want)
+        assert rel <= REL_TOL and (cos >= COS_TOL or not want.any()), (r, s, c, rel, cos)
+    kv.close()
