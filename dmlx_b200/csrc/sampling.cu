@@ -2,35 +2,74 @@
 // (src/sampling.zig:42-72, 175-242, 258-268, 298-322, 328-375), so that only one token id per
 // request crosses PCIe for non-greedy requests too.  The uniform variate of each draw is an input.
 //
-// One CTA of 1024 threads per row.  The row is read from L2 several times (first maximum,
-// log-sum-exp, the digit passes of a radix select, one gather pass); nothing of vocabulary size is
-// kept on chip.  Ordering follows the reference's stable descending sort: a candidate is the
-// 64-bit key (descending score bits << 32 | token id), so equal scores keep index order.  The
-// candidates are taken from that order kChunk at a time: one pass over the row bounds the chunk
-// (the kChunk-th smallest per-thread minimum), a second gathers the few keys under the bound, a
-// bitonic network in shared memory sorts them; a radix select over the key backs this up for rows
-// that defeat the bound.  The sums over the sorted prefix (softmax denominator, nucleus cut,
-// renormalised draw) run on one thread in the reference's order in f32.
+// A row belongs to a cluster of up to eight CTAs, a contiguous part of the vocabulary each; it is read from L2 a few times and what has to be
+// known of the whole row goes through distributed shared memory to the cluster's first CTA.  Ordering follows the reference's stable
+// descending sort: a candidate is the 64-bit key (descending score bits << 32 | token id), so equal scores keep index order.
+//
+// Nothing of vocabulary size is sorted.  The scores are counted in 2048 bins by their distance from the maximum (1/64 each, the last one for
+// all beyond 32), with the bins' weights; the k-th candidate, the end of the nucleus and the drawn token are each found first by bin, from
+// the bins' running sums, and then inside it, among its few keys, sorted in shared memory.  Where all bins up to the one that matters hold
+// no more than 2048 keys they are sorted at once and everything is decided on that list; for up to 512 candidates that is tried first on the
+// bins that hold as many of the threads' maxima, without counting the row.  A bin with more keys than that is counted again
+// in 2048 finer ranges of keys, as often as it takes (keys are unique, so at most five times).
+//
+// A bin's weight is edge * (count - deficit): 1 - exp(-x), x the distance behind the bin's near edge, is below 2^-6 and is summed in units of
+// 2^-22 in an integer, so sums do not depend on the order of the additions.  Running sums over bins and candidates are f64.
+//
+// Bound by the latency of its passes (loads, cluster barriers), not by bytes.  64 rows of 128256 bf16 words on one B200: greedy 20 us, top-k 50 40,
+// the whole distribution 54, a nucleus of 0.9 over all words 87 (thousands of words: 140).  One CTA per row that walked the sorted order 512
+// candidates at a time, one thread adding, took 800 to 1760 us for a mixture of these rows; this takes 87 to 100.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "common.h"
 
+namespace cg = cooperative_groups;
+
 namespace {
 
-constexpr int kThreads = 1024;
-constexpr int kCap = 2048;    // keys held in shared memory
-constexpr int kChunk = 512;   // candidates taken from the sorted order at a time
+constexpr int kThreads = 512, kWarps = kThreads / 32;
+constexpr int kBins = 2048, kPerThread = kBins / kThreads;
+constexpr int kCap = 2048;     // keys sorted in shared memory
+constexpr int kMaxCluster = 8;
+constexpr int kFew = 512;      // candidates that the threads' maxima are asked for
+constexpr float kBinsPerUnit = 64.f;
+
+struct Bins {  // running sums over the bins, inclusive
+  unsigned n[kBins];
+  double m[kBins];
+};
 
 struct Shared {
-  unsigned long long key[kCap];
-  float e[kChunk];
-  int hist[256];
-  float red_f[32];
-  int red_i[32];
-  int sel_digit, sel_below, sel_count, sel_total, count;
-  float acc, sum_exp, nucleus, carry;
-  int cutoff, done, seg;
-  unsigned token, last_idx;
+  unsigned hist_n[kBins], hist_d[kBins];  // this CTA's part: keys, deficits
+  Bins row;                               // (first CTA)
+  union {
+    Bins fine;                            // of the ranges inside one bin
+    struct {
+      unsigned long long key[kCap];
+      float weight[kCap];
+    } list;
+  };
+  double red_d[kWarps];
+  float red_f[kWarps];
+  int red_i[kWarps];
+  unsigned red_u[kWarps];
+  unsigned long long red_k[2 * kWarps];
+  // what a CTA hands to the others
+  float part_max;
+  int part_arg;
+  double part_sum[2];                     // of exp(logit - max), and of exp((logit - max) / temperature)
+  double warp_sum[kWarps];                // the latter by warp, in the order of the vocabulary
+  unsigned long long part_lo, part_hi;
+  // what the first CTA found
+  unsigned found, count;
+  double before, mass;
+  unsigned n_before;
+  unsigned token;
+  int owner;
+  double target;
 };
 
 template <typename T> struct Row {
@@ -73,10 +112,9 @@ __device__ __forceinline__ int load8(const Row<float>& r, int i0, float (&v)[8])
 
 // (score descending, token id ascending) as one ascending 64-bit key; -0 is folded into +0 so that
 // scores that compare equal share their bits.
-__device__ __forceinline__ unsigned long long cand_key(float logit, float temperature, int idx) {
-  float s = logit / temperature;
-  s += 0.0f;
-  unsigned u = __float_as_uint(s);
+__device__ __forceinline__ float score_of(float logit, float temperature) { return logit / temperature + 0.0f; }
+__device__ __forceinline__ unsigned long long key_of(float score, int idx) {
+  unsigned u = __float_as_uint(score);
   u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
   return ((unsigned long long)(~u) << 32) | (unsigned)idx;
 }
@@ -84,415 +122,588 @@ __device__ __forceinline__ float key_score(unsigned long long c) {
   const unsigned u = ~(unsigned)(c >> 32);
   return __uint_as_float((u & 0x80000000u) ? (u ^ 0x80000000u) : ~u);
 }
+__device__ __forceinline__ int bin_of(float distance) { return (int)fminf(fmaxf(distance * kBinsPerUnit, 0.f), (float)(kBins - 1)); }
 
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
+// One row's work: the CTA's threads, its part of the vocabulary, and the cluster it belongs to.
+template <typename T>
+struct Sampler {
+  cg::cluster_group cluster;
+  Shared& s;
+  Row<T> r;
+  int ranks, rank, tid, lane, warp;
+  int warp_part, lo, hi;  // a warp's part of the vocabulary (a multiple of 8), and this warp's
+  int unit_shift;         // deficits are in units of 2^-(22 - unit_shift)
+  float units;
 
-__device__ float block_sum(float v, Shared& s) {
-  __syncthreads();
-  v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) s.red_f[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    float t = warp_sum(s.red_f[threadIdx.x]);
-    if (threadIdx.x == 0) s.red_f[0] = t;
+  __device__ Sampler(Shared& sh, const Row<T>& row) : cluster(cg::this_cluster()), s(sh), r(row) {
+    ranks = cluster.num_blocks();
+    rank = cluster.block_rank();
+    tid = threadIdx.x; lane = tid & 31; warp = tid >> 5;
+    warp_part = ((r.V + ranks * kWarps - 1) / (ranks * kWarps) + 7) / 8 * 8;
+    lo = min((rank * kWarps + warp) * warp_part, r.V);
+    hi = min(lo + warp_part, r.V);
+    // a CTA's deficits of one bin stay below 2^32: 2^16 units each at most
+    unit_shift = 0;
+    while (((long long)warp_part * kWarps >> unit_shift) > 65535) ++unit_shift;
+    units = exp2f((float)(22 - unit_shift));
   }
-  __syncthreads();
-  return s.red_f[0];
-}
+  __device__ Shared& of(int q) { return *cluster.map_shared_rank(&s, q); }
 
-// First strict maximum of the row (src/sampling.zig:22-39): value through *out_max, index returned.
-template <typename T> __device__ int block_first_max(const Row<T>& r, Shared& s, float* out_max) {
-  float best = -INFINITY;
-  int bi = 0x7fffffff;
-  for (int base = 0; base < r.V; base += kThreads * 8) {
-    const int i0 = base + threadIdx.x * 8;
-    float v[8];
-    const int n = load8(r, i0, v);
+  // f(logits, first token, how many) over the thread's elements, eight neighbours at a time; Q of these loads are in flight
+  template <int Q, typename F>
+  __device__ __forceinline__ void each8(F f) {
+    int base = lo;
+    for (; base + Q * 256 <= hi; base += Q * 256) {
+      float v[Q][8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (j < n && v[j] > best) { best = v[j]; bi = i0 + j; }
-  }
-  auto better = [](float va, int ia, float vb, int ib) { return va > vb || (va == vb && ia < ib); };
+      for (int q = 0; q < Q; ++q) load8(r, base + (q * 32 + lane) * 8, v[q]);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (better(ov, oi, best, bi)) { best = ov; bi = oi; }
+      for (int q = 0; q < Q; ++q) f(v[q], base + (q * 32 + lane) * 8, 8);
+    }
+#pragma unroll 1
+    for (int i0 = base + lane * 8; i0 < hi; i0 += 256) {
+      float v[8];
+      load8(r, i0, v);
+      f(v, i0, min(hi - i0, 8));
+    }
   }
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) { s.red_f[threadIdx.x >> 5] = best; s.red_i[threadIdx.x >> 5] = bi; }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    best = s.red_f[threadIdx.x];
-    bi = s.red_i[threadIdx.x];
+  // f(logit, token) over the thread's elements with a logit from `least` to `most`
+  template <typename F>
+  __device__ __forceinline__ void each_within(float least, float most, F f) {
+    each8<2>([&](const float (&v)[8], int i0, int n) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j < n && !(v[j] < least) && !(v[j] > most)) f(v[j], i0 + j);
+    });
+  }
+  // Logits whose scores may fall into bins first..last (a little wider: rounding).
+  __device__ __forceinline__ void logits_of(int first, int last, float temperature, float gmax, float* least, float* most) {
+    const float slack = 1e-5f * (fabsf(gmax) + 32.f * temperature);
+    *most = first == 0 ? INFINITY : gmax - (float)first * (1.f / kBinsPerUnit) * temperature + slack;
+    *least = last == kBins - 1 ? -INFINITY : gmax - (float)(last + 1) * (1.f / kBinsPerUnit) * temperature - slack;
+  }
+
+  __device__ double block_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if (lane == 0) s.red_d[warp] = v;
+    __syncthreads();
+    double t = 0.0;
+    for (int w = 0; w < kWarps; ++w) t += s.red_d[w];
+    return t;
+  }
+
+  // First strict maximum of the row (src/sampling.zig:22-39).
+  __device__ int first_max(float* out_max, float* thread_max) {
+    float best = -INFINITY;
+    int bi = 0x7fffffff;
+    each8<4>([&](const float (&v)[8], int i0, int n) {
+      float top = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j < n) top = fmaxf(top, v[j]);
+      if (top > best) {
+        best = top;
+#pragma unroll
+        for (int j = 7; j >= 0; --j)
+          if (j < n && v[j] == top) bi = i0 + j;
+      }
+    });
+    *thread_max = best;
+    auto better = [](float va, int ia, float vb, int ib) { return va > vb || (va == vb && ia < ib); };
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, best, o);
       const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (better(ov, oi, best, bi)) { best = ov; bi = oi; }
     }
-    if (threadIdx.x == 0) { s.red_f[0] = best; s.red_i[0] = bi == 0x7fffffff ? 0 : bi; }
-  }
-  __syncthreads();
-  *out_max = s.red_f[0];
-  return s.red_i[0];
-}
-
-// Ascending bitonic sort of s.key[0, n2), n2 a power of two <= kCap.  All threads call.
-__device__ void sort_keys(Shared& s, int n2) {
-  for (int k = 2; k <= n2; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = threadIdx.x; i < n2; i += kThreads) {
-        const int x = i ^ j;
-        if (x > i) {
-          const unsigned long long a = s.key[i], c = s.key[x];
-          if ((a > c) == ((i & k) == 0)) { s.key[i] = c; s.key[x] = a; }
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-// Largest key of the m smallest keys >= lo_bound (most-significant-digit radix select over the whole
-// row); *out_count = how many keys lie in [lo_bound, result] (m, or fewer when the row runs out).
-// This is the general path: every element takes part in the first digit passes.
-template <typename T>
-__device__ unsigned long long radix_threshold(const Row<T>& r, float temperature, unsigned long long lo_bound, int m,
-                                              Shared& s, int* out_count) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  unsigned long long prefix = 0, mask = 0, thr = 0;
-  int need = m, taken = 0;
-  bool closed = false;
-  for (int b = 7; b >= 0 && !closed; --b) {
-    // digits of the token id that are zero for every element of the row
-    if (b == 3 || (b == 2 && r.V <= (1 << 16)) || (b == 1 && r.V <= (1 << 8))) continue;
-    const int shift = 8 * b;
-    __syncthreads();
-    if (tid < 256) s.hist[tid] = 0;
-    __syncthreads();
-    for (int base = 0; base < r.V; base += kThreads * 8) {
-      const int i0 = base + tid * 8;
-      float v[8];
-      const int n = load8(r, i0, v);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        unsigned long long c = 0;
-        bool valid = j < n;
-        if (valid) {
-          c = cand_key(v[j], temperature, i0 + j);
-          valid = c >= lo_bound && (c & mask) == prefix;
-        }
-        if (__any_sync(0xffffffffu, valid)) {
-          const unsigned digit = (unsigned)(c >> shift) & 255u;
-          // one shared-memory atomic per distinct digit of the warp: the leading digits of a row's
-          // scores fall into a handful of bins
-          const unsigned peers = __match_any_sync(0xffffffffu, valid ? digit : 256u + lane);
-          if (valid && lane == __ffs(peers) - 1) atomicAdd(&s.hist[digit], __popc(peers));
-        }
-      }
-    }
-    __syncthreads();
-    if (tid < 32) {
-      int loc[8], sum = 0;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { loc[q] = s.hist[lane * 8 + q]; sum += loc[q]; }
-      int incl = sum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-      }
-      const int total = __shfl_sync(0xffffffffu, incl, 31);
-      const int want = min(need, total), excl = incl - sum;
-      if (total > 0 && excl < want && want <= incl) {
-        int run = excl;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          if (run + loc[q] >= want) { s.sel_digit = lane * 8 + q; s.sel_below = run; s.sel_count = loc[q]; break; }
-          run += loc[q];
-        }
-      }
-      if (lane == 0) s.sel_total = total;
-    }
-    __syncthreads();
-    if (s.sel_total == 0) { *out_count = 0; return 0; }
-    need = min(need, s.sel_total) - s.sel_below;
-    taken += s.sel_below;
-    prefix |= (unsigned long long)s.sel_digit << shift;
-    mask |= 255ull << shift;
-    if (s.sel_count == need) {  // the whole bin is taken: no need to look at lower digits
-      thr = prefix | (shift ? ((1ull << shift) - 1) : 0ull);
-      closed = true;
-    }
-  }
-  if (!closed) thr = prefix;
-  *out_count = taken + need;
-  return thr;
-}
-
-// Appends every key in [lo_bound, hi_bound] to s.key (unordered); returns how many there are, which
-// may exceed kCap (only the first kCap are stored).
-template <typename T>
-__device__ int gather_keys(const Row<T>& r, float temperature, unsigned long long lo_bound, unsigned long long hi_bound,
-                           Shared& s) {
-  __syncthreads();
-  if (threadIdx.x == 0) s.count = 0;
-  __syncthreads();
-  for (int base = 0; base < r.V; base += kThreads * 8) {
-    const int i0 = base + threadIdx.x * 8;
-    float v[8];
-    const int n = load8(r, i0, v);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (j < n) {
-        const unsigned long long c = cand_key(v[j], temperature, i0 + j);
-        if (c >= lo_bound && c <= hi_bound) {
-          const int pos = atomicAdd(&s.count, 1);
-          if (pos < kCap) s.key[pos] = c;
-        }
-      }
-    }
-  }
-  __syncthreads();
-  return s.count;
-}
-
-// The m (<= kChunk) smallest keys >= lo_bound, sorted ascending into s.key[0, m); returns how many
-// there were.  Fast path: the m-th smallest of the 1024 per-thread minima bounds the m-th smallest of
-// the row from above, and for m <= kChunk only a few more than m keys lie under that bound, so one
-// pass finds the bound and a second gathers the candidates.  Rows that defeat the bound (a run of
-// equal scores longer than the buffer, or fewer eligible keys than threads) take the radix select.
-template <typename T>
-__device__ int next_chunk(const Row<T>& r, float temperature, unsigned long long lo_bound, int m, Shared& s) {
-  const int tid = threadIdx.x;
-  unsigned long long best = ~0ull;
-  for (int base = 0; base < r.V; base += kThreads * 8) {
-    const int i0 = base + tid * 8;
-    float v[8];
-    const int n = load8(r, i0, v);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (j < n) {
-        const unsigned long long c = cand_key(v[j], temperature, i0 + j);
-        if (c >= lo_bound && c < best) best = c;
-      }
-    }
-  }
-  __syncthreads();
-  s.key[tid] = best;
-  __syncthreads();
-  sort_keys(s, kThreads);
-  const unsigned long long tau = s.key[m - 1];  // ~0 when fewer than m threads saw an eligible key
-  int count = gather_keys(r, temperature, lo_bound, tau, s);
-  if (count > kCap) {
-    int exact = 0;
-    const unsigned long long thr = radix_threshold(r, temperature, lo_bound, m, s, &exact);
-    count = exact > 0 ? gather_keys(r, temperature, lo_bound, thr, s) : 0;
-  }
-  if (count == 0) return 0;
-  int n2 = 2;
-  while (n2 < count) n2 <<= 1;
-  for (int i = count + tid; i < n2; i += kThreads) s.key[i] = ~0ull;
-  __syncthreads();
-  sort_keys(s, n2);
-  return min(count, m);
-}
-
-// temperatureSample (src/sampling.zig:42-72): softmax of (logit - max) / T in index order, first
-// index whose cumulative probability exceeds u.  Each warp owns a contiguous segment of the row.
-template <typename T>
-__device__ unsigned sample_full_softmax(const Row<T>& r, float temperature, float gmax, float u, Shared& s) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  float part = 0.f;
-  for (int base = 0; base < r.V; base += kThreads * 8) {
-    float v[8];
-    const int n = load8(r, base + tid * 8, v);
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (j < n) part += expf((v[j] - gmax) / temperature);
-  }
-  const float sum = block_sum(part, s);
-  const int seg = ((r.V + 31) / 32 + 31) / 32 * 32;
-  const int lo = min(warp * seg, r.V), hi = min(lo + seg, r.V);
-  float ls = 0.f;
-  for (int i = lo + lane; i < hi; i += 32) ls += expf((to_f32(r.p[i]) - gmax) / temperature) / sum;
-  ls = warp_sum(ls);
-  __syncthreads();
-  if (lane == 0) s.red_f[warp] = ls;
-  __syncthreads();
-  if (tid == 0) {
-    float cum = 0.f;
-    s.seg = -1;
-    for (int w = 0; w < 32; ++w) {
-      const float c2 = cum + s.red_f[w];
-      if (u < c2) { s.seg = w; s.carry = cum; break; }
-      cum = c2;
-    }
-    s.token = (unsigned)(r.V - 1);  // sampleFromProbs returns n - 1 when u is never exceeded (:267)
-  }
-  __syncthreads();
-  if (s.seg == warp) {
-    float carry = s.carry;
-    unsigned tok = (unsigned)(hi - 1);
-    for (int base = lo; base < hi; base += 32) {
-      const int i = base + lane;
-      const float p = i < hi ? expf((to_f32(r.p[i]) - gmax) / temperature) / sum : 0.f;
-      float incl = p;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-      }
-      const unsigned hit = __ballot_sync(0xffffffffu, i < hi && u < carry + incl);
-      if (hit) { tok = (unsigned)(base + __ffs(hit) - 1); break; }
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) s.token = tok;
-  }
-  __syncthreads();
-  return s.token;
-}
-
-// Sum of exp(score - max_score) over every key <= hi_bound, as a parallel reduction.
-template <typename T>
-__device__ float sum_exp_below(const Row<T>& r, float temperature, unsigned long long hi_bound, float max_score, Shared& s) {
-  float part = 0.f;
-  for (int base = 0; base < r.V; base += kThreads * 8) {
-    const int i0 = base + threadIdx.x * 8;
-    float v[8];
-    const int n = load8(r, i0, v);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (j < n) {
-        const unsigned long long c = cand_key(v[j], temperature, i0 + j);
-        if (c <= hi_bound) part += expf(key_score(c) - max_score);
-      }
-    }
-  }
-  return block_sum(part, s);
-}
-
-// topKTopPSampler (src/sampling.zig:175-242).  The sorted order is walked kChunk candidates at a time.
-// Up to kChunk candidates (the usual top-k) everything, the softmax denominator included, is summed on
-// one thread in sorted order like the reference; above that the denominator is a parallel reduction
-// and only the nucleus cut and the draw walk the order, normally inside the first chunk.
-template <typename T>
-__device__ unsigned sample_top_k_top_p(const Row<T>& r, float temperature, int k_eff, float top_p, float u, float gmax,
-                                       Shared& s) {
-  const int tid = threadIdx.x;
-  const bool single = k_eff <= kChunk;
-  bool have_chunk = false;
-  int chunk_cnt = 0;
-  // the largest score is the largest logit's: division by a positive temperature keeps the order
-  const float max_score = gmax / temperature + 0.0f;
-  if (!single) {
-    unsigned long long hi = ~0ull;
-    if (k_eff < r.V) {
-      int exact = 0;
-      hi = radix_threshold(r, temperature, 0ull, k_eff, s, &exact);
-    }
-    const float total = sum_exp_below(r, temperature, hi, max_score, s);
-    if (tid == 0) s.sum_exp = total;
-    __syncthreads();
-  }
-  for (int pass = single ? 0 : 1; pass < 3; ++pass) {
-    // pass 0: softmax denominator over the top k; 1: nucleus cut; 2: the draw inside the nucleus
-    unsigned long long lo = 0;
-    int taken = 0;
-    const int limit = pass == 2 ? s.cutoff : k_eff;
-    __syncthreads();
-    if (tid == 0) { s.acc = 0.f; s.done = 0; }
-    __syncthreads();
-    while (taken < limit) {
-      int cnt;
-      if (single && have_chunk) {
-        cnt = chunk_cnt;
-      } else {
-        cnt = next_chunk(r, temperature, lo, min(kChunk, k_eff - taken), s);
-        if (cnt == 0) break;
-        for (int i = tid; i < cnt; i += kThreads) s.e[i] = expf(key_score(s.key[i]) - max_score);
-        __syncthreads();
-        have_chunk = true;
-        chunk_cnt = cnt;
-      }
-      const int use = min(cnt, limit - taken);
-      if (tid == 0) {
-        float acc = s.acc;
-        if (pass == 0) {
-          for (int i = 0; i < use; ++i) acc += s.e[i];
-        } else if (pass == 1) {
-          for (int i = 0; i < use; ++i) {
-            acc += s.e[i] / s.sum_exp;
-            if (acc > top_p) { s.cutoff = taken + i + 1; s.done = 1; break; }
-          }
-        } else {
-          for (int i = 0; i < use; ++i) {
-            acc += (s.e[i] / s.sum_exp) / s.nucleus;
-            s.last_idx = (unsigned)s.key[i];
-            if (u < acc) { s.token = s.last_idx; s.done = 1; break; }
-          }
-        }
-        s.acc = acc;
-      }
-      __syncthreads();
-      lo = s.key[cnt - 1] + 1;
-      taken += cnt;
-      const int done = s.done;
-      __syncthreads();  // everyone has read the flag and the last key before either is rewritten
-      if (done) break;
-    }
+    if (lane == 0) { s.red_f[warp] = best; s.red_i[warp] = bi; }
     __syncthreads();
     if (tid == 0) {
-      if (pass == 0) s.sum_exp = s.acc;
-      if (pass == 1) { s.nucleus = s.acc; if (!s.done) s.cutoff = min(taken, k_eff); }
-      if (pass == 2 && !s.done) s.token = s.last_idx;
+      for (int w = 1; w < kWarps; ++w)
+        if (better(s.red_f[w], s.red_i[w], best, bi)) { best = s.red_f[w]; bi = s.red_i[w]; }
+      s.part_max = best;
+      s.part_arg = bi;
     }
+    cluster.sync();
+    best = of(0).part_max;
+    bi = of(0).part_arg;
+    for (int q = 1; q < ranks; ++q) {
+      const float ov = of(q).part_max;
+      const int oi = of(q).part_arg;
+      if (better(ov, oi, best, bi)) { best = ov; bi = oi; }
+    }
+    *out_max = best;
+    return bi == 0x7fffffff ? 0 : bi;
+  }
+
+  __device__ void clear_hist() {
+    for (int b = tid; b < kBins; b += kThreads) { s.hist_n[b] = 0; s.hist_d[b] = 0; }
     __syncthreads();
   }
-  return s.token;
-}
-
-template <typename T>
-__device__ void sample_row(const Row<T>& r, const b200_sample_params& p, Shared& s, uint32_t* out_token, float* out_logprob) {
-  float gmax;
-  const int garg = block_first_max(r, s, &gmax);
-  unsigned token;
-  if (!(p.temperature > 0.0f)) {
-    token = (unsigned)garg;
-  } else if (p.top_p >= 1.0f && (p.top_k <= 0 || p.top_k >= r.V)) {
-    token = sample_full_softmax(r, p.temperature, gmax, p.uniform, s);
-  } else {
-    const int k_eff = (p.top_k <= 0 || p.top_k > r.V) ? r.V : p.top_k;
-    token = sample_top_k_top_p(r, p.temperature, k_eff, p.top_p, p.uniform, gmax, s);
+  __device__ void count(int bin, float x) {  // x: distance behind the near edge of the score's bin, below 1/64
+    const float deficit = x * (1.f - x * (0.5f - x * (1.f / 6.f - x * (1.f / 24.f))));
+    atomicAdd(&s.hist_n[bin], 1u);
+    atomicAdd(&s.hist_d[bin], (unsigned)(deficit * units + 0.5f));
   }
-  if (out_logprob != nullptr) {
-    float part = 0.f;
-    for (int base = 0; base < r.V; base += kThreads * 8) {
-      float v[8];
-      const int n = load8(r, base + threadIdx.x * 8, v);
+  // First CTA: running sums of the whole row's bins.  `edge`: weight at the near edge of bin b; `counted` false: the bin weighs nothing.
+  template <typename F>
+  __device__ void sum_bins(Bins& out, F edge) {
+    cluster.sync();
+    if (rank == 0) {
+      unsigned n[kPerThread], d[kPerThread];
+      double m[kPerThread];
+#pragma unroll
+      for (int k = 0; k < kPerThread; ++k) n[k] = d[k] = 0;
+      double deficit[kPerThread] = {};
+      for (int q = 0; q < ranks; ++q) {
+        const Shared& o = of(q);
+#pragma unroll
+        for (int k = 0; k < kPerThread; ++k) {
+          n[k] += o.hist_n[tid * kPerThread + k];
+          deficit[k] += (double)o.hist_d[tid * kPerThread + k];
+        }
+      }
+      const double unit = exp2((double)(unit_shift - 22));
+      unsigned nt = 0;
+      double mt = 0.0;
+#pragma unroll
+      for (int k = 0; k < kPerThread; ++k) {
+        m[k] = edge(tid * kPerThread + k) * ((double)n[k] - deficit[k] * unit);
+        nt += n[k]; n[k] = nt;
+        mt += m[k]; m[k] = mt;
+      }
+      unsigned ni = nt;
+      double mi = mt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned a = __shfl_up_sync(0xffffffffu, ni, o);
+        const double b = __shfl_up_sync(0xffffffffu, mi, o);
+        if (lane >= o) { ni += a; mi += b; }
+      }
+      if (lane == 31) { s.red_u[warp] = ni; s.red_d[warp] = mi; }
+      __syncthreads();
+      unsigned nb = ni - nt;
+      double mb = mi - mt;
+      for (int w = 0; w < warp; ++w) { nb += s.red_u[w]; mb += s.red_d[w]; }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < kPerThread; ++k) { out.n[tid * kPerThread + k] = nb + n[k]; out.m[tid * kPerThread + k] = mb + m[k]; }
+    }
+    cluster.sync();
+  }
+
+  // A set of keys that follow one another in the order: a range inside a bin, with what lies ahead of it.
+  struct Range {
+    int bin;
+    unsigned long long lo, hi;
+    unsigned n_before, n;
+    double m_before;
+  };
+  // The first bin whose running count reaches `rank_wanted` (by_mass false) or whose running weight exceeds `target`.  All CTAs get the answer.
+  __device__ unsigned search(const Bins& bins, bool by_mass, unsigned rank_wanted, double target, unsigned last) {
+    if (rank == 0) {
+      if (tid == 0) s.found = last;
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < kPerThread; ++k) {
+        const int b = tid * kPerThread + k;
+        const bool here = by_mass ? bins.m[b] > target && (b == 0 || !(bins.m[b - 1] > target)) : bins.n[b] >= rank_wanted && (b == 0 || bins.n[b - 1] < rank_wanted);
+        if (here) atomicMin(&s.found, (unsigned)b);
+      }
+      __syncthreads();
+      if (tid == 0) {
+        // (a bin that adds nothing but rounding is passed over)
+        unsigned b = s.found;
+        while (b > 0 && bins.n[b] == bins.n[b - 1]) --b;
+        s.found = b;
+        s.n_before = b ? bins.n[b - 1] : 0;
+        s.count = bins.n[b] - s.n_before;
+        s.before = b ? bins.m[b - 1] : 0.0;
+      }
+    }
+    cluster.sync();
+    return of(0).found;
+  }
+  // Narrows a search down to at most kCap keys.
+  __device__ Range find(float temperature, float gmax, float max_score, bool by_mass, unsigned rank_wanted, double target, unsigned last) {
+    Range g;
+    g.bin = (int)search(s.row, by_mass, rank_wanted, target, last);
+    g.lo = 0;
+    g.hi = ~0ull;
+    const Shared& f = of(0);
+    g.n_before = f.n_before;
+    g.n = f.count;
+    g.m_before = f.before;
+    cluster.sync();
+    const double edge = g.bin == kBins - 1 ? 0.0 : exp(-(double)g.bin / (double)kBinsPerUnit);
+    while (g.n > kCap) {
+      // the range's first and last key, then its keys counted in 2048 parts
+      unsigned long long kl = ~0ull, kh = 0ull;
+      auto mine = [&](float v, int i, auto f) {
+        const float sc = score_of(v, temperature), dist = max_score - sc;
+        if (bin_of(dist) != g.bin) return;
+        const unsigned long long k = key_of(sc, i);
+        if (k >= g.lo && k <= g.hi) f(k, dist);
+      };
+      float least, most;
+      logits_of(g.bin, g.bin, temperature, gmax, &least, &most);
+      each_within(least, most, [&](float v, int i) { mine(v, i, [&](unsigned long long k, float) { kl = min(kl, k); kh = max(kh, k); }); });
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        kl = min(kl, __shfl_xor_sync(0xffffffffu, kl, o));
+        kh = max(kh, __shfl_xor_sync(0xffffffffu, kh, o));
+      }
+      __syncthreads();
+      if (lane == 0) { s.red_k[warp] = kl; s.red_k[kWarps + warp] = kh; }
+      __syncthreads();
+      if (tid == 0) {
+        for (int w = 0; w < kWarps; ++w) { kl = min(kl, s.red_k[w]); kh = max(kh, s.red_k[kWarps + w]); }
+        s.part_lo = kl;
+        s.part_hi = kh;
+      }
+      cluster.sync();
+      for (int q = 0; q < ranks; ++q) { kl = min(kl, of(q).part_lo); kh = max(kh, of(q).part_hi); }
+      int shift = 0;
+      while (((kh - kl) >> shift) >= kBins) ++shift;
+      clear_hist();
+      each_within(least, most, [&](float v, int i) {
+        mine(v, i, [&](unsigned long long k, float dist) { count((int)((k - kl) >> shift), g.bin == kBins - 1 ? 0.f : fmaxf(dist - (float)g.bin * (1.f / kBinsPerUnit), 0.f)); });
+      });
+      sum_bins(s.fine, [&](int) { return edge; });
+      const unsigned part = search(s.fine, by_mass, rank_wanted - g.n_before, target - g.m_before, (unsigned)((kh - kl) >> shift));
+      g.lo = kl + ((unsigned long long)part << shift);
+      g.hi = g.lo + ((1ull << shift) - 1);
+      g.n_before += f.n_before;
+      g.n = f.count;
+      g.m_before += f.before;
+      cluster.sync();
+    }
+    return g;
+  }
+
+  // The keys of bins first..last between klo and khi, sorted, into the first CTA's list; returns how many.
+  __device__ int gather(float temperature, float gmax, float max_score, int first, int last, unsigned long long klo, unsigned long long khi) {
+    return gather(temperature, gmax, max_score, first, last, klo, khi, [](const float (&)[8], int) {});
+  }
+  // `also`: done to all the thread's elements on the way.  More keys than fit: the list is not made.
+  template <typename F>
+  __device__ int gather(float temperature, float gmax, float max_score, int first, int last, unsigned long long klo, unsigned long long khi, F also) {
+    Shared& f = of(0);
+    if (rank == 0 && tid == 0) s.count = 0;
+    cluster.sync();
+    float least, most;
+    logits_of(first, last, temperature, gmax, &least, &most);
+    each8<2>([&](const float (&v)[8], int i0, int n) {
+      also(v, n);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (j >= n || v[j] < least || v[j] > most) continue;
+        const float sc = score_of(v[j], temperature);
+        const int b = bin_of(max_score - sc);
+        if (b < first || b > last) continue;
+        const unsigned long long k = key_of(sc, i0 + j);
+        if (k < klo || k > khi) continue;
+        const unsigned at = atomicAdd(&f.count, 1u);
+        if (at < kCap) f.list.key[at] = k;
+      }
+    });
+    cluster.sync();
+    const int n = (int)f.count;
+    if (rank == 0 && n <= kCap) {
+      int n2 = 2;
+      while (n2 < n) n2 <<= 1;
+      for (int i = n + tid; i < n2; i += kThreads) s.list.key[i] = ~0ull;
+      __syncthreads();
+      for (int k = 2; k <= n2; k <<= 1) {
+        for (int j = k >> 1; j > 0; j >>= 1) {
+          for (int i = tid; i < n2; i += kThreads) {
+            const int x = i ^ j;
+            if (x > i) {
+              const unsigned long long a = s.list.key[i], c = s.list.key[x];
+              if ((a > c) == ((i & k) == 0)) { s.list.key[i] = c; s.list.key[x] = a; }
+            }
+          }
+          __syncthreads();
+        }
+      }
+      for (int i = tid; i < n; i += kThreads) s.list.weight[i] = expf(key_score(s.list.key[i]) - max_score);
+      __syncthreads();
+    }
+    return n;
+  }
+
+  // First CTA, all its threads: the first of list[0, n) at which base + running weight exceeds target, n if none does; *upto gets the
+  // running sum with it (or all).  A thread takes four neighbours.
+  __device__ int walk(int n, double base, double target, double* upto) {
+    constexpr int E = kCap / kThreads;
+    double w[E], t = 0.0;
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+      const int i = tid * E + k;
+      t += i < n ? (double)s.list.weight[i] : 0.0;
+      w[k] = t;
+    }
+    double incl = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double a = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += a;
+    }
+    __syncthreads();
+    if (lane == 31) s.red_d[warp] = incl;
+    if (tid == 0) s.found = (unsigned)n;
+    __syncthreads();
+    double ahead = base + incl - t;
+    for (int q = 0; q < warp; ++q) ahead += s.red_d[q];
+    int at = n;
+#pragma unroll
+    for (int k = E - 1; k >= 0; --k)
+      if (tid * E + k < n && ahead + w[k] > target) at = tid * E + k;
+    if (at < n) atomicMin(&s.found, (unsigned)at);
+    __syncthreads();
+    const int found = (int)s.found;
+    const int last = min(found, n - 1);  // whose running sum is wanted
+#pragma unroll
+    for (int k = 0; k < E; ++k)
+      if (tid * E + k == last) s.mass = ahead + w[k];
+    if (n == 0 && tid == 0) s.mass = base;
+    __syncthreads();
+    *upto = s.mass;
+    __syncthreads();
+    return found;
+  }
+
+  // First CTA: end of the nucleus and draw on the sorted list, whose first `keep` keys are the candidates; total: their weight.
+  __device__ void decide(int keep, double total, bool cut, float top_p, float u) {
+    double nucleus, drawn;
+    const int end = walk(keep, 0.0, cut ? (double)top_p * total : (double)INFINITY, &nucleus), members = min(end + 1, keep);
+    const int at = min(walk(members, 0.0, (double)u * nucleus, &drawn), members - 1);
+    if (tid == 0) s.token = (unsigned)s.list.key[at];
+    __syncthreads();
+  }
+
+  // topKTopPSampler (src/sampling.zig:175-242).  `part` gets the thread's sum of exp(logit - max) where sums is set.
+  __device__ unsigned top_k_top_p(float temperature, int k_eff, float top_p, float u, float gmax, float max_score, float thread_max, bool sums, double* part) {
+    const Shared& f = of(0);
+    const bool all = k_eff >= r.V;
+    const bool cut = top_p < 1.0f;
+    if (k_eff <= kFew) {
+      // The few best: as many threads' maxima as candidates are wanted lie in the bins up to some bin, hence as many words; all words of
+      // those bins are a prefix of the order, little longer than wanted.
+      clear_hist();
+      if (lo < hi) atomicAdd(&s.hist_n[bin_of(max_score - score_of(thread_max, temperature))], 1u);
+      sum_bins(s.row, [](int) { return 0.0; });
+      const unsigned last = search(s.row, false, (unsigned)k_eff, 0.0, kBins - 1);
+      const int n = gather(temperature, gmax, max_score, 0, (int)last, 0ull, ~0ull, [&](const float (&v)[8], int m) {
+        if (!sums) return;
+        float a = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (j < m) a += expf(v[j] - gmax);
+        *part += (double)a;
+      });
+      if (n <= kCap) {
+        if (rank == 0) {
+          const int keep = min(n, k_eff);
+          double total;
+          walk(keep, 0.0, INFINITY, &total);
+          decide(keep, total, cut, top_p, u);
+        }
+        cluster.sync();
+        return f.token;
+      }
+      sums = false;
+      cluster.sync();
+    }
+    clear_hist();
+    each8<2>([&](const float (&v)[8], int i0, int n) {
+      float a = 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j)
-        if (j < n) part += expf(v[j] - gmax);
+        if (j < n) {
+          if (sums) a += expf(v[j] - gmax);
+          const float dist = max_score - score_of(v[j], temperature);
+          const int b = bin_of(dist);
+          count(b, b == kBins - 1 ? 0.f : fmaxf(dist - (float)b * (1.f / kBinsPerUnit), 0.f));
+        }
+      *part += (double)a;
+    });
+    sum_bins(s.row, [](int b) { return b == kBins - 1 ? 0.0 : exp(-(double)b / (double)kBinsPerUnit); });
+    // the bin that ends the list of candidates: by rank, or by weight where every word is one
+    double total = f.row.m[kBins - 1];
+    const unsigned last = search(s.row, all && cut, (unsigned)k_eff, (double)top_p * total, kBins - 1);
+    const unsigned upto = f.n_before + f.count;
+    cluster.sync();
+    unsigned token = 0;
+    if (upto <= kCap) {
+      // they fit: everything is decided on the sorted list
+      const int n = gather(temperature, gmax, max_score, 0, (int)last, 0ull, ~0ull);
+      if (rank == 0) {
+        const int keep = min(n, k_eff);
+        if (!all) walk(keep, 0.0, INFINITY, &total);
+        decide(keep, total, cut, top_p, u);
+      }
+    } else {
+      // position by position: the last candidate, the end of the nucleus (s.token is the last member so far), the draw
+      Range k_end{};
+      unsigned n_keep = (unsigned)r.V;
+      if (!all) {
+        k_end = find(temperature, gmax, max_score, false, (unsigned)k_eff, 0.0, kBins - 1);
+        const int n = gather(temperature, gmax, max_score, k_end.bin, k_end.bin, k_end.lo, k_end.hi);
+        if (rank == 0) {
+          double sum;
+          const int here = min(n, k_eff - (int)k_end.n_before);
+          walk(here, k_end.m_before, INFINITY, &sum);
+          if (tid == 0) { s.target = sum; s.token = (unsigned)s.list.key[here - 1]; }
+          __syncthreads();
+        }
+        cluster.sync();
+        total = f.target;
+        n_keep = (unsigned)k_eff;
+        cluster.sync();
+      }
+      unsigned members = n_keep;
+      double nucleus = total;
+      if (cut) {
+        const Range g = find(temperature, gmax, max_score, true, 0u, (double)top_p * total, all ? kBins - 1 : (unsigned)k_end.bin);
+        const int n = gather(temperature, gmax, max_score, g.bin, g.bin, g.lo, g.hi);
+        if (rank == 0) {
+          double sum;
+          const int here = (int)min((unsigned)n, n_keep - min(n_keep, g.n_before));
+          const int at = walk(here, g.m_before, (double)top_p * total, &sum);
+          if (tid == 0) {
+            s.target = sum;
+            s.n_before = min(n_keep, g.n_before + (unsigned)min(at + 1, here));
+            if (here > 0) s.token = (unsigned)s.list.key[min(at, here - 1)];
+          }
+          __syncthreads();
+        }
+        cluster.sync();
+        nucleus = f.target;
+        members = f.n_before;
+        cluster.sync();
+      }
+      const Range g = find(temperature, gmax, max_score, true, 0u, (double)u * nucleus, kBins - 1);
+      const int n = gather(temperature, gmax, max_score, g.bin, g.bin, g.lo, g.hi);
+      if (rank == 0) {
+        double sum;
+        // (behind the last member, by rounding: s.token is that one already)
+        const int here = (int)min((unsigned)n, members - min(members, g.n_before));
+        const int at = min(walk(here, g.m_before, (double)u * nucleus, &sum), here - 1);
+        if (tid == 0 && here > 0) s.token = (unsigned)s.list.key[at];
+        __syncthreads();
+      }
     }
-    const float sum = block_sum(part, s);
-    if (threadIdx.x == 0) *out_logprob = token < (unsigned)r.V ? to_f32(r.p[token]) - (gmax + logf(sum)) : -INFINITY;
+    cluster.sync();
+    token = f.token;
+    return token;
   }
-  if (threadIdx.x == 0) *out_token = token;
-}
+
+  // temperatureSample (src/sampling.zig:42-72): softmax of (logit - max) / T in index order, first index whose cumulative probability
+  // exceeds u.  The warps' sums say which warp's part it falls into; there a lane takes a run of neighbours.
+  __device__ unsigned full_softmax(float temperature, float gmax, float u) {
+    cluster.sync();
+    if (rank == 0 && tid == 0) {
+      double sum = 0.0, cum = 0.0;
+      for (int q = 0; q < ranks; ++q) sum += of(q).part_sum[1];
+      const double target = (double)u * sum;
+      s.owner = -1;
+      s.token = (unsigned)(r.V - 1);  // sampleFromProbs returns n - 1 when u is never exceeded (:267)
+      for (int q = 0; q < ranks && s.owner < 0; ++q)
+        for (int w = 0; w < kWarps; ++w) {
+          const double next = cum + of(q).warp_sum[w];
+          if (next > target) { s.owner = q * kWarps + w; s.target = target - cum; break; }
+          cum = next;
+        }
+    }
+    cluster.sync();
+    Shared& f = of(0);
+    if (f.owner == rank * kWarps + warp) {
+      const double target = f.target;
+      const int run = (warp_part + 31) / 32, b = min(lo + lane * run, hi), e = min(b + run, hi);
+      double mine = 0.0;
+      for (int i = b; i < e; ++i) mine += (double)expf((to_f32(r.p[i]) - gmax) / temperature);
+      double incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      const unsigned over = __ballot_sync(0xffffffffu, incl > target && e > b);
+      if (over == 0) {
+        if (lane == 0) f.token = (unsigned)(hi - 1);
+      } else if (lane == __ffs(over) - 1) {
+        double cum = incl - mine;
+        int i = b;
+        for (; i < e - 1; ++i) {
+          cum += (double)expf((to_f32(r.p[i]) - gmax) / temperature);
+          if (cum > target) break;
+        }
+        f.token = (unsigned)i;
+      }
+    }
+    cluster.sync();
+    return f.token;
+  }
+
+  __device__ void run(const b200_sample_params& p, uint32_t* out_token, float* out_logprob) {
+    float gmax, thread_max;
+    unsigned token = (unsigned)first_max(&gmax, &thread_max);
+    const bool sums = out_logprob != nullptr, greedy = !(p.temperature > 0.0f), whole = !greedy && p.top_p >= 1.0f && (p.top_k <= 0 || p.top_k >= r.V);
+    double part = 0.0, part_t = 0.0;
+    if (!greedy && !whole) {
+      // the largest score is the largest logit's: division by a positive temperature keeps the order
+      token = top_k_top_p(p.temperature, (p.top_k <= 0 || p.top_k > r.V) ? r.V : p.top_k, p.top_p, p.uniform, gmax, score_of(gmax, p.temperature), thread_max, sums, &part);
+    } else if (sums || whole) {
+      each8<2>([&](const float (&v)[8], int i0, int n) {
+        float a = 0.f, b = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (sums && j < n) a += expf(v[j] - gmax);
+          if (whole && j < n) b += expf((v[j] - gmax) / p.temperature);
+        }
+        part += (double)a;
+        part_t += (double)b;
+      });
+    }
+    const double sum = block_sum(part);
+    if (tid == 0) s.part_sum[0] = sum;
+    if (whole) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) part_t += __shfl_xor_sync(0xffffffffu, part_t, o);
+      if (lane == 0) s.warp_sum[warp] = part_t;
+      __syncthreads();
+      if (tid == 0) {
+        double t = 0.0;
+        for (int w = 0; w < kWarps; ++w) t += s.warp_sum[w];
+        s.part_sum[1] = t;
+      }
+      token = full_softmax(p.temperature, gmax, p.uniform);
+    }
+    cluster.sync();
+    if (rank == 0 && tid == 0) {
+      if (out_logprob != nullptr) {
+        double all = 0.0;
+        for (int q = 0; q < ranks; ++q) all += of(q).part_sum[0];
+        *out_logprob = token < (unsigned)r.V ? to_f32(r.p[token]) - (gmax + logf((float)all)) : -INFINITY;
+      }
+      *out_token = token;
+    }
+    cluster.sync();  // nobody leaves while its shared memory may be read
+  }
+};
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) sample_rows_kernel(const T* __restrict__ logits, int V,
-                                                               const b200_sample_params* __restrict__ params,
-                                                               const uint32_t* __restrict__ ctx, const int* __restrict__ ctx_off,
-                                                               float* __restrict__ scratch, uint32_t* __restrict__ tokens,
-                                                               float* __restrict__ logprobs) {
-  __shared__ Shared s;
-  const int row = blockIdx.x;
+__global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(const T* __restrict__ logits, int V, const b200_sample_params* __restrict__ params,
+                                                                  const uint32_t* __restrict__ ctx, const int* __restrict__ ctx_off,
+                                                                  float* __restrict__ scratch, uint32_t* __restrict__ tokens,
+                                                                  float* __restrict__ logprobs) {
+  extern __shared__ __align__(16) unsigned char sample_dyn[];
+  Shared& s = *reinterpret_cast<Shared*>(sample_dyn);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ranks = cluster.num_blocks(), rank = cluster.block_rank(), row = blockIdx.x / ranks;
   const b200_sample_params p = params[row];
   const T* x = logits + (size_t)row * V;
   float* lp = logprobs ? logprobs + row : nullptr;
@@ -501,13 +712,14 @@ __global__ void __launch_bounds__(kThreads) sample_rows_kernel(const T* __restri
     // applyRepetitionPenalty (src/sampling.zig:328-354): every occurrence of a token divides a positive
     // logit by the penalty or multiplies a non-positive one; occurrences commute, so they may race.
     float* y = scratch + (size_t)row * V;
-    for (int i = threadIdx.x; i < V; i += kThreads) y[i] = to_f32(x[i]);
-    __syncthreads();
-    for (int c = threadIdx.x; c < ctx_n; c += kThreads) {
+    for (int i = rank * kThreads + threadIdx.x; i < V; i += ranks * kThreads) y[i] = to_f32(x[i]);
+    __threadfence();
+    cluster.sync();
+    for (int c = rank * kThreads + threadIdx.x; c < ctx_n; c += ranks * kThreads) {
       const uint32_t tok = ctx[ctx_lo + c];
       if (tok < (uint32_t)V) {
         unsigned* a = reinterpret_cast<unsigned*>(y + tok);
-        unsigned old = *a, assumed;
+        unsigned old = *reinterpret_cast<volatile unsigned*>(a), assumed;
         do {
           assumed = old;
           const float f = __uint_as_float(assumed);
@@ -515,13 +727,39 @@ __global__ void __launch_bounds__(kThreads) sample_rows_kernel(const T* __restri
         } while (old != assumed);
       }
     }
-    __syncthreads();
-    const Row<float> r{y, V, V % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0};
-    sample_row(r, p, s, tokens + row, lp);
+    __threadfence();
+    cluster.sync();
+    Sampler<float>(s, Row<float>{y, V, V % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0}).run(p, tokens + row, lp);
   } else {
-    const Row<T> r{x, V, V % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0};
-    sample_row(r, p, s, tokens + row, lp);
+    Sampler<T>(s, Row<T>{x, V, V % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0}).run(p, tokens + row, lp);
   }
+}
+
+template <typename T>
+b200_status launch(const T* logits, int rows, int vocab, const b200_sample_params* params, const uint32_t* ctx, const int* ctx_off, float* scratch,
+                   uint32_t* tokens, float* logprobs, cudaStream_t s) {
+  static bool configured = false;
+  if (!configured) {
+    B200_CUDA_TRY(cudaFuncSetAttribute(sample_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared)));
+    configured = true;
+  }
+  // CTAs per row: 8192 words each at least (16 a thread), and no more than two per SM altogether (what registers allow: more would wait)
+  int ranks = 1;
+  while (ranks < kMaxCluster && vocab > ranks * 8192 && (long long)rows * ranks * 2 <= 296) ranks *= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)rows * ranks);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = sizeof(Shared);
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = ranks;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, sample_rows_kernel<T>, logits, vocab, params, ctx, ctx_off, scratch, tokens, logprobs));
+  B200_LAUNCH_CHECK();
+  return B200_OK;
 }
 
 }  // namespace
@@ -543,14 +781,8 @@ b200_status b200_sample_rows(const void* d_logits, int32_t logits_f32, int32_t r
     return B200_ERR_INVALID_ARGUMENT;
   }
   cudaStream_t cs = (cudaStream_t)stream;
-  if (logits_f32)
-    sample_rows_kernel<float><<<rows, kThreads, 0, cs>>>((const float*)d_logits, vocab, d_params, d_ctx_tokens, d_ctx_offsets,
-                                                         d_scratch, d_tokens, d_logprobs);
-  else
-    sample_rows_kernel<__nv_bfloat16><<<rows, kThreads, 0, cs>>>((const __nv_bfloat16*)d_logits, vocab, d_params, d_ctx_tokens,
-                                                                 d_ctx_offsets, d_scratch, d_tokens, d_logprobs);
-  B200_LAUNCH_CHECK();
-  return B200_OK;
+  return logits_f32 ? launch((const float*)d_logits, rows, vocab, d_params, d_ctx_tokens, d_ctx_offsets, d_scratch, d_tokens, d_logprobs, cs)
+                    : launch((const __nv_bfloat16*)d_logits, rows, vocab, d_params, d_ctx_tokens, d_ctx_offsets, d_scratch, d_tokens, d_logprobs, cs);
 }
 
 }  // extern "C"

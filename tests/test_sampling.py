@@ -232,3 +232,68 @@ def test_engine_request_with_sampler():
     g1, g2 = run(7, with_sampler=False)
     assert a1 == b1 and a2 == b2 == c2 == g2
     assert a1 != g1 or c1 != g1  # sampling at temperature 0.9 leaves the greedy path for some seed
+
+
+def _tokens_in_64_bits(x, temperature, top_k, top_p, u, tol):
+    """Tokens that f64 sums over the stable order of the f32 scores allow when cumulative probabilities are off by up to tol."""
+    x = x.astype(np.float32)
+    if temperature <= 0.0:
+        return {int(np.argmax(x))}
+    z = (x / np.float32(temperature)).astype(np.float64)
+    whole = top_p >= 1.0 and (top_k <= 0 or top_k >= len(x))
+    order = np.arange(len(x)) if whole else np.argsort(-z, kind="stable")[:len(x) if top_k <= 0 else top_k]
+    e = np.exp(z[order] - z.max())
+    cum = np.cumsum(e) / e.sum()
+    if whole or top_p >= 1.0:
+        cutoffs = {len(order)}
+    else:
+        p = float(np.float32(top_p))
+        cutoffs = {min(int(np.searchsorted(cum, p + d, side="right")) + 1, len(order)) for d in (-tol, 0.0, tol)}
+    out = set()
+    for c in cutoffs:
+        inner = cum[:c] / cum[c - 1]
+        lo, hi = np.concatenate([[-np.inf], inner[:-1]]), inner.copy()
+        hi[-1] = np.inf
+        out |= {int(t) for t in order[:c][(u >= lo - tol) & (u < hi + tol)]}
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype_name", ["bfloat16", "float32"])
+@pytest.mark.parametrize("vocab", [8192, 8193, 16392, 65537, 131080])
+def test_rows_spread_over_clusters_and_bins_counted_again(dtype_name, vocab):
+    """Vocabularies at the borders of the cluster sizes (a row over one to eight CTAs, parts that do not divide evenly, rows that do not
+    start on 16 bytes), with distributions that reach every way of finding a position: nuclei of thousands of words, bins of 1/64 with more keys
+    than the list holds (thousands of equal scores, scores a hair apart), candidates beyond the bins (distances over 32), and the end of the
+    nucleus and the draw in the same bin or far apart.  Against f64 sums: weights are f32 exponentials (2 ulp) and deficits in units of 2^-22 at
+    most, so cumulative probabilities are within 2^-20 (the sequential f32 sums of the oracle drift further over thousands of words)."""
+    import torch
+
+    from dmlx_b200 import device as dev
+
+    rng = np.random.default_rng(vocab)
+    u = lambda: float(np.float32(rng.random()))
+    flat = rng.normal(0.0, 1.0, vocab)
+    equal = np.where(rng.random(vocab) < 0.5, 1.0, -3.0)           # half of the words alike
+    near = 5.0 + rng.random(vocab) * 1e-3                          # all in one bin (f32; alike in bf16)
+    steep = rng.normal(0.0, 4.0, vocab)
+    plans = [(flat, 1.0, 0, 0.9), (flat, 2.5, 0, 0.5), (flat, 1.0, 5000, 0.95), (flat, 1.0, 6000, 1.0), (equal, 1.0, 0, 0.7), (equal, 1.0, 3000, 0.5),
+             (equal, 1.0, 2500, 1.0), (near, 1.0, 0, 0.3), (near, 1.0, 4000, 0.9), (steep, 0.05, 3000, 1.0), (steep, 0.05, 7000, 0.999999), (flat, 1.0, 0, 1.0),
+             (steep, 1.0, 40, 0.8), (flat, 0.0, 0, 1.0)]
+    x = np.stack([a for a, *_ in plans for _ in range(2)]).astype(np.float32)
+    rows = [(t, k, p, u()) for _, t, k, p in plans for _ in range(2)]
+    rows[1], rows[9] = (*rows[1][:3], float(np.nextafter(np.float32(1), np.float32(0)))), (*rows[9][:3], 0.0)
+    logits = torch.tensor(x, device="cuda").to(getattr(torch, dtype_name)).contiguous()
+    x32 = logits.float().cpu().numpy()
+    tokens, lp = dev.sample_rows(logits, rows)
+    again, lp2 = dev.sample_rows(logits, rows)
+    assert torch.equal(tokens, again) and torch.equal(lp, lp2)
+    tokens, lp, exact = tokens.cpu().numpy(), lp.cpu().numpy(), 0
+    for i, row in enumerate(rows):
+        want = _tokens_in_64_bits(x32[i], *row, 0.0)
+        exact += int(tokens[i]) in want
+        assert int(tokens[i]) in _tokens_in_64_bits(x32[i], *row, 2.0 ** -20), (i, row, int(tokens[i]), want)
+        z = x32[i].astype(np.float64)
+        true = z[tokens[i]] - z.max() - math.log(np.exp(z - z.max()).sum())
+        assert abs(float(lp[i]) - true) < 2e-6 * max(1.0, abs(true)), (i, row, float(lp[i]), true)
+    assert exact >= len(rows) - 3, (exact, len(rows))
