@@ -759,6 +759,10 @@ b200_status b200_moe_forward(b200_moe* m, const void* d_x, int32_t n_tokens, voi
   if (n_tokens > c.max_tokens) { b200_set_error("moe: %d tokens > max_tokens %d", n_tokens, c.max_tokens); return B200_ERR_CAPACITY; }
   if (n_tokens <= 0) return B200_OK;
   const int A = n_tokens * c.top_k;
+  // A token chooses an expert at most once, so no expert has more rows than there are tokens: a tile no larger than that leaves the
+  // block-scaled kernel five stages of weights in flight instead of three (24 tokens on 32 experts of 4096 x 2048, top 6:
+  // 248 -> 194 us a layer).
+  const int tile_rows = c.tile_rows <= 128 ? std::min(c.tile_rows, (n_tokens + 15) / 16 * 16) : c.tile_rows;
   b200_status st;
 #define STEP(call) do { if ((st = (call)) != B200_OK) return st; } while (0)
   if (m->sh_gu) {  // shared expert on every token (deepseek_v4.zig:1017-1022, 489-517)
@@ -768,23 +772,23 @@ b200_status b200_moe_forward(b200_moe* m, const void* d_x, int32_t n_tokens, voi
   STEP(b200_qmm(m->gate, d_x, n_tokens, m->logits, B200_EPI_NONE, nullptr, 0.f, B200_QMM_AUTO, stream));
   STEP(b200_moe_route(m->logits, 0, m->d_bias, n_tokens, c.n_experts, c.top_k, c.scoring, c.route_scale, m->indices,
                       m->weights, m->counts, stream));
-  STEP(b200_moe_group(m->indices, m->counts, n_tokens, c.top_k, c.n_experts, c.tile_rows, m->offsets, m->order,
+  STEP(b200_moe_group(m->indices, m->counts, n_tokens, c.top_k, c.n_experts, tile_rows, m->offsets, m->order,
                       m->inv_order, m->items, m->n_items, stream));
   // gate/up with clipped SwiGLU and the routing score folded in before the down projection (:787-805)
-  if (b200_qmm_grouped_takes_tokens(m->exp_gu, c.tile_rows)) {
+  if (b200_qmm_grouped_takes_tokens(m->exp_gu, tile_rows)) {
     // the block-scaled path re-encodes every activation row anyway: it reads the rows from the token
     // matrix through `order`, and no expert-sorted bf16 copy is made
     row_scales_kernel<<<(A + 255) / 256, 256, 0, (cudaStream_t)stream>>>(m->order, m->weights, A, m->row_scales, nullptr);
     B200_LAUNCH_CHECK();
     STEP(b200_qmm_grouped_from_tokens(m->exp_gu, d_x, m->order, c.top_k, A, m->act_sorted, B200_EPI_SWIGLU, m->row_scales,
-                                      c.swiglu_limit, m->items, m->n_items, m->max_items, c.tile_rows, stream));
+                                      c.swiglu_limit, m->items, m->n_items, m->max_items, tile_rows, stream));
   } else {
     STEP(b200_moe_gather(d_x, m->order, m->weights, A, c.top_k, c.hidden, m->x_sorted, m->row_scales, stream));
     STEP(b200_qmm_grouped(m->exp_gu, m->x_sorted, A, m->act_sorted, B200_EPI_SWIGLU, m->row_scales, c.swiglu_limit, m->items,
-                          m->n_items, m->max_items, c.tile_rows, stream));
+                          m->n_items, m->max_items, tile_rows, stream));
   }
   STEP(b200_qmm_grouped(m->exp_down, m->act_sorted, A, m->y_sorted, B200_EPI_NONE, nullptr, 0.f, m->items, m->n_items,
-                        m->max_items, c.tile_rows, stream));
+                        m->max_items, tile_rows, stream));
   STEP(b200_moe_combine(m->y_sorted, m->inv_order, n_tokens, c.top_k, c.hidden, m->sh_out, d_out, stream));
 #undef STEP
   return B200_OK;
