@@ -312,13 +312,63 @@ __global__ void __launch_bounds__(kTileN) qmm_simt_kernel(QmmArgs a) {
   for (int t = 0; t < TT; ++t) wsp[(size_t)t * kTileN + r] = acc[t];
 }
 
+// One 32-token batch of accumulators (v[j] = token c0+j, weight row n) to scratch or to the output.  y_col: first output column of a
+// block-diagonal launch.  The residual may be y itself, so its 32 values are asked for ahead of the first store: one by one between the
+// stores their latencies added up (52 of the 124 us of o at 2105 rows of 4096 x 4096, 144 CTAs).
+__device__ __forceinline__ void tile_epilogue_store(const QmmArgs& a, const uint32_t (&v)[32], int c0, int rows_here, int t0, int n, int lane, bool direct,
+                                                    float* wsp, size_t n_pad, int y_col = 0) {
+  const int left = rows_here - c0;
+  if (!direct) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < left) wsp[(size_t)(c0 + j) * n_pad] = __uint_as_float(v[j]);
+  } else if (a.epilogue == B200_EPI_SWIGLU) {
+    // rows 2i / 2i+1 of the tile are gate_i / up_i: neighbouring lanes.  The even lane takes token j,
+    // the odd lane token j+1 (one exchange per token pair, no lane idles in the arithmetic).
+    const bool odd = lane & 1;
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      const float a0 = __uint_as_float(v[j]), a1 = __uint_as_float(v[j + 1]);
+      const float got = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
+      const int tok = c0 + j + (int)odd;
+      if (tok < rows_here && n < a.n) {
+        const int token = t0 + tok;
+        a.y[(size_t)token * a.out_stride(a.n / 2) + n / 2] = __float2bfloat16(gated(a, odd ? got : a0, odd ? a1 : got) * a.row_scale(token));
+      }
+    }
+  } else if (n < a.n) {
+    const size_t stride = a.out_stride(a.n), o = (size_t)(t0 + c0) * stride + y_col + n;
+    if (a.y_f32) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < left) reinterpret_cast<float*>(a.y)[o + j * stride] = __uint_as_float(v[j]);
+    } else if (a.epilogue == B200_EPI_RESIDUAL) {
+      __nv_bfloat16 r[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < left) r[j] = a.residual[o + j * stride];
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < left) a.y[o + j * stride] = __float2bfloat16((__uint_as_float(v[j]) + __bfloat162float(r[j])) * a.row_scale(t0 + c0 + j));
+    } else if (!elementwise(a.epilogue) && !a.row_scales) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < left) a.y[o + j * stride] = __float2bfloat16(__uint_as_float(v[j]));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < left) a.y[o + j * stride] = __float2bfloat16(activate(a.epilogue, __uint_as_float(v[j])) * a.row_scale(t0 + c0 + j));
+    }
+  }
+}
+
 // ---- tcgen05 kernel ------------------------------------------------------------------------------
-constexpr int kTcThreads = 320;  // warps 0-7 dequantise (0-3 also run the epilogue), 8 loads, 9 issues MMAs
+constexpr int kTcThreads = 320;  // warps 0-7 dequantise and run the epilogue, 8 loads, 9 issues MMAs
 constexpr int kRawStride = 5120;  // weight block padded to a multiple of 1024
 constexpr int kPrefetchAhead = 12;  // weight blocks requested into L2 ahead of the copy
 
 template <int MODE>
-__global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
+__global__ void __launch_bounds__(kTcThreads, 2) qmm_tc_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
   extern __shared__ unsigned char smem_raw[];
   // 1024-byte alignment: the 128B swizzle pattern is a function of the shared-memory address.
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -447,54 +497,23 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const __grid_cons
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&a_ready[s]);
     }
-    // ---- accumulator -> f32 partial tile in scratch ----
-    if (ok && warp < 4) ok = ptx::mbar_wait(accum_ready, 0);
-    if (ok && warp < 4) {
+    // ---- accumulator -> output, or f32 partial tile in scratch; warps 0-3 and 4-7 take the 32-token batches in turn ----
+    if (ok) ok = ptx::mbar_wait(accum_ready, 0);
+    if (ok) {
       ptx::tc_fence_after_sync();
-      const int n = nt * kTileN + warp * 32 + lane;
+      const int row = (warp & 3) * 32 + lane, n = nt * kTileN + row;
       // One K split and a small token tile: apply the epilogue here and skip the finish kernel.  With
       // large token tiles the strided 64-byte row stores cost more than the extra pass.
       // (Dense weights in groups: their tiles are never split, and the pass would move the whole output twice more.)
       const bool direct = gridDim.y == 1 && !a.keep_f32 && (tn <= 64 || (MODE == B200_Q_BF16 && (a.items || a.groups > 0)));
       const size_t n_pad = a.items ? (size_t)a.nt * kTileN : (size_t)kTileN;  // stride between token rows
       float* wsp = a.items ? a.ws + ((size_t)split * a.rows + t0) * n_pad + n
-                           : a.ws + (((size_t)(nt * gridDim.z + blockIdx.z) * gridDim.y + split) * tn) * kTileN + warp * 32 + lane;
-      for (int c0 = 0; c0 < rows_here; c0 += 32) {
+                           : a.ws + (((size_t)(nt * gridDim.z + blockIdx.z) * gridDim.y + split) * tn) * kTileN + row;
+      for (int c0 = (warp >> 2) * 32; c0 < rows_here; c0 += 64) {
         uint32_t v[32];
-        ptx::tmem_ld32(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+        ptx::tmem_ld32(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
         ptx::tmem_ld_wait();
-        if (!direct) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (c0 + j < rows_here) wsp[(size_t)(c0 + j) * n_pad] = __uint_as_float(v[j]);
-        } else if (a.epilogue == B200_EPI_SWIGLU) {
-          // rows 2i / 2i+1 of the tile are gate_i / up_i: neighbouring lanes
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float mine = __uint_as_float(v[j]);
-            const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
-            if ((lane & 1) == 0 && c0 + j < rows_here && n < a.n) {
-              const int token = t0 + c0 + j;
-              a.y[(size_t)token * a.out_stride(a.n / 2) + n / 2] = __float2bfloat16(gated(a, mine, other) * a.row_scale(token));
-            }
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (c0 + j < rows_here && n < a.n) {
-              const int token = t0 + c0 + j;
-              const size_t o = (size_t)token * a.out_stride(a.n) + y_col + n;
-              float acc = __uint_as_float(v[j]);
-              if (MODE == B200_Q_BF16 && a.y_f32) {
-                reinterpret_cast<float*>(a.y)[o] = acc;
-                continue;
-              }
-              if (a.epilogue == B200_EPI_RESIDUAL) acc += __bfloat162float(a.residual[o]);
-              else if (MODE == B200_Q_BF16) acc = activate(a.epilogue, acc);
-              a.y[o] = __float2bfloat16(acc * a.row_scale(token));
-            }
-          }
-        }
+        tile_epilogue_store(a, v, c0, rows_here, t0, n, lane, direct, wsp, n_pad, y_col);
       }
     }
   }
@@ -503,42 +522,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) qmm_tc_kernel(const __grid_cons
   const int any_bad = __syncthreads_or(!ok);
   if (warp == 9) ptx::tmem_dealloc(tmem_base, ncols);
   (void)any_bad;
-}
-
-// One 32-token batch of accumulators (v[j] = token c0+j, weight row n) to scratch or to the output.
-__device__ __forceinline__ void tile_epilogue_store(const QmmArgs& a, const uint32_t (&v)[32], int c0, int rows_here, int t0,
-                                                    int n, int lane, bool direct, float* wsp, size_t n_pad) {
-  if (!direct) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (c0 + j < rows_here) wsp[(size_t)(c0 + j) * n_pad] = __uint_as_float(v[j]);
-  } else if (a.epilogue == B200_EPI_SWIGLU) {
-    // rows 2i / 2i+1 of the tile are gate_i / up_i: neighbouring lanes.  The even lane takes token j,
-    // the odd lane token j+1 (one exchange per token pair, no lane idles in the arithmetic).
-    const bool odd = lane & 1;
-#pragma unroll
-    for (int j = 0; j < 32; j += 2) {
-      const float a0 = __uint_as_float(v[j]), a1 = __uint_as_float(v[j + 1]);
-      const float got = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
-      const int tok = c0 + j + (int)odd;
-      if (tok < rows_here && n < a.n) {
-        const int token = t0 + tok;
-        a.y[(size_t)token * a.out_stride(a.n / 2) + n / 2] = __float2bfloat16(gated(a, odd ? got : a0, odd ? a1 : got) * a.row_scale(token));
-      }
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      if (c0 + j < rows_here && n < a.n) {
-        const int token = t0 + c0 + j;
-        const size_t o = (size_t)token * a.out_stride(a.n) + n;
-        float acc = __uint_as_float(v[j]);
-        if (a.epilogue == B200_EPI_RESIDUAL) acc += __bfloat162float(a.residual[o]);
-        else acc = activate(a.epilogue, acc);
-        a.y[o] = __float2bfloat16(acc * a.row_scale(token));
-      }
-    }
-  }
 }
 
 // ---- tcgen05 kernel with the weight operand in tensor memory -----------------------------------
@@ -979,6 +962,60 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
           if (tile < n_tiles && col < n_out)
             *reinterpret_cast<uint4*>(a.y + (size_t)(t0 + tok) * a.out_stride(n_out) + col) = *reinterpret_cast<const uint4*>(stage_h + (size_t)idx * 8);
         }
+      }
+    } else if (gridDim.y == 1 && !a.keep_f32 && a.epilogue != B200_EPI_SWIGLU && a.n % 8 == 0 && a.out_stride(a.n) % 8 == 0 &&
+               (((uintptr_t)a.y | (uintptr_t)a.residual) & 15) == 0) {
+      // The other epilogues written by this kernel, likewise through the idle stage buffers: bf16 [token][256 columns of the pair].  The
+      // residual is brought in first, 16 bytes at a time, and the sums replace it in place (o at 2105 rows of 4096 x 4096: 124 us with
+      // a 2-byte residual load ahead of each 2-byte store, 70 this way).
+      uint32_t all_ok;
+      asm volatile(
+          "{\n\t.reg .pred p, q;\n\t"
+          "setp.ne.b32 p, %1, 0;\n\t"
+          "bar.red.and.pred q, 1, 512, p;\n\t"
+          "selp.u32 %0, 1, 0, q;\n\t}"
+          : "=r"(all_ok)
+          : "r"((uint32_t)ok)
+          : "memory");
+      if (all_ok) {
+        ptx::tc_fence_after_sync();
+        __nv_bfloat16* stage_h = reinterpret_cast<__nv_bfloat16*>(smem);
+        const size_t stride = a.out_stride(a.n), o0 = (size_t)t0 * stride + nt0 * kTileN;
+        const int cols = min(a.n - nt0 * kTileN, 2 * kTileN);
+        const bool add = a.epilogue == B200_EPI_RESIDUAL;
+        if (add) {
+          for (int idx = tid; idx < rows_here * 32; idx += kTc2DequantThreads)
+            if ((idx & 31) * 8 < cols)
+              *reinterpret_cast<uint4*>(stage_h + (size_t)idx * 8) = *reinterpret_cast<const uint4*>(a.residual + o0 + (size_t)(idx >> 5) * stride + (idx & 31) * 8);
+          asm volatile("bar.sync 1, 512;" ::: "memory");
+        }
+        if (etile < n_tiles) {
+          const int lq = warp & 3;
+          const int ch = ((tn / 2 + 31) / 32) * 32;
+          const int c_end = min(rows_here, (half + 1) * ch);
+          for (int c0 = half * ch; c0 < c_end; c0 += 32) {
+            uint32_t v[32];
+            ptx::tmem_ld32(tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(etile * 256 + c0), v);
+            const float rs_mine = c0 + lane < rows_here ? a.row_scale(t0 + c0 + lane) : 0.f;
+            ptx::tmem_ld_wait();
+            __nv_bfloat16* mine = stage_h + (size_t)c0 * 256 + etile * kTileN + lq * 32 + lane;
+            const int left = rows_here - c0;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const float rs = __shfl_sync(0xffffffffu, rs_mine, j);
+              if (j < left) {
+                float acc = __uint_as_float(v[j]);
+                if (add) acc += __bfloat162float(mine[j * 256]);
+                else acc = activate(a.epilogue, acc);
+                mine[j * 256] = __float2bfloat16(acc * rs);
+              }
+            }
+          }
+        }
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+        for (int idx = tid; idx < rows_here * 32; idx += kTc2DequantThreads)
+          if ((idx & 31) * 8 < cols)
+            *reinterpret_cast<uint4*>(a.y + o0 + (size_t)(idx >> 5) * stride + (idx & 31) * 8) = *reinterpret_cast<const uint4*>(stage_h + (size_t)idx * 8);
       }
     } else if (ok && etile < n_tiles) {
       ptx::tc_fence_after_sync();
