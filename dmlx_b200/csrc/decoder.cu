@@ -1118,12 +1118,13 @@ b200_status b200_decoder::attention(b200_kv* kv, int run, int rows, void* stream
   return b200_window_attn_run(kv, c, d_row_seq, d_row_ctx, rows, attn_mma, stream);
 }
 
-// Token tile of the experts' matmuls: the rows an expert gets on average, rounded up.
+// Most rows of a work item of the experts' matmuls: the rows an expert gets on average, rounded up; above 64 the tile-pair kernel's 256, which
+// costs an item no more than the rows it has.
 int b200_decoder::moe_tile_rows(int T) const {
   if (f32()) return 64;
   int rows = 0;
   for (int i : moe_layers) rows = std::max(rows, (T * layers[i].s.top_k + layers[i].s.n_experts - 1) / layers[i].s.n_experts);
-  return std::min(128, std::max(16, (rows + 15) / 16 * 16));
+  return rows > 64 ? 256 : std::max(16, (rows + 15) / 16 * 16);
 }
 
 // What the layers of a step share: attention plans, chunks of the recurrent layers, rotations, experts.

@@ -269,3 +269,33 @@ def test_expert_parallel_layer_with_a_group_of_one_equals_the_plain_layer(mode_n
     layer.close()
     comm.close()
     plain.close()
+
+
+@pytest.mark.parametrize("n,epilogue", [(256, "swiglu"), (384, "swiglu"), (384, "none"), (136, "none"), (132, "none")])
+def test_dense_experts_by_pairs_of_weight_tiles(n, epilogue):
+    """Grouped matmul of dense bf16 weights with items of up to 256 rows (two weight tiles share an item's rows, which are loaded 64 at a time):
+    experts with no row, one, and one more or less than a copy, a half and a whole item; an odd number of weight tiles; outputs that cannot leave
+    in 16-byte pieces; row scales.  Every row against an f64 product of the same bf16 operands; results are rounded to bf16 once
+    (2^-8 of the value, 2^-7 with the scale and the gate in front)."""
+    from dmlx_b200 import device as dev
+
+    rng = np.random.default_rng(n + len(epilogue))
+    k, counts = 192, [0, 1, 15, 16, 17, 63, 64, 65, 127, 128, 129, 255, 256, 257, 300, 0, 40]
+    e, rows = len(counts), sum(counts)
+    wf = ref_math.bf16_round(rng.normal(0, k ** -0.5, (e, n, k)))
+    w = dev.QWeight(dev.Q_BF16, _bits(wf.reshape(e * n, k)), np.zeros(1, np.uint8), None, n, k, n_experts=e)
+    x = ref_math.bf16_round(rng.normal(0, 1, (rows, k)))
+    scales = rng.uniform(0.5, 2.0, rows).astype(np.float32)
+    first = np.concatenate([[0], np.cumsum(counts)])
+    items = [(i, first[i] + at, min(256, c - at), 0) for i, c in enumerate(counts) for at in range(0, c, 256)]
+    items_d = torch.tensor(items + [(0, 0, 0, 0)] * 5, dtype=torch.int32, device="cuda")
+    got = dev.moe_grouped_qmm(w, torch.tensor(x, device="cuda").bfloat16(), items_d, torch.tensor([len(items)], dtype=torch.int32, device="cuda"), 256,
+                              epilogue=dev.EPI_SWIGLU if epilogue == "swiglu" else dev.EPI_NONE, row_scales=torch.tensor(scales, device="cuda")).float().cpu().numpy()
+    assert dev.qmm_error_word() == 0
+    for i in range(e):
+        part = slice(first[i], first[i + 1])
+        y = x[part].astype(np.float64) @ wf[i].astype(np.float64).T
+        if epilogue == "swiglu":
+            y = y[:, 0::2] / (1 + np.exp(-y[:, 0::2])) * y[:, 1::2]
+        y = y * scales[part, None]
+        assert np.all(np.abs(got[part] - y) <= 2.0 ** -7 * np.abs(y) + 1e-4), (i, counts[i], np.abs(got[part] - y).max())

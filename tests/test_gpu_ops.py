@@ -414,3 +414,32 @@ def test_qmm_integer_small_batch_kernel_keeps_small_elements_beside_an_outlier()
         assert rel <= 2e-2 and cos >= 0.9995, (r, rel, cos)
         rel, cos = _close(got[r, : n // 2], want[r, : n // 2])
         assert rel <= 2e-2 and cos >= 0.9995, (r, "small elements", rel, cos)
+
+
+@pytest.mark.parametrize("mode_name", ["affine4", "bf16"])
+@pytest.mark.parametrize("rows", [130, 256, 257, 300, 513])
+@pytest.mark.parametrize("n", [256, 384, 1160, 1156])   # whole pairs of weight tiles, an odd one, rows that end inside a tile, rows of 8-byte multiples
+def test_tile_pair_kernel_adds_the_residual_in_place(mode_name, rows, n):
+    """Tile-pair matmul with the residual epilogue where y is the residual itself: token tiles with a remainder, odd numbers of weight tiles, rows
+    that cannot be moved in 16-byte pieces.  Against f64 products of the same operands: one rounding to bf16 (2^-8 of the value), f32 sums of
+    128 products, and for affine weights their rounding to bf16 (2^-9 of each weight)."""
+    from dmlx_b200 import device as dev
+
+    _bits = lambda a: (np.ascontiguousarray(a, np.float32).view(np.uint32) >> 16).astype(np.uint16)
+    rng = np.random.default_rng(rows + n)
+    k = 128
+    wf = rng.normal(0, 0.1, (n, k)).astype(np.float32)
+    if mode_name == "affine4":
+        packed, s, b = ref_math.quantize_affine4(wf)
+        w, deq = dev.QWeight(dev.Q_AFFINE4_G64, packed, _bits(s), _bits(b), n, k), ref_math.dequantize_affine4(packed, s, b)
+    else:
+        deq = ref_math.bf16_round(wf)
+        w = dev.QWeight(dev.Q_BF16, _bits(deq), np.zeros(1, np.uint8), None, n, k)
+    x = ref_math.bf16_round(rng.normal(0, 1, (rows, k)).astype(np.float32))
+    res = ref_math.bf16_round(rng.normal(0, 1, (rows, n)).astype(np.float32))
+    y = torch.tensor(res, device="cuda").bfloat16()
+    dev.qmm(w, torch.tensor(x, device="cuda").bfloat16(), epilogue=dev.EPI_RESIDUAL, residual=y, path=dev.QMM_TCGEN05_X2, out=y)
+    got, want = y.float().cpu().numpy(), res + x.astype(np.float64) @ deq.astype(np.float64).T
+    assert dev.qmm_error_word() == 0
+    bound = 2.0 ** -8 * np.abs(want) + 2.0 ** -9 * (np.abs(x).astype(np.float64) @ np.abs(deq).T.astype(np.float64)) * (1 if mode_name == "affine4" else 2.0 ** -10) + 1e-6
+    assert np.all(np.abs(got - want) <= bound), np.abs(got - want).max()
