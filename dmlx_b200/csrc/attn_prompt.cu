@@ -17,7 +17,7 @@
 // counter, since contexts differ.  A batch too small to fill the chip has its key ranges split, f32 partial sums, and a combine pass.
 //
 // Measured on one B200, bf16, 32/8 heads of 128: 3 portions of 683 tokens over 700..8000 cached 985 us in groups of 16 rows per warp on mma.sync
-// (paged_attn.cu), 171 us here; a step of four 512-token portions and 57 decoding requests 733 and 169 us per layer.
+// (paged_attn.cu), 165 us here; a step of four 512-token portions and 57 decoding requests 733 and 169 us per layer.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -548,32 +548,32 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
           }
         }
-        // A score that is no number weighs nothing, as a hidden one: it shows in the sum, and the block is done again without it.
-#pragma unroll 1
-        for (bool again = true, clean = false; again; clean = true) {
-          const float2 k2 = make_float2(a.scale_log2, a.scale_log2), m2 = make_float2(-m, -m);
+        const float2 k2 = make_float2(a.scale_log2, a.scale_log2), m2 = make_float2(-m, -m);
+        auto weigh = [&]() {  // P, and its sum
           float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             uint32_t p[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
-              const float2 x = fma2(make_float2(s[c * 64 + 2 * i], s[c * 64 + 2 * i + 1]), k2, m2), e = make_float2(ex2(x.x), ex2(x.y));
+              const float2 x = fma2(make_float2(s[c * 64 + 2 * i], s[c * 64 + 2 * i + 1]), k2, m2);
+              const float2 e = make_float2(ex2(x.x), ex2(x.y));
               sum[i & 1] = add2(sum[i & 1], e);
               p[i] = pack2(e.x, e.y);
             }
             ptx::tmem_st32(tmem_s(g) + lanes + c * 32, p);
           }
           const float2 both = add2(sum[0], sum[1]);
-          const float total = both.x + both.y;
-          again = !clean && __any_sync(0xffffffffu, total != total);
-          if (again) {
+          return both.x + both.y;
+        };
+        float total = weigh();
+        // A score that is no number weighs nothing, as a hidden one: it shows in the sum, and the block is done again without it.
+        if (__any_sync(0xffffffffu, total != total)) {
 #pragma unroll
-            for (int i = 0; i < kBlockKeys; ++i) s[i] = fmaxf(s[i], kHidden);
-          } else {
-            l += total;
-          }
+          for (int i = 0; i < kBlockKeys; ++i) s[i] = fmaxf(s[i], kHidden);
+          total = weigh();
         }
+        l += total;
         ptx::tmem_st_wait();
         ptx::tc_fence_before_sync();
         ptx::mbar_arrive(&sh.p_ready[g]);
