@@ -1467,21 +1467,37 @@ __global__ void __launch_bounds__(D) attn_combine_groups_kernel(AttnArgs a, __nv
   out[((size_t)row * a.n_q_heads + qh) * D + d] = __float2bfloat16(ll > 0.f ? acc / ll : 0.f);
 }
 
-// D threads per (row, query head): merge the row's chunks and write bf16.
+// D threads per (row, query head): merge the row's chunks and write bf16.  The lanes of a warp look at 32 chunks' maxima and sums at once and
+// hand the weights around; eight chunks' sums are in flight per thread.  (Bound by latency: with both loads in the loop over the chunks, four
+// at a time, 61 rows of 32 heads over 1..8192 tokens took 10.3-11.3 us per layer; 6.3-6.6 now.)
 template <int D>
 __global__ void __launch_bounds__(D) attn_combine_kernel(AttnArgs a, __nv_bfloat16* __restrict__ out) {
-  const int row = blockIdx.x / a.n_q_heads, qh = blockIdx.x - row * a.n_q_heads, d = threadIdx.x;
+  const int row = blockIdx.x / a.n_q_heads, qh = blockIdx.x - row * a.n_q_heads, d = threadIdx.x, lane = d & 31;
   if (a.d.state[ST_ATTN_ERR] != 0) return;
   const int c0 = a.chunk_start[row], c1 = a.chunk_start[row + 1];
-  float mm = -1e30f;
-  for (int c = c0; c < c1; ++c) mm = fmaxf(mm, a.part_ml[((size_t)c * a.n_q_heads + qh) * 2]);
-  float ll = 0.f, acc = 0.f;
-#pragma unroll 4
-  for (int c = c0; c < c1; ++c) {
-    const size_t pidx = (size_t)c * a.n_q_heads + qh;
-    const float w = exp2f(a.part_ml[pidx * 2] - mm);
-    ll += a.part_ml[pidx * 2 + 1] * w;
-    acc += a.part_o[pidx * D + d] * w;
+  const float2* ml = reinterpret_cast<const float2*>(a.part_ml);
+  const float* po = a.part_o + d;
+  float mm = -1e30f, ll = 0.f, acc = 0.f;
+  for (int base = c0; base < c1; base += 32) {
+    const int n = min(32, c1 - base);
+    const float2 mine = lane < n ? ml[(size_t)(base + lane) * a.n_q_heads + qh] : make_float2(-1e30f, 0.f);
+    float top = mine.x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    const float m_new = fmaxf(mm, top), corr = exp2f(mm - m_new), w = lane < n ? exp2f(mine.x - m_new) : 0.f;
+    float l = mine.y * w;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    ll = ll * corr + l;
+    acc *= corr;
+    mm = m_new;
+    for (int c = 0; c < n; c += 8) {
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = c + e < n ? po[((size_t)(base + c + e) * a.n_q_heads + qh) * D] : 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc = fmaf(v[e], __shfl_sync(0xffffffffu, w, (c + e) & 31), acc);
+    }
   }
   out[((size_t)row * a.n_q_heads + qh) * D + d] = __float2bfloat16(ll > 0.f ? acc / ll : 0.f);
 }
