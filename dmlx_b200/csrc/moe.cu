@@ -456,22 +456,34 @@ __global__ void gather_sorted_kernel(const __nv_bfloat16* __restrict__ x, const 
 __global__ void combine_kernel(const __nv_bfloat16* __restrict__ y_sorted, const int* __restrict__ inv_order, int k, int hidden,
                                const __nv_bfloat16* __restrict__ shared_out, __nv_bfloat16* __restrict__ out) {
   const int t = blockIdx.x;
-  if (hidden % 8 == 0 && k <= 16) {  // 16-byte loads, the row indices read once
-    int rows[16];
-    for (int j = 0; j < k; ++j) rows[j] = inv_order[t * k + j];
-    for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) {
+  if (hidden % 8 == 0 && k <= 16) {
+    // 16-byte loads, the rows of eight experts (and the shared one) asked for at once: one after the other they took 8.2 us at 24 tokens of
+    // 4096, top 6 (3.2 now), where a part of a row is a block's
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < hidden / 8; i += gridDim.y * blockDim.x) {
       float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int j = 0; j <= k; ++j) {
-        if (j == k && !shared_out) break;
-        const __nv_bfloat16* src = j < k ? y_sorted + (size_t)rows[j] * hidden : shared_out + (size_t)t * hidden;
-        const uint4 q = reinterpret_cast<const uint4*>(src)[i];
+      auto add = [&](const uint4& q) {
         const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           acc[2 * e] += __uint_as_float(w[e] << 16);
           acc[2 * e + 1] += __uint_as_float(w[e] & 0xFFFF0000u);
         }
+      };
+      uint4 shared_q = make_uint4(0u, 0u, 0u, 0u);
+      if (shared_out) shared_q = reinterpret_cast<const uint4*>(shared_out + (size_t)t * hidden)[i];
+      for (int j0 = 0; j0 < k; j0 += 8) {
+        int rows[8];
+        uint4 q[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) rows[j] = j0 + j < k ? inv_order[t * k + j0 + j] : 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (j0 + j < k) q[j] = reinterpret_cast<const uint4*>(y_sorted + (size_t)rows[j] * hidden)[i];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (j0 + j < k) add(q[j]);
       }
+      if (shared_out) add(shared_q);
       uint4 o;
       __nv_bfloat162 p0 = __floats2bfloat162_rn(acc[0], acc[1]), p1 = __floats2bfloat162_rn(acc[2], acc[3]);
       __nv_bfloat162 p2 = __floats2bfloat162_rn(acc[4], acc[5]), p3 = __floats2bfloat162_rn(acc[6], acc[7]);
@@ -481,6 +493,7 @@ __global__ void combine_kernel(const __nv_bfloat16* __restrict__ y_sorted, const
     }
     return;
   }
+  if (blockIdx.y > 0) return;
   for (int i = threadIdx.x; i < hidden / 2; i += blockDim.x) {
     float2 acc = make_float2(0.f, 0.f);
     for (int j = 0; j < k; ++j) {
@@ -612,7 +625,9 @@ b200_status b200_moe_combine(const void* d_y_sorted, const int32_t* d_inv_order,
   if (st != B200_OK) return st;
   if (hidden % 2) { b200_set_error("combine: hidden must be even"); return B200_ERR_INVALID_ARGUMENT; }
   if (n_tokens <= 0) return B200_OK;
-  combine_kernel<<<n_tokens, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)d_y_sorted, d_inv_order, k, hidden,
+  // (few tokens: a block per 2048 columns)
+  const int parts = n_tokens <= 512 && hidden % 8 == 0 && k <= 16 ? (hidden / 8 + 255) / 256 : 1;
+  combine_kernel<<<dim3(n_tokens, parts), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)d_y_sorted, d_inv_order, k, hidden,
                                                              (const __nv_bfloat16*)d_shared_out, (__nv_bfloat16*)d_out);
   B200_LAUNCH_CHECK();
   return B200_OK;
