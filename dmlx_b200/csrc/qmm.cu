@@ -32,6 +32,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <cstring>
 #include <vector>
 
@@ -1301,6 +1302,109 @@ __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma_kernel
     }
   }
   if (!ok) atomicExch(a.err, B200_ERR_DEVICE_FLAGGED);
+}
+
+// ---- dense bf16 weights, up to 16 rows ------------------------------------------------------------
+// A stream of weights with next to no arithmetic.  A CTA owns MT groups of 16 weight rows; its eight warps share K and add up through shared
+// memory, so nothing is split across CTAs and the epilogue is applied here.  Weights go straight from memory to mma.sync registers: lane t
+// of a quad takes the 16-byte pieces t and t + 4 of a block's 128-byte rows (K slots are a free permutation as long as both operands agree, and
+// the activations are read in the same pieces).  Many light CTAs, 32 to 64 KB of weights in flight per SM and CTA-wide set-up of nothing,
+// against a tensor-memory allocation, barriers, a ring and a finish pass per launch in qmm_tc_kernel: with 8 rows, 1536 x 512 outputs x K took
+// 5.3 + 2.2 us there and 2.5 here, 2816 x 512 2.9; experts of a step of 16 rows 56 -> 45 us (gate/up) and 37 -> 25 (down).
+constexpr int kFewRows = 16, kFewWarps = 8;
+
+template <int MT, int NT>
+__global__ void __launch_bounds__(kFewWarps * 32) qmm_few_kernel(QmmArgs a) {
+  constexpr int R = MT * 16, TOK = NT * 8, U = 2 / MT;
+  __shared__ float red[kFewWarps][TOK][R + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  int t0 = 0, rows_here = a.rows;
+  const unsigned char* blocks = a.blocks;
+  if (a.items) {
+    if ((int)blockIdx.z >= *a.n_items) return;
+    const int4 it = a.items[blockIdx.z];
+    blocks += (size_t)it.x * a.expert_stride;
+    t0 = it.y;
+    rows_here = it.z;
+  }
+  const int r0 = blockIdx.x * R, tile = r0 / kTileN, rr = r0 % kTileN;
+  const unsigned char* w = blocks + (size_t)tile * a.kc * (kTileN * 128) + (size_t)(rr + g) * 128;
+  const int piece[2] = {(t ^ g) << 4, ((t + 4) ^ g) << 4};  // swizzled place of pieces t and t + 4 (rr and 8 leave the row's low bits alone)
+  const __nv_bfloat16* x[NT];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) x[j] = a.x + (size_t)(t0 + min(j * 8 + g, rows_here - 1)) * a.k + t * 8;
+  float acc[MT][NT][4];
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) { acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f; }
+  // chunks warp, warp + 8, ...: the CTA's warps read neighbouring blocks at a time
+  auto work = [&](int c, auto count) {
+    constexpr int N = decltype(count)::value;
+    uint4 wv[N][MT][2][2], xv[N][NT][2];
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int half = 0; half < 2; ++half)
+            wv[u][i][h][half] = __ldcs(reinterpret_cast<const uint4*>(w + (size_t)(c + u * kFewWarps) * (kTileN * 128) + (i * 16 + half * 8) * 128 + piece[h]));
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) xv[u][j][h] = *reinterpret_cast<const uint4*>(x[j] + (size_t)(c + u * kFewWarps) * kChunkK + h * 32);
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint4 lo = wv[u][i][h][0], hi = wv[u][i][h][1];
+          const uint32_t f0[4] = {lo.x, hi.x, lo.y, hi.y}, f1[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            mma_bf16_full(acc[i][j], f1, xv[u][j][h].z, xv[u][j][h].w);
+            mma_bf16_full(acc[i][j], f0, xv[u][j][h].x, xv[u][j][h].y);
+          }
+        }
+  };
+  int c = warp;
+  for (; c + (U - 1) * kFewWarps < a.kc; c += U * kFewWarps) work(c, std::integral_constant<int, U>{});
+  for (; U > 1 && c < a.kc; c += kFewWarps) work(c, std::integral_constant<int, 1>{});
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) red[warp][j * 8 + 2 * t + (e & 1)][i * 16 + g + (e & 2) * 4] = acc[i][j][e];
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < R * TOK; idx += kFewWarps * 32) {  // (a multiple of the warp: its lanes stay together)
+    const int tok = idx / R, r = idx - tok * R, n = r0 + r, token = t0 + tok;
+    float part[kFewWarps];
+#pragma unroll
+    for (int q = 0; q < kFewWarps; ++q) part[q] = red[q][tok][r];
+#pragma unroll
+    for (int q = 1; q < kFewWarps; ++q) part[0] += part[q];
+    float v = part[0];
+    const float other = __shfl_xor_sync(0xffffffffu, v, 1);
+    if (tok >= rows_here) continue;
+    if (a.keep_f32) {  // the sums wait in scratch, as those of one K split
+      a.ws[((size_t)tile * a.tn + tok) * kTileN + rr + r] = v;
+    } else if (n < a.n) {
+      if (a.epilogue == B200_EPI_SWIGLU) {
+        if ((r & 1) == 0) a.y[(size_t)token * a.out_stride(a.n / 2) + n / 2] = __float2bfloat16(gated(a, v, other) * a.row_scale(token));
+      } else {
+        const size_t o = (size_t)token * a.out_stride(a.n) + n;
+        if (a.epilogue == B200_EPI_RESIDUAL) v += __bfloat162float(a.residual[o]);
+        else v = activate(a.epilogue, v);
+        a.y[o] = __float2bfloat16(v * a.row_scale(token));
+      }
+    }
+  }
 }
 
 // ---- small-batch kernel, integer variant (affine int4) --------------------------------------------
@@ -2736,6 +2840,37 @@ static b200_status launch_mma_nt(QmmArgs& a, int rows, cudaStream_t s) {
   return launch_finish(a, splits, s);
 }
 
+// Dense bf16 weights, up to 16 rows (of a batch, or of every work item).  Two groups of weight rows per CTA share the activations' loads where
+// that leaves at least two CTAs per SM.  Up to K = 2048 only: longer rows keep the tensor-memory kernels' deeper stream busy (K = 8192, 2048
+// outputs: 11.7 us there against 14.8 here; K = 5120: 7.9 against 10.6; K = 2048, 3072 outputs: 7.1 against 5.6).  The experts of one step are
+// many short grids at once and always come here.
+static bool takes_few(const QmmArgs& a, int rows) {
+  return rows <= kFewRows && ((uintptr_t)a.x & 15) == 0 && !a.y_f32 && a.groups == 0 && (a.items || a.kc <= 32);
+}
+static b200_status launch_few(QmmArgs& a, int rows, cudaStream_t s) {
+  a.tn = (rows + 15) / 16 * 16;
+  // A caller that takes partial sums gets f32 sums for the matrices whose K the tensor-memory kernels would split (17 rows and more do), and a
+  // bf16 result for the others, so that what follows rounds alike whatever the rows of the step.
+  const bool deferred = a.defer && a.epilogue == B200_EPI_NONE && !a.items && !a.row_scales && !a.norm_w &&
+                        (a.keep_f32 || (ensure_state(0) == B200_OK && pick_splits(a.nt, a.kc, g_sms, 2, 12) > 1));
+  if (deferred) a.keep_f32 = 1;
+  b200_status st = ensure_state(a.keep_f32 ? (size_t)a.tn * a.nt * kTileN * sizeof(float) : 0);
+  if (st != B200_OK) return st;
+  a.ws = g_ws[g_place]; a.err = g_err;
+  const int z = a.items ? a.max_items : 1;
+  const bool wide = (long long)((a.n + 31) / 32) * z >= 2 * g_sms;
+  const dim3 grid((a.n + (wide ? 31 : 15)) / (wide ? 32 : 16), 1, z);
+  if (rows <= 8) {
+    if (wide) qmm_few_kernel<2, 1><<<grid, kFewWarps * 32, 0, s>>>(a);
+    else qmm_few_kernel<1, 1><<<grid, kFewWarps * 32, 0, s>>>(a);
+  } else {
+    if (wide) qmm_few_kernel<2, 2><<<grid, kFewWarps * 32, 0, s>>>(a);
+    else qmm_few_kernel<1, 2><<<grid, kFewWarps * 32, 0, s>>>(a);
+  }
+  B200_LAUNCH_CHECK();
+  return a.keep_f32 ? launch_finish(a, 1, s) : B200_OK;
+}
+
 template <int NT8>
 static b200_status launch_mma8_nt(QmmArgs& a, int rows, cudaStream_t s) {
   const int tile = NT8 * 8;
@@ -2875,6 +3010,7 @@ static b200_status qmm_entry(const b200_qweight* w, const void* d_x, int32_t row
   // where its grid is one well-filled wave without a K split (gate/up-sized matrices: 74 vs 85 us at
   // 256 rows; elsewhere the tensor-memory kernel measured 3-8 % faster).  Dense bf16 weights: the
   // shared-memory-operand kernels.
+  const int32_t asked = path;
   if (path == B200_QMM_AUTO) {
     // MXFP4 at prefill-sized batches: the block-scaled tensor-core path once its grid (tile pairs x
     // 128-row token tiles, no K split) fills most of the GPU: 188 vs 261 us at 4096 x 4096 x 4096,
@@ -2916,7 +3052,9 @@ static b200_status qmm_entry(const b200_qweight* w, const void* d_x, int32_t row
   a.swiglu_alpha = g_shape.alpha; a.swiglu_shift = g_shape.shift;
   a.keep_f32 = g_defer_always ? 1 : 0;
   cudaStream_t s = (cudaStream_t)stream;
+  const bool few = asked == B200_QMM_AUTO && w->mode == B200_Q_BF16 && takes_few(a, rows);
   auto dispatch = [&]() -> b200_status {
+    if (few) return launch_few(a, rows, s);
     if (path == B200_QMM_MXFP4_BLOCK_SCALED) return launch_mx(w, a, rows, s);
     if (path == B200_QMM_MMA_I8) {
       if (w->mode != B200_Q_AFFINE4_G64) { b200_set_error("qmm: the integer small-batch kernel serves affine int4 weights"); return B200_ERR_UNSUPPORTED; }
@@ -3135,6 +3273,7 @@ b200_status b200_qmm_grouped(const b200_qweight* w, const void* d_x, int32_t row
     return w->mode == B200_Q_AFFINE4_G64 ? launch_tca<B200_Q_AFFINE4_G64>(a, rows, s) : launch_tca<B200_Q_MXFP4_G32>(a, rows, s);
   if (w->mode == B200_Q_AFFINE4_G64) return launch_tc<B200_Q_AFFINE4_G64>(a, rows, s);
   if (w->mode == B200_Q_MXFP4_G32) return launch_tc<B200_Q_MXFP4_G32>(a, rows, s);
+  if (takes_few(a, tile_rows)) return launch_few(a, tile_rows, s);
   // dense weights, items of more than 128 rows: two weight tiles share the item's rows (32 experts of 1024 x 2048 with 253 rows on average:
   // gate/up 175 -> 99 us, down 141 -> 64)
   return tile_rows > 128 ? launch_tc2<B200_Q_BF16>(a, rows, s) : launch_tc<B200_Q_BF16>(a, rows, s);

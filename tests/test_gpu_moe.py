@@ -299,3 +299,32 @@ def test_dense_experts_by_pairs_of_weight_tiles(n, epilogue):
             y = y[:, 0::2] / (1 + np.exp(-y[:, 0::2])) * y[:, 1::2]
         y = y * scales[part, None]
         assert np.all(np.abs(got[part] - y) <= 2.0 ** -7 * np.abs(y) + 1e-4), (i, counts[i], np.abs(got[part] - y).max())
+
+
+@pytest.mark.parametrize("n,k,epilogue", [(256, 64, "swiglu"), (384, 576, "swiglu"), (132, 192, "none"), (1160, 2176, "none")])
+def test_dense_experts_with_few_rows(n, k, epilogue):
+    """Grouped matmul of dense bf16 weights with items of up to 16 rows: experts with no row, one, and one more or less than a half and a whole
+    item; K in fewer chunks than warps and in a remainder of them.  Bounds as for the items of pairs of tiles."""
+    from dmlx_b200 import device as dev
+
+    rng = np.random.default_rng(n + k)
+    tile_rows, counts = 16, [0, 1, 7, 8, 9, 15, 16, 17, 0, 40, 3]
+    e, rows = len(counts), sum(counts)
+    wf = ref_math.bf16_round(rng.normal(0, k ** -0.5, (e, n, k)))
+    w = dev.QWeight(dev.Q_BF16, _bits(wf.reshape(e * n, k)), np.zeros(1, np.uint8), None, n, k, n_experts=e)
+    x = ref_math.bf16_round(rng.normal(0, 1, (rows, k)))
+    scales = rng.uniform(0.5, 2.0, rows).astype(np.float32)
+    first = np.concatenate([[0], np.cumsum(counts)])
+    items = [(i, first[i] + at, min(tile_rows, c - at), 0) for i, c in enumerate(counts) for at in range(0, c, tile_rows)]
+    items_d = torch.tensor(items + [(0, 0, 0, 0)] * 5, dtype=torch.int32, device="cuda")
+    got = dev.moe_grouped_qmm(w, torch.tensor(x, device="cuda").bfloat16(), items_d, torch.tensor([len(items)], dtype=torch.int32, device="cuda"),
+                              tile_rows, epilogue=dev.EPI_SWIGLU if epilogue == "swiglu" else dev.EPI_NONE,
+                              row_scales=torch.tensor(scales, device="cuda")).float().cpu().numpy()
+    assert dev.qmm_error_word() == 0
+    for i in range(e):
+        part = slice(first[i], first[i + 1])
+        y = x[part].astype(np.float64) @ wf[i].astype(np.float64).T
+        if epilogue == "swiglu":
+            y = y[:, 0::2] / (1 + np.exp(-y[:, 0::2])) * y[:, 1::2]
+        y = y * scales[part, None]
+        assert np.all(np.abs(got[part] - y) <= 2.0 ** -7 * np.abs(y) + 1e-4), (i, counts[i], np.abs(got[part] - y).max())

@@ -443,3 +443,36 @@ def test_tile_pair_kernel_adds_the_residual_in_place(mode_name, rows, n):
     assert dev.qmm_error_word() == 0
     bound = 2.0 ** -8 * np.abs(want) + 2.0 ** -9 * (np.abs(x).astype(np.float64) @ np.abs(deq).T.astype(np.float64)) * (1 if mode_name == "affine4" else 2.0 ** -10) + 1e-6
     assert np.all(np.abs(got - want) <= bound), np.abs(got - want).max()
+
+
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(128, 64), (1156, 320), (1160, 576), (4128, 1088), (10000, 2048), (384, 2112)])
+def test_dense_weights_with_few_rows(rows, n, k):
+    """Dense bf16 weights under up to 16 rows: half and whole groups of 8 rows, K in fewer chunks than warps, in a remainder of them and at either
+    side of the longest that the kernel without tensor memory takes, outputs that end inside a weight tile, one and two groups of weight rows
+    per block, every epilogue and the residual in place.  Against f64 products of the same operands: f32 sums (K 2^-24 of the absolute products)
+    and one rounding to bf16 (2^-8 of the value; 2^-7 behind the gate and the activation, whose slopes stay under 1.2)."""
+    from dmlx_b200 import device as dev
+
+    rng = np.random.default_rng(rows + n + k)
+    wf = ref_math.bf16_round(rng.normal(0, 1, (n, k)) * k ** -0.5)
+    w = dev.QWeight(dev.Q_BF16, (wf.view(np.uint32) >> 16).astype(np.uint16), np.zeros(1, np.uint8), None, n, k)
+    x = ref_math.bf16_round(rng.normal(0, 1, (rows, k)).astype(np.float32))
+    res = ref_math.bf16_round(rng.normal(0, 1, (rows, n)).astype(np.float32))
+    xd, y = torch.tensor(x, device="cuda").bfloat16(), torch.tensor(res, device="cuda").bfloat16()
+    s = x.astype(np.float64) @ wf.astype(np.float64).T
+    sums = 2.0 ** -24 * k * (np.abs(x).astype(np.float64) @ np.abs(wf).T.astype(np.float64))
+    g, u = s[:, 0::2], s[:, 1::2]
+    dev.qmm(w, xd, epilogue=dev.EPI_RESIDUAL, residual=y, out=y)
+    for name, got, want, tol in (
+            ("none", dev.qmm(w, xd), s, 2.0 ** -8 * np.abs(s) + sums),
+            ("residual", y, s + res, 2.0 ** -8 * np.abs(s + res) + sums),
+            ("swiglu", dev.qmm(w, xd, epilogue=dev.EPI_SWIGLU), g / (1 + np.exp(-g)) * u,
+             2.0 ** -7 * np.abs(g * u) + 1.2 * (np.abs(g) * sums[:, 1::2] + np.abs(u) * sums[:, 0::2]) + 1e-5),
+            ("gelu", dev.qmm(w, xd, epilogue=dev.EPI_GELU), None, 2.0 ** -7 * np.abs(s) + 1.2 * sums + 1e-5)):
+        got = got.double().cpu().numpy()
+        if want is None:
+            want = torch.nn.functional.gelu(torch.tensor(s)).numpy()
+        bad = np.abs(got - want) > tol
+        assert not bad.any(), (name, np.abs(got - want)[bad].max())
+    assert dev.qmm_error_word() == 0
