@@ -123,6 +123,33 @@ def test_pool_random_workload_bit_exact():
         kv.close()
 
 
+@pytest.mark.parametrize("n_req", [1, 32, 33, 255, 256, 257, 600])
+def test_reservation_of_many_requests_at_once(n_req):
+    """A step of as many requests as either block size of the reservation takes, one more and one less: growth, pages shared with a sequence
+    of the same step (copied once), then a step that the pool cannot serve, which changes nothing."""
+    dev = _dev()
+    rng = np.random.default_rng(n_req)
+    n_seqs, n_pages = n_req + 4, 2 * n_req + 8
+    kv = dev.PagedKVCache(1, 2, 64, n_pages, n_seqs, 64, 8, max_rows=4096)
+    ref = ref_host.PagedKVTables(n_pages, n_seqs)
+    seqs = rng.permutation(n_seqs - 4)[:n_req].tolist()
+    steps = [rng.integers(1, 7, n_req).tolist(), rng.integers(1, 7, n_req).tolist(), [66] * n_req, [1] * n_req]
+    for step, counts in enumerate(steps):
+        try:
+            ref.reserve(seqs, counts)
+            expect_err = 0
+        except ref_host.InsufficientBlocks:
+            expect_err = 1
+        kv.reserve(_desc(dev, [(s, c, 0, -1) for s, c in zip(seqs, counts)]))
+        assert kv.error_word() == expect_err
+        _check_tables(kv, ref, n_seqs)
+        if step == 0 and n_req > 2:  # the last request of the step shares the page of the first one
+            for side in (ref, kv):
+                side.release(seqs[-1]) if side is ref else kv.release([seqs[-1]])
+                side.fork(seqs[0], seqs[-1], ref.lens[seqs[0]])
+    kv.close()
+
+
 def test_cow_two_sharers_same_step():
     """Two sequences that share a partially filled page and both append in one step: the first
     (in batch order) takes a private copy, the second keeps the original (paged.zig:167-206)."""
