@@ -31,7 +31,10 @@ namespace {
 
 constexpr int kBlockKeys = 128, kBlockPages = 4, kTileRows = 128;
 constexpr int kThreads = 320;
-constexpr float kGrow = 8.f;            // log2 units a row's scale may lag behind its scores
+// log2 units a row's scale may lag behind its scores.  0 takes 193 us instead of 160 (3 portions of 683 tokens over 700..8000).  P is bf16 either
+// way, as in the groups of paged_attn.cu; the scale decides which weights are exact: a row's largest one is 1 where the scale follows every 32
+// keys.  Error of the results against 64 bits there 2.13e-3, here 2.19e-3 (0: 2.15e-3), of which 1.7e-3 are the rounding of the results.
+constexpr float kGrow = 8.f;
 constexpr float kHidden = -1e30f;       // score of a key that a row does not see
 constexpr float kNoScale = -1e28f;      // scale of a row that has seen no key: exp2 of any hidden score against it is 0
 constexpr uint32_t kPolls = 1u << 21;   // a wait inside a CTA is microseconds
