@@ -769,6 +769,8 @@ __global__ void __launch_bounds__(kTcaThreads, 2) qmm_tca_kernel(const __grid_co
 constexpr int kTc2Threads = 19 * 32;  // warps 0-15 dequantise, 16 streams the weights, 17 issues MMAs, 18 loads activation tiles
 constexpr int kTc2DequantThreads = 16 * 32;
 constexpr int kGroupBox = 64;  // rows of expert-sorted activations per copy
+// Rows that a stage's activation tile has room for: a work item's arrive in whole copies, so its tile is as many of them as cover tn.
+__host__ __device__ constexpr int tc2_x_rows(bool grouped, int tn) { return grouped ? (tn + kGroupBox - 1) / kGroupBox * kGroupBox : tn; }
 
 // Quantised weights: the raw 4-bit blocks have a ring of their own (SR slots of two blocks), released as
 // soon as the dequantising warps hold the words in registers, so the weight stream runs ahead of the
@@ -784,7 +786,7 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
   constexpr bool kDense = MODE == B200_Q_BF16;
   constexpr int RB = kDense ? 0 : ((BB + 127) / 128) * 128;
   const int tn = a.tn, stages = a.stages, SR = a.x_slots;
-  const int stage_stride = 2 * kTileN * 128 + tn * 128;
+  const int stage_stride = 2 * kTileN * 128 + tc2_x_rows(a.items != nullptr, tn) * 128;
   auto a_tile = [&](int s, int tile) { return smem + (size_t)s * stage_stride + tile * (kTileN * 128); };
   auto x_tile = [&](int s) { return smem + (size_t)s * stage_stride + 2 * kTileN * 128; };
   auto raw_blk = [&](int sr, int tile) { return smem + (size_t)stages * stage_stride + (size_t)(sr * 2 + tile) * RB; };
@@ -2756,7 +2758,7 @@ static b200_status launch_tc2(QmmArgs& a, int rows, cudaStream_t s) {
   if (st != B200_OK) return st;
   constexpr int BB = block_bytes(MODE);
   constexpr int RB = MODE == B200_Q_BF16 ? 0 : ((BB + 127) / 128) * 128;
-  const int stage_stride = 2 * kTileN * 128 + tn * 128;
+  const int stage_stride = 2 * kTileN * 128 + tc2_x_rows(a.items != nullptr, tn) * 128;
   static int smem_budget[3] = {0, 0, 0};
   if (smem_budget[MODE] == 0) {
     int dev = 0, optin = 0;

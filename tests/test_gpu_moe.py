@@ -328,3 +328,60 @@ def test_dense_experts_with_few_rows(n, k, epilogue):
             y = y[:, 0::2] / (1 + np.exp(-y[:, 0::2])) * y[:, 1::2]
         y = y * scales[part, None]
         assert np.all(np.abs(got[part] - y) <= 2.0 ** -7 * np.abs(y) + 1e-4), (i, counts[i], np.abs(got[part] - y).max())
+
+
+@pytest.mark.parametrize("tile_rows", [144, 160, 176, 192, 208, 224, 240, 256])
+@pytest.mark.parametrize("epilogue", ["swiglu", "none"])
+def test_dense_experts_at_every_item_size_above_128(tile_rows, epilogue):
+    """Items of any accepted size above 128 rows, which arrive 64 rows at a time: full ones, a row short of it, a row more than whole copies, and
+    K of more chunks than a block has stages.  Bounds as for the items of pairs of tiles."""
+    from dmlx_b200 import device as dev
+
+    rng = np.random.default_rng(tile_rows)
+    n, k, counts = 384, 448, [tile_rows, tile_rows - 1, tile_rows - 15, tile_rows - 16, 64, 65, 128, 129, 0, tile_rows + 1, 1, 2 * tile_rows]
+    e, rows = len(counts), sum(counts)
+    wf = ref_math.bf16_round(rng.normal(0, k ** -0.5, (e, n, k)))
+    w = dev.QWeight(dev.Q_BF16, _bits(wf.reshape(e * n, k)), np.zeros(1, np.uint8), None, n, k, n_experts=e)
+    x = ref_math.bf16_round(rng.normal(0, 1, (rows, k)))
+    first = np.concatenate([[0], np.cumsum(counts)])
+    items = [(i, first[i] + at, min(tile_rows, c - at), 0) for i, c in enumerate(counts) for at in range(0, c, tile_rows)]
+    got = dev.moe_grouped_qmm(w, torch.tensor(x, device="cuda").bfloat16(), torch.tensor(items, dtype=torch.int32, device="cuda"),
+                              torch.tensor([len(items)], dtype=torch.int32, device="cuda"), tile_rows,
+                              epilogue=dev.EPI_SWIGLU if epilogue == "swiglu" else dev.EPI_NONE).float().cpu().numpy()
+    assert dev.qmm_error_word() == 0
+    for i in range(e):
+        part = slice(first[i], first[i + 1])
+        y = x[part].astype(np.float64) @ wf[i].astype(np.float64).T
+        if epilogue == "swiglu":
+            y = y[:, 0::2] / (1 + np.exp(-y[:, 0::2])) * y[:, 1::2]
+        assert np.all(np.abs(got[part] - y) <= 2.0 ** -7 * np.abs(y) + 1e-4), (i, counts[i], np.abs(got[part] - y).max())
+
+
+@pytest.mark.parametrize("tile_rows", [208, 256])
+def test_layer_of_dense_experts_with_large_items(tile_rows):
+    """MoELayer over dense experts whose items hold more than 128 rows: a few popular experts, every token against f64 sums over the routing that
+    the layer reports (two matmuls of bf16 operands, the gated rows and the results rounded to bf16)."""
+    from dmlx_b200 import device as dev
+
+    rng = np.random.default_rng(tile_rows)
+    hidden, e, inter, k, n = 256, 5, 128, 2, 500
+    mats = [ref_math.bf16_round(rng.normal(0, 1, s) * s[-1] ** -0.5) for s in ((e, hidden), (e, 2 * inter, hidden), (e, hidden, inter))]
+    wg, wu, wd = mats
+    qw = lambda m, ne=1: dev.QWeight(dev.Q_BF16, _bits(m.reshape(-1, m.shape[-1])), np.zeros(1, np.uint8), None, m.shape[-2], m.shape[-1], n_experts=ne)
+    bias = np.array([0.3, 0.2, 0.0, -0.1, -0.2], np.float32)
+    layer = dev.MoELayer(hidden, e, inter, k, qw(wg), qw(wu, e), qw(wd, e), bias=bias, swiglu_limit=0.0, tile_rows=tile_rows, max_tokens=n)
+    x = ref_math.bf16_round(rng.normal(0, 1, (n, hidden)))
+    got = layer.forward(torch.tensor(x, device="cuda").bfloat16()).float().cpu().numpy()
+    assert dev.qmm_error_word() == 0
+    idx, wts, off = layer.last_routing(n)
+    assert np.diff(off).max() > tile_rows
+    want = np.zeros((n, hidden))
+    for j in range(k):
+        for ex in range(e):
+            t = np.where(idx[:, j] == ex)[0]
+            y = x[t].astype(np.float64) @ wu[ex].astype(np.float64).T
+            a = y[:, 0::2] / (1 + np.exp(-y[:, 0::2])) * y[:, 1::2] * wts[t, j][:, None]
+            want[t] += a @ wd[ex].astype(np.float64).T
+    rel, cos = _close(got, want)
+    assert rel <= 2e-2 and cos >= 0.9999, (rel, cos)
+    layer.close()
