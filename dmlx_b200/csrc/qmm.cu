@@ -809,6 +809,7 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
     blocks += (size_t)it.x * a.expert_stride;
     t0 = it.y;
     rows_here = it.z;
+    if (rows_here <= 0) return;  // (an MMA of no columns does not exist)
   }
   const int tn_here = (rows_here + 15) / 16 * 16;  // only the rows that exist are multiplied
   const int nt0 = 2 * pair;
@@ -1328,6 +1329,7 @@ __global__ void __launch_bounds__(kFewWarps * 32) qmm_few_kernel(QmmArgs a) {
     blocks += (size_t)it.x * a.expert_stride;
     t0 = it.y;
     rows_here = it.z;
+    if (rows_here <= 0) return;  // (there is no row to stand in for the missing ones)
   }
   const int r0 = blockIdx.x * R, tile = r0 / kTileN, rr = r0 % kTileN;
   const unsigned char* w = blocks + (size_t)tile * a.kc * (kTileN * 128) + (size_t)(rr + g) * 128;

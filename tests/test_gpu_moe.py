@@ -385,3 +385,22 @@ def test_layer_of_dense_experts_with_large_items(tile_rows):
     rel, cos = _close(got, want)
     assert rel <= 2e-2 and cos >= 0.9999, (rel, cos)
     layer.close()
+
+
+@pytest.mark.parametrize("tile_rows", [16, 64, 128, 256])
+def test_dense_items_without_rows_write_nothing(tile_rows):
+    """Work items of no rows among the others, the first one at row 0: skipped by every kernel that serves dense experts."""
+    from dmlx_b200 import device as dev
+
+    rng = np.random.default_rng(tile_rows)
+    n, k, e, count = 256, 128, 3, min(tile_rows, 40)
+    wf = ref_math.bf16_round(rng.normal(0, k ** -0.5, (e, n, k)))
+    w = dev.QWeight(dev.Q_BF16, _bits(wf.reshape(e * n, k)), np.zeros(1, np.uint8), None, n, k, n_experts=e)
+    x = ref_math.bf16_round(rng.normal(0, 1, (2 * count, k)))
+    items = [(0, 0, 0, 0), (1, 0, count, 0), (2, count, 0, 0), (2, count, count, 0), (0, 2 * count, 0, 0)]
+    got = dev.moe_grouped_qmm(w, torch.tensor(x, device="cuda").bfloat16(), torch.tensor(items, dtype=torch.int32, device="cuda"),
+                              torch.tensor([len(items)], dtype=torch.int32, device="cuda"), tile_rows).float().cpu().numpy()
+    assert dev.qmm_error_word() == 0
+    for ex, part in ((1, slice(0, count)), (2, slice(count, 2 * count))):
+        y = x[part].astype(np.float64) @ wf[ex].astype(np.float64).T
+        assert np.all(np.abs(got[part] - y) <= 2.0 ** -8 * np.abs(y) + 1e-4)
