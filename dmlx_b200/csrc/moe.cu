@@ -14,6 +14,7 @@
 //             (src/models/deepseek_v4.zig:809-819,1051).
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "common.h"
@@ -726,7 +727,8 @@ b200_status b200_moe_create(const b200_moe_config* c, const b200_qweight* gate, 
   // with expert parallelism every rank routes the tokens of all ranks; a rank's matmul rows are the
   // assignments that fall on its experts, at most all of them
   const size_t N = (size_t)c->max_tokens * world, A = N * c->top_k;
-  m->max_items = n_local + (int)((A + c->tile_rows - 1) / c->tile_rows);
+  // (a step of few tokens has items of no more rows than tokens: up to top_k of them beyond one per expert, where a token chose experts twice)
+  m->max_items = n_local + std::max(c->top_k, (int)((A + c->tile_rows - 1) / c->tile_rows));
 #define M_ALLOC(ptr, bytes)                                                                  \
   do {                                                                                       \
     if (cudaMalloc((void**)&(ptr), (bytes)) != cudaSuccess) {                                \
@@ -774,9 +776,9 @@ b200_status b200_moe_forward(b200_moe* m, const void* d_x, int32_t n_tokens, voi
   if (n_tokens > c.max_tokens) { b200_set_error("moe: %d tokens > max_tokens %d", n_tokens, c.max_tokens); return B200_ERR_CAPACITY; }
   if (n_tokens <= 0) return B200_OK;
   const int A = n_tokens * c.top_k;
-  // A token chooses an expert at most once, so no expert has more rows than there are tokens: a tile no larger than that leaves the
-  // block-scaled kernel five stages of weights in flight instead of three (24 tokens on 32 experts of 4096 x 2048, top 6:
-  // 248 -> 194 us a layer).
+  // A token chooses an expert once (more often only where fewer than top_k logits are numbers), so hardly an expert has more rows than there
+  // are tokens: a tile no larger than that leaves the block-scaled kernel five stages of weights in flight instead of three (24 tokens on
+  // 32 experts of 4096 x 2048, top 6: 248 -> 194 us a layer).
   const int tile_rows = c.tile_rows <= 128 ? std::min(c.tile_rows, (n_tokens + 15) / 16 * 16) : c.tile_rows;
   b200_status st;
 #define STEP(call) do { if ((st = (call)) != B200_OK) return st; } while (0)

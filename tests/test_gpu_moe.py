@@ -404,3 +404,31 @@ def test_dense_items_without_rows_write_nothing(tile_rows):
     for ex, part in ((1, slice(0, count)), (2, slice(count, 2 * count))):
         y = x[part].astype(np.float64) @ wf[ex].astype(np.float64).T
         assert np.all(np.abs(got[part] - y) <= 2.0 ** -8 * np.abs(y) + 1e-4)
+
+
+def test_layer_whose_router_finds_one_number_per_token():
+    """Router logits that are no number but for one expert per token: that expert is chosen top_k times, so experts have more rows than the step
+    has tokens and more work items than one each.  The layer's item list holds them, and every token gets its expert's output."""
+    from dmlx_b200 import device as dev
+
+    rng = np.random.default_rng(3)
+    hidden, e, inter, k, n = 128, 6, 64, 6, 16
+    pick = np.arange(n) // 3   # three tokens of six choices each: 18 rows for items of 16
+    gate = np.zeros((e, hidden), np.float32)
+    gate[np.arange(e), np.arange(e)] = np.inf
+    x = ref_math.bf16_round(rng.normal(0, 1, (n, hidden)))
+    x[:, :e] = np.eye(e, dtype=np.float32)[pick]
+    wu, wd = (ref_math.bf16_round(rng.normal(0, 1, s) * s[-1] ** -0.5) for s in ((e, 2 * inter, hidden), (e, hidden, inter)))
+    qw = lambda m, ne=1: dev.QWeight(dev.Q_BF16, (np.ascontiguousarray(m, np.float32).reshape(-1, m.shape[-1]).view(np.uint32) >> 16).astype(np.uint16),
+                                     np.zeros(1, np.uint8), None, m.shape[-2], m.shape[-1], n_experts=ne)
+    layer = dev.MoELayer(hidden, e, inter, k, qw(gate), qw(wu, e), qw(wd, e), scoring=dev.SCORE_SIGMOID, swiglu_limit=0.0, tile_rows=128, max_tokens=n)
+    got = layer.forward(torch.tensor(x, device="cuda").bfloat16()).float().cpu().numpy()
+    assert dev.qmm_error_word() == 0
+    idx, wts, off = layer.last_routing(n)
+    assert (idx == pick[:, None]).all() and np.allclose(wts, 1.0 / k)
+    assert sum(-(-c // 16) for c in np.diff(off)) > e + 1
+    y = np.einsum("nh,nih->ni", x.astype(np.float64), wu[pick].astype(np.float64))
+    a = y[:, 0::2] / (1 + np.exp(-y[:, 0::2])) * y[:, 1::2]
+    rel, cos = _close(got, np.einsum("ni,nhi->nh", a, wd[pick].astype(np.float64)))
+    assert rel <= 2e-2 and cos >= 0.9999, (rel, cos)
+    layer.close()
