@@ -453,3 +453,21 @@ def test_admission_budget_in_pages_keeps_arrival_order(H):
     s.set_admission_budget(None)
     r = s.schedule()
     assert [q.id for q in r.prefill_requests] == [1, 2, 3, 4]
+
+
+# ---- numbers of a step, as the Python layer hands them over ----------------------------------------
+
+
+@pytest.mark.parametrize("name", ["list", "tuple", "range", "bytes", "bytearray", "memoryview", "int16", "uint32", "int64", "strided", "floats", "strings", "wrapped", "empty", "empty_bytes"])
+def test_tokens_of_a_step_are_taken_one_by_one(name):
+    """Whatever holds the tokens of a step, each element is a token as int() sees it, wrapped to 32 bits like a ctypes field; bytes are a
+    token each (their lengths: those that eight-byte words divide, and others)."""
+    from dmlx_b200 import device as dev
+
+    values = {"list": [3, 1, 2], "tuple": (7, 8), "range": range(5), "bytes": bytes(range(16)), "bytearray": bytearray(b"\x01\x02\xff"),
+              "memoryview": memoryview(bytes(range(8))), "int16": np.array([1, 2, 3], np.int16), "uint32": np.array([1, 2 ** 32 - 1], np.uint32),
+              "int64": np.array([5, 6]), "strided": np.arange(10, dtype=np.uint32)[::3], "floats": [1.0, 2.9], "strings": "407",
+              "wrapped": [-1, 2 ** 32 + 5, 2 ** 70 + 9], "empty": [], "empty_bytes": b""}[name]
+    got = dev._packed(values, np.uint32)
+    assert got.dtype == np.uint32 and got.flags.c_contiguous
+    assert got.tolist() == [int(t) & 0xFFFFFFFF for t in values]
