@@ -13,6 +13,12 @@
 // softmax groups take the blocks in turn, with sums of their own, and put them together at the end.  Such items are bound by the stream of
 // pages, 64 KB per block.
 //
+// A key that a row does not see has weight 0 there, and 0 times a value that is no finite number is no number: a group's rows share their blocks
+// of values, so one such value would reach up to 256 / G tokens ahead of its own.  The softmax threads therefore look through the values of the
+// blocks that some row does not see whole (one or two of an item, the rest of its last page among them), clear what is not finite, and a row
+// that does see it gets it back at the end.  The look costs 64 packed multiply-adds per thread and such block: 3 portions of 683 tokens over
+// 700..8000 160 us with and without.
+//
 // Two tiles of 128 rows: a CTA reads 64 KB of pages per block for 256 rows; one tile would read them twice.  Items go longest first, from a
 // counter, since contexts differ.  A batch too small to fill the chip has its key ranges split, f32 partial sums, and a combine pass.
 //
@@ -62,12 +68,14 @@ struct Args {
   float *part_o, *part_ml;
   __nv_bfloat16* out;
   float scale_log2;
+  bool may_split;  // such batches give 0 for a row whose sum is no number, as the decode kernels do; the others what comes out
 };
 
 template <int D>
 struct Shared {
   uint64_t full[Shape<D>::kSlots], free[Shape<D>::kSlots], q_full, q_free, s_full[2], p_ready[2], o_full[2], item_full[2], item_free[2], merged[2], drain;
   Item items[2];
+  uint32_t cleared[4];  // item n of this CTA had values cleared: [n % 4] is n + 1 (a softmax group is never three items ahead of the other)
   uint32_t tmem;
   float m[2][kTileRows], l[2][kTileRows];
 };
@@ -260,10 +268,43 @@ __global__ void __launch_bounds__(1024) prompt_plan_kernel(const int* __restrict
   }
 }
 
+// ---- values that are not finite ------------------------------------------------------------------------------------
+// Pieces of 16 bytes from `first` on, one for each thread of a tile in turn, in every box of a block of values: what is not finite becomes 0.
+template <int D>
+__device__ __noinline__ void clear_pieces(uint4* v, int first, int pieces, uint32_t* mark, uint32_t value) {
+  auto clear = [](uint32_t w) { return ((w & 0x7F80u) == 0x7F80u ? 0u : w & 0xFFFFu) | ((w & 0x7F800000u) == 0x7F800000u ? 0u : w & 0xFFFF0000u); };
+  for (int i = first; i < pieces; i += kTileRows)
+    for (int x = 0; x < Shape<D>::kBoxes; ++x) {
+      const uint4 q = v[x * (kBlockKeys * 8) + i], z = make_uint4(clear(q.x), clear(q.y), clear(q.z), clear(q.w));
+      if (q.x == z.x && q.y == z.y && q.z == z.z && q.w == z.w) continue;
+      *reinterpret_cast<volatile uint32_t*>(mark) = value;
+      __threadfence_block();  // (who finds the values cleared finds the mark)
+      v[x * (kBlockKeys * 8) + i] = z;
+    }
+}
+// (Written out where it is used, in loops that stay loops: as a function it cost the whole kernel 9 %, for the registers that a call takes.)
+// The cleared values that a row sees, onto its columns c_begin..c_end as they were written.
+template <int D>
+__device__ __forceinline__ void add_cleared(const Args& a, const Item& it, int ctx, int c_begin, int c_end, __nv_bfloat16* row, float* partial) {
+  const int begin = it.page_begin * 32, first = max(begin, begin + (it.ctx0 - begin) / kBlockKeys * kBlockKeys);
+#pragma unroll 1
+  for (int key = first; key < min(ctx, it.page_end * 32); ++key) {
+    const size_t page = (size_t)a.layer * a.d.n_pages + a.d.block_table[(size_t)it.seq * a.d.max_pages_per_seq + key / 32];
+    const __nv_bfloat16* v = reinterpret_cast<const __nv_bfloat16*>(a.d.v_pool) + ((page * a.d.n_kv_heads + it.head) * 32 + key % 32) * D;
+#pragma unroll 1
+    for (int c = c_begin; c < c_end; ++c) {
+      const float value = __bfloat162float(v[c]);
+      if (isfinite(value)) continue;
+      if (row) row[c] = __float2bfloat16(__bfloat162float(row[c]) + value);
+      else partial[c] += value;
+    }
+  }
+}
+
 // ---- the kernel ---------------------------------------------------------------------------------------------------
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
-    prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap qmap, Args a) {
+    prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ Args a) {
   using Z = Shape<D>;
   extern __shared__ __align__(1024) unsigned char smem[];  // (there is no room for a base that has to be rounded up)
   unsigned char* qbuf = smem;                        // [tile][box][128 rows][128 B]
@@ -283,6 +324,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       ptx::mbar_init(&sh.merged[t], 2 * kTileRows);
     }
     ptx::mbar_init(&sh.drain, 1);
+    for (int i = 0; i < 4; ++i) sh.cleared[i] = 0;
     ptx::mbar_fence_init();
   }
   if (warp == 9) {
@@ -494,7 +536,27 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ---- softmax: a thread per row ----
     const int g = warp >> 2, row = (warp & 3) * 32 + lane;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    uint32_t n_s = 0, n_o[2] = {0, 0}, n_m = 0;
+    uint32_t n_s = 0, n_o[2] = {0, 0}, n_m = 0, loads = 0;  // loads: of the items before
+    // Clears what is not finite among the values of a block (the group's threads a 16-byte piece each, in turn).
+    auto clear_values = [&](uint32_t load, int pages, uint32_t n) {
+      wait(&sh.full[load % Z::kSlots], (load / Z::kSlots) & 1u, ok);
+      uint4* v = reinterpret_cast<uint4*>(ring + (load % Z::kSlots) * Z::kSlotBytes);
+      const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+      __nv_bfloat162 seen = zero;  // 0 as long as every factor is finite
+      for (int i = row; i < pages * 256; i += kTileRows)
+#pragma unroll
+        for (int x = 0; x < Z::kBoxes; ++x) {
+          uint4 q = v[x * (kBlockKeys * 8) + i];
+          const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) seen = __hfma2(h[e], zero, seen);
+        }
+      if (__any_sync(0xffffffffu, __low2float(seen) != 0.f || __high2float(seen) != 0.f)) {
+        clear_pieces<D>(v, row, pages * 256, &sh.cleared[n & 3u], n + 1);
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+      }
+    };
     for (uint32_t n = 0;; ++n) {
       const int b = n & 1u;
       wait(&sh.item_full[b], (n >> 1) & 1u, ok);
@@ -516,6 +578,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         ++n_s;
         ptx::tc_fence_after_sync();
         __syncwarp();
+        const int tok0 = (it.page_begin + j * kBlockPages) * 32;
+        const bool partly = tok0 + kBlockKeys > it.ctx0;  // some row does not see all of the block's keys
+        if (partly) clear_values(loads + 2 * j + 1, min(kBlockPages, n_pages - j * kBlockPages), n);
         float s[kBlockKeys];
         {
           uint32_t u[4][32];
@@ -525,8 +590,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int i = 0; i < kBlockKeys; ++i) s[i] = __uint_as_float(u[i >> 5][i & 31]);
         }
-        const int tok0 = (it.page_begin + j * kBlockPages) * 32;
-        if (tok0 + kBlockKeys > it.ctx0) {
+        if (partly) {
           const int seen = ctx - tok0;
 #pragma unroll
           for (int i = 0; i < kBlockKeys; ++i) s[i] = i < seen ? s[i] : kHidden;
@@ -536,7 +600,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int i = 0; i < kBlockKeys; ++i) mx[i & 3] = fmaxf(mx[i & 3], s[i]);
         const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * a.scale_log2;
         if (__any_sync(0xffffffffu, top > m + kGrow)) {
-          const float m_new = fmaxf(m, top), corr = ex2(m - m_new);
+          const float m_new = top > m + kGrow ? top : m, corr = ex2(m - m_new);  // (by the row's own scores, whatever its neighbours do)
           m = m_new;
           l *= corr;
           if (j != j0) {  // (the scores' arrival says that the product before them is done)
@@ -611,7 +675,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (writes) {
         const int c_begin = both ? g * (D / 2) : 0, c_end = both ? c_begin + D / 2 : D, tile = shared_tile ? 0 : g;
         const bool direct = it.slot0 < 0;
-        const float inv = direct ? (l > 0.f ? 1.0f / l : (l == 0.f ? 0.f : l)) : 1.f;
+        const float inv = direct ? (l > 0.f ? 1.0f / l : 0.f) : 1.f;
+        const bool drop = direct && a.may_split && !(l > 0.f);
+        const bool cleared = nb > 0 && l > 0.f && *reinterpret_cast<const volatile uint32_t*>(&sh.cleared[n & 3u]) == n + 1;
         const size_t qh = (size_t)it.head * a.group + head;
         __nv_bfloat16* dst = a.out + ((size_t)(it.first_row + tok) * a.n_q_heads + qh) * D;
         const size_t pidx = (size_t)(max(it.slot0, 0) + tok) * a.n_q_heads + qh;
@@ -638,6 +704,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int i = 0; i < 32; ++i) x[i] = 0.f;
           }
+          if (drop) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) x[i] = 0.f;
+          }
           if (on) {
             if (direct) {
 #pragma unroll
@@ -649,6 +719,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
           }
         }
+        if (cleared && on) add_cleared<D>(a, it, ctx, c_begin, c_end, direct ? dst : nullptr, po);
       }
       if (both) {  // neither group's sums are written again before the other has read them
         ptx::tc_fence_before_sync();
@@ -657,6 +728,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         ptx::tc_fence_after_sync();
         ++n_m;
       }
+      loads += 2 * nb;
     }
   }
   if (!ok) atomicExch(a.d.state + ST_ATTN_ERR, B200_ERR_DEVICE_FLAGGED);
@@ -686,10 +758,10 @@ __global__ void __launch_bounds__(256) prompt_combine_kernel(Args a, const int* 
 #pragma unroll
     for (int e = 0; e < V; ++e) acc[e] = fmaf(a.part_o[pidx * D + lane * V + e], w, acc[e]);
   }
-  const float inv = ll > 0.f ? 1.0f / ll : (ll == 0.f ? 0.f : ll);
+  const float inv = ll > 0.f ? 1.0f / ll : 0.f;
   uint32_t* dst = reinterpret_cast<uint32_t*>(a.out + ((size_t)row * a.n_q_heads + qh) * D + lane * V);
 #pragma unroll
-  for (int e = 0; e < V; e += 2) dst[e / 2] = pack2(acc[e] * inv, acc[e + 1] * inv);
+  for (int e = 0; e < V; e += 2) dst[e / 2] = ll > 0.f ? pack2(acc[e] * inv, acc[e + 1] * inv) : 0u;
 }
 
 template <int D>
@@ -740,6 +812,7 @@ b200_status b200_attn_prompt(b200_kv* kv, int32_t layer, const void* d_q, int32_
   a.items = reinterpret_cast<const int2*>(kv->d_prompt + kHdr);
   a.part_o = kv->d_part_o; a.part_ml = kv->d_part_ml; a.out = (__nv_bfloat16*)d_out;
   a.scale_log2 = 1.4426950408889634f / sqrtf((float)c.head_dim);
+  a.may_split = may_split;
   if (!reuse_plan) {
     prompt_plan_kernel<<<1, 1024, 0, s>>>(d_row_seq, d_row_ctx, total_rows, c.page_size, 2 * kTileRows / g, kTileRows / g, c.n_kv_heads, g_prompt_sms,
                                           may_split ? 1 : 0, kv->max_chunks, may_split ? 16 / g : 0, kv->d_chunk_start, kv->d_groups, kv->d_groups + stride,

@@ -309,3 +309,68 @@ def test_portions_at_the_edges_of_the_row_tiles(hq, hkv, d, scratch, rows):
         rel, cos = _close(got[r], want)
         assert rel <= REL_TOL and (cos >= COS_TOL or not want.any()), (r, s, c, rel, cos)
     kv.close()
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(32, 8, 128), (8, 1, 128), (4, 4, 64), (8, 4, 64)])
+@pytest.mark.parametrize("portions", [((2000, 300), (1500, 260), (700, 1)), ((1200, 640), (1000, 400), (90, 2))])   # below 1024 rows, and above
+def test_values_that_are_not_finite_reach_only_the_rows_that_see_them(hq, hkv, d, portions):
+    """Infinities and NaN in V of tokens inside prompt portions and behind the last token of a page: a row that does not see the token is the same
+    to the last bit as without them, a row that sees it is not finite in just those columns of just those heads.  Keys of a token that no row
+    sees change nothing; a row whose score is +inf has no sum (0 below 1024 rows, as from the row-by-row kernel); rows without context are 0."""
+    from dmlx_b200 import device as dev
+
+    rng = np.random.default_rng(hq + d + len(portions))
+    totals, extra = [c + n for c, n in portions], 7    # tokens behind the contexts, in the last page or the one behind it
+    held, n_rows = [t + extra for t in totals], sum(n for _, n in portions)
+    k = torch.tensor(rng.normal(0, 1, (sum(held), hkv, d)), device="cuda").bfloat16()
+    v = torch.tensor(rng.normal(0, 1, (sum(held), hkv, d)), device="cuda").bfloat16()
+    q = torch.tensor(rng.normal(0, 1, (n_rows + 2, hq, d)), device="cuda").bfloat16()
+    first = np.concatenate([[0], np.cumsum(held)])
+    row_seq = np.concatenate([np.full(n, s, np.int32) for s, (_, n) in enumerate(portions)] + [[0, 1]]).astype(np.int32)
+    row_ctx = np.concatenate([np.arange(c + 1, c + n + 1, dtype=np.int32) for c, n in portions] + [[0, 0]]).astype(np.int32)
+    rs, rc = torch.tensor(row_seq, device="cuda"), torch.tensor(row_ctx, device="cuda")
+
+    def run(kd, vd, prefill=True):
+        kv = dev.PagedKVCache(1, hkv, d, sum(-(-t // 32) for t in held) + 4, len(held), -(-max(held) // 32), hq, max_rows=sum(held), attn_scratch_chunks=40 * n_rows)
+        kv.reserve(dev.pack_desc_array([(s, t, 0, -1) for s, t in enumerate(held)]).cuda())
+        kv.append(0, kd, vd)
+        out = kv.attention(0, q, rs, rc, prefill=prefill).float()
+        assert kv.error_word() == 0
+        kv.close()
+        return out
+
+    nan, inf = float("nan"), float("inf")
+    # (request, token, head, column, value): in the middle and at the end of portions, twice in one column with either sign, behind the contexts
+    c0, n0 = portions[0]
+    c1, n1 = portions[1]
+    bad = [(0, c0 + n0 // 2, 0, 3, nan), (0, c0 + n0 // 2 + 1, hkv - 1, 5, inf), (0, c0 + n0 - 2, 0, 7, -inf), (0, c0 + n0 - 2, 0, d - 1, inf), (0, c0 + n0 - 1, 0, d - 1, -inf),
+           (1, c1 + n1 - 1, hkv - 1, 0, nan), (1, c1 + 130, 0, 9, inf), (2, portions[2][0] + portions[2][1] - 1, 0, 1, nan)]
+    bad += [(s, totals[s] + e, h, 2, val) for s in range(3) for e, val in ((0, nan), (extra - 1, inf)) for h in (0, hkv - 1)]
+    clean, dirty = v.clone(), v.clone()
+    for s, t, h, c, val in bad:
+        clean[first[s] + t, h, c], dirty[first[s] + t, h, c] = 0.0, val
+    want, got = run(k, clean), run(k, dirty)
+    assert torch.isfinite(want).all() and (want[n_rows:] == 0).all() and (got[n_rows:] == 0).all()
+    added = torch.zeros_like(want)
+    g = hq // hkv
+    for s, t, h, c, val in bad:
+        sees = (rs == s) & (rc > t)
+        added[sees, h * g:(h + 1) * g, c] += val
+    hit = ~torch.isfinite(added)
+    assert hit.any()
+    assert torch.equal(got[~hit], want[~hit])
+    assert torch.equal(torch.isnan(got[hit]), torch.isnan(added[hit])) and torch.equal(got[hit & (added == inf)], added[hit & (added == inf)])
+    # keys: behind the contexts nothing happens; inside, the rows behind the token whose score is +inf have no sum
+    kd = k.clone()
+    for s in range(3):
+        kd[first[s] + totals[s]:first[s] + held[s], :, 1] = inf
+    assert torch.equal(run(kd, clean), want)
+    at = c0 + n0 // 2
+    kd[first[0] + at, :, 3] = inf
+    got, hidden = run(kd, clean), (rs != 0) | (rc <= at)
+    assert torch.equal(got[hidden], want[hidden])
+    up = ~hidden[:, None] & (q[:, :, 3] > 0)
+    if n_rows < 1022:
+        assert (got[up] == 0).all() and (run(kd, clean, prefill=False)[up] == 0).all()
+    down = ~hidden[:, None] & (q[:, :, 3] < 0)
+    assert torch.isfinite(got[down]).all()
