@@ -6,8 +6,15 @@
 //   warp 9      issues the products: S = Q K^T into tensor memory, O += P V with P read from there, where it replaces S;
 //   warps 0-3   softmax of tile 0, a thread per row; warps 4-7 the same for tile 1.
 // While one tile's scores go through softmax the tensor cores work for the other, so the products (2 x 1024 cycles per block) and the
-// exponentials (32768 per block, 16 a cycle) overlap.  A row's scale moves only when a score exceeds it by 2^8; then the row's thread, whose
-// tensor-memory lane holds its sums, rescales them itself.
+// exponentials (32768 per block, 16 a cycle) overlap.
+//
+// P is bf16, and which of a row's weights are exact depends on its scale.  A block's weights are scaled by the row's largest score in that block
+// (or 2^-8 of its largest so far, if that is more), so that the block's largest weight is 1; the rows' threads, whose tensor-memory lanes hold the
+// sums, rescale them to it behind the weights.  The groups of paged_attn.cu scale by the largest of every 32 keys, anew every 256.  What the
+// coarser step costs is made good in the blocks that some row does not see whole, which are all the keys of a short context: there the MMAs also
+// get what the rounding of P leaves.  Error against 64 bits, as a multiple of theirs, scores of standard deviation 1 / 4: 200 tokens 0.85 / 0.97,
+// 512 over 256 cached 0.98 / 1.00, 683 over 700 0.98 / 1.00, 300 over 3000 1.00 / 1.00.  A scale that may lag its scores by 2^8, the published
+// way round most of the rescaling, is 1.02 to 1.2 there.
 //
 // A group that fits one tile (the decoding requests of the batch are groups of one token) would leave half of the CTA idle: there the two
 // softmax groups take the blocks in turn, with sums of their own, and put them together at the end.  Such items are bound by the stream of
@@ -16,14 +23,13 @@
 // A key that a row does not see has weight 0 there, and 0 times a value that is no finite number is no number: a group's rows share their blocks
 // of values, so one such value would reach up to 256 / G tokens ahead of its own.  The softmax threads therefore look through the values of the
 // blocks that some row does not see whole (one or two of an item, the rest of its last page among them), clear what is not finite, and a row
-// that does see it gets it back at the end.  The look costs 64 packed multiply-adds per thread and such block: 3 portions of 683 tokens over
-// 700..8000 160 us with and without.
+// that does see it gets it back at the end.  The look, 64 packed multiply-adds per thread and such block, did not show in the time.
 //
 // Two tiles of 128 rows: a CTA reads 64 KB of pages per block for 256 rows; one tile would read them twice.  Items go longest first, from a
 // counter, since contexts differ.  A batch too small to fill the chip has its key ranges split, f32 partial sums, and a combine pass.
 //
 // Measured on one B200, bf16, 32/8 heads of 128: 3 portions of 683 tokens over 700..8000 cached 985 us in groups of 16 rows per warp on mma.sync
-// (paged_attn.cu), 165 us here; a step of four 512-token portions and 57 decoding requests 733 and 169 us per layer.
+// (paged_attn.cu), 171 us here; a step of four 512-token portions and 57 decoding requests 733 and 169 us per layer.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -37,10 +43,7 @@ namespace {
 
 constexpr int kBlockKeys = 128, kBlockPages = 4, kTileRows = 128;
 constexpr int kThreads = 320;
-// log2 units a row's scale may lag behind its scores.  0 takes 193 us instead of 160 (3 portions of 683 tokens over 700..8000).  P is bf16 either
-// way, as in the groups of paged_attn.cu; the scale decides which weights are exact: a row's largest one is 1 where the scale follows every 32
-// keys.  Error of the results against 64 bits there 2.13e-3, here 2.19e-3 (0: 2.15e-3), of which 1.7e-3 are the rounding of the results.
-constexpr float kGrow = 8.f;
+constexpr float kBelow = 8.f;            // log2 units that the scale of a block may lie below a row's largest score so far
 constexpr float kHidden = -1e30f;       // score of a key that a row does not see
 constexpr float kNoScale = -1e28f;      // scale of a row that has seen no key: exp2 of any hidden score against it is 0
 constexpr uint32_t kPolls = 1u << 21;   // a wait inside a CTA is microseconds
@@ -301,6 +304,69 @@ __device__ __forceinline__ void add_cleared(const Args& a, const Item& it, int c
   }
 }
 
+// A tile's sums, rescaled by its rows' threads.
+template <int D>
+__device__ __forceinline__ void rescale(uint32_t t_o, float corr) {
+#pragma unroll
+  for (int c = 0; c < D; c += 32) {
+    uint32_t u[32];
+    ptx::tmem_ld32(t_o + c, u);
+    ptx::tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) u[i] = __float_as_uint(__uint_as_float(u[i]) * corr);
+    ptx::tmem_st32(t_o + c, u);
+  }
+}
+// A row's sums: their scale, the largest score so far (both log2), the sum of its weights.
+struct Row {
+  float m = kNoScale, most = kNoScale, l = 0.f;
+  // Takes the scale of a block whose largest score is `top`; returns the factor of what was summed before.
+  __device__ __forceinline__ float next(float top) {
+    most = fmaxf(most, top);
+    const float scale = fmaxf(top, most - kBelow), corr = ex2(m - scale);
+    m = scale;
+    return corr;
+  }
+};
+// One block of keys, some of which some rows of the tile do not see: the scores from tensor memory, P into place of the scores, and what its rounding leaves behind it, 64 columns further on.  The blocks that all rows see take the same steps in the kernel itself.
+template <int D>
+__device__ __noinline__ Row partly_seen_block(uint32_t t_s, uint32_t t_o, int seen, bool first, float scale_log2, Row r) {
+  float s[kBlockKeys];
+  {
+    uint32_t u[4][32];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) ptx::tmem_ld32(t_s + c * 32, u[c]);
+    ptx::tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < kBlockKeys; ++i) s[i] = i < seen ? fmaxf(__uint_as_float(u[i >> 5][i & 31]), kHidden) : kHidden;
+  }
+  float mx[4] = {kHidden, kHidden, kHidden, kHidden};
+#pragma unroll
+  for (int i = 0; i < kBlockKeys; ++i) mx[i & 3] = fmaxf(mx[i & 3], s[i]);
+  const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;
+  const float corr = r.next(top);
+  const float2 k2 = make_float2(scale_log2, scale_log2), m2 = make_float2(-r.m, -r.m);
+  float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t p[16], left[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float2 x = fma2(make_float2(s[c * 32 + 2 * i], s[c * 32 + 2 * i + 1]), k2, m2), e = make_float2(ex2(x.x), ex2(x.y));
+      sum[i & 1] = add2(sum[i & 1], e);
+      p[i] = pack2(e.x, e.y);
+      const float2 rest = add2(e, make_float2(-__uint_as_float(p[i] << 16), -__uint_as_float(p[i] & 0xFFFF0000u)));
+      left[i] = pack2(rest.x, rest.y);
+    }
+    ptx::tmem_st16(t_s + c * 16, p);
+    ptx::tmem_st16(t_s + 64 + c * 16, left);
+  }
+  const float2 both = add2(sum[0], sum[1]);
+  if (!first) rescale<D>(t_o, corr);
+  r.l = fmaf(r.l, corr, both.x + both.y);
+  return r;
+}
+
 // ---- the kernel ---------------------------------------------------------------------------------------------------
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -444,6 +510,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         wait(&sh.item_full[b], (n >> 1) & 1u, ok);
         if (!ok) break;
         const int kind = sh.items[b].kind, n_pages = sh.items[b].page_end - sh.items[b].page_begin;
+        const int first_partly = (sh.items[b].ctx0 - sh.items[b].page_begin * 32) / kBlockKeys;  // the first block that some row does not see whole
         ptx::mbar_arrive(&sh.item_free[b]);
         if (kind == 0) break;
         if (n_pages <= 0) continue;
@@ -474,6 +541,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int k = 0; k < steps; ++k)
               ptx::umma_bf16_tmem_a(tmem_o(t), tmem_s(t) + k * 8, v0 + k * (2048 >> 4), id_o, first && k == 0 ? 0u : 1u);
           }
+          if (j >= first_partly)
+            for (int k = 0; k < steps; ++k) ptx::umma_bf16_tmem_a(tmem_o(t), tmem_s(t) + 64 + k * 8, v0 + k * (2048 >> 4), id_o, 1u);
         };
         if (kind == 2) {
           arrived(0);
@@ -571,7 +640,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const bool on = tok < it.n_rows;
       const int ctx = on ? it.ctx0 + tok : 0;
       const int n_pages = it.page_end - it.page_begin, nb = n_pages > 0 ? (n_pages + kBlockPages - 1) / kBlockPages : 0;
-      float m = kNoScale, l = 0.f;
+      Row r;
       const int j0 = shared_tile ? g : 0, step = shared_tile ? 2 : 1;
       for (int j = j0; j < nb; j += step) {
         wait(&sh.s_full[g], n_s & 1u, ok);
@@ -580,74 +649,59 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         const int tok0 = (it.page_begin + j * kBlockPages) * 32;
         const bool partly = tok0 + kBlockKeys > it.ctx0;  // some row does not see all of the block's keys
-        if (partly) clear_values(loads + 2 * j + 1, min(kBlockPages, n_pages - j * kBlockPages), n);
-        float s[kBlockKeys];
-        {
-          uint32_t u[4][32];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) ptx::tmem_ld32(tmem_s(g) + lanes + c * 32, u[c]);
-          ptx::tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < kBlockKeys; ++i) s[i] = __uint_as_float(u[i >> 5][i & 31]);
-        }
         if (partly) {
-          const int seen = ctx - tok0;
+          clear_values(loads + 2 * j + 1, min(kBlockPages, n_pages - j * kBlockPages), n);
+          r = partly_seen_block<D>(tmem_s(g) + lanes, tmem_o(g) + lanes, ctx - tok0, j == j0, a.scale_log2, r);
+        } else {
+          float s[kBlockKeys];
+          {
+            uint32_t u[4][32];
 #pragma unroll
-          for (int i = 0; i < kBlockKeys; ++i) s[i] = i < seen ? s[i] : kHidden;
-        }
-        float mx[4] = {kHidden, kHidden, kHidden, kHidden};
+            for (int c = 0; c < 4; ++c) ptx::tmem_ld32(tmem_s(g) + lanes + c * 32, u[c]);
+            ptx::tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < kBlockKeys; ++i) mx[i & 3] = fmaxf(mx[i & 3], s[i]);
-        const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * a.scale_log2;
-        if (__any_sync(0xffffffffu, top > m + kGrow)) {
-          const float m_new = top > m + kGrow ? top : m, corr = ex2(m - m_new);  // (by the row's own scores, whatever its neighbours do)
-          m = m_new;
-          l *= corr;
-          if (j != j0) {  // (the scores' arrival says that the product before them is done)
-#pragma unroll 1
-            for (int c = 0; c < D; c += 32) {
-              uint32_t u[32];
-              ptx::tmem_ld32(tmem_o(g) + lanes + c, u);
-              ptx::tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) u[i] = __float_as_uint(__uint_as_float(u[i]) * corr);
-              ptx::tmem_st32(tmem_o(g) + lanes + c, u);
-            }
+            for (int i = 0; i < kBlockKeys; ++i) s[i] = __uint_as_float(u[i >> 5][i & 31]);
           }
-        }
-        const float2 k2 = make_float2(a.scale_log2, a.scale_log2), m2 = make_float2(-m, -m);
-        auto weigh = [&]() {  // P, and its sum
-          float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+          float mx[4] = {kHidden, kHidden, kHidden, kHidden};
 #pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            uint32_t p[32];
+          for (int i = 0; i < kBlockKeys; ++i) mx[i & 3] = fmaxf(mx[i & 3], s[i]);
+          const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * a.scale_log2;
+          const float corr = r.next(top);  // (by the row's own scores, whatever its neighbours do)
+          const float2 k2 = make_float2(a.scale_log2, a.scale_log2), m2 = make_float2(-r.m, -r.m);
+          auto weigh = [&]() {  // P, and its sum
+            float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const float2 x = fma2(make_float2(s[c * 64 + 2 * i], s[c * 64 + 2 * i + 1]), k2, m2);
-              const float2 e = make_float2(ex2(x.x), ex2(x.y));
-              sum[i & 1] = add2(sum[i & 1], e);
-              p[i] = pack2(e.x, e.y);
+            for (int c = 0; c < 2; ++c) {
+              uint32_t p[32];
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                const float2 x = fma2(make_float2(s[c * 64 + 2 * i], s[c * 64 + 2 * i + 1]), k2, m2);
+                const float2 e = make_float2(ex2(x.x), ex2(x.y));
+                sum[i & 1] = add2(sum[i & 1], e);
+                p[i] = pack2(e.x, e.y);
+              }
+              ptx::tmem_st32(tmem_s(g) + lanes + c * 32, p);
             }
-            ptx::tmem_st32(tmem_s(g) + lanes + c * 32, p);
-          }
-          const float2 both = add2(sum[0], sum[1]);
-          return both.x + both.y;
-        };
-        float total = weigh();
-        // A score that is no number weighs nothing, as a hidden one: it shows in the sum, and the block is done again without it.
-        if (__any_sync(0xffffffffu, total != total)) {
+            const float2 both = add2(sum[0], sum[1]);
+            return both.x + both.y;
+          };
+          float total = weigh();
+          // A score that is no number weighs nothing, as a hidden one: it shows in the sum, and the block is done again without it.
+          if (__any_sync(0xffffffffu, total != total)) {
 #pragma unroll
-          for (int i = 0; i < kBlockKeys; ++i) s[i] = fmaxf(s[i], kHidden);
-          total = weigh();
+            for (int i = 0; i < kBlockKeys; ++i) s[i] = fmaxf(s[i], kHidden);
+            total = weigh();
+          }
+          r.l = fmaf(r.l, corr, total);
+          if (j != j0) rescale<D>(tmem_o(g) + lanes, corr);  // (the scores' arrival says that the product before them is done)
         }
-        l += total;
         ptx::tmem_st_wait();
         ptx::tc_fence_before_sync();
         ptx::mbar_arrive(&sh.p_ready[g]);
       }
       // ---- the rows leave: all columns of this thread's row, or half of them from both groups' sums ----
       const bool both = shared_tile && nb > 1;
-      float w0 = 1.f, w1 = 0.f;
+      float w0 = 1.f, w1 = 0.f, m = r.m, l = r.l;
       if (nb > 0 && (j0 < nb || both)) wait(&sh.o_full[g], n_o[g] & 1u, ok);
       if (both) {
         wait(&sh.o_full[g ^ 1], n_o[g ^ 1] & 1u, ok);
