@@ -14,7 +14,8 @@
 // in 2048 finer ranges of keys, as often as it takes (keys are unique, so at most five times).
 //
 // A bin's weight is edge * (count - deficit): 1 - exp(-x), x the distance behind the bin's near edge, is below 2^-6 and is summed in units of
-// 2^-22 in an integer, so sums do not depend on the order of the additions.  Running sums over bins and candidates are f64.
+// 2^-22 in an integer, so sums do not depend on the order of the additions.  (Equal scores round alike, so the unit is the same for every
+// vocabulary: a CTA of more than 65535 words counts how often a bin's 32 bits are full.)  Running sums over bins and candidates are f64.
 //
 // Bound by the latency of its passes (loads, cluster barriers), not by bytes.  64 rows of 128256 bf16 words on one B200: greedy 20 us, top-k 50 40,
 // the whole distribution 54, a nucleus of 0.9 over all words 87 (thousands of words: 140).  One CTA per row that walked the sorted order 512
@@ -36,6 +37,8 @@ constexpr int kCap = 2048;     // keys sorted in shared memory
 constexpr int kMaxCluster = 8;
 constexpr int kFew = 512;      // candidates that the threads' maxima are asked for
 constexpr float kBinsPerUnit = 64.f;
+constexpr float kUnits = 4194304.f;  // of a deficit: 2^-22
+constexpr int kFullWords = 65535;    // whose deficits, below 2^16 units each, add up in 32 bits
 
 struct Bins {  // running sums over the bins, inclusive
   unsigned n[kBins];
@@ -44,6 +47,7 @@ struct Bins {  // running sums over the bins, inclusive
 
 struct Shared {
   unsigned hist_n[kBins], hist_d[kBins];  // this CTA's part: keys, deficits
+  unsigned hist_c[kBins];                 // multiples of 2^32 of the deficits, where the CTA has more than kFullWords
   Bins row;                               // (first CTA)
   union {
     Bins fine;                            // of the ranges inside one bin
@@ -132,8 +136,7 @@ struct Sampler {
   Row<T> r;
   int ranks, rank, tid, lane, warp;
   int warp_part, lo, hi;  // a warp's part of the vocabulary (a multiple of 8), and this warp's
-  int unit_shift;         // deficits are in units of 2^-(22 - unit_shift)
-  float units;
+  bool carries;           // deficits of one bin may exceed 32 bits
 
   __device__ Sampler(Shared& sh, const Row<T>& row) : cluster(cg::this_cluster()), s(sh), r(row) {
     ranks = cluster.num_blocks();
@@ -142,10 +145,7 @@ struct Sampler {
     warp_part = ((r.V + ranks * kWarps - 1) / (ranks * kWarps) + 7) / 8 * 8;
     lo = min((rank * kWarps + warp) * warp_part, r.V);
     hi = min(lo + warp_part, r.V);
-    // a CTA's deficits of one bin stay below 2^32: 2^16 units each at most
-    unit_shift = 0;
-    while (((long long)warp_part * kWarps >> unit_shift) > 65535) ++unit_shift;
-    units = exp2f((float)(22 - unit_shift));
+    carries = warp_part * kWarps > kFullWords;
   }
   __device__ Shared& of(int q) { return *cluster.map_shared_rank(&s, q); }
 
@@ -239,23 +239,28 @@ struct Sampler {
   }
 
   __device__ void clear_hist() {
-    for (int b = tid; b < kBins; b += kThreads) { s.hist_n[b] = 0; s.hist_d[b] = 0; }
+    for (int b = tid; b < kBins; b += kThreads) { s.hist_n[b] = 0; s.hist_d[b] = 0; s.hist_c[b] = 0; }
     __syncthreads();
   }
   __device__ void count(int bin, float x) {  // x: distance behind the near edge of the score's bin, below 1/64
     const float deficit = x * (1.f - x * (0.5f - x * (1.f / 6.f - x * (1.f / 24.f))));
     atomicAdd(&s.hist_n[bin], 1u);
-    atomicAdd(&s.hist_d[bin], (unsigned)(deficit * units + 0.5f));
+    const unsigned d = (unsigned)(deficit * kUnits + 0.5f);
+    if (!carries) {
+      atomicAdd(&s.hist_d[bin], d);
+    } else if (const unsigned old = atomicAdd(&s.hist_d[bin], d); old + d < old) {
+      atomicAdd(&s.hist_c[bin], 1u);
+    }
   }
   // First CTA: running sums of the whole row's bins.  `edge`: weight at the near edge of bin b; `counted` false: the bin weighs nothing.
   template <typename F>
   __device__ void sum_bins(Bins& out, F edge) {
     cluster.sync();
     if (rank == 0) {
-      unsigned n[kPerThread], d[kPerThread];
+      unsigned n[kPerThread];
       double m[kPerThread];
 #pragma unroll
-      for (int k = 0; k < kPerThread; ++k) n[k] = d[k] = 0;
+      for (int k = 0; k < kPerThread; ++k) n[k] = 0;
       double deficit[kPerThread] = {};
       for (int q = 0; q < ranks; ++q) {
         const Shared& o = of(q);
@@ -263,14 +268,14 @@ struct Sampler {
         for (int k = 0; k < kPerThread; ++k) {
           n[k] += o.hist_n[tid * kPerThread + k];
           deficit[k] += (double)o.hist_d[tid * kPerThread + k];
+          if (carries) deficit[k] += 4294967296.0 * (double)o.hist_c[tid * kPerThread + k];
         }
       }
-      const double unit = exp2((double)(unit_shift - 22));
       unsigned nt = 0;
       double mt = 0.0;
 #pragma unroll
       for (int k = 0; k < kPerThread; ++k) {
-        m[k] = edge(tid * kPerThread + k) * ((double)n[k] - deficit[k] * unit);
+        m[k] = edge(tid * kPerThread + k) * ((double)n[k] - deficit[k] * (1.0 / (double)kUnits));
         nt += n[k]; n[k] = nt;
         mt += m[k]; m[k] = mt;
       }

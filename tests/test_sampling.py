@@ -297,3 +297,52 @@ def test_rows_spread_over_clusters_and_bins_counted_again(dtype_name, vocab):
         true = z[tokens[i]] - z.max() - math.log(np.exp(z - z.max()).sum())
         assert abs(float(lp[i]) - true) < 2e-6 * max(1.0, abs(true)), (i, row, float(lp[i]), true)
     assert exact >= len(rows) - 3, (exact, len(rows))
+
+
+def _share_ahead(values, counts, first_of, temperature, k, value):
+    """Cumulative probability (64 bits) ahead of a token and with it in the stable descending order of a row that holds `counts[i]` words of
+    `values[i]` (descending): among the k best."""
+    z = (np.asarray(values, np.float32) / np.float32(temperature)).astype(np.float64)
+    n = np.minimum(np.cumsum(counts), k) - np.minimum(np.cumsum(counts) - counts, k)
+    cum = np.concatenate([[0.0], np.cumsum(np.exp(z - z[0]) * n)])
+    at = values.index(value)
+    ahead = cum[at] + np.exp(z[at] - z[0]) * first_of
+    return ahead / cum[-1], (ahead + np.exp(z[at] - z[0])) / cum[-1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype_name,vocab,rows", [("bfloat16", 1 << 24, 8), ("float32", (1 << 24) - 3, 8), ("bfloat16", 1 << 22, 152), ("bfloat16", 262144, 160), ("float32", 524281, 16)])
+def test_bins_of_vocabularies_beyond_65535_words_per_block(dtype_name, vocab, rows):
+    """Nuclei and lists of candidates of most of a large vocabulary whose words share a few scores, so that all words of a bin round alike: a bin's
+    deficits are in units of 2^-22 whatever the words of a thread block, so every weight is off by half a unit (2^-23) at most, and a draw's place in the
+    sum, which is a share of such weights in a share of such weights, by 2^-22 beside the words at either end.  (In units that grow with the words
+    of a block it was 6 x 2^-21 at 4 million words.)"""
+    import torch
+
+    from dmlx_b200 import device as dev
+
+    values = [2.0, 1.6875, 0.70703125, 0.1328125, -3.0]   # distances 0 and others inside their bins, exact in bf16
+    gen = torch.Generator("cuda").manual_seed(vocab + rows)
+    kind = torch.multinomial(torch.tensor([0.02, 0.38, 0.3, 0.2, 0.1], device="cuda"), 1 << 16, replacement=True, generator=gen)
+    kind = kind.repeat(-(-vocab // (1 << 16)))[:vocab]
+    x = torch.tensor(values, device="cuda")[kind].to(getattr(torch, dtype_name))
+    logits = x.expand(rows, vocab).contiguous()
+    counts = [int((kind == i).sum()) for i in range(len(values))]
+    rng = np.random.default_rng(vocab)
+    plans = [(1.0, 0, 0.9), (1.0, vocab - vocab // 8, 1.0), (0.75, 0, 0.625), (1.25, vocab // 2, 0.8125)]
+    params = [(*plans[i % 4], float(np.float32(rng.random()))) for i in range(rows)]
+    tokens, _ = dev.sample_rows(logits, params)
+    again, _ = dev.sample_rows(logits, params)
+    assert torch.equal(tokens, again)
+    kind = kind.cpu().numpy()
+    worst = 0.0
+    for (t, k, p, u), token in zip(params, tokens.cpu().numpy().astype(np.int64)):
+        k = k or vocab
+        place = int((kind[:token] == kind[token]).sum())
+        lo, hi = _share_ahead(values, counts, place, t, k, values[kind[token]])
+        # the nucleus ends with the word that takes its share beyond p; a word more or less there is inside the bound
+        mass = 1.0 if p >= 1.0 else float(np.float32(p))
+        drawn = u * mass
+        off = max(lo - drawn, drawn - hi, 0.0) - (hi - lo)
+        worst = max(worst, off)
+    assert worst <= 2.0 ** -22, worst * 2.0 ** 22
