@@ -743,11 +743,8 @@ __global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(const T* __res
 template <typename T>
 b200_status launch(const T* logits, int rows, int vocab, const b200_sample_params* params, const uint32_t* ctx, const int* ctx_off, float* scratch,
                    uint32_t* tokens, float* logprobs, cudaStream_t s) {
-  static bool configured = false;
-  if (!configured) {
-    B200_CUDA_TRY(cudaFuncSetAttribute(sample_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared)));
-    configured = true;
-  }
+  // (asked for at every launch: the attribute belongs to the device that the calling thread uses)
+  B200_CUDA_TRY(cudaFuncSetAttribute(sample_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared)));
   // CTAs per row: 8192 words each at least (16 a thread), and no more than two per SM altogether (what registers allow: more would wait)
   int ranks = 1;
   while (ranks < kMaxCluster && vocab > ranks * 8192 && (long long)rows * ranks * 2 <= 296) ranks *= 2;

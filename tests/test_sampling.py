@@ -346,3 +346,21 @@ def test_bins_of_vocabularies_beyond_65535_words_per_block(dtype_name, vocab, ro
         off = max(lo - drawn, drawn - hi, 0.0) - (hi - lo)
         worst = max(worst, off)
     assert worst <= 2.0 ** -22, worst * 2.0 ** 22
+
+
+@pytest.mark.gpu
+def test_rows_on_every_device_of_the_process():
+    """A process that uses several devices: the kernel's dynamic shared memory is asked for on each of them, whichever comes first."""
+    import torch
+
+    from dmlx_b200 import device as dev
+
+    if torch.cuda.device_count() < 2:
+        pytest.skip("one device")
+    x = torch.tensor(np.random.default_rng(1).normal(0.0, 2.0, (4, 20000)), dtype=torch.float32)
+    rows = [(0.0, 0, 1.0, 0.5), (1.0, 40, 0.9, 0.25), (1.0, 0, 0.8, 0.75), (0.7, 0, 1.0, 0.125)]
+    seen = []
+    for i in range(torch.cuda.device_count()):
+        with torch.cuda.device(i):
+            seen.append(dev.sample_rows(x.cuda(), rows)[0].cpu().tolist())
+    assert all(s == seen[0] for s in seen)
