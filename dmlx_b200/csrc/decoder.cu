@@ -1119,7 +1119,7 @@ b200_status b200_decoder::attention(b200_kv* kv, int run, int rows, void* stream
 }
 
 // Most rows of a work item of the experts' matmuls: the rows an expert gets on average, rounded up; above 64 the tile-pair kernel's 256, which
-// costs an item no more than the rows it has.
+// costs an item no more than the rows it has (measured at 253 rows on average, 175 -> 99 and 141 -> 64 us; 65 to 128 are not).
 int b200_decoder::moe_tile_rows(int T) const {
   if (f32()) return 64;
   int rows = 0;

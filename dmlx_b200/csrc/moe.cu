@@ -494,7 +494,6 @@ __global__ void combine_kernel(const __nv_bfloat16* __restrict__ y_sorted, const
     }
     return;
   }
-  if (blockIdx.y > 0) return;
   for (int i = threadIdx.x; i < hidden / 2; i += blockDim.x) {
     float2 acc = make_float2(0.f, 0.f);
     for (int j = 0; j < k; ++j) {

@@ -15,16 +15,21 @@
 // The kernels share the layout, the split-K scratch and the epilogue:
 //   * qmm_mma_kernel  (up to 16 rows): weight streaming.  Persistent CTAs, a producer warp keeping a
 //     ring of raw 4-bit blocks in flight, 8 consumer warps feeding mma.sync from registers.
+//   * qmm_mma8_kernel (affine int4, up to 8 rows): the same on int8 mma.sync, from the raw codes.
+//   * qmm_few_kernel  (dense bf16, up to 16 rows, and experts' items of up to 16 rows): a CTA's eight
+//     warps share K of 16 or 32 weight rows, memory to mma.sync registers; no ring, no K split.
+//   * qmm_tca_kernel  (17..256 rows, quantised weights): qmm_tc_kernel with the dequantised weights in
+//     tensor memory.  qmm_mx_kernel, qmm_mxp_kernel: block-scaled MMAs on MXFP4 codes.
 //   * qmm_tc_kernel   (17..128 rows per token tile, and the grouped MoE launches): "swap-AB" tcgen05
 //     GEMM.  The 128 weight rows are the MMA M dimension, the packed tokens (16..256 per tile) the N
 //     dimension, so small and large batches both map to dense tensor-core tiles.  Per 64-column
 //     chunk: warp 8 issues one bulk copy for the weight block and one 2-D TMA load (128B swizzle)
 //     for the activation tile; warps 0-7 dequantise the block to bf16 into a 128B-swizzled K-major
 //     tile (one row and one 32-column plane per thread); warp 9 issues 4 tcgen05.mma (M128 x N x
-//     K16) accumulating in tensor memory and commits to free the stage.  After the last chunk warps
-//     0-3 read the accumulator with tcgen05.ld.
-//   * qmm_tc2_kernel  (129..256 rows per token tile): the same with two weight tiles per CTA
-//     sharing one activation tile.
+//     K16) accumulating in tensor memory and commits to free the stage.  After the last chunk all
+//     eight dequantising warps read the accumulator with tcgen05.ld, 32 tokens in turn per half.
+//   * qmm_tc2_kernel  (129..256 rows per token tile, and dense experts' items of more than 128): the
+//     same with two weight tiles per CTA sharing one activation tile.
 //   * qmm_simt_kernel : CUDA-core GEMV kept as a forced path for tests.
 // Split-K partials go to an f32 scratch; a finish kernel sums them in split order (deterministic),
 // applies the epilogue (residual add, SwiGLU) and writes bf16.  No CTA waits on another.
@@ -2847,7 +2852,7 @@ static b200_status launch_mma_nt(QmmArgs& a, int rows, cudaStream_t s) {
 // Dense bf16 weights, up to 16 rows (of a batch, or of every work item).  Two groups of weight rows per CTA share the activations' loads where
 // that leaves at least two CTAs per SM.  Up to K = 2048 only: longer rows keep the tensor-memory kernels' deeper stream busy (K = 8192, 2048
 // outputs: 11.7 us there against 14.8 here; K = 5120: 7.9 against 10.6; K = 2048, 3072 outputs: 7.1 against 5.6).  The experts of one step are
-// many short grids at once and always come here.
+// many short grids at once and always come here (measured with K of 1024 and 2048: 56 -> 45 us and 37 -> 25; experts of longer K are not).
 static bool takes_few(const QmmArgs& a, int rows) {
   return rows <= kFewRows && ((uintptr_t)a.x & 15) == 0 && !a.y_f32 && a.groups == 0 && (a.items || a.kc <= 32);
 }

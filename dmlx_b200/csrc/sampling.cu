@@ -19,7 +19,8 @@
 //
 // Bound by the latency of its passes (loads, cluster barriers), not by bytes.  64 rows of 128256 bf16 words on one B200: greedy 20 us, top-k 50 40,
 // the whole distribution 54, a nucleus of 0.9 over all words 87 (thousands of words: 140).  One CTA per row that walked the sorted order 512
-// candidates at a time, one thread adding, took 800 to 1760 us for a mixture of these rows; this takes 87 to 100.
+// candidates at a time, one thread adding, took 1286 us for a mixture of these rows (800 to 1760 from call to call); this takes 102, upload of
+// the rows' parameters included.  More than 148 rows are a CTA each, whose times are not measured.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 

@@ -392,8 +392,10 @@ typedef struct b200_sample_params {
  * astype (src/generation.zig:124-141).  d_ctx_tokens / d_ctx_offsets[rows+1] (optional) give each row's
  * token history for the repetition penalty, applied once per occurrence; d_scratch [rows, vocab] f32
  * is required with them.  d_logprobs (optional) receives log softmax of the (penalised, unscaled)
- * logits at the sampled token (computeLogprob, :355-375).  Sums over the whole vocabulary are
- * parallel reductions; sums over the sorted top-k prefix run in the reference's order. */
+ * logits at the sampled token (computeLogprob, :355-375).  All sums are parallel reductions of f32
+ * weights (f64 running sums, the same for the same row whatever shares the batch): a cumulative
+ * probability is within 2^-20 of the exact one, where sums in the reference's order, f32 and one
+ * by one, drift further over thousands of words. */
 b200_status b200_sample_rows(const void* d_logits, int32_t logits_f32, int32_t rows, int32_t vocab,
                              const b200_sample_params* d_params, const uint32_t* d_ctx_tokens,
                              const int32_t* d_ctx_offsets, float* d_scratch, uint32_t* d_tokens,
