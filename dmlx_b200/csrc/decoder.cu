@@ -1119,7 +1119,9 @@ b200_status b200_decoder::attention(b200_kv* kv, int run, int rows, void* stream
 }
 
 // Most rows of a work item of the experts' matmuls: the rows an expert gets on average, rounded up; above 64 the tile-pair kernel's 256, which
-// costs an item no more than the rows it has (measured at 253 rows on average, 175 -> 99 and 141 -> 64 us; 65 to 128 are not).
+// costs an item no more than the rows it has (items of up to 128 against 256, us:
+// 16 experts of 4096 x 4096, 65 rows each 120 / 103, 128 rows 134 / 115, uneven 153 / 120; of 2048 x 2048 36 / 34, 40 / 37, 49 / 44; 64 of
+// 2048 x 1024 71 / 77, 82 / 85, 90 / 82; at 253 rows 188 / 149, 54 / 46, 125 / 112).
 int b200_decoder::moe_tile_rows(int T) const {
   if (f32()) return 64;
   int rows = 0;

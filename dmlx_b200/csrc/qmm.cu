@@ -2852,7 +2852,9 @@ static b200_status launch_mma_nt(QmmArgs& a, int rows, cudaStream_t s) {
 // Dense bf16 weights, up to 16 rows (of a batch, or of every work item).  Two groups of weight rows per CTA share the activations' loads where
 // that leaves at least two CTAs per SM.  Up to K = 2048 only: longer rows keep the tensor-memory kernels' deeper stream busy (K = 8192, 2048
 // outputs: 11.7 us there against 14.8 here; K = 5120: 7.9 against 10.6; K = 2048, 3072 outputs: 7.1 against 5.6).  The experts of one step are
-// many short grids at once and always come here (measured with K of 1024 and 2048: 56 -> 45 us and 37 -> 25; experts of longer K are not).
+// many short grids at once and always come here (16 experts of
+// 1024 outputs, 8 rows, against qmm_tc_kernel: K = 1024 17.0 -> 13.3 us, 2048 24.1 -> 20.0, 4096 35.3 -> 34.3; 4096 outputs, K = 7168 192 -> 145;
+// only 8 experts of 2048 outputs and K = 8192 lose, 57.7 -> 61.3).
 static bool takes_few(const QmmArgs& a, int rows) {
   return rows <= kFewRows && ((uintptr_t)a.x & 15) == 0 && !a.y_f32 && a.groups == 0 && (a.items || a.kc <= 32);
 }
