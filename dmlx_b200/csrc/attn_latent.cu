@@ -18,6 +18,7 @@
 #include "attn_latent.cuh"
 #include "attn_plan.cuh"
 #include "common.h"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "tma.cuh"
 
@@ -26,6 +27,7 @@ namespace {
 // Angles in f64, brought into one turn before they become f32: positions far out keep their accuracy.
 __global__ void __launch_bounds__(256) rotation_table_kernel(const double* __restrict__ freq, int half, float size, const int* __restrict__ pos, int rows,
                                                              float2* __restrict__ out) {
+  after_previous();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= (long long)rows * half) return;
   const int row = (int)(i / half), p = (int)(i - (long long)row * half);
@@ -46,6 +48,7 @@ struct PrepArgs {
 // One warp per (row, query head); blocks of their own for the row's latent and its query latent.
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) latent_prep_kernel(PrepArgs a) {
+  after_previous();
   const LatentPrep& p = a.p;
   __shared__ float part[32];
   const int row = blockIdx.x, lane = threadIdx.x & 31, head_blocks = (p.heads + 7) / 8, u = blockIdx.y * 8 + (threadIdx.x >> 5);
@@ -121,7 +124,7 @@ __global__ void __launch_bounds__(256) latent_prep_kernel(PrepArgs a) {
 b200_status b200_rotation_table(const double* d_freq, int dims, double size, const int32_t* d_pos, int rows, float2* d_out, void* stream) {
   if (rows <= 0 || dims < 2) return B200_OK;
   const long long n = (long long)rows * (dims / 2);
-  rotation_table_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(d_freq, dims / 2, (float)size, d_pos, rows, d_out);
+  launch_after(rotation_table_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, d_freq, dims / 2, (float)size, d_pos, rows, d_out);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -138,7 +141,7 @@ b200_status b200_latent_prep(b200_kv* kv, const LatentPrep& p, const int32_t* d_
   const bool v4 = p.dim % 4 == 0 && p.rot % 4 == 0 && p.rank % 4 == 0 && p.plain_stride % 4 == 0 && p.q_rank % 4 == 0 && p.q_latent_stride % 4 == 0 && (p.src.ws || p.src.y_stride % 4 == 0);
   auto* kernel = kv->dev.elem_bytes == 4 ? (v4 ? latent_prep_kernel<float, 4> : latent_prep_kernel<float, 1>)
                                          : (v4 ? latent_prep_kernel<__nv_bfloat16, 4> : latent_prep_kernel<__nv_bfloat16, 1>);
-  kernel<<<dim3(rows, (p.heads + 7) / 8 + (p.keys ? 1 : 0) + (p.q_rank > 0 ? 1 : 0)), 256, 0, (cudaStream_t)stream>>>(a);
+  launch_after(kernel, dim3(rows, (p.heads + 7) / 8 + (p.keys ? 1 : 0) + (p.q_rank > 0 ? 1 : 0)), 256, 0, (cudaStream_t)stream, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -228,6 +231,7 @@ struct LatentShared {
 template <int NR>
 __global__ void __launch_bounds__(kLatentThreads, 1)
     latent_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap qmap, LatentArgs la) {
+  after_previous();
   const WinArgs& a = la.w;
   extern __shared__ unsigned char latent_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(latent_dyn) + 1023) & ~(uintptr_t)1023);
@@ -652,7 +656,7 @@ b200_status launch(const b200_kv* kv, LatentArgs& la, int layer, cudaStream_t s)
     B200_CUDA_TRY(cudaFuncSetAttribute(latent_attn_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     configured = true;
   }
-  latent_attn_kernel<NR><<<g_sms, kLatentThreads, smem_of<NR>(la.n_kb, stages), s>>>(kv->lay_kmap[layer], qmap, la);
+  launch_after(latent_attn_kernel<NR>, g_sms, kLatentThreads, smem_of<NR>(la.n_kb, stages), s, kv->lay_kmap[layer], qmap, la);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }

@@ -39,6 +39,7 @@
 
 #include "attn_prompt.cuh"
 #include "common.h"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "tma.cuh"
 
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(1024) prompt_plan_kernel(const int* __restrict
                                                            int old_tokens, int* __restrict__ chunk_start, int* __restrict__ group_first,
                                                            int* __restrict__ part_base, int* __restrict__ row_group, int2* __restrict__ items,
                                                            int* __restrict__ hdr, int* __restrict__ err) {
+  after_previous();
   __shared__ int warp_buf[32], hist[256], carry[4];
   __shared__ int s_max[kLengths], s_items[kLengths], s_total[kLengths], s_slots[kLengths], s_old, s_pick, s_longest;
   __shared__ int2 s_group[1024];  // {rows, blocks} of the first groups
@@ -374,6 +376,7 @@ __device__ __noinline__ Row partly_seen_block(uint32_t t_s, uint32_t t_o, int se
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
     prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ Args a) {
+  after_previous();
   using Z = Shape<D>;
   extern __shared__ __align__(1024) unsigned char smem[];  // (there is no room for a base that has to be rounded up)
   unsigned char* qbuf = smem;                        // [tile][box][128 rows][128 B]
@@ -798,6 +801,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // A warp per (row, query head): merges the chunks of rows whose key range was split.
 template <int D>
 __global__ void __launch_bounds__(256) prompt_combine_kernel(Args a, const int* __restrict__ row_group) {
+  after_previous();
   const int u = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (u >= a.total_rows * a.n_q_heads || a.hdr[4] == 0 || a.d.state[ST_ATTN_ERR] != 0) return;
   const int row = u / a.n_q_heads, qh = u - row * a.n_q_heads;
@@ -830,10 +834,10 @@ b200_status launch(b200_kv* kv, const CUtensorMap& qmap, const Args& a, const in
     B200_CUDA_TRY(cudaFuncSetAttribute(prompt_attn_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = true;
   }
-  prompt_attn_kernel<D><<<sms, kThreads, smem, s>>>(kv->kmap, kv->vmap, qmap, a);
+  launch_after(prompt_attn_kernel<D>, sms, kThreads, smem, s, kv->kmap, kv->vmap, qmap, a);
   B200_LAUNCH_CHECK();
   if (!may_split) return B200_OK;
-  prompt_combine_kernel<D><<<(a.total_rows * a.n_q_heads + 7) / 8, 256, 0, s>>>(a, row_group);
+  launch_after(prompt_combine_kernel<D>, (a.total_rows * a.n_q_heads + 7) / 8, 256, 0, s, a, row_group);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -871,7 +875,7 @@ b200_status b200_attn_prompt(b200_kv* kv, int32_t layer, const void* d_q, int32_
   a.scale_log2 = 1.4426950408889634f / sqrtf((float)c.head_dim);
   a.may_split = may_split;
   if (!reuse_plan) {
-    prompt_plan_kernel<<<1, 1024, 0, s>>>(d_row_seq, d_row_ctx, total_rows, c.page_size, 2 * kTileRows / g, kTileRows / g, c.n_kv_heads, g_prompt_sms,
+    launch_after(prompt_plan_kernel, 1, 1024, 0, s, d_row_seq, d_row_ctx, total_rows, c.page_size, 2 * kTileRows / g, kTileRows / g, c.n_kv_heads, g_prompt_sms,
                                           may_split ? 1 : 0, kv->max_chunks, may_split ? 16 / g : 0, kv->d_chunk_start, kv->d_groups, kv->d_groups + stride,
                                           kv->d_groups + 2 * stride, reinterpret_cast<int2*>(kv->d_prompt + kHdr), kv->d_prompt, kv->dev.state + ST_ATTN_ERR);
     B200_LAUNCH_CHECK();

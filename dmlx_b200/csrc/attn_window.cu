@@ -24,6 +24,7 @@
 #include "attn_plan.cuh"
 #include "common.h"
 #include "kv_pool.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "tma.cuh"
 
@@ -85,6 +86,7 @@ __global__ void __launch_bounds__(1024) window_plan_kernel(const int* __restrict
                                                            int n_workers, int forced_ppc, int max_slots, float item_cost, float slot_cost, int* __restrict__ group_first,
                                                            int* __restrict__ chunk_start, int* __restrict__ part_base,
                                                            int* __restrict__ row_group, int* __restrict__ page_base, int* __restrict__ hdr) {
+  after_previous();
   __shared__ int warp_buf[32];
   __shared__ int carry_start, carry_groups, carry_chunks, carry_slots, carry_pages, s_share;
   const int tid = threadIdx.x;
@@ -261,6 +263,7 @@ constexpr int most_warps(int kb, int vb) { return kb + vb == 2 ? 12 : (kb + vb =
 template <int KB, int VB, bool TABLE>
 __global__ void __launch_bounds__(most_warps(KB, VB) * 32, 1)
     window_attn_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, WinArgs a) {
+  after_previous();
   constexpr int KS = KB * 4;  // 16-column steps of Q K^T
   constexpr int NO = VB * 8;  // 8-column tiles of the output
   const int n_kb = (a.L.kd + 63) / 64, n_vb = (a.L.vd + 63) / 64, n_ks = a.L.kd / 16, n_vs = a.L.vd / 16;
@@ -509,6 +512,7 @@ __global__ void __launch_bounds__(most_warps(KB, VB) * 32, 1)
 
 // One warp per (row, query head) of the groups that were cut into several chunks.
 __global__ void __launch_bounds__(256) window_combine_kernel(WinArgs a) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (w >= (long long)a.total_rows * a.n_q_heads || a.d.state[ST_ATTN_ERR] != 0) return;
@@ -574,6 +578,7 @@ struct SimtArgs {
 // weighted sum; query and output row in shared memory.
 template <typename T>
 __global__ void __launch_bounds__(128) attn_simt_kernel(SimtArgs a) {
+  after_previous();
   extern __shared__ float sh[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kd = a.L.key_dim, vd = a.L.value_dim;
   float* q = sh + warp * (kd + vd);
@@ -684,7 +689,7 @@ b200_status launch_mma(const b200_kv* kv, WinArgs& a, int layer, cudaStream_t s)
     B200_CUDA_TRY((cudaFuncSetAttribute(window_attn_mma_kernel<KB, VB, TABLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024)));
     configured = true;
   }
-  window_attn_mma_kernel<KB, VB, TABLE><<<g_sms, sh.warps * 32, smem, s>>>(kv->lay_kmap[layer], kv->lay_vmap[layer], a);
+  launch_after(window_attn_mma_kernel<KB, VB, TABLE>, g_sms, sh.warps * 32, smem, s, kv->lay_kmap[layer], kv->lay_vmap[layer], a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -720,7 +725,7 @@ b200_status b200_attn_make_plan(b200_kv* kv, int32_t window, int32_t qt, int32_t
   }
   const int forced = b200_attn_pages_per_chunk <= 0 ? 0 : std::min(std::max(b200_attn_pages_per_chunk, 1), 1 << 20);
   auto* kernel = fine ? window_plan_kernel<FineLengths> : window_plan_kernel<CoarseLengths>;
-  kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(d_row_seq, d_row_ctx, total_rows, kv->cfg.page_size, window, qt,
+  launch_after(kernel, 1, 1024, 0, (cudaStream_t)stream, d_row_seq, d_row_ctx, total_rows, kv->cfg.page_size, window, qt,
                                                           items_per_chunk, n_workers, forced, kv->max_chunks, item_cost, slot_cost,
                                                           p->buf, p->buf + R, p->buf + 2 * R, p->buf + 3 * R, p->buf + 4 * R, p->buf + 5 * R);
   B200_LAUNCH_CHECK();
@@ -740,7 +745,7 @@ bool b200_attn_use_plan(b200_kv* kv, int32_t window, int32_t q_tokens, bool fine
 b200_status b200_attn_combine(b200_kv* kv, const WinArgs& a, void* stream) {
   const long long rows = (long long)a.total_rows * a.n_q_heads;
   // few rows (decode): their columns over several blocks
-  window_combine_kernel<<<dim3((unsigned)((rows + 7) / 8), rows <= 8192 ? (a.L.vd + 127) / 128 : 1), 256, 0, (cudaStream_t)stream>>>(a);
+  launch_after(window_combine_kernel, dim3((unsigned)((rows + 7) / 8), rows <= 8192 ? (a.L.vd + 127) / 128 : 1), 256, 0, (cudaStream_t)stream, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -778,7 +783,7 @@ b200_status b200_window_attn_run(b200_kv* kv, const WindowAttnCall& c, const int
     const unsigned grid = (unsigned)(((long long)total_rows * c.n_q_heads + 3) / 4);
     auto* kernel = kv->dev.elem_bytes == 4 ? attn_simt_kernel<float> : attn_simt_kernel<__nv_bfloat16>;
     if (smem > 48 * 1024) B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, 128, smem, s>>>(a);
+    launch_after(kernel, grid, 128, smem, s, a);
     B200_LAUNCH_CHECK();
     return B200_OK;
   }

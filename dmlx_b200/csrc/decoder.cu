@@ -45,6 +45,7 @@
 #include "delta.cuh"
 #include "gla.cuh"
 #include "kv_pool.cuh"
+#include "launch.cuh"
 #include "lru.cuh"
 #include "model_step.cuh"
 #include "moe.cuh"
@@ -119,6 +120,7 @@ __device__ __forceinline__ float as_stored(float x) {
 constexpr int kStateAhead = 3;  // entries of its state that are asked for before the row's sums are known
 template <typename T, int VEC, int NQ, bool FEW>
 __global__ void __launch_bounds__(512, FEW ? 1 : 2) decoder_rows_kernel(RowArgs a) {
+  after_previous();
   extern __shared__ float row_sh[];
   __shared__ float part[32];
   __shared__ float4 part4[32];
@@ -349,6 +351,7 @@ struct InputConvArgs {
 
 template <typename T, int VEC, int TAPS, int R>
 __global__ void __launch_bounds__(256) input_conv_kernel(InputConvArgs a, int rows) {
+  after_previous();
   const int begin = blockIdx.x * R, end = min(begin + R, rows), ch = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
   if (ch >= a.hidden || a.pool_state[ST_ERR] != 0) return;
   auto value = [&](int row, int col) { return load_vec<VEC>((const T*)a.h + (size_t)row * a.stride + col); };
@@ -380,7 +383,7 @@ b200_status launch_input_conv(const InputConvArgs& a, int rows, bool f32, cudaSt
   const bool v4 = a.hidden % 4 == 0 && a.stride % 4 == 0 && a.conv.slot_elems % 4 == 0, many = rows >= 256 && v4 && !f32;
   const int groups = v4 ? a.hidden / 4 : a.hidden, threads = std::min(256, (groups + 31) / 32 * 32);
   auto run = [&](auto* kernel, int per) -> b200_status {
-    kernel<<<dim3((rows + per - 1) / per, (groups + threads - 1) / threads), threads, 0, s>>>(a, rows);
+    launch_after(kernel, dim3((rows + per - 1) / per, (groups + threads - 1) / threads), threads, 0, s, a, rows);
     B200_LAUNCH_CHECK();
     return B200_OK;
   };
@@ -396,6 +399,7 @@ b200_status launch_input_conv(const InputConvArgs& a, int rows, bool f32, cudaSt
 template <typename T>
 __global__ void __launch_bounds__(256) decoder_final_kernel(const float* __restrict__ x, const int* __restrict__ idx, const float* __restrict__ w,
                                                             T* __restrict__ out, int hidden, int out_stride, float eps) {
+  after_previous();
   __shared__ float part[32];
   const float* xr = x + (size_t)max(idx[blockIdx.x], 0) * hidden;
   float ss = 0.f;
@@ -405,6 +409,7 @@ __global__ void __launch_bounds__(256) decoder_final_kernel(const float* __restr
 }
 
 __global__ void __launch_bounds__(256) decoder_logits_kernel(MatSrc src, float* __restrict__ logits, int vocab) {
+  after_previous();
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c < vocab) logits[(size_t)blockIdx.y * vocab + c] = mat_value<float, 1>(src, blockIdx.y, c).v[0];
 }
@@ -448,6 +453,7 @@ __device__ __forceinline__ T* page_row(const QkvArgs& a, int row, int head, bool
 // One warp per (row, head); q heads, then k heads, then v heads.  Grid y covers the heads, eight at a time.
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) decoder_qkv_kernel(QkvArgs a) {
+  after_previous();
   constexpr int KEEP = VEC == 4 ? 2 : 4;  // passes of 32 x VEC columns kept in registers; wider heads are read again
   const int row = blockIdx.x, lane = threadIdx.x & 31, H = a.L.heads;
   const int u = blockIdx.y * 8 + (threadIdx.x >> 5);
@@ -512,6 +518,7 @@ __global__ void __launch_bounds__(256) decoder_qkv_kernel(QkvArgs a) {
 // that read the convolution's state (short_conv.cuh).
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) decoder_qkv_conv_kernel(QkvArgs a) {
+  after_previous();
   extern __shared__ float row_sh[];
   const int first = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, H = a.L.heads, u = blockIdx.y * 8 + warp;
   if (u >= a.hq + 2 * H || a.d.state[ST_ERR] != 0) return;
@@ -565,6 +572,7 @@ __global__ void __launch_bounds__(256) decoder_qkv_conv_kernel(QkvArgs a) {
 // rotated, and rows of one request that lie next to each other share the loads of their inputs and of the weights.
 template <typename T, int KEEP, int R>
 __global__ void __launch_bounds__(256, KEEP == 1 ? 3 : 2) decoder_qkv_conv4_kernel(QkvArgs a, int rows) {
+  after_previous();
   extern __shared__ float row_sh[];  // [warp][rot]
   const int begin = blockIdx.x * R, end = min(begin + R, rows);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, H = a.L.heads, u = blockIdx.y * 8 + warp;
@@ -701,6 +709,7 @@ __global__ void __launch_bounds__(256, KEEP == 1 ? 3 : 2) decoder_qkv_conv4_kern
 // also scaled by a temperature that grows with the position; without keys there are queries only.
 template <typename T, int VEC, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) decoder_qkv_row_kernel(QkvArgs a) {
+  after_previous();
   extern __shared__ __align__(16) float row_sh[];
   __shared__ float part[32];
   const int row = blockIdx.x, H = a.keys ? a.L.heads : 0, dim = a.L.key_dim, nq = a.hq * dim, nqk = nq + H * dim, all = nqk + H * a.L.value_dim;
@@ -770,7 +779,7 @@ b200_status launch_qkv(const QkvArgs& a, int rows, cudaStream_t s) {
     if (few) kernel = a.d.elem_bytes == 4 ? (vec ? decoder_qkv_row_kernel<float, 4, 1024> : decoder_qkv_row_kernel<float, 1, 1024>)
                                           : (vec ? decoder_qkv_row_kernel<__nv_bfloat16, 4, 1024> : decoder_qkv_row_kernel<__nv_bfloat16, 1, 1024>);
     if (smem > 48 * 1024) B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<rows, few ? 1024 : 256, smem, s>>>(a);
+    launch_after(kernel, rows, few ? 1024 : 256, smem, s, a);
     B200_LAUNCH_CHECK();
     return B200_OK;
   }
@@ -780,7 +789,7 @@ b200_status launch_qkv(const QkvArgs& a, int rows, cudaStream_t s) {
     if (vec && a.conv.taps == 4 && !a.conv.bias && a.L.key_dim <= 256 && a.L.value_dim <= 256) {
       const bool narrow = a.L.key_dim <= 128 && a.L.value_dim <= 128, many = rows >= 1024;
       auto run = [&](auto* kernel, int per) {
-        kernel<<<dim3((rows + per - 1) / per, (a.hq + 2 * a.L.heads + 7) / 8), 256, sizeof(float) * 8 * std::max(a.rot, 1), s>>>(a, rows);
+        launch_after(kernel, dim3((rows + per - 1) / per, (a.hq + 2 * a.L.heads + 7) / 8), 256, sizeof(float) * 8 * std::max(a.rot, 1), s, a, rows);
       };
       auto pick = [&](auto tag) {
         using T = decltype(tag);
@@ -797,14 +806,14 @@ b200_status launch_qkv(const QkvArgs& a, int rows, cudaStream_t s) {
     auto* kernel = a.d.elem_bytes == 4 ? (vec ? decoder_qkv_conv_kernel<float, 4> : decoder_qkv_conv_kernel<float, 1>)
                                        : (vec ? decoder_qkv_conv_kernel<__nv_bfloat16, 4> : decoder_qkv_conv_kernel<__nv_bfloat16, 1>);
     if (smem > 48 * 1024) B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<dim3(rows, (a.hq + 2 * a.L.heads + 7) / 8), 256, smem, s>>>(a);
+    launch_after(kernel, dim3(rows, (a.hq + 2 * a.L.heads + 7) / 8), 256, smem, s, a);
     B200_LAUNCH_CHECK();
     return B200_OK;
   }
   const bool v4 = a.L.key_dim % 4 == 0 && a.L.value_dim % 4 == 0 && a.src.y_stride % 4 == 0;
   auto* kernel = a.d.elem_bytes == 4 ? (v4 ? decoder_qkv_kernel<float, 4> : decoder_qkv_kernel<float, 1>)
                                      : (v4 ? decoder_qkv_kernel<__nv_bfloat16, 4> : decoder_qkv_kernel<__nv_bfloat16, 1>);
-  kernel<<<dim3(rows, (a.hq + 2 * a.L.heads + 7) / 8), 256, 0, s>>>(a);
+  launch_after(kernel, dim3(rows, (a.hq + 2 * a.L.heads + 7) / 8), 256, 0, s, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -1090,7 +1099,7 @@ b200_status b200_decoder::rows_step(RowArgs a, int rows, int next, cudaStream_t 
   auto* kernel = f32() ? (few ? rows_kernel<float, true>(vec, nq) : rows_kernel<float, false>(vec, nq))
                        : (few ? rows_kernel<__nv_bfloat16, true>(vec, nq) : rows_kernel<__nv_bfloat16, false>(vec, nq));
   if (smem > 47 * 1024) B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<rows, threads, smem, s>>>(a);
+  launch_after(kernel, rows, threads, smem, s, a);
   B200_LAUNCH_CHECK();
   return ic.hc ? launch_input_conv(ic, rows, f32(), s) : B200_OK;
 }
@@ -1378,8 +1387,8 @@ b200_status b200_decoder::run_layers(b200_kv* kv, int n_req, int T, int n_logits
       B200_CUDA_TRY(cudaMemcpyAsync(rec + r * (size_t)max_rows * cfg.hidden, x, sizeof(float) * (size_t)T * cfg.hidden, cudaMemcpyDeviceToDevice, cs));
   }
   auto head_rows = [&]() -> b200_status {
-    if (f32()) decoder_final_kernel<float><<<n_logits, 256, 0, cs>>>(x, d_logit_row, final_norm, (float*)last, cfg.hidden, hp, cfg.norm_eps);
-    else decoder_final_kernel<__nv_bfloat16><<<n_logits, 256, 0, cs>>>(x, d_logit_row, final_norm, (__nv_bfloat16*)last, cfg.hidden, hp, cfg.norm_eps);
+    if (f32()) launch_after(decoder_final_kernel<float>, n_logits, 256, 0, cs, x, d_logit_row, final_norm, (float*)last, cfg.hidden, hp, cfg.norm_eps);
+    else launch_after(decoder_final_kernel<__nv_bfloat16>, n_logits, 256, 0, cs, x, d_logit_row, final_norm, (__nv_bfloat16*)last, cfg.hidden, hp, cfg.norm_eps);
     B200_LAUNCH_CHECK();
     return B200_OK;
   };
@@ -1390,7 +1399,7 @@ b200_status b200_decoder::run_layers(b200_kv* kv, int n_req, int T, int n_logits
   }
   MODEL_STEP_CAT(1, matmul(head, last, n_logits, 2, &src, stream));
   auto finish = [&]() -> b200_status {
-    decoder_logits_kernel<<<dim3((cfg.vocab + 255) / 256, n_logits), 256, 0, cs>>>(src, (float*)logits, cfg.vocab);
+    launch_after(decoder_logits_kernel, dim3((cfg.vocab + 255) / 256, n_logits), 256, 0, cs, src, (float*)logits, cfg.vocab);
     B200_LAUNCH_CHECK();
     return B200_OK;
   };

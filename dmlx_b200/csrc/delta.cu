@@ -22,6 +22,7 @@
 #include "common.h"
 #include "delta.cuh"
 #include "gla_chunks.cuh"
+#include "launch.cuh"
 
 namespace {
 
@@ -43,6 +44,7 @@ struct PrepArgs {
 // One warp per (R rows, unit): a head of q or k, 32 * VEC columns of v, or the gates of a row.
 template <typename T, int VEC, int TAPS, int R>
 __global__ void __launch_bounds__(256) delta_prep_kernel(PrepArgs a, int n_rows) {
+  after_previous();
   const DeltaCall& c = a.c;
   const int begin = blockIdx.x * R, end = min(begin + R, n_rows), lane = threadIdx.x & 31, unit = blockIdx.y * 8 + (threadIdx.x >> 5);
   const int heads_qk = 2 * c.kv_heads, KD = c.kv_heads * c.dk, VD = c.heads * c.dv;
@@ -135,6 +137,7 @@ struct Delta {
 // stays in memory.
 template <typename T, int VEC, int KEEP>
 __global__ void __launch_bounds__(256, KEEP == 32 ? 1 : 2) delta_step_kernel(Delta a) {
+  after_previous();
   extern __shared__ float sh[];
   __shared__ float part[32];
   const int req = blockIdx.x, head = blockIdx.y, dk = a.g.dk, dv = a.g.dv;
@@ -273,6 +276,7 @@ __device__ __forceinline__ float dot16(const float* x, int dx, const float* y, i
 }
 
 __global__ void __launch_bounds__(256, 3) delta_chunk_kernel(Delta a) {
+  after_previous();
   extern __shared__ __align__(16) float sh[];
   __shared__ float s_L[kC], s_beta[kC];
   const int chunk = blockIdx.x, head = blockIdx.y;
@@ -527,7 +531,7 @@ b200_status b200_delta_prep(b200_kv* kv, const GlaScratch& g, const DeltaCall& c
   auto* kernel = f32 ? (v4 ? delta_prep_kernel<float, 4, 0, 1> : delta_prep_kernel<float, 1, 0, 1>)
                      : (v4 ? delta_prep_kernel<__nv_bfloat16, 4, 0, 1> : delta_prep_kernel<__nv_bfloat16, 1, 0, 1>);
   if (many) kernel = delta_prep_kernel<__nv_bfloat16, 4, 4, 4>;
-  kernel<<<dim3(many ? (total_rows + 3) / 4 : total_rows, (2 * c.kv_heads + a.v_units + 1 + 7) / 8), 256, 0, (cudaStream_t)stream>>>(a, total_rows);
+  launch_after(kernel, dim3(many ? (total_rows + 3) / 4 : total_rows, (2 * c.kv_heads + a.v_units + 1 + 7) / 8), 256, 0, (cudaStream_t)stream, a, total_rows);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -563,7 +567,7 @@ b200_status b200_delta_run(b200_kv* kv, const GlaScratch& g, const DeltaCall& c,
     if (smem > 200 * 1024) { b200_set_error("delta rule: head widths %d / %d are too large", c.dk, c.dv); return B200_ERR_UNSUPPORTED; }
     auto run = [&](auto* kernel) -> b200_status {
       if (smem > 48 * 1024) B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      kernel<<<dim3(n_req, c.heads), (z.cols * z.groups + 31) / 32 * 32, smem, s>>>(a);
+      launch_after(kernel, dim3(n_req, c.heads), (z.cols * z.groups + 31) / 32 * 32, smem, s, a);
       B200_LAUNCH_CHECK();
       return B200_OK;
     };
@@ -585,7 +589,7 @@ b200_status b200_delta_run(b200_kv* kv, const GlaScratch& g, const DeltaCall& c,
     B200_CUDA_TRY(cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     configured = true;
   }
-  delta_chunk_kernel<<<dim3(chunks, c.heads), 256, smem, s>>>(a);
+  launch_after(delta_chunk_kernel, dim3(chunks, c.heads), 256, smem, s, a);
   B200_LAUNCH_CHECK();
   if ((st = b200_gla_scan(z, n_req, true, s)) != B200_OK) return st;
   return b200_gla_out(z, chunks, by_four(kv, c) && c.out_stride % 4 == 0, s);

@@ -3,6 +3,7 @@
 #include <cuda_bf16.h>
 
 #include "common.h"
+#include "launch.cuh"
 
 namespace {
 
@@ -15,6 +16,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // One CTA per row; hidden % 8 == 0.
 __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                __nv_bfloat16* __restrict__ out, int hidden, float eps) {
+  after_previous();
   __shared__ float s_part[32];
   const int row = blockIdx.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * hidden);
@@ -60,6 +62,7 @@ __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ k,
                             const int* __restrict__ positions, int rows, int hq, int hkv, int D, int q_stride,
                             int k_stride, float log2_theta) {
+  after_previous();
   const int half = D / 2;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long total = (long long)rows * (hq + hkv) * half;
@@ -79,6 +82,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __rest
 
 __global__ void embed_kernel(const __nv_bfloat16* __restrict__ table, const uint32_t* __restrict__ ids,
                              __nv_bfloat16* __restrict__ out, int hidden) {
+  after_previous();
   const int row = blockIdx.x;
   const uint4* src = reinterpret_cast<const uint4*>(table + (size_t)ids[row] * hidden);
   uint4* dst = reinterpret_cast<uint4*>(out + (size_t)row * hidden);
@@ -88,6 +92,7 @@ __global__ void embed_kernel(const __nv_bfloat16* __restrict__ table, const uint
 // First strict maximum of each row (ties keep the smaller index).
 template <typename T>
 __global__ void argmax_kernel(const T* __restrict__ logits, int vocab, uint32_t* __restrict__ out) {
+  after_previous();
   __shared__ float s_val[32];
   __shared__ int s_idx[32];
   const int row = blockIdx.x;
@@ -140,6 +145,7 @@ __global__ void argmax_kernel(const T* __restrict__ logits, int vocab, uint32_t*
 
 __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ idx,
                                    __nv_bfloat16* __restrict__ dst, int hidden) {
+  after_previous();
   const int row = blockIdx.x;
   const int s = max(idx[row], 0);
   const uint4* sp = reinterpret_cast<const uint4*>(src + (size_t)s * hidden);
@@ -153,6 +159,7 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const 
 __global__ void scatter_tokens_kernel(const uint32_t* __restrict__ next, const b200_pack_desc* __restrict__ desc,
                                       uint32_t* __restrict__ last_token, int n_req, const int* __restrict__ flags,
                                       int flag_a, int flag_b) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (flags && (flags[flag_a] != 0 || flags[flag_b] != 0)) return;
   if (i < n_req && desc[i].count > 0) last_token[desc[i].seq_slot] = next[i];
@@ -163,7 +170,7 @@ __global__ void scatter_tokens_kernel(const uint32_t* __restrict__ next, const b
 // Rows idx[r] of src -> row r of dst (the last position of every request, src/generation.zig:124-131).
 b200_status b200_gather_rows(const void* d_src, const int32_t* d_idx, void* d_dst, int32_t rows, int32_t hidden, void* stream) {
   if (rows <= 0) return B200_OK;
-  gather_rows_kernel<<<rows, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)d_src, d_idx, (__nv_bfloat16*)d_dst, hidden);
+  launch_after(gather_rows_kernel, rows, 128, 0, (cudaStream_t)stream, (const __nv_bfloat16*)d_src, d_idx, (__nv_bfloat16*)d_dst, hidden);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -172,7 +179,7 @@ b200_status b200_gather_rows(const void* d_src, const int32_t* d_idx, void* d_ds
 b200_status b200_scatter_tokens(const uint32_t* d_next, const b200_pack_desc* d_desc, uint32_t* d_last_token, int32_t n_req,
                                 const int* d_flags, int flag_a, int flag_b, void* stream) {
   if (n_req <= 0) return B200_OK;
-  scatter_tokens_kernel<<<(n_req + 127) / 128, 128, 0, (cudaStream_t)stream>>>(d_next, d_desc, d_last_token, n_req, d_flags,
+  launch_after(scatter_tokens_kernel, (n_req + 127) / 128, 128, 0, (cudaStream_t)stream, d_next, d_desc, d_last_token, n_req, d_flags,
                                                                               flag_a, flag_b);
   B200_LAUNCH_CHECK();
   return B200_OK;
@@ -186,7 +193,7 @@ b200_status b200_rmsnorm(const void* d_x, const void* d_weight, void* d_out, int
   if (st != B200_OK) return st;
   if (hidden % 8 != 0) { b200_set_error("rmsnorm: hidden must be a multiple of 8"); return B200_ERR_INVALID_ARGUMENT; }
   if (rows <= 0) return B200_OK;
-  rmsnorm_kernel<<<rows, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)d_x, (const __nv_bfloat16*)d_weight,
+  launch_after(rmsnorm_kernel, rows, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)d_x, (const __nv_bfloat16*)d_weight,
                                                         (__nv_bfloat16*)d_out, hidden, eps);
   B200_LAUNCH_CHECK();
   return B200_OK;
@@ -199,7 +206,7 @@ b200_status b200_rope(void* d_q, void* d_k, const int32_t* d_positions, int32_t 
   if (st != B200_OK) return st;
   if (rows <= 0) return B200_OK;
   long long total = (long long)rows * (n_q_heads + n_kv_heads) * (head_dim / 2);
-  rope_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+  launch_after(rope_kernel, (unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream,
       (__nv_bfloat16*)d_q, (__nv_bfloat16*)d_k, d_positions, rows, n_q_heads, n_kv_heads, head_dim, q_stride, k_stride,
       log2f(theta));
   B200_LAUNCH_CHECK();
@@ -212,7 +219,7 @@ b200_status b200_embed_gather(const void* d_table, const uint32_t* d_ids, void* 
   if (st != B200_OK) return st;
   if (hidden % 8 != 0) { b200_set_error("embed: hidden must be a multiple of 8"); return B200_ERR_INVALID_ARGUMENT; }
   if (rows <= 0) return B200_OK;
-  embed_kernel<<<rows, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)d_table, d_ids, (__nv_bfloat16*)d_out, hidden);
+  launch_after(embed_kernel, rows, 128, 0, (cudaStream_t)stream, (const __nv_bfloat16*)d_table, d_ids, (__nv_bfloat16*)d_out, hidden);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -221,7 +228,7 @@ b200_status b200_argmax(const void* d_logits, int32_t rows, int32_t vocab, uint3
   b200_status st = b200_require_device();
   if (st != B200_OK) return st;
   if (rows <= 0) return B200_OK;
-  argmax_kernel<<<rows, 1024, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)d_logits, vocab, d_out);
+  launch_after(argmax_kernel<__nv_bfloat16>, rows, 1024, 0, (cudaStream_t)stream, (const __nv_bfloat16*)d_logits, vocab, d_out);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -230,7 +237,7 @@ b200_status b200_argmax_f32(const float* d_logits, int32_t rows, int32_t vocab, 
   b200_status st = b200_require_device();
   if (st != B200_OK) return st;
   if (rows <= 0) return B200_OK;
-  argmax_kernel<<<rows, 1024, 0, (cudaStream_t)stream>>>(d_logits, vocab, d_out);
+  launch_after(argmax_kernel<float>, rows, 1024, 0, (cudaStream_t)stream, d_logits, vocab, d_out);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }

@@ -23,6 +23,7 @@
 
 #include "common.h"
 #include "gla_chunks.cuh"
+#include "launch.cuh"
 
 namespace {
 
@@ -41,6 +42,7 @@ __device__ __forceinline__ Vec<VEC> memory_value(const Gla& a, int row, int head
 // ---- token by token ------------------------------------------------------------------------------------------
 template <typename T, int VEC, bool MEM>
 __global__ void __launch_bounds__(256, 3) gla_step_kernel(Gla a) {
+  after_previous();
   extern __shared__ float sh[];
   __shared__ float part[32];
   const int req = blockIdx.x, head = blockIdx.y, dk = a.dk, dv = a.dv, dvs = MEM ? a.dvs : dv, dva = MEM && VEC == 1 ? a.dva : dvs;
@@ -149,6 +151,7 @@ struct GateArgs {
 // One CTA per (request, head).  m_t = max(m_(t-1) + f_t, i_t) is a scan: the pair (F, M) stands for m -> max(m + F, M).
 template <typename T>
 __global__ void __launch_bounds__(1024) memory_gates_kernel(GateArgs a) {
+  after_previous();
   __shared__ float2 total[32];
   __shared__ float s_m[1025];
   const int req = blockIdx.x, head = blockIdx.y, H = a.g.heads, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
@@ -201,6 +204,7 @@ __global__ void __launch_bounds__(1024) memory_gates_kernel(GateArgs a) {
 // One CTA: the chunks of every portion that goes chunk by chunk, and where each request's start.
 __global__ void __launch_bounds__(1024) gla_plan_kernel(const int* __restrict__ cu, int n_req, int max_chunks, int4* __restrict__ plan,
                                                         int* __restrict__ first_chunk) {
+  after_previous();
   __shared__ int sums[32];
   __shared__ int base;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -243,6 +247,7 @@ constexpr float kMaxGrowth = 60.f;
 
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) gla_chunk_kernel(Gla a) {
+  after_previous();
   extern __shared__ __align__(16) float sh[];
   __shared__ int s_range;
   const int chunk = blockIdx.x, head = blockIdx.y;
@@ -375,6 +380,7 @@ __global__ void __launch_bounds__(256) gla_chunk_kernel(Gla a) {
 // delta_chunk_kernel (delta.cu); u is f32 and enters the tensor cores as two terms.
 template <int NT, bool DELTA>  // NT: 8-channel tiles of the state a warp holds
 __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
+  after_previous();
   extern __shared__ unsigned char scan_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(scan_dyn) + 127) & ~(uintptr_t)127);
   const int req = blockIdx.x, head = blockIdx.y, slice = blockIdx.z;
@@ -567,6 +573,7 @@ __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
 // ---- chunks: norm and gate -------------------------------------------------------------------------------------------
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) gla_out_kernel(Gla a) {
+  after_previous();
   const int chunk = blockIdx.x, head = blockIdx.y, lane = threadIdx.x & 31;
   if (chunk >= a.first_chunk[a.n_req] || a.d.state[ST_ERR] != 0) return;
   const int4 it = a.plan[chunk];
@@ -596,6 +603,7 @@ __global__ void __launch_bounds__(256) gla_out_kernel(Gla a) {
 // any strength take this route.
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) memory_chunk_kernel(Gla a) {
+  after_previous();
   extern __shared__ __align__(16) float sh[];
   __shared__ float s_L[kC], s_w[kC];
   const int chunk = blockIdx.x, head = blockIdx.y;
@@ -689,6 +697,7 @@ __global__ void __launch_bounds__(256) memory_chunk_kernel(Gla a) {
 
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) memory_out_kernel(Gla a) {
+  after_previous();
   const int chunk = blockIdx.x, head = blockIdx.y, lane = threadIdx.x & 31;
   if (chunk >= a.first_chunk[a.n_req] || a.d.state[ST_ERR] != 0) return;
   const int4 it = a.plan[chunk];
@@ -724,7 +733,7 @@ b200_status launch_scan(Gla& a, int n_req, cudaStream_t s) {
     B200_CUDA_TRY((cudaFuncSetAttribute(gla_scan_kernel<NT, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024)));
     configured = true;
   }
-  gla_scan_kernel<NT, DELTA><<<dim3(n_req, a.heads, a.n_slices), kScanWarps * 32, smem, s>>>(a);
+  launch_after(gla_scan_kernel<NT, DELTA>, dim3(n_req, a.heads, a.n_slices), kScanWarps * 32, smem, s, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -742,7 +751,7 @@ b200_status b200_gla_scan(Gla& a, int n_req, bool delta, cudaStream_t s) { retur
 
 b200_status b200_gla_out(const Gla& a, int chunks, bool wide, cudaStream_t s) {
   auto* kernel = wide ? gla_out_kernel<__nv_bfloat16, 4> : gla_out_kernel<__nv_bfloat16, 1>;
-  kernel<<<dim3(chunks, a.heads), 256, 0, s>>>(a);
+  launch_after(kernel, dim3(chunks, a.heads), 256, 0, s, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -776,7 +785,7 @@ void GlaScratch::free() {
 
 b200_status b200_gla_plan(GlaScratch& g, const int32_t* d_cu, int n_req, int total_rows, void* stream) {
   if (n_req > g.max_reqs || total_rows > g.max_rows) { b200_set_error("gla: %d requests / %d rows exceed the scratch", n_req, total_rows); return B200_ERR_CAPACITY; }
-  gla_plan_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(d_cu, n_req, g.max_chunks, g.plan, g.first_chunk);
+  launch_after(gla_plan_kernel, 1, 1024, 0, (cudaStream_t)stream, d_cu, n_req, g.max_chunks, g.plan, g.first_chunk);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -792,7 +801,7 @@ b200_status b200_memory_gates(b200_kv* kv, const MemoryGates& g, const int32_t* 
   a.d = kv->dev; a.g = g; a.state = kv->dev.rec_pool + kv->lay[g.layer].rec_off; a.rec_elems = kv->lay[g.layer].rec_elems;
   a.cu = d_cu; a.row_seq = d_row_seq; a.pos = d_pos;
   auto* kernel = kv->dev.elem_bytes == 4 ? memory_gates_kernel<float> : memory_gates_kernel<__nv_bfloat16>;
-  kernel<<<dim3(n_req, g.heads), total_rows > 256 * n_req ? 1024 : (total_rows > 4 * n_req ? 256 : 32), 0, (cudaStream_t)stream>>>(a);
+  launch_after(kernel, dim3(n_req, g.heads), total_rows > 256 * n_req ? 1024 : (total_rows > 4 * n_req ? 256 : 32), 0, (cudaStream_t)stream, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -836,7 +845,7 @@ b200_status b200_gla_run(b200_kv* kv, const GlaScratch& g, const GlaCall& c, con
     if (mem) kernel = f32 ? (v4 ? gla_step_kernel<float, 4, true> : gla_step_kernel<float, 1, true>)
                           : (v4 ? gla_step_kernel<__nv_bfloat16, 4, true> : gla_step_kernel<__nv_bfloat16, 1, true>);
     if (smem > 48 * 1024) B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<dim3(n_req, c.heads), (a.cols * a.groups + 31) / 32 * 32, smem, s>>>(a);
+    launch_after(kernel, dim3(n_req, c.heads), (a.cols * a.groups + 31) / 32 * 32, smem, s, a);
     B200_LAUNCH_CHECK();
   }
   if (!a.chunked || total_rows <= n_req) return B200_OK;
@@ -854,13 +863,13 @@ b200_status b200_gla_run(b200_kv* kv, const GlaScratch& g, const GlaCall& c, con
   const bool wide = v4 && c.out_stride % 4 == 0;
   auto* chunk_kernel = mem ? (wide ? memory_chunk_kernel<__nv_bfloat16, 4> : memory_chunk_kernel<__nv_bfloat16, 1>)
                            : (wide ? gla_chunk_kernel<__nv_bfloat16, 4> : gla_chunk_kernel<__nv_bfloat16, 1>);
-  chunk_kernel<<<dim3(chunks, c.heads), 256, smem, s>>>(a);
+  launch_after(chunk_kernel, dim3(chunks, c.heads), 256, smem, s, a);
   B200_LAUNCH_CHECK();
   b200_status st = b200_gla_scan(a, n_req, false, s);
   if (st != B200_OK) return st;
   if (!mem) return b200_gla_out(a, chunks, wide, s);
   auto* out_kernel = wide ? memory_out_kernel<__nv_bfloat16, 4> : memory_out_kernel<__nv_bfloat16, 1>;
-  out_kernel<<<dim3(chunks, c.heads), 256, 0, s>>>(a);
+  launch_after(out_kernel, dim3(chunks, c.heads), 256, 0, s, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }

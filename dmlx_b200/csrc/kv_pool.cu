@@ -24,6 +24,7 @@
 #include "attn_prompt.cuh"
 #include "common.h"
 #include "kv_pool.cuh"
+#include "launch.cuh"
 #include "tma.cuh"
 
 static int g_device_state = -1;  // -1 unknown, 0 none, 1 ok
@@ -71,6 +72,7 @@ constexpr int kReserveThreads = 1024;
 constexpr int kReserveItems = 4;  // requests per thread -> 4096 requests per step
 
 __global__ void init_pool_kernel(KvDev d) {
+  after_previous();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < d.n_pages) {
     d.free_stack[i] = d.n_pages - 1 - i;
@@ -119,6 +121,7 @@ __device__ int4 block_exscan4(int4 v, int4* total, int4* warp_sums) {
 // in a block of 256: 8 requests 9.0 -> 3.4 us, 61 requests 13.7 -> 5.2.
 template <int THREADS, int ITEMS>
 __global__ void __launch_bounds__(THREADS) reserve_kernel(KvDev d, const b200_pack_desc* desc, int n_req) {
+  after_previous();
   __shared__ int4 warp_sums[32], s_total;  // {pages needed, pages touched, copies, rows}
   __shared__ int s_any_cow;
   const int tid = threadIdx.x;
@@ -251,6 +254,7 @@ __global__ void __launch_bounds__(THREADS) reserve_kernel(KvDev d, const b200_pa
 
 // Copies every queued CoW page (all layers, K and V, scales for FP8 pools).
 __global__ void cow_copy_kernel(KvDev d) {
+  after_previous();
   const int n_cow = d.state[ST_N_COW];
   const int layer = blockIdx.y >> 1, is_v = blockIdx.y & 1;
   const KvLayerDev L = d.layer[layer];
@@ -273,6 +277,7 @@ __global__ void cow_copy_kernel(KvDev d) {
 // bf16 append: one CTA per (page touch, kv head) copies rows into the page tile.
 __global__ void append_bf16_kernel(KvDev d, int layer, const __nv_bfloat16* __restrict__ k_rows,
                                    const __nv_bfloat16* __restrict__ v_rows, int k_stride, int v_stride) {
+  after_previous();
   const int n_touch = d.state[ST_N_TOUCH];
   const int head = blockIdx.y, D = d.head_dim, H = d.n_kv_heads;
   const int vec_per_row = D / 8;
@@ -299,6 +304,7 @@ __global__ void __launch_bounds__(256) rope_append_bf16_kernel(KvDev d, int laye
                                                                int q_stride, int k_stride, int v_stride,
                                                                const int* __restrict__ positions, const int* __restrict__ row_seq, int hq,
                                                                float log2_theta) {
+  after_previous();
   const int row = blockIdx.x, D = d.head_dim, H = d.n_kv_heads, half = D / 2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int pos = positions[row], seq = row_seq[row];
@@ -356,6 +362,7 @@ __device__ __forceinline__ float from_e4m3(unsigned char b) {
 // rows already in the tile are re-encoded at the new scale; then the new rows are encoded.
 __global__ void append_fp8_kernel(KvDev d, int layer, const __nv_bfloat16* __restrict__ k_rows,
                                   const __nv_bfloat16* __restrict__ v_rows, int k_stride, int v_stride) {
+  after_previous();
   __shared__ float s_red[32];
   __shared__ float s_scale[2];
   const int n_touch = d.state[ST_N_TOUCH];
@@ -406,6 +413,7 @@ __global__ void append_fp8_kernel(KvDev d, int layer, const __nv_bfloat16* __res
 // Test helper: contiguous [len, H, key_dim] and [len, H, value_dim] views of one sequence of one layer (bf16, or f32 for
 // an f32 pool).
 __global__ void gather_kernel(KvDev d, int layer, int seq, void* k_out, void* v_out, int cap_rows) {
+  after_previous();
   const int len = min(d.seq_len[seq], cap_rows);
   const KvLayerDev L = d.layer[layer];
   for (int is_v = 0; is_v < 2; ++is_v) {
@@ -444,6 +452,7 @@ __device__ void release_page(KvDev& d, int page) {
 
 // args: op-specific; `list` is a device array (sequence slots, or page ids); out: device ints.
 __global__ void admin_kernel(KvDev d, int op, int a0, int a1, int a2, const int* list, int* out) {
+  after_previous();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   out[0] = B200_OK;
   switch (op) {
@@ -810,11 +819,11 @@ b200_status b200_kv_reserve(b200_kv* kv, const b200_pack_desc* d_desc, int32_t n
     return B200_ERR_INVALID_ARGUMENT;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  if (n_req <= 256) reserve_kernel<256, 1><<<1, 256, 0, s>>>(kv->dev, d_desc, n_req);
-  else reserve_kernel<kReserveThreads, kReserveItems><<<1, kReserveThreads, 0, s>>>(kv->dev, d_desc, n_req);
+  if (n_req <= 256) launch_after(reserve_kernel<256, 1>, 1, 256, 0, s, kv->dev, d_desc, n_req);
+  else launch_after(reserve_kernel<kReserveThreads, kReserveItems>, 1, kReserveThreads, 0, s, kv->dev, d_desc, n_req);
   B200_LAUNCH_CHECK();
   dim3 grid(std::min(kv->cfg.max_seqs, 256), kv->cfg.n_layers * 2);
-  cow_copy_kernel<<<grid, 256, 0, s>>>(kv->dev);
+  launch_after(cow_copy_kernel, grid, 256, 0, s, kv->dev);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -835,10 +844,10 @@ b200_status b200_kv_append_strided(b200_kv* kv, int32_t layer, const void* d_k_r
   cudaStream_t s = (cudaStream_t)stream;
   int gx = std::min(total_rows, 2048);
   if (kv->cfg.kv_dtype == B200_KV_BF16) {
-    append_bf16_kernel<<<dim3(gx, kv->cfg.n_kv_heads), 128, 0, s>>>(kv->dev, layer, (const __nv_bfloat16*)d_k_rows,
+    launch_after(append_bf16_kernel, dim3(gx, kv->cfg.n_kv_heads), 128, 0, s, kv->dev, layer, (const __nv_bfloat16*)d_k_rows,
                                                                     (const __nv_bfloat16*)d_v_rows, k_stride, v_stride);
   } else {
-    append_fp8_kernel<<<dim3(gx, kv->cfg.n_kv_heads, 2), 128, 0, s>>>(kv->dev, layer, (const __nv_bfloat16*)d_k_rows,
+    launch_after(append_fp8_kernel, dim3(gx, kv->cfg.n_kv_heads, 2), 128, 0, s, kv->dev, layer, (const __nv_bfloat16*)d_k_rows,
                                                                       (const __nv_bfloat16*)d_v_rows, k_stride, v_stride);
   }
   B200_LAUNCH_CHECK();
@@ -861,6 +870,7 @@ extern "C" b200_status b200_kv_rope_append(b200_kv* kv, int32_t layer, void* d_q
 __global__ void __launch_bounds__(256) rope_append_partials_bf16_kernel(KvDev d, int layer, b200_qmm_partials p, __nv_bfloat16* __restrict__ q,
                                                                         int q_stride, const int* __restrict__ positions,
                                                                         const int* __restrict__ row_seq, int hq, float log2_theta) {
+  after_previous();
   constexpr int D = 128, half = 64;
   const int row = blockIdx.x, H = d.n_kv_heads;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -927,7 +937,7 @@ extern "C" b200_status b200_kv_rope_append_partials(b200_kv* kv, int32_t layer, 
   }
   if (layer < 0 || layer >= c.n_layers) { b200_set_error("append: layer %d out of range", layer); return B200_ERR_INVALID_ARGUMENT; }
   if (total_rows <= 0) return B200_OK;
-  rope_append_partials_bf16_kernel<<<dim3(total_rows, (n_q_heads + 2 * c.n_kv_heads + 7) / 8), 256, 0, (cudaStream_t)stream>>>(
+  launch_after(rope_append_partials_bf16_kernel, dim3(total_rows, (n_q_heads + 2 * c.n_kv_heads + 7) / 8), 256, 0, (cudaStream_t)stream,
       kv->dev, layer, *parts, (__nv_bfloat16*)d_q, q_stride, d_positions, d_row_seq, n_q_heads, log2f(theta));
   B200_LAUNCH_CHECK();
   return B200_OK;
@@ -947,7 +957,7 @@ b200_status b200_kv_rope_append_strided(b200_kv* kv, int32_t layer, void* d_q, c
   }
   if (layer < 0 || layer >= c.n_layers) { b200_set_error("append: layer %d out of range", layer); return B200_ERR_INVALID_ARGUMENT; }
   if (total_rows <= 0) return B200_OK;
-  rope_append_bf16_kernel<<<dim3(total_rows, (n_q_heads + c.n_kv_heads + 7) / 8), 256, 0, (cudaStream_t)stream>>>(kv->dev, layer, (__nv_bfloat16*)d_q, (const __nv_bfloat16*)d_k_rows,
+  launch_after(rope_append_bf16_kernel, dim3(total_rows, (n_q_heads + c.n_kv_heads + 7) / 8), 256, 0, (cudaStream_t)stream, kv->dev, layer, (__nv_bfloat16*)d_q, (const __nv_bfloat16*)d_k_rows,
                                                                          (const __nv_bfloat16*)d_v_rows, q_stride, k_stride, v_stride,
                                                                          d_positions, d_row_seq, n_q_heads, log2f(theta));
   B200_LAUNCH_CHECK();
@@ -1004,7 +1014,7 @@ b200_status b200_kv_gather(b200_kv* kv, int32_t layer, int32_t seq, void* d_k_ou
     b200_set_error("gather: layer/slot out of range");
     return B200_ERR_INVALID_BATCH_INDEX;
   }
-  gather_kernel<<<296, 256, 0, (cudaStream_t)stream>>>(kv->dev, layer, seq, d_k_out, d_v_out, cap_rows);
+  launch_after(gather_kernel, 296, 256, 0, (cudaStream_t)stream, kv->dev, layer, seq, d_k_out, d_v_out, cap_rows);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -1034,6 +1044,7 @@ b200_status b200_kv_page_load(b200_kv* kv, int32_t layer, int32_t page, const vo
 // page (and, for FP8 pools, the per-head scales); grid = (pages of the sequence, layers).
 __global__ void __launch_bounds__(256) copy_pages_kernel(KvDev src, KvDev dst, const int* __restrict__ src_table,
                                                          const int* __restrict__ dst_table) {
+  after_previous();
   const int layer = blockIdx.y, sp = src_table[blockIdx.x], dp = dst_table[blockIdx.x];
   if (sp < 0 || sp >= src.n_pages || dp < 0 || dp >= dst.n_pages) return;
   const KvLayerDev L = src.layer[layer], M = dst.layer[layer];  // the same shapes; the pools may differ in page count

@@ -9,6 +9,7 @@
 #include <algorithm>
 
 #include "common.h"
+#include "launch.cuh"
 #include "lru.cuh"
 
 namespace {
@@ -29,6 +30,7 @@ __device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-
 // One thread per (R rows, VEC channels).
 template <typename T, int VEC, int R>
 __global__ void __launch_bounds__(256) lru_prep_kernel(LruArgs a, int rows) {
+  after_previous();
   const LruCall& c = a.c;
   const int begin = blockIdx.x * R, end = min(begin + R, rows), ch = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
   if (ch >= c.width) return;
@@ -78,6 +80,7 @@ __global__ void __launch_bounds__(256) lru_prep_kernel(LruArgs a, int rows) {
 // warps take a segment of the tokens each.
 template <typename T, int SEG>
 __global__ void __launch_bounds__(SEG == 1 ? 128 : 32 * SEG) lru_scan_kernel(LruArgs a) {
+  after_previous();
   __shared__ float s_log[SEG][33], s_sum[SEG][33];
   const LruCall& c = a.c;
   const int req = blockIdx.y, lane = threadIdx.x & 31, seg = SEG == 1 ? 0 : threadIdx.x >> 5;
@@ -163,7 +166,7 @@ b200_status b200_lru_prep(b200_kv* kv, LruCall c, const int32_t* d_cu, const int
   const bool many = total_rows >= 1024, f32 = kv->dev.elem_bytes == 4;
   auto* kernel = f32 ? (v4 ? lru_prep_kernel<float, 4, 1> : lru_prep_kernel<float, 1, 1>) : (v4 ? lru_prep_kernel<__nv_bfloat16, 4, 1> : lru_prep_kernel<__nv_bfloat16, 1, 1>);
   if (many) kernel = f32 ? (v4 ? lru_prep_kernel<float, 4, 4> : lru_prep_kernel<float, 1, 4>) : (v4 ? lru_prep_kernel<__nv_bfloat16, 4, 4> : lru_prep_kernel<__nv_bfloat16, 1, 4>);
-  kernel<<<dim3(many ? (total_rows + 3) / 4 : total_rows, (groups + threads - 1) / threads), threads, 0, (cudaStream_t)stream>>>(a, total_rows);
+  launch_after(kernel, dim3(many ? (total_rows + 3) / 4 : total_rows, (groups + threads - 1) / threads), threads, 0, (cudaStream_t)stream, a, total_rows);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -179,10 +182,10 @@ b200_status b200_lru_scan(b200_kv* kv, const LruCall& c, const int32_t* d_cu, co
   cudaStream_t s = (cudaStream_t)stream;
   if (total_rows <= 8 * n_req) {
     auto* kernel = f32 ? lru_scan_kernel<float, 1> : lru_scan_kernel<__nv_bfloat16, 1>;
-    kernel<<<dim3((c.width + 127) / 128, n_req), 128, 0, s>>>(a);
+    launch_after(kernel, dim3((c.width + 127) / 128, n_req), 128, 0, s, a);
   } else {
     auto* kernel = f32 ? lru_scan_kernel<float, 16> : lru_scan_kernel<__nv_bfloat16, 16>;
-    kernel<<<dim3((c.width + 31) / 32, n_req), 512, 0, s>>>(a);
+    launch_after(kernel, dim3((c.width + 31) / 32, n_req), 512, 0, s, a);
   }
   B200_LAUNCH_CHECK();
   return B200_OK;

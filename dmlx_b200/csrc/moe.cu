@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "common.h"
+#include "launch.cuh"
 #include "moe.cuh"
 #include "qmm.cuh"
 
@@ -37,6 +38,7 @@ template <typename LogitT>
 __global__ void route_kernel(const LogitT* __restrict__ logits, const float* __restrict__ bias, int n_tokens, int n_experts,
                              int k, int scoring, float route_scale, uint32_t* __restrict__ out_idx,
                              float* __restrict__ out_w, int* __restrict__ counts) {
+  after_previous();
   const int token = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (token >= n_tokens) return;
   constexpr int PER = kMaxExperts / 32;
@@ -116,6 +118,7 @@ __global__ void route_kernel(const LogitT* __restrict__ logits, const float* __r
 // offsets = exclusive scan of counts; work items {expert, first row, rows} for tiles of `tile_rows`.
 __global__ void offsets_items_kernel(const int* __restrict__ counts, int n_experts, int tile_rows, int* __restrict__ offsets,
                                      int4* __restrict__ items, int* __restrict__ n_items) {
+  after_previous();
   __shared__ int s_off[kMaxExperts + 1], s_item[kMaxExperts + 1];
   if (threadIdx.x == 0) {
     int o = 0, it = 0;
@@ -200,6 +203,7 @@ __device__ __forceinline__ void place_assignments(const uint32_t* __restrict__ i
 __global__ void __launch_bounds__(1024) place_kernel(const uint32_t* __restrict__ indices, int n_assign,
                                                      const int* __restrict__ offsets, int* __restrict__ order,
                                                      int* __restrict__ inv_order) {
+  after_previous();
   place_assignments(indices, n_assign, offsets, order, inv_order);
 }
 
@@ -208,6 +212,7 @@ __global__ void __launch_bounds__(1024) place_kernel(const uint32_t* __restrict_
 // them and lays out the work items; one CTA per (expert, layer) then places the assignments.
 __global__ void __launch_bounds__(1024) table_route_kernel(const MoeTableLayer* __restrict__ layers, const uint32_t* __restrict__ tokens, int n_tokens,
                                                            int vocab, int tile_rows) {
+  after_previous();
   __shared__ int s_count[kMaxExperts], s_off[kMaxExperts + 1], s_item[kMaxExperts + 1];
   const MoeTableLayer L = layers[blockIdx.x];
   const int tid = threadIdx.x, n = n_tokens * L.top;
@@ -241,6 +246,7 @@ __global__ void __launch_bounds__(1024) table_route_kernel(const MoeTableLayer* 
 }
 
 __global__ void __launch_bounds__(1024) table_place_kernel(const MoeTableLayer* __restrict__ layers, int n_tokens) {
+  after_previous();
   const MoeTableLayer L = layers[blockIdx.y];
   if ((int)blockIdx.x >= L.n_experts) return;
   place_assignments(L.indices, n_tokens * L.top, L.offsets, L.order, L.inv_order);
@@ -252,6 +258,7 @@ __global__ void __launch_bounds__(1024) table_place_kernel(const MoeTableLayer* 
 template <typename T, int PER>
 __global__ void __launch_bounds__(256) route_src_kernel(MatSrc logits, int n_tokens, int n_experts, int k, int n_groups, int keep, RouterScores scores,
                                                         uint32_t* __restrict__ out_idx, float* __restrict__ out_w) {
+  after_previous();
   const int token = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (token >= n_tokens) return;
   float sc[PER], ch[PER];
@@ -337,6 +344,7 @@ __global__ void __launch_bounds__(256) route_src_kernel(MatSrc logits, int n_tok
 // The plan of one layer in one launch, a CTA per expert: it counts the assignments of the experts before its own and places its
 // own; the first also lays out the work items.
 __global__ void __launch_bounds__(1024) plan_kernel(MoeTableLayer L, int n_tokens, int tile_rows) {
+  after_previous();
   __shared__ int s_count[kMaxExperts], s_item[kMaxExperts + 1];
   const int n = n_tokens * L.top, tid = threadIdx.x, e = blockIdx.x;
   for (int i = tid; i < L.n_experts; i += blockDim.x) s_count[i] = 0;
@@ -372,6 +380,7 @@ __global__ void __launch_bounds__(1024) plan_kernel(MoeTableLayer L, int n_token
 // Rows of x in the experts' order, 16 bytes at a time.
 __global__ void __launch_bounds__(128) gather_rows_by_order_kernel(const uint4* __restrict__ x, const int* __restrict__ order, int top, int vecs,
                                                                    uint4* __restrict__ out) {
+  after_previous();
   const uint4* src = x + (size_t)(order[blockIdx.x] / top) * vecs;
   uint4* dst = out + (size_t)blockIdx.x * vecs;
   for (int i = threadIdx.x; i < vecs; i += blockDim.x) dst[i] = src[i];
@@ -381,6 +390,7 @@ __global__ void __launch_bounds__(128) gather_rows_by_order_kernel(const uint4* 
 // n_valid (optional, device): rows that exist when n is only the capacity.
 __global__ void row_scales_kernel(const int* __restrict__ order, const float* __restrict__ weights, int n, float* __restrict__ out,
                                   const int* __restrict__ n_valid) {
+  after_previous();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p < n && (!n_valid || p < *n_valid)) out[p] = weights[order[p]];
 }
@@ -389,6 +399,7 @@ __global__ void row_scales_kernel(const int* __restrict__ order, const float* __
 // "not mine" (a value no expert matches, so the counting sort leaves those assignments out).
 __global__ void localize_kernel(const uint32_t* __restrict__ idx, int n_assign, int first_expert, int n_local,
                                 uint32_t* __restrict__ local_idx) {
+  after_previous();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n_assign) return;
   const int e = (int)idx[a] - first_expert;
@@ -399,6 +410,7 @@ __global__ void localize_kernel(const uint32_t* __restrict__ idx, int n_assign, 
 // token's experts lives here).  inv_order[a] < 0 marks an assignment served by another rank.
 __global__ void combine_partial_kernel(const __nv_bfloat16* __restrict__ y_sorted, const int* __restrict__ inv_order, int k,
                                        int hidden, float* __restrict__ out) {
+  after_previous();
   const int t = blockIdx.x;
   int rows[kMaxTopK];
   for (int j = 0; j < k; ++j) rows[j] = inv_order[t * k + j];
@@ -423,6 +435,7 @@ __global__ void combine_partial_kernel(const __nv_bfloat16* __restrict__ y_sorte
 // Expert parallelism: out = bf16(routed sum (f32, reduced over the ranks) + shared expert).
 __global__ void add_shared_kernel(const float* __restrict__ routed, const __nv_bfloat16* __restrict__ shared_out, size_t n8,
                                   __nv_bfloat16* __restrict__ out) {
+  after_previous();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n8) return;
   const float4 a = reinterpret_cast<const float4*>(routed)[2 * i], b = reinterpret_cast<const float4*>(routed)[2 * i + 1];
@@ -445,6 +458,7 @@ __global__ void gather_sorted_kernel(const __nv_bfloat16* __restrict__ x, const 
                                      const float* __restrict__ weights, int k, int hidden,
                                      __nv_bfloat16* __restrict__ x_sorted, float* __restrict__ row_scales,
                                      const int* __restrict__ n_valid) {
+  after_previous();
   const int p = blockIdx.x;
   if (n_valid && p >= *n_valid) return;
   const int a = order[p];
@@ -456,6 +470,7 @@ __global__ void gather_sorted_kernel(const __nv_bfloat16* __restrict__ x, const 
 
 __global__ void combine_kernel(const __nv_bfloat16* __restrict__ y_sorted, const int* __restrict__ inv_order, int k, int hidden,
                                const __nv_bfloat16* __restrict__ shared_out, __nv_bfloat16* __restrict__ out) {
+  after_previous();
   const int t = blockIdx.x;
   if (hidden % 8 == 0 && k <= 16) {
     // 16-byte loads, the rows of eight experts (and the shared one) asked for at once: one after the other they took 8.2 us at 24 tokens of
@@ -518,9 +533,9 @@ b200_status b200_moe_table_plan(const MoeTableLayer* d_layers, int n_layers, int
                                 int tile_rows, void* stream) {
   if (n_layers <= 0 || n_tokens <= 0) return B200_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  table_route_kernel<<<n_layers, 1024, 0, s>>>(d_layers, d_tokens, n_tokens, vocab, tile_rows);
+  launch_after(table_route_kernel, n_layers, 1024, 0, s, d_layers, d_tokens, n_tokens, vocab, tile_rows);
   B200_LAUNCH_CHECK();
-  table_place_kernel<<<dim3(most_experts, n_layers), 1024, 0, s>>>(d_layers, n_tokens);
+  launch_after(table_place_kernel, dim3(most_experts, n_layers), 1024, 0, s, d_layers, n_tokens);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -534,19 +549,19 @@ b200_status b200_moe_route_plan(const MoeTableLayer& L, const MatSrc& logits, bo
   }
   if (n_tokens <= 0) return B200_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  auto route = [&](auto* kernel) { kernel<<<(n_tokens + 7) / 8, 256, 0, s>>>(logits, n_tokens, L.n_experts, L.top, n_groups, keep_groups, scores, L.indices, d_weights); };
+  auto route = [&](auto* kernel) { launch_after(kernel, (n_tokens + 7) / 8, 256, 0, s, logits, n_tokens, L.n_experts, L.top, n_groups, keep_groups, scores, L.indices, d_weights); };
   const int per = (L.n_experts + 31) / 32;
   if (f32) route(per <= 1 ? route_src_kernel<float, 1> : (per <= 4 ? route_src_kernel<float, 4> : (per <= 8 ? route_src_kernel<float, 8> : route_src_kernel<float, 32>)));
   else route(per <= 1 ? route_src_kernel<__nv_bfloat16, 1> : (per <= 4 ? route_src_kernel<__nv_bfloat16, 4> : (per <= 8 ? route_src_kernel<__nv_bfloat16, 8> : route_src_kernel<__nv_bfloat16, 32>)));
   B200_LAUNCH_CHECK();
-  plan_kernel<<<L.n_experts, 1024, 0, s>>>(L, n_tokens, tile_rows);
+  launch_after(plan_kernel, L.n_experts, 1024, 0, s, L, n_tokens, tile_rows);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
 
 b200_status b200_moe_gather_order(const void* d_x, const int* d_order, int top, int n_assign, int width, void* d_out, void* stream) {
   if (n_assign <= 0) return B200_OK;
-  gather_rows_by_order_kernel<<<n_assign, 128, 0, (cudaStream_t)stream>>>((const uint4*)d_x, d_order, top, width / 8, (uint4*)d_out);
+  launch_after(gather_rows_by_order_kernel, n_assign, 128, 0, (cudaStream_t)stream, (const uint4*)d_x, d_order, top, width / 8, (uint4*)d_out);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -567,10 +582,10 @@ b200_status b200_moe_route(const void* d_logits, int32_t logits_are_f32, const f
   if (d_counts) B200_CUDA_TRY(cudaMemsetAsync(d_counts, 0, sizeof(int) * n_experts, s));
   const int blocks = (n_tokens * 32 + 255) / 256;
   if (logits_are_f32)
-    route_kernel<float><<<blocks, 256, 0, s>>>((const float*)d_logits, d_bias, n_tokens, n_experts, k, scoring, route_scale,
+    launch_after(route_kernel<float>, blocks, 256, 0, s, (const float*)d_logits, d_bias, n_tokens, n_experts, k, scoring, route_scale,
                                                d_indices, d_weights, d_counts);
   else
-    route_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>((const __nv_bfloat16*)d_logits, d_bias, n_tokens, n_experts, k, scoring,
+    launch_after(route_kernel<__nv_bfloat16>, blocks, 256, 0, s, (const __nv_bfloat16*)d_logits, d_bias, n_tokens, n_experts, k, scoring,
                                                        route_scale, d_indices, d_weights, d_counts);
   B200_LAUNCH_CHECK();
   return B200_OK;
@@ -584,9 +599,9 @@ b200_status b200_moe_group(const uint32_t* d_indices, const int32_t* d_counts, i
   if (n_experts <= 0 || n_experts > kMaxExperts || tile_rows <= 0) { b200_set_error("group: bad expert count or tile"); return B200_ERR_INVALID_ARGUMENT; }
   if (n_tokens <= 0) return B200_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  offsets_items_kernel<<<1, 256, 0, s>>>(d_counts, n_experts, tile_rows, d_offsets, (int4*)d_items, d_n_items);
+  launch_after(offsets_items_kernel, 1, 256, 0, s, d_counts, n_experts, tile_rows, d_offsets, (int4*)d_items, d_n_items);
   B200_LAUNCH_CHECK();
-  place_kernel<<<n_experts, 1024, 0, s>>>(d_indices, n_tokens * k, d_offsets, d_order, d_inv_order);
+  launch_after(place_kernel, n_experts, 1024, 0, s, d_indices, n_tokens * k, d_offsets, d_order, d_inv_order);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -597,7 +612,7 @@ b200_status b200_moe_gather(const void* d_x, const int32_t* d_order, const float
   if (st != B200_OK) return st;
   if (hidden % 8) { b200_set_error("gather: hidden must be a multiple of 8"); return B200_ERR_INVALID_ARGUMENT; }
   if (n_assign <= 0) return B200_OK;
-  gather_sorted_kernel<<<n_assign, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)d_x, d_order, d_weights, k, hidden,
+  launch_after(gather_sorted_kernel, n_assign, 128, 0, (cudaStream_t)stream, (const __nv_bfloat16*)d_x, d_order, d_weights, k, hidden,
                                                                   (__nv_bfloat16*)d_x_sorted, d_row_scales, nullptr);
   B200_LAUNCH_CHECK();
   return B200_OK;
@@ -627,7 +642,7 @@ b200_status b200_moe_combine(const void* d_y_sorted, const int32_t* d_inv_order,
   if (n_tokens <= 0) return B200_OK;
   // (few tokens: a block per 2048 columns)
   const int parts = n_tokens <= 512 && hidden % 8 == 0 && k <= 16 ? (hidden / 8 + 255) / 256 : 1;
-  combine_kernel<<<dim3(n_tokens, parts), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)d_y_sorted, d_inv_order, k, hidden,
+  launch_after(combine_kernel, dim3(n_tokens, parts), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)d_y_sorted, d_inv_order, k, hidden,
                                                              (const __nv_bfloat16*)d_shared_out, (__nv_bfloat16*)d_out);
   B200_LAUNCH_CHECK();
   return B200_OK;
@@ -651,12 +666,12 @@ b200_status b200_ep_plan(const uint32_t* d_indices, const int32_t* d_counts, int
   if (n_tokens <= 0) return B200_OK;
   const int n_local = n_experts / world, A = n_tokens * k;
   cudaStream_t s = (cudaStream_t)stream;
-  localize_kernel<<<(A + 255) / 256, 256, 0, s>>>(d_indices, A, rank * n_local, n_local, d_local_idx);
+  launch_after(localize_kernel, (A + 255) / 256, 256, 0, s, d_indices, A, rank * n_local, n_local, d_local_idx);
   B200_LAUNCH_CHECK();
   B200_CUDA_TRY(cudaMemsetAsync(d_inv_order, 0xFF, sizeof(int) * (size_t)A, s));
-  offsets_items_kernel<<<1, 256, 0, s>>>(d_counts + rank * n_local, n_local, tile_rows, d_offsets, (int4*)d_items, d_n_items);
+  launch_after(offsets_items_kernel, 1, 256, 0, s, d_counts + rank * n_local, n_local, tile_rows, d_offsets, (int4*)d_items, d_n_items);
   B200_LAUNCH_CHECK();
-  place_kernel<<<n_local, 1024, 0, s>>>(d_local_idx, A, d_offsets, d_order, d_inv_order);
+  launch_after(place_kernel, n_local, 1024, 0, s, d_local_idx, A, d_offsets, d_order, d_inv_order);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -794,7 +809,7 @@ b200_status b200_moe_forward(b200_moe* m, const void* d_x, int32_t n_tokens, voi
   if (b200_qmm_grouped_takes_tokens(m->exp_gu, tile_rows)) {
     // the block-scaled path re-encodes every activation row anyway: it reads the rows from the token
     // matrix through `order`, and no expert-sorted bf16 copy is made
-    row_scales_kernel<<<(A + 255) / 256, 256, 0, (cudaStream_t)stream>>>(m->order, m->weights, A, m->row_scales, nullptr);
+    launch_after(row_scales_kernel, (A + 255) / 256, 256, 0, (cudaStream_t)stream, m->order, m->weights, A, m->row_scales, nullptr);
     B200_LAUNCH_CHECK();
     STEP(b200_qmm_grouped_from_tokens(m->exp_gu, d_x, m->order, c.top_k, A, m->act_sorted, B200_EPI_SWIGLU, m->row_scales,
                                       c.swiglu_limit, m->items, m->n_items, m->max_items, tile_rows, stream));
@@ -849,24 +864,24 @@ b200_status b200_moe_forward_ep(b200_moe* m, b200_ep* ep, const void* d_x, int32
   STEP(b200_ep_plan(m->indices, m->counts, N, c.top_k, c.n_experts, c.ep_rank, world, c.tile_rows, m->local_idx, m->offsets,
                     m->order, m->inv_order, m->items, m->n_items, stream));
   const int* rows_valid = m->offsets + m->n_local;  // assignments served here
-  row_scales_kernel<<<(A + 255) / 256, 256, 0, s>>>(m->order, m->weights, A, m->row_scales, rows_valid);
+  launch_after(row_scales_kernel, (A + 255) / 256, 256, 0, s, m->order, m->weights, A, m->row_scales, rows_valid);
   B200_LAUNCH_CHECK();
   if (b200_qmm_grouped_takes_tokens(m->exp_gu, c.tile_rows)) {
     STEP(b200_qmm_grouped_from_tokens(m->exp_gu, m->x_all, m->order, c.top_k, A, m->act_sorted, B200_EPI_SWIGLU, m->row_scales,
                                       c.swiglu_limit, m->items, m->n_items, m->max_items, c.tile_rows, stream, rows_valid));
   } else {
-    gather_sorted_kernel<<<A, 128, 0, s>>>(m->x_all, m->order, m->weights, c.top_k, c.hidden, m->x_sorted, nullptr, rows_valid);
+    launch_after(gather_sorted_kernel, A, 128, 0, s, m->x_all, m->order, m->weights, c.top_k, c.hidden, m->x_sorted, nullptr, rows_valid);
     B200_LAUNCH_CHECK();
     STEP(b200_qmm_grouped(m->exp_gu, m->x_sorted, A, m->act_sorted, B200_EPI_SWIGLU, m->row_scales, c.swiglu_limit, m->items,
                           m->n_items, m->max_items, c.tile_rows, stream));
   }
   STEP(b200_qmm_grouped(m->exp_down, m->act_sorted, A, m->y_sorted, B200_EPI_NONE, nullptr, 0.f, m->items, m->n_items,
                         m->max_items, c.tile_rows, stream));
-  combine_partial_kernel<<<N, 256, 0, s>>>(m->y_sorted, m->inv_order, c.top_k, c.hidden, m->partial);
+  launch_after(combine_partial_kernel, N, 256, 0, s, m->y_sorted, m->inv_order, c.top_k, c.hidden, m->partial);
   B200_LAUNCH_CHECK();
   STEP(b200_ep_combine(ep, m->partial, m->reduced, n_tokens, c.hidden, stream));
   const size_t n8 = (size_t)n_tokens * c.hidden / 8;
-  add_shared_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, s>>>(m->reduced, m->sh_out, n8, (__nv_bfloat16*)d_out);
+  launch_after(add_shared_kernel, (unsigned)((n8 + 255) / 256), 256, 0, s, m->reduced, m->sh_out, n8, (__nv_bfloat16*)d_out);
   B200_LAUNCH_CHECK();
 #undef STEP
   return B200_OK;

@@ -2,6 +2,7 @@
 // descriptors the attention kernel consumes.  Replaces the host loops and the T x T mask of
 // src/batch_builder.zig:122-205 — the mask is implied by (row_seq, row_ctx).
 #include "common.h"
+#include "launch.cuh"
 
 namespace {
 
@@ -10,6 +11,7 @@ constexpr int kScanItems = 4;
 
 __global__ void __launch_bounds__(kScanThreads) pack_scan_kernel(const b200_pack_desc* __restrict__ desc, int n_req,
                                                                  int* __restrict__ cu_seqlens, int* __restrict__ last_row) {
+  after_previous();
   __shared__ int warp_sums[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int c[kScanItems], sum = 0;
@@ -55,6 +57,7 @@ __global__ void pack_fill_kernel(const b200_pack_desc* __restrict__ desc, int n_
                                  uint32_t* __restrict__ token_ids, int* __restrict__ position_ids,
                                  int* __restrict__ row_to_req, int* __restrict__ row_seq, int* __restrict__ row_ctx,
                                  int total_rows) {
+  after_previous();
   int row = blockIdx.x * blockDim.x + threadIdx.x;
   if (row >= total_rows) return;
   // last request r with cu[r] <= row
@@ -86,10 +89,10 @@ extern "C" b200_status b200_pack_batch(const b200_pack_desc* d_desc, int32_t n_r
     return B200_ERR_INVALID_ARGUMENT;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  pack_scan_kernel<<<1, kScanThreads, 0, s>>>(d_desc, n_req, d_cu_seqlens, d_last_row);
+  launch_after(pack_scan_kernel, 1, kScanThreads, 0, s, d_desc, n_req, d_cu_seqlens, d_last_row);
   B200_LAUNCH_CHECK();
   if (total_rows > 0 && n_req > 0) {
-    pack_fill_kernel<<<(total_rows + 255) / 256, 256, 0, s>>>(d_desc, n_req, d_cu_seqlens, d_prefill_tokens, d_last_token,
+    launch_after(pack_fill_kernel, (total_rows + 255) / 256, 256, 0, s, d_desc, n_req, d_cu_seqlens, d_prefill_tokens, d_last_token,
                                                             d_token_ids, d_position_ids, d_row_to_req, d_row_seq,
                                                             d_row_ctx, total_rows);
     B200_LAUNCH_CHECK();

@@ -22,6 +22,7 @@
 #include "attn_prompt.cuh"
 #include "common.h"
 #include "kv_pool.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "tma.cuh"
 
@@ -68,6 +69,7 @@ __device__ __forceinline__ int attn_pages_per_chunk(const AttnArgs& a) { return 
 // launch at 32 against 0.377 at 8).  The choice is written to *ppc_out for the kernels that follow.
 __global__ void attn_plan_kernel(const int* __restrict__ row_ctx, int total_rows, int page_size, int pages_per_chunk,
                                  int* __restrict__ chunk_start, int max_chunks, int* __restrict__ err, int* __restrict__ ppc_out) {
+  after_previous();
   __shared__ int warp_sums[32];
   __shared__ int carry;
   __shared__ int s_ppc;
@@ -196,6 +198,7 @@ __device__ __forceinline__ void load_row(const unsigned char* tile, int tok, int
 
 template <int D, bool FP8>
 __global__ void __launch_bounds__(kAttnThreads, 3) paged_attn_kernel(AttnArgs a) {
+  after_previous();
   constexpr int ELEM = FP8 ? 1 : 2;
   constexpr int TILE = 32 * D * ELEM;  // bytes of one (page, kv head) K or V tile
   constexpr int VEC = D / 16;          // dims per lane
@@ -478,6 +481,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 template <int D>
 __global__ void __launch_bounds__(kMmaWarps * 32, 1)
     paged_attn_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, AttnArgs a) {
+  after_previous();
   constexpr int BOXES = D / 64;     // 128-byte wide TMA boxes per tile
   constexpr int TILE = 32 * D * 2;  // bytes of one K or V tile
   constexpr int KS = D / 16;        // k-steps of Q K^T
@@ -675,6 +679,7 @@ __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
 template <int STAGES, int MINB>
 __global__ void __launch_bounds__(kMmaWarps * 32, MINB)
     paged_attn_mma_fp8_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, AttnArgs a) {
+  after_previous();
   constexpr int D = 128;
   constexpr int TILE = 32 * D;  // bytes of one K or V tile
   constexpr int KS = D / 16;    // k-steps of Q K^T = 16-byte chunks of a row
@@ -903,6 +908,7 @@ __global__ void __launch_bounds__(1024) attn_plan_groups_kernel(const int* __res
                                                                 int* __restrict__ chunk_start, int* __restrict__ group_first,
                                                                 int* __restrict__ part_base, int* __restrict__ row_group,
                                                                 int* __restrict__ n_groups_out, int max_slots, int* __restrict__ err) {
+  after_previous();
   __shared__ int warp_buf[32];
   __shared__ int carry_start, carry_groups, carry_chunks, carry_slots;
   const int tid = threadIdx.x;
@@ -989,6 +995,7 @@ __device__ __forceinline__ void mma_bf16_16816_full(float (&d)[4], uint32_t a0, 
 template <int D>
 __global__ void __launch_bounds__(kMmaWarps * 32, 1)
     paged_attn_prefill_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, AttnArgs a) {
+  after_previous();
   constexpr int BOXES = D / 64;
   constexpr int TILE = 32 * D * 2;
   constexpr int KS = D / 16;
@@ -1206,6 +1213,7 @@ __device__ __forceinline__ void mma_f16_16816_full(float (&d)[4], uint32_t a0, u
 // slots permuted to match ldmatrix on byte tiles, K scale on the scores, relative V scale on P).
 __global__ void __launch_bounds__(kMmaWarps * 32, 1)
     paged_attn_prefill_fp8_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, AttnArgs a) {
+  after_previous();
   constexpr int D = 128, TILE = 32 * D, KS = D / 16, NO = D / 8, STAGES = kMmaStages;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -1449,6 +1457,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 1)
 // D threads per (row, query head): merge the partials of the row's group chunks and write bf16.
 template <int D>
 __global__ void __launch_bounds__(D) attn_combine_groups_kernel(AttnArgs a, __nv_bfloat16* __restrict__ out) {
+  after_previous();
   const int row = blockIdx.x / a.n_q_heads, qh = blockIdx.x - row * a.n_q_heads, d = threadIdx.x;
   if (a.d.state[ST_ATTN_ERR] != 0) return;
   const int grp = a.row_group[row], first = a.group_first[grp], size = a.group_first[grp + 1] - first;
@@ -1472,6 +1481,7 @@ __global__ void __launch_bounds__(D) attn_combine_groups_kernel(AttnArgs a, __nv
 // at a time, 61 rows of 32 heads over 1..8192 tokens took 10.3-11.3 us per layer; 6.3-6.6 now.)
 template <int D>
 __global__ void __launch_bounds__(D) attn_combine_kernel(AttnArgs a, __nv_bfloat16* __restrict__ out) {
+  after_previous();
   const int row = blockIdx.x / a.n_q_heads, qh = blockIdx.x - row * a.n_q_heads, d = threadIdx.x, lane = d & 31;
   if (a.d.state[ST_ATTN_ERR] != 0) return;
   const int c0 = a.chunk_start[row], c1 = a.chunk_start[row + 1];
@@ -1516,9 +1526,9 @@ b200_status launch_attn(const AttnArgs& a, void* d_out, int grid, cudaStream_t s
     B200_CUDA_TRY(cudaFuncSetAttribute(paged_attn_kernel<D, FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = true;
   }
-  paged_attn_kernel<D, FP8><<<grid, kAttnThreads, smem, s>>>(a);
+  launch_after(paged_attn_kernel<D, FP8>, grid, kAttnThreads, smem, s, a);
   B200_LAUNCH_CHECK();
-  attn_combine_kernel<D><<<a.total_rows * a.n_q_heads, D, 0, s>>>(a, (__nv_bfloat16*)d_out);
+  launch_after(attn_combine_kernel<D>, a.total_rows * a.n_q_heads, D, 0, s, a, (__nv_bfloat16*)d_out);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -1533,9 +1543,9 @@ b200_status launch_attn_mma(const b200_kv* kv, const AttnArgs& a, void* d_out, i
     configured = true;
   }
   const int ctas_per_sm = smem <= 100 * 1024 ? 2 : 1;
-  paged_attn_mma_kernel<D><<<sms * ctas_per_sm, kMmaWarps * 32, smem, s>>>(kv->kmap, kv->vmap, a);
+  launch_after(paged_attn_mma_kernel<D>, sms * ctas_per_sm, kMmaWarps * 32, smem, s, kv->kmap, kv->vmap, a);
   B200_LAUNCH_CHECK();
-  attn_combine_kernel<D><<<a.total_rows * a.n_q_heads, D, 0, s>>>(a, (__nv_bfloat16*)d_out);
+  launch_after(attn_combine_kernel<D>, a.total_rows * a.n_q_heads, D, 0, s, a, (__nv_bfloat16*)d_out);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -1549,9 +1559,9 @@ b200_status launch_attn_mma_fp8_cfg(const b200_kv* kv, const AttnArgs& a, void* 
     B200_CUDA_TRY((cudaFuncSetAttribute(paged_attn_mma_fp8_kernel<STAGES, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)));
     configured = true;
   }
-  paged_attn_mma_fp8_kernel<STAGES, MINB><<<sms * MINB, kMmaWarps * 32, smem, s>>>(kv->kmap, kv->vmap, a);
+  launch_after(paged_attn_mma_fp8_kernel<STAGES, MINB>, sms * MINB, kMmaWarps * 32, smem, s, kv->kmap, kv->vmap, a);
   B200_LAUNCH_CHECK();
-  attn_combine_kernel<128><<<a.total_rows * a.n_q_heads, 128, 0, s>>>(a, (__nv_bfloat16*)d_out);
+  launch_after(attn_combine_kernel<128>, a.total_rows * a.n_q_heads, 128, 0, s, a, (__nv_bfloat16*)d_out);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -1572,10 +1582,10 @@ b200_status launch_attn_prefill(const b200_kv* kv, const AttnArgs& a, void* d_ou
     configured = true;
   }
   const int ctas_per_sm = smem <= 100 * 1024 ? 2 : 1;
-  paged_attn_prefill_kernel<D><<<sms * ctas_per_sm, kMmaWarps * 32, smem, s>>>(kv->kmap, kv->vmap, a);
+  launch_after(paged_attn_prefill_kernel<D>, sms * ctas_per_sm, kMmaWarps * 32, smem, s, kv->kmap, kv->vmap, a);
   B200_LAUNCH_CHECK();
   if (a.direct_out) return B200_OK;  // one chunk per group: the kernel wrote the rows itself
-  attn_combine_groups_kernel<D><<<a.total_rows * a.n_q_heads, D, 0, s>>>(a, (__nv_bfloat16*)d_out);
+  launch_after(attn_combine_groups_kernel<D>, a.total_rows * a.n_q_heads, D, 0, s, a, (__nv_bfloat16*)d_out);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -1588,10 +1598,10 @@ b200_status launch_attn_prefill_fp8(const b200_kv* kv, const AttnArgs& a, void* 
     B200_CUDA_TRY(cudaFuncSetAttribute(paged_attn_prefill_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = true;
   }
-  paged_attn_prefill_fp8_kernel<<<sms * 2, kMmaWarps * 32, smem, s>>>(kv->kmap, kv->vmap, a);
+  launch_after(paged_attn_prefill_fp8_kernel, sms * 2, kMmaWarps * 32, smem, s, kv->kmap, kv->vmap, a);
   B200_LAUNCH_CHECK();
   if (a.direct_out) return B200_OK;  // one chunk per group: the kernel wrote the rows itself
-  attn_combine_groups_kernel<128><<<a.total_rows * a.n_q_heads, 128, 0, s>>>(a, (__nv_bfloat16*)d_out);
+  launch_after(attn_combine_groups_kernel<128>, a.total_rows * a.n_q_heads, 128, 0, s, a, (__nv_bfloat16*)d_out);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -1650,7 +1660,7 @@ b200_status b200_paged_attn_decode_strided(b200_kv* kv, int32_t layer, const voi
   a.scale_log2 = 1.4426950408889634f / sqrtf((float)c.head_dim);
   a.ppc_dev = kv->d_chunk_start + c.max_rows + 1;  // the last word of the array: the plan kernel's choice
   if (!reuse_plan) {  // the chunk plan depends on the row arrays only: the layers of one step share it
-    attn_plan_kernel<<<1, 1024, 0, s>>>(d_row_ctx, total_rows, c.page_size, ppc, kv->d_chunk_start, kv->max_chunks,
+    launch_after(attn_plan_kernel, 1, 1024, 0, s, d_row_ctx, total_rows, c.page_size, ppc, kv->d_chunk_start, kv->max_chunks,
                                         kv->dev.state + ST_ATTN_ERR, kv->d_chunk_start + c.max_rows + 1);
     B200_LAUNCH_CHECK();
   }
@@ -1709,7 +1719,7 @@ b200_status b200_paged_attn_prefill_strided(b200_kv* kv, int32_t layer, const vo
   a.q_tokens = 16 / G;
   a.direct_out = single_chunk ? (__nv_bfloat16*)d_out : nullptr;
   if (!reuse_plan) {
-    attn_plan_groups_kernel<<<1, 1024, 0, s>>>(d_row_seq, d_row_ctx, total_rows, c.page_size, ppc, a.q_tokens, kv->d_chunk_start,
+    launch_after(attn_plan_groups_kernel, 1, 1024, 0, s, d_row_seq, d_row_ctx, total_rows, c.page_size, ppc, a.q_tokens, kv->d_chunk_start,
                                                kv->d_groups, kv->d_groups + stride, kv->d_groups + 2 * stride,
                                                kv->d_groups + 3 * stride - 1, kv->max_chunks, kv->dev.state + ST_ATTN_ERR);
     B200_LAUNCH_CHECK();

@@ -42,6 +42,7 @@
 #include <vector>
 
 #include "common.h"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "qmm.cuh"
 #include "tma.cuh"
@@ -146,6 +147,7 @@ __device__ __forceinline__ void finish_store(const QmmArgs& a, int token, int n,
 // writes bf16.  One thread per 4 consecutive output columns of one row, so the whole GPU takes
 // part and every thread has `splits` independent 16-byte loads in flight.
 __global__ void qmm_finish_kernel(QmmArgs a, int splits) {
+  after_previous();
   const int n4 = a.nt * (kTileN / 4);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)a.rows * n4) return;
@@ -189,6 +191,7 @@ __global__ void qmm_finish_kernel(QmmArgs a, int splits) {
 // it has just written forms the row's mean square and writes rmsnorm(y) * weight: one launch and one
 // pass over y less per projection.  N <= 4 * 4 * blockDim (each thread keeps up to 4 quads).
 __global__ void __launch_bounds__(1024) qmm_finish_rmsnorm_kernel(QmmArgs a, int splits) {
+  after_previous();
   __shared__ float s_part[32];
   const int token = blockIdx.x, n4 = a.n / 4;
   const int tts = (a.rows + a.tn - 1) / a.tn, tt = token / a.tn, t = token - tt * a.tn;
@@ -254,6 +257,7 @@ __global__ void __launch_bounds__(1024) qmm_finish_rmsnorm_kernel(QmmArgs a, int
 // ---- GEMV kernel ---------------------------------------------------------------------------------
 template <int MODE, int TT>
 __global__ void __launch_bounds__(kTileN) qmm_simt_kernel(QmmArgs a) {
+  after_previous();
   __shared__ __align__(16) float xs[TT][kChunkK];
   const int nt = blockIdx.x, split = blockIdx.y, tt = blockIdx.z;
   const int r = threadIdx.x, t0 = tt * TT;
@@ -375,6 +379,7 @@ constexpr int kPrefetchAhead = 12;  // weight blocks requested into L2 ahead of 
 
 template <int MODE>
 __global__ void __launch_bounds__(kTcThreads, 2) qmm_tc_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
+  after_previous();
   extern __shared__ unsigned char smem_raw[];
   // 1024-byte alignment: the 128B swizzle pattern is a function of the shared-memory address.
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -552,6 +557,7 @@ constexpr int kTcaMaxWeightSlots = 24;
 
 template <int MODE>
 __global__ void __launch_bounds__(kTcaThreads, 2) qmm_tca_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
+  after_previous();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   constexpr int BB = block_bytes(MODE);
@@ -785,6 +791,7 @@ __host__ __device__ constexpr int tc2_x_rows(bool grouped, int tn) { return grou
 // dequantisation runs.  Dense bf16 blocks land in the stage's MMA tiles directly (SR = stages there).
 template <int MODE>
 __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
+  after_previous();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   constexpr int BB = block_bytes(MODE);
@@ -1112,6 +1119,7 @@ __device__ __forceinline__ uint32_t operand_pair(uint32_t word, int i, __nv_bflo
 
 template <int MODE, int NT8>
 __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma_kernel(QmmArgs a) {
+  after_previous();
   extern __shared__ __align__(128) unsigned char gsm[];
   const int stages = a.stages;
   constexpr int kSlotBytes = 2 * kRawStride;  // a ring slot holds the blocks of two adjacent weight tiles
@@ -1323,6 +1331,7 @@ constexpr int kFewRows = 16, kFewWarps = 8;
 
 template <int MT, int NT>
 __global__ void __launch_bounds__(kFewWarps * 32) qmm_few_kernel(QmmArgs a) {
+  after_previous();
   constexpr int R = MT * 16, TOK = NT * 8, U = 2 / MT;
   __shared__ float red[kFewWarps][TOK][R + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -1451,6 +1460,7 @@ __host__ __device__ constexpr int slab8_stride(int chunks) { return (chunks * kC
 
 template <int NT8>
 __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma8_kernel(QmmArgs a) {
+  after_previous();
   extern __shared__ __align__(128) unsigned char gsm[];
   const int stages = a.stages;
   constexpr int kSlotBytes = 2 * kRawStride;
@@ -1692,6 +1702,7 @@ __global__ void __launch_bounds__(256) mx_split_activations_kernel(const __nv_bf
                                                                    unsigned char* __restrict__ hi, unsigned char* __restrict__ lo,
                                                                    float* __restrict__ unscale, const int* __restrict__ gather,
                                                                    int gather_div, const int* __restrict__ rows_valid) {
+  after_previous();
   __shared__ float s_max[8];
   const int row = blockIdx.x;
   if (rows_valid && row >= *rows_valid) return;  // capacity beyond the rows that exist: nothing to read
@@ -1736,6 +1747,7 @@ __global__ void __launch_bounds__(256) mx_split_activations_kernel(const __nv_bf
 // Tile-major blocks -> row-major codes + scale atoms (see b200_qweight).  One thread per 32-bit word of a plane.
 __global__ void mx_from_blocks_kernel(const unsigned char* __restrict__ blocks, unsigned char* __restrict__ codes,
                                       unsigned char* __restrict__ sf, int nt_total, int kc, int k) {
+  after_previous();
   constexpr int BB = block_bytes(B200_Q_MXFP4_G32);
   const size_t n_words = (size_t)nt_total * kc * 2 * kTileN * 4;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_words; i += (size_t)gridDim.x * blockDim.x) {
@@ -1798,6 +1810,7 @@ struct MxActMaps {
 
 __global__ void __launch_bounds__(kMxThreads, 1)
     qmm_mx_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ MxActMaps amaps, QmmArgs a) {
+  after_previous();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int tn = a.tn, P = a.stages;
@@ -1987,6 +2000,7 @@ constexpr int kMxpStageTokens = 16;
 
 __global__ void __launch_bounds__(kMxpThreads, 1)
     qmm_mxp_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ MxActMaps amaps, QmmArgs a) {
+  after_previous();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int tn = a.tn, P = a.stages;
@@ -2364,6 +2378,7 @@ __device__ __forceinline__ uint32_t mix32(uint32_t x) {
 // Fills blocks with pseudo-random codes and plausible scales: affine weights land in about
 // [-0.04, 0.035], MXFP4 scales are 2^-6, dense weights are small bf16 values.
 __global__ void random_blocks_kernel(unsigned char* blocks, size_t n_blocks, int mode, uint32_t seed) {
+  after_previous();
   const int bb = block_bytes(mode);
   const size_t words = n_blocks * (size_t)(bb / 4);
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (size_t)gridDim.x * blockDim.x) {
@@ -2471,13 +2486,13 @@ static b200_status launch_finish(QmmArgs& a, int splits, cudaStream_t s) {
   if (a.norm_w && a.rows <= 256 && a.epilogue == B200_EPI_RESIDUAL && !a.items && !a.row_scales && a.n % 4 == 0 && a.n <= 16384) {
     int threads = ((a.n / 4 + 31) / 32) * 32;
     while (threads > 1024) threads = (((threads + 1) / 2 + 31) / 32) * 32;
-    qmm_finish_rmsnorm_kernel<<<a.rows, threads, 0, s>>>(a, splits);
+    launch_after(qmm_finish_rmsnorm_kernel, a.rows, threads, 0, s, a, splits);
     B200_LAUNCH_CHECK();
     a.did_norm = 1;
     return B200_OK;
   }
   const long long threads = (long long)a.rows * a.nt * (kTileN / 4);
-  qmm_finish_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(a, splits);
+  launch_after(qmm_finish_kernel, (unsigned)((threads + 255) / 256), 256, 0, s, a, splits);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -2496,7 +2511,7 @@ static b200_status launch_simt(QmmArgs& a, int rows, cudaStream_t s) {
   st = ensure_state((size_t)splits * (size_t)tts * TT * a.nt * kTileN * sizeof(float));
   if (st != B200_OK) return st;
   a.ws = g_ws[g_place]; a.err = g_err;
-  qmm_simt_kernel<MODE, TT><<<dim3(a.nt, splits, tts), kTileN, 0, s>>>(a);
+  launch_after(qmm_simt_kernel<MODE, TT>, dim3(a.nt, splits, tts), kTileN, 0, s, a);
   B200_LAUNCH_CHECK();
   return launch_finish(a, splits, s);
 }
@@ -2547,7 +2562,7 @@ static b200_status launch_tc(QmmArgs& a, int rows, cudaStream_t s, int x_stride 
   st = make_x_map(&xmap, a.x, rows, x_stride > 0 ? x_stride : a.k, tn);
   if (st != B200_OK) return st;
   a.x_row0 = 0;
-  qmm_tc_kernel<MODE><<<dim3(a.nt, splits, a.items ? a.max_items : tts * std::max(a.groups, 1)), kTcThreads, smem, s>>>(xmap, a);
+  launch_after(qmm_tc_kernel<MODE>, dim3(a.nt, splits, a.items ? a.max_items : tts * std::max(a.groups, 1)), kTcThreads, smem, s, xmap, a);
   B200_LAUNCH_CHECK();
   if (grouped_bf16) return B200_OK;
   return (splits == 1 && tn <= 64 && !a.keep_f32) ? B200_OK : launch_finish(a, splits, s);  // a single small split writes its output itself
@@ -2607,7 +2622,7 @@ static b200_status launch_tca(QmmArgs& a, int rows, cudaStream_t s) {
   st = make_x_map(&xmap, a.x, rows, a.k, tn);
   if (st != B200_OK) return st;
   a.x_row0 = 0;
-  qmm_tca_kernel<MODE><<<dim3(a.nt, splits, a.items ? a.max_items : tts), kTcaThreads, smem, s>>>(xmap, a);
+  launch_after(qmm_tca_kernel<MODE>, dim3(a.nt, splits, a.items ? a.max_items : tts), kTcaThreads, smem, s, xmap, a);
   B200_LAUNCH_CHECK();
   return direct ? B200_OK : launch_finish(a, splits, s);
 }
@@ -2683,7 +2698,7 @@ static b200_status launch_mx(const b200_qweight* w, QmmArgs& a, int rows, cudaSt
   unsigned char* hi = g_mx_act;
   unsigned char* lo = hi + (size_t)rows * a.k;
   float* unscale = reinterpret_cast<float*>(lo + (((size_t)rows * a.k + 255) / 256) * 256);
-  mx_split_activations_kernel<<<rows, 256, 0, s>>>(a.x, a.k, hi, lo, unscale, a.x_gather, a.x_gather_div, a.rows_valid);
+  launch_after(mx_split_activations_kernel, rows, 256, 0, s, a.x, a.k, hi, lo, unscale, a.x_gather, a.x_gather_div, a.rows_valid);
   B200_LAUNCH_CHECK();
   MxActMaps amaps;
   std::memset(&amaps, 0, sizeof(amaps));
@@ -2739,7 +2754,7 @@ static b200_status launch_mx(const b200_qweight* w, QmmArgs& a, int rows, cudaSt
     }
     const long long n_work = a.items ? (long long)pairs * a.max_items : (long long)pairs * tts * real_splits;
     const int grid = (int)std::max<long long>(1, std::min<long long>(g_sms, n_work));
-    qmm_mxp_kernel<<<grid, kMxpThreads, smem, s>>>(*reinterpret_cast<const CUtensorMap*>(w->mx_map), amaps, a);
+    launch_after(qmm_mxp_kernel, grid, kMxpThreads, smem, s, *reinterpret_cast<const CUtensorMap*>(w->mx_map), amaps, a);
     B200_LAUNCH_CHECK();
     return real_splits > 1 ? launch_finish(a, real_splits, s) : B200_OK;
   }
@@ -2748,7 +2763,7 @@ static b200_status launch_mx(const b200_qweight* w, QmmArgs& a, int rows, cudaSt
   a.stages = std::min(a.stages, std::max(2, a.k / kMxK));
   const size_t smem = (size_t)a.stages * stage + fixed;
   if ((int)smem > smem_budget) { b200_set_error("block-scaled path: %zu bytes of shared memory needed, %d available", smem, smem_budget); return B200_ERR_CAPACITY; }
-  qmm_mx_kernel<<<dim3((a.nt + 1) / 2, 1, a.items ? a.max_items : tts), kMxThreads, smem, s>>>(
+  launch_after(qmm_mx_kernel, dim3((a.nt + 1) / 2, 1, a.items ? a.max_items : tts), kMxThreads, smem, s,
       *reinterpret_cast<const CUtensorMap*>(w->mx_map), amaps, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
@@ -2799,7 +2814,7 @@ static b200_status launch_tc2(QmmArgs& a, int rows, cudaStream_t s) {
   st = make_x_map(&xmap, a.x, rows, a.k, a.items ? kGroupBox : tn);
   if (st != B200_OK) return st;
   a.x_row0 = 0;
-  qmm_tc2_kernel<MODE><<<dim3(pairs, splits, tts), kTc2Threads, smem, s>>>(xmap, a);
+  launch_after(qmm_tc2_kernel<MODE>, dim3(pairs, splits, tts), kTc2Threads, smem, s, xmap, a);
   B200_LAUNCH_CHECK();
   return splits == 1 && !a.keep_f32 ? B200_OK : launch_finish(a, splits, s);
 }
@@ -2844,7 +2859,7 @@ static b200_status launch_mma_nt(QmmArgs& a, int rows, cudaStream_t s) {
                                        (int)(base_smem + 48 * 1024)));
     configured = true;
   }
-  qmm_mma_kernel<MODE, NT8><<<dim3(best_groups * splits, tts), kGemvThreads, smem, s>>>(a);
+  launch_after(qmm_mma_kernel<MODE, NT8>, dim3(best_groups * splits, tts), kGemvThreads, smem, s, a);
   B200_LAUNCH_CHECK();
   return launch_finish(a, splits, s);
 }
@@ -2872,11 +2887,11 @@ static b200_status launch_few(QmmArgs& a, int rows, cudaStream_t s) {
   const bool wide = (long long)((a.n + 31) / 32) * z >= 2 * g_sms;
   const dim3 grid((a.n + (wide ? 31 : 15)) / (wide ? 32 : 16), 1, z);
   if (rows <= 8) {
-    if (wide) qmm_few_kernel<2, 1><<<grid, kFewWarps * 32, 0, s>>>(a);
-    else qmm_few_kernel<1, 1><<<grid, kFewWarps * 32, 0, s>>>(a);
+    if (wide) launch_after(qmm_few_kernel<2, 1>, grid, kFewWarps * 32, 0, s, a);
+    else launch_after(qmm_few_kernel<1, 1>, grid, kFewWarps * 32, 0, s, a);
   } else {
-    if (wide) qmm_few_kernel<2, 2><<<grid, kFewWarps * 32, 0, s>>>(a);
-    else qmm_few_kernel<1, 2><<<grid, kFewWarps * 32, 0, s>>>(a);
+    if (wide) launch_after(qmm_few_kernel<2, 2>, grid, kFewWarps * 32, 0, s, a);
+    else launch_after(qmm_few_kernel<1, 2>, grid, kFewWarps * 32, 0, s, a);
   }
   B200_LAUNCH_CHECK();
   return a.keep_f32 ? launch_finish(a, 1, s) : B200_OK;
@@ -2921,7 +2936,7 @@ static b200_status launch_mma8_nt(QmmArgs& a, int rows, cudaStream_t s) {
     B200_CUDA_TRY(cudaFuncSetAttribute(qmm_mma8_kernel<NT8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(base_smem + 48 * 1024)));
     configured = true;
   }
-  qmm_mma8_kernel<NT8><<<dim3(best_groups * splits, tts), kGemvThreads, smem, s>>>(a);
+  launch_after(qmm_mma8_kernel<NT8>, dim3(best_groups * splits, tts), kGemvThreads, smem, s, a);
   B200_LAUNCH_CHECK();
   return launch_finish(a, splits, s);
 }
@@ -3114,6 +3129,7 @@ struct F32Args {
 };
 
 __global__ void __launch_bounds__(256) qmm_f32_kernel(F32Args a) {
+  after_previous();
   __shared__ float xs[kF32K][kF32Rows + 4];
   __shared__ float ws[kF32K][kTileN + 4];
   const int nt = blockIdx.x, tid = threadIdx.x, kc = a.kc, n_valid = a.n_valid, y_stride = a.y_stride;
@@ -3207,7 +3223,7 @@ b200_status b200_qmm_f32_shaped(const b200_qweight* w, const float* d_x, int32_t
   a.blocks = w->d_blocks; a.x = d_x; a.y = d_y; a.rows = rows; a.kc = w->kc; a.x_stride = w->k; a.y_stride = y_stride; a.n_valid = n_valid;
   a.epilogue = epilogue;
   a.shape = shape;
-  qmm_f32_kernel<<<dim3(w->nt, (rows + kF32Rows - 1) / kF32Rows), 256, 0, (cudaStream_t)stream>>>(a);
+  launch_after(qmm_f32_kernel, dim3(w->nt, (rows + kF32Rows - 1) / kF32Rows), 256, 0, (cudaStream_t)stream, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -3226,7 +3242,7 @@ b200_status b200_qmm_f32_blocks(const b200_qweight* w, const float* d_x, int32_t
   F32Args a{};
   a.blocks = w->d_blocks; a.x = d_x; a.y = d_y; a.rows = rows; a.kc = w->kc; a.x_stride = x_stride; a.y_stride = y_stride; a.n_valid = w->n;
   a.expert_stride = (size_t)w->nt * w->kc * w->block_bytes; a.x_group = x_group; a.y_group = y_group;
-  qmm_f32_kernel<<<dim3(w->nt, (rows + kF32Rows - 1) / kF32Rows, w->n_experts), 256, 0, (cudaStream_t)stream>>>(a);
+  launch_after(qmm_f32_kernel, dim3(w->nt, (rows + kF32Rows - 1) / kF32Rows, w->n_experts), 256, 0, (cudaStream_t)stream, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -3242,7 +3258,7 @@ b200_status b200_qmm_f32_grouped(const b200_qweight* w, const float* d_x, const 
   a.blocks = w->d_blocks; a.x = d_x; a.y = d_y; a.kc = w->kc; a.x_stride = w->k; a.y_stride = y_stride; a.n_valid = swiglu ? w->n / 2 : w->n;
   a.epilogue = epilogue; a.expert_stride = (size_t)w->nt * w->kc * w->block_bytes;
   a.items = d_items; a.n_items = d_n_items; a.order = d_order; a.order_div = order_div > 0 ? order_div : 1;
-  qmm_f32_kernel<<<dim3(w->nt, max_items), 256, 0, (cudaStream_t)stream>>>(a);
+  launch_after(qmm_f32_kernel, dim3(w->nt, max_items), 256, 0, (cudaStream_t)stream, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -3358,6 +3374,7 @@ namespace {
 // out, the thread records that in the error word exactly as the matmul kernels do, and the kernel
 // returns.  Nothing faults or spins for ever; the context stays usable.
 __global__ void wait_runs_out_kernel(int* err, uint32_t polls) {
+  after_previous();
   __shared__ uint64_t bar;
   if (threadIdx.x == 0) {
     ptx::mbar_init(&bar, 1);
@@ -3462,7 +3479,7 @@ b200_status launch_tc_static(QmmArgs& a, int rows, int dev, cudaStream_t s) {
   b200_status st = make_x_map(&xmap, a.x, rows, a.k, tn);
   if (st != B200_OK) return st;
   a.x_row0 = 0;
-  qmm_tc_kernel<MODE><<<dim3(a.nt, splits, tts), kTcThreads, smem, s>>>(xmap, a);
+  launch_after(qmm_tc_kernel<MODE>, dim3(a.nt, splits, tts), kTcThreads, smem, s, xmap, a);
   B200_LAUNCH_CHECK();
   return (splits == 1 && tn <= 64 && !a.keep_f32) ? B200_OK : launch_finish(a, splits, s);
 }

@@ -28,6 +28,7 @@
 #include <algorithm>
 
 #include "common.h"
+#include "launch.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -707,6 +708,7 @@ __global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(const T* __res
                                                                   const uint32_t* __restrict__ ctx, const int* __restrict__ ctx_off,
                                                                   float* __restrict__ scratch, uint32_t* __restrict__ tokens,
                                                                   float* __restrict__ logprobs) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char sample_dyn[];
   Shared& s = *reinterpret_cast<Shared*>(sample_dyn);
   cg::cluster_group cluster = cg::this_cluster();
@@ -755,12 +757,14 @@ b200_status launch(const T* logits, int rows, int vocab, const b200_sample_param
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = sizeof(Shared);
   cfg.stream = s;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = ranks;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ranks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (as launch_after)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
   B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, sample_rows_kernel<T>, logits, vocab, params, ctx, ctx_off, scratch, tokens, logprobs));
   B200_LAUNCH_CHECK();
   return B200_OK;
