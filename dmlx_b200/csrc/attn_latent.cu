@@ -231,7 +231,7 @@ struct LatentShared {
 template <int NR>
 __global__ void __launch_bounds__(kLatentThreads, 1)
     latent_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap qmap, LatentArgs la) {
-  after_previous();
+  wait_previous();
   const WinArgs& a = la.w;
   extern __shared__ unsigned char latent_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(latent_dyn) + 1023) & ~(uintptr_t)1023);

@@ -376,7 +376,7 @@ __device__ __noinline__ Row partly_seen_block(uint32_t t_s, uint32_t t_o, int se
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
     prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ Args a) {
-  after_previous();
+  wait_previous();
   using Z = Shape<D>;
   extern __shared__ __align__(1024) unsigned char smem[];  // (there is no room for a base that has to be rounded up)
   unsigned char* qbuf = smem;                        // [tile][box][128 rows][128 B]

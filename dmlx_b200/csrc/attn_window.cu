@@ -263,7 +263,7 @@ constexpr int most_warps(int kb, int vb) { return kb + vb == 2 ? 12 : (kb + vb =
 template <int KB, int VB, bool TABLE>
 __global__ void __launch_bounds__(most_warps(KB, VB) * 32, 1)
     window_attn_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, WinArgs a) {
-  after_previous();
+  wait_previous();
   constexpr int KS = KB * 4;  // 16-column steps of Q K^T
   constexpr int NO = VB * 8;  // 8-column tiles of the output
   const int n_kb = (a.L.kd + 63) / 64, n_vb = (a.L.vd + 63) / 64, n_ks = a.L.kd / 16, n_vs = a.L.vd / 16;

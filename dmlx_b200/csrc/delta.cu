@@ -276,7 +276,7 @@ __device__ __forceinline__ float dot16(const float* x, int dx, const float* y, i
 }
 
 __global__ void __launch_bounds__(256, 3) delta_chunk_kernel(Delta a) {
-  after_previous();
+  wait_previous();
   extern __shared__ __align__(16) float sh[];
   __shared__ float s_L[kC], s_beta[kC];
   const int chunk = blockIdx.x, head = blockIdx.y;

@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(256) gla_chunk_kernel(Gla a) {
 // delta_chunk_kernel (delta.cu); u is f32 and enters the tensor cores as two terms.
 template <int NT, bool DELTA>  // NT: 8-channel tiles of the state a warp holds
 __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
-  after_previous();
+  wait_previous();
   extern __shared__ unsigned char scan_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(scan_dyn) + 127) & ~(uintptr_t)127);
   const int req = blockIdx.x, head = blockIdx.y, slice = blockIdx.z;

@@ -2,10 +2,10 @@
 //
 // A step is a chain of dozens of kernels of a few microseconds.  Launched plainly, each waits until the one before has drained and its
 // writes are flushed, and only then are its blocks scheduled.  With this attribute a kernel's blocks are scheduled as soon as every block of
-// the kernel before has passed `after_previous` and there is room; they set up what needs no memory and wait inside `after_previous`.
+// the kernel before has passed `let_next_start` and there is room; they set up what needs no memory and wait.
 //
-// Every kernel that is launched through `launch_after` runs `after_previous` in all of its threads, before any return and before it reads or
-// writes global memory or allocates tensor memory.  So the bodies of two kernels of a stream never overlap, and as a kernel ends only after its
+// In every kernel that is launched through `launch_after`, each thread that reads or writes global memory (weights apart, which nothing writes
+// after their creation) or allocates tensor memory runs `wait_previous` before it does, and so does some thread of every block before it ends.  So the bodies of two kernels of a stream never overlap, and as a kernel ends only after its
 // own wait did, the wait of the next one covers all that came before.
 #pragma once
 #include <cuda_runtime.h>
@@ -13,10 +13,16 @@
 #include <utility>
 
 #ifdef __CUDACC__
-// Waits until the kernels before this one in the stream have ended and their writes are visible, then lets the next one be scheduled.
+// Waits until the kernels before this one in the stream have ended and their writes are visible.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel be scheduled once every block has come here (one thread of a block is enough) or ended.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Both.  For kernels of a few microseconds, or of many blocks per SM.  Blocks that wait take issue slots from those that work, so one long wave
+// waits alone and lets the next kernel start when its main loop is done (the block-scaled matmul of 24576 expert rows: 372 us with 54 waiting
+// warps on every SM, 334 without).
 __device__ __forceinline__ void after_previous() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  wait_previous();
+  let_next_start();
 }
 
 // kernel<<<grid, block, smem, s>>>(args...); a failure is left for cudaGetLastError.

@@ -198,7 +198,7 @@ __device__ __forceinline__ void load_row(const unsigned char* tile, int tok, int
 
 template <int D, bool FP8>
 __global__ void __launch_bounds__(kAttnThreads, 3) paged_attn_kernel(AttnArgs a) {
-  after_previous();
+  wait_previous();
   constexpr int ELEM = FP8 ? 1 : 2;
   constexpr int TILE = 32 * D * ELEM;  // bytes of one (page, kv head) K or V tile
   constexpr int VEC = D / 16;          // dims per lane
@@ -481,7 +481,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 template <int D>
 __global__ void __launch_bounds__(kMmaWarps * 32, 1)
     paged_attn_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, AttnArgs a) {
-  after_previous();
+  wait_previous();
   constexpr int BOXES = D / 64;     // 128-byte wide TMA boxes per tile
   constexpr int TILE = 32 * D * 2;  // bytes of one K or V tile
   constexpr int KS = D / 16;        // k-steps of Q K^T
@@ -643,6 +643,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 1)
       if (t == 0) { a.part_ml[pidx * 2] = m_run; a.part_ml[pidx * 2 + 1] = l_run; }
     }
   }
+  let_next_start();
   if (!alive && lane == 0) atomicExch(a.d.state + ST_ATTN_ERR, B200_ERR_DEVICE_FLAGGED);
 }
 
@@ -679,7 +680,7 @@ __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
 template <int STAGES, int MINB>
 __global__ void __launch_bounds__(kMmaWarps * 32, MINB)
     paged_attn_mma_fp8_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, AttnArgs a) {
-  after_previous();
+  wait_previous();
   constexpr int D = 128;
   constexpr int TILE = 32 * D;  // bytes of one K or V tile
   constexpr int KS = D / 16;    // k-steps of Q K^T = 16-byte chunks of a row
@@ -863,6 +864,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, MINB)
       if (t == 0) { a.part_ml[pidx * 2] = m_run; a.part_ml[pidx * 2 + 1] = l_run; }
     }
   }
+  let_next_start();
   if (!alive && lane == 0) atomicExch(a.d.state + ST_ATTN_ERR, B200_ERR_DEVICE_FLAGGED);
 }
 
@@ -995,7 +997,7 @@ __device__ __forceinline__ void mma_bf16_16816_full(float (&d)[4], uint32_t a0, 
 template <int D>
 __global__ void __launch_bounds__(kMmaWarps * 32, 1)
     paged_attn_prefill_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, AttnArgs a) {
-  after_previous();
+  wait_previous();
   constexpr int BOXES = D / 64;
   constexpr int TILE = 32 * D * 2;
   constexpr int KS = D / 16;
@@ -1199,6 +1201,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 1)
       if (t == 0) { a.part_ml[pidx * 2] = mB; a.part_ml[pidx * 2 + 1] = lB; }
     }
   }
+  let_next_start();
   if (!alive && lane == 0) atomicExch(a.d.state + ST_ATTN_ERR, B200_ERR_DEVICE_FLAGGED);
 }
 
@@ -1213,7 +1216,7 @@ __device__ __forceinline__ void mma_f16_16816_full(float (&d)[4], uint32_t a0, u
 // slots permuted to match ldmatrix on byte tiles, K scale on the scores, relative V scale on P).
 __global__ void __launch_bounds__(kMmaWarps * 32, 1)
     paged_attn_prefill_fp8_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, AttnArgs a) {
-  after_previous();
+  wait_previous();
   constexpr int D = 128, TILE = 32 * D, KS = D / 16, NO = D / 8, STAGES = kMmaStages;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -1451,6 +1454,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 1)
       if (t == 0) { a.part_ml[pidx * 2] = mB; a.part_ml[pidx * 2 + 1] = lB; }
     }
   }
+  let_next_start();
   if (!alive && lane == 0) atomicExch(a.d.state + ST_ATTN_ERR, B200_ERR_DEVICE_FLAGGED);
 }
 

@@ -63,17 +63,19 @@ __device__ __forceinline__ uint4 dequant_word(uint32_t word, __nv_bfloat162 s2, 
   uint32_t out[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const uint32_t t = (word >> (4 * i)) & 0x000F000Fu;
     __nv_bfloat162 r;
     if (MODE == B200_Q_AFFINE4_G64) {
-      // 0x4300 | q is the bf16 128+q; subtracting 128 leaves q exactly, then one fused q*s+b.
-      uint32_t u = t | 0x43004300u;
+      // 0x4300 | q is the bf16 128+q; subtracting 128 leaves q exactly, then one fused q*s+b.  (And-or as one instruction: written apart, the
+      // compiler issues two, 32 more of some 300 a warp for two chunks.)
       const uint32_t c128 = 0x43004300u;
+      uint32_t u;
+      asm("lop3.b32 %0, %1, 0x000F000F, %2, 0xEA;" : "=r"(u) : "r"(word >> (4 * i)), "r"(c128));
       __nv_bfloat162 q = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&u), *reinterpret_cast<const __nv_bfloat162*>(&c128));
       r = __hfma2(q, s2, b2);
     } else {
       // sign | (e,m) << 6 is the E2M1 value times 2^-126 (exact, subnormals included); two exact
       // power-of-two multiplies bring it to value * 2^(scale-127).
+      const uint32_t t = (word >> (4 * i)) & 0x000F000Fu;
       uint32_t u = ((t & 0x00080008u) << 12) | ((t & 0x00070007u) << 6);
       const uint32_t c64 = 0x5F805F80u;  // 2^64
       r = __hmul2(__hmul2(*reinterpret_cast<__nv_bfloat162*>(&u), *reinterpret_cast<const __nv_bfloat162*>(&c64)), s2);
@@ -379,7 +381,7 @@ constexpr int kPrefetchAhead = 12;  // weight blocks requested into L2 ahead of 
 
 template <int MODE>
 __global__ void __launch_bounds__(kTcThreads, 2) qmm_tc_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
-  after_previous();
+  wait_previous();
   extern __shared__ unsigned char smem_raw[];
   // 1024-byte alignment: the 128B swizzle pattern is a function of the shared-memory address.
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -481,6 +483,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) qmm_tc_kernel(const __grid_cons
         ptx::umma_commit(&mma_done[s]);
       }
       if (ok) ptx::umma_commit(accum_ready);
+      let_next_start();
     }
   } else {
     // ---- dequantise: thread (r, plane) owns one 32-column half of weight row r ----
@@ -557,7 +560,7 @@ constexpr int kTcaMaxWeightSlots = 24;
 
 template <int MODE>
 __global__ void __launch_bounds__(kTcaThreads, 2) qmm_tca_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
-  after_previous();
+  wait_previous();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   constexpr int BB = block_bytes(MODE);
@@ -680,6 +683,7 @@ __global__ void __launch_bounds__(kTcaThreads, 2) qmm_tca_kernel(const __grid_co
         if (++q == Q) { q = 0; qh ^= 1u; }
       }
       if (ok) ptx::umma_commit(accum_ready);
+      let_next_start();
     }
   } else {
     // ---- dequantise: thread (r, plane) owns one 32-column half of weight row r = tensor-memory lane r ----
@@ -778,10 +782,138 @@ __global__ void __launch_bounds__(kTcaThreads, 2) qmm_tca_kernel(const __grid_co
 // the latency and the L2 -> SM activation traffic per flop halves.  16 dequant warps (one thread
 // per weight row and 32-column plane of either tile), one loader warp, one MMA warp.
 constexpr int kTc2Threads = 19 * 32;  // warps 0-15 dequantise, 16 streams the weights, 17 issues MMAs, 18 loads activation tiles
-constexpr int kTc2DequantThreads = 16 * 32;
+constexpr int kPairThreads = 16 * 32;  // the dequantising warps
 constexpr int kGroupBox = 64;  // rows of expert-sorted activations per copy
 // Rows that a stage's activation tile has room for: a work item's arrive in whole copies, so its tile is as many of them as cover tn.
 __host__ __device__ constexpr int tc2_x_rows(bool grouped, int tn) { return grouped ? (tn + kGroupBox - 1) / kGroupBox * kGroupBox : tn; }
+
+// Accumulators of a pair of weight tiles (tensor memory: tile 0 at column 0, tile 1 at `acc_stride`) to the output or to f32 partial tiles; the
+// calling CTA's first 16 warps, all of them.  Warp w reads lanes 32*(w%4); warps 4g..4g+3 take tile g/2, column half g%2.  `smem`: the idle
+// stage buffers, 512 bytes per row.
+__device__ __forceinline__ void pair_epilogue(const QmmArgs& a, unsigned char* smem, uint32_t tmem_base, uint32_t acc_stride, bool ok, int rows_here,
+                                              int tn_here, int t0, int nt0, int n_tiles, int tt, int split) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tn = a.tn;
+  const int grp = warp >> 2, etile = grp >> 1, half = grp & 1;
+  // SwiGLU written by this kernel (no K split): the outputs go through the idle stage buffers as
+  // bf16 [token][tile][64] and leave as 16-byte stores, 256 contiguous bytes per token for the tile
+  // pair.  Stores of 64 bytes per token straight from the accumulator layout (one instruction per
+  // token and warp) took a quarter of the kernel's time at 256 rows.
+  const bool staged = gridDim.y == 1 && !a.keep_f32 && a.epilogue == B200_EPI_SWIGLU && a.n % 16 == 0 && a.out_stride(a.n / 2) % 8 == 0 &&
+                      ((uintptr_t)a.y & 15) == 0;
+  if (staged) {
+    uint32_t all_ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, 1, 512, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all_ok)
+        : "r"((uint32_t)ok)
+        : "memory");
+    if (all_ok) {
+      ptx::tc_fence_after_sync();
+      __nv_bfloat16* stage_h = reinterpret_cast<__nv_bfloat16*>(smem);
+      if (etile < n_tiles) {
+        const int lq = warp & 3;
+        const int ch = ((tn_here / 2 + 31) / 32) * 32;
+        const int c_end = min(rows_here, (half + 1) * ch);
+        for (int c0 = half * ch; c0 < c_end; c0 += 32) {
+          uint32_t v[32];
+          ptx::tmem_ld32(tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(etile * acc_stride + c0), v);
+          const float rs_mine = c0 + lane < rows_here ? a.row_scale(t0 + c0 + lane) : 0.f;
+          ptx::tmem_ld_wait();
+          // lanes 2i / 2i+1 hold gate_i / up_i of every token: the even lane takes token j, the odd
+          // lane token j+1, one exchange per token pair and no idle lanes in the arithmetic
+          const bool odd = lane & 1;
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float a0 = __uint_as_float(v[j]), a1 = __uint_as_float(v[j + 1]);
+            const float got = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
+            const float rs = __shfl_sync(0xffffffffu, rs_mine, j + (int)odd);
+            stage_h[((size_t)(c0 + j + (int)odd) * 2 + etile) * 64 + lq * 16 + (lane >> 1)] =
+                __float2bfloat16(gated(a, odd ? got : a0, odd ? a1 : got) * rs);
+          }
+        }
+      }
+      asm volatile("bar.sync 1, 512;" ::: "memory");
+      const int n_out = a.n / 2;
+      for (int idx = tid; idx < rows_here * 16; idx += kPairThreads) {
+        const int tok = idx >> 4, c16 = idx & 15, tile = c16 >> 3;
+        const int col = (nt0 + tile) * 64 + (c16 & 7) * 8;
+        if (tile < n_tiles && col < n_out)
+          *reinterpret_cast<uint4*>(a.y + (size_t)(t0 + tok) * a.out_stride(n_out) + col) = *reinterpret_cast<const uint4*>(stage_h + (size_t)idx * 8);
+      }
+    }
+  } else if (gridDim.y == 1 && !a.keep_f32 && a.epilogue != B200_EPI_SWIGLU && a.n % 8 == 0 && a.out_stride(a.n) % 8 == 0 &&
+             (((uintptr_t)a.y | (uintptr_t)a.residual) & 15) == 0) {
+    // The other epilogues written by this kernel, likewise through the idle stage buffers: bf16 [token][256 columns of the pair].  The
+    // residual is brought in first, 16 bytes at a time, and the sums replace it in place (o at 2105 rows of 4096 x 4096: 124 us with
+    // a 2-byte residual load ahead of each 2-byte store, 70 this way).
+    uint32_t all_ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, 1, 512, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all_ok)
+        : "r"((uint32_t)ok)
+        : "memory");
+    if (all_ok) {
+      ptx::tc_fence_after_sync();
+      __nv_bfloat16* stage_h = reinterpret_cast<__nv_bfloat16*>(smem);
+      const size_t stride = a.out_stride(a.n), o0 = (size_t)t0 * stride + nt0 * kTileN;
+      const int cols = min(a.n - nt0 * kTileN, 2 * kTileN);
+      const bool add = a.epilogue == B200_EPI_RESIDUAL;
+      if (add) {
+        for (int idx = tid; idx < rows_here * 32; idx += kPairThreads)
+          if ((idx & 31) * 8 < cols)
+            *reinterpret_cast<uint4*>(stage_h + (size_t)idx * 8) = *reinterpret_cast<const uint4*>(a.residual + o0 + (size_t)(idx >> 5) * stride + (idx & 31) * 8);
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+      }
+      if (etile < n_tiles) {
+        const int lq = warp & 3;
+        const int ch = ((tn_here / 2 + 31) / 32) * 32;
+        const int c_end = min(rows_here, (half + 1) * ch);
+        for (int c0 = half * ch; c0 < c_end; c0 += 32) {
+          uint32_t v[32];
+          ptx::tmem_ld32(tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(etile * acc_stride + c0), v);
+          const float rs_mine = c0 + lane < rows_here ? a.row_scale(t0 + c0 + lane) : 0.f;
+          ptx::tmem_ld_wait();
+          __nv_bfloat16* mine = stage_h + (size_t)c0 * 256 + etile * kTileN + lq * 32 + lane;
+          const int left = rows_here - c0;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const float rs = __shfl_sync(0xffffffffu, rs_mine, j);
+            if (j < left) {
+              float acc = __uint_as_float(v[j]);
+              if (add) acc += __bfloat162float(mine[j * 256]);
+              else acc = activate(a.epilogue, acc);
+              mine[j * 256] = __float2bfloat16(acc * rs);
+            }
+          }
+        }
+      }
+      asm volatile("bar.sync 1, 512;" ::: "memory");
+      for (int idx = tid; idx < rows_here * 32; idx += kPairThreads)
+        if ((idx & 31) * 8 < cols)
+          *reinterpret_cast<uint4*>(a.y + o0 + (size_t)(idx >> 5) * stride + (idx & 31) * 8) = *reinterpret_cast<const uint4*>(stage_h + (size_t)idx * 8);
+    }
+  } else if (ok && etile < n_tiles) {
+    ptx::tc_fence_after_sync();
+    const int lq = warp & 3;
+    const int nt = nt0 + etile, n = nt * kTileN + lq * 32 + lane;
+    const bool direct = gridDim.y == 1 && !a.keep_f32;
+    float* wsp = a.ws + (((size_t)(nt * gridDim.z + tt) * gridDim.y + split) * tn) * kTileN + lq * 32 + lane;
+    const int ch = ((tn_here / 2 + 31) / 32) * 32;
+    const int c_end = min(rows_here, (half + 1) * ch);
+    for (int c0 = half * ch; c0 < c_end; c0 += 32) {
+      uint32_t v[32];
+      ptx::tmem_ld32(tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(etile * acc_stride + c0), v);
+      ptx::tmem_ld_wait();
+      tile_epilogue_store(a, v, c0, rows_here, t0, n, lane, direct, wsp, (size_t)kTileN);
+    }
+  }
+}
 
 // Quantised weights: the raw 4-bit blocks have a ring of their own (SR slots of two blocks), released as
 // soon as the dequantising warps hold the words in registers, so the weight stream runs ahead of the
@@ -791,7 +923,7 @@ __host__ __device__ constexpr int tc2_x_rows(bool grouped, int tn) { return grou
 // dequantisation runs.  Dense bf16 blocks land in the stage's MMA tiles directly (SR = stages there).
 template <int MODE>
 __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
-  after_previous();
+  wait_previous();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   constexpr int BB = block_bytes(MODE);
@@ -833,12 +965,12 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
   if (tid == 0) {
     for (int s = 0; s < stages; ++s) {
       ptx::mbar_init(&x_loaded[s], 1);
-      ptx::mbar_init(&a_ready[s], kTc2DequantThreads / 32);  // one arrival per dequantising warp
+      ptx::mbar_init(&a_ready[s], kPairThreads / 32);  // one arrival per dequantising warp
       ptx::mbar_init(&mma_done[s], 1);
     }
     for (int s = 0; s < SR; ++s) {
       ptx::mbar_init(&raw_full[s], 1);
-      ptx::mbar_init(&raw_free[s], kTc2DequantThreads / 32);
+      ptx::mbar_init(&raw_free[s], kPairThreads / 32);
     }
     ptx::mbar_init(accum_ready, 1);
     ptx::mbar_fence_init();
@@ -907,6 +1039,7 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
         if (++s == stages) { s = 0; ph ^= 1u; }
       }
       if (ok) ptx::umma_commit(accum_ready);
+      let_next_start();
     }
   } else {
     // ---- dequantise: thread (r, plane, tile) owns one 32-column half of weight row r of a tile ----
@@ -944,132 +1077,192 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
       if (++s == stages) { s = 0; ph ^= 1u; }
       if (++sr == SR) { sr = 0; phr ^= 1u; }
     }
-    // ---- accumulators: warp w reads lanes 32*(w%4); warps 4g..4g+3 take tile g/2, column half g%2 ----
     if (ok) ok = ptx::mbar_wait(accum_ready, 0);
-    const int grp = warp >> 2, etile = grp >> 1, half = grp & 1;
-    // SwiGLU written by this kernel (no K split): the outputs go through the idle stage buffers as
-    // bf16 [token][tile][64] and leave as 16-byte stores, 256 contiguous bytes per token for the tile
-    // pair.  Stores of 64 bytes per token straight from the accumulator layout (one instruction per
-    // token and warp) took a quarter of the kernel's time at 256 rows.
-    const bool staged = gridDim.y == 1 && a.epilogue == B200_EPI_SWIGLU && a.n % 16 == 0;
-    if (staged) {
-      uint32_t all_ok;
-      asm volatile(
-          "{\n\t.reg .pred p, q;\n\t"
-          "setp.ne.b32 p, %1, 0;\n\t"
-          "bar.red.and.pred q, 1, 512, p;\n\t"
-          "selp.u32 %0, 1, 0, q;\n\t}"
-          : "=r"(all_ok)
-          : "r"((uint32_t)ok)
-          : "memory");
-      if (all_ok) {
-        ptx::tc_fence_after_sync();
-        __nv_bfloat16* stage_h = reinterpret_cast<__nv_bfloat16*>(smem);
-        if (etile < n_tiles) {
-          const int lq = warp & 3;
-          const int ch = ((tn_here / 2 + 31) / 32) * 32;
-          const int c_end = min(rows_here, (half + 1) * ch);
-          for (int c0 = half * ch; c0 < c_end; c0 += 32) {
-            uint32_t v[32];
-            ptx::tmem_ld32(tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(etile * 256 + c0), v);
-            const float rs_mine = c0 + lane < rows_here ? a.row_scale(t0 + c0 + lane) : 0.f;
-            ptx::tmem_ld_wait();
-            // lanes 2i / 2i+1 hold gate_i / up_i of every token: the even lane takes token j, the odd
-            // lane token j+1, one exchange per token pair and no idle lanes in the arithmetic
-            const bool odd = lane & 1;
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              const float a0 = __uint_as_float(v[j]), a1 = __uint_as_float(v[j + 1]);
-              const float got = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
-              const float rs = __shfl_sync(0xffffffffu, rs_mine, j + (int)odd);
-              stage_h[((size_t)(c0 + j + (int)odd) * 2 + etile) * 64 + lq * 16 + (lane >> 1)] =
-                  __float2bfloat16(gated(a, odd ? got : a0, odd ? a1 : got) * rs);
-            }
-          }
-        }
-        asm volatile("bar.sync 1, 512;" ::: "memory");
-        const int n_out = a.n / 2;
-        for (int idx = tid; idx < rows_here * 16; idx += kTc2DequantThreads) {
-          const int tok = idx >> 4, c16 = idx & 15, tile = c16 >> 3;
-          const int col = (nt0 + tile) * 64 + (c16 & 7) * 8;
-          if (tile < n_tiles && col < n_out)
-            *reinterpret_cast<uint4*>(a.y + (size_t)(t0 + tok) * a.out_stride(n_out) + col) = *reinterpret_cast<const uint4*>(stage_h + (size_t)idx * 8);
-        }
-      }
-    } else if (gridDim.y == 1 && !a.keep_f32 && a.epilogue != B200_EPI_SWIGLU && a.n % 8 == 0 && a.out_stride(a.n) % 8 == 0 &&
-               (((uintptr_t)a.y | (uintptr_t)a.residual) & 15) == 0) {
-      // The other epilogues written by this kernel, likewise through the idle stage buffers: bf16 [token][256 columns of the pair].  The
-      // residual is brought in first, 16 bytes at a time, and the sums replace it in place (o at 2105 rows of 4096 x 4096: 124 us with
-      // a 2-byte residual load ahead of each 2-byte store, 70 this way).
-      uint32_t all_ok;
-      asm volatile(
-          "{\n\t.reg .pred p, q;\n\t"
-          "setp.ne.b32 p, %1, 0;\n\t"
-          "bar.red.and.pred q, 1, 512, p;\n\t"
-          "selp.u32 %0, 1, 0, q;\n\t}"
-          : "=r"(all_ok)
-          : "r"((uint32_t)ok)
-          : "memory");
-      if (all_ok) {
-        ptx::tc_fence_after_sync();
-        __nv_bfloat16* stage_h = reinterpret_cast<__nv_bfloat16*>(smem);
-        const size_t stride = a.out_stride(a.n), o0 = (size_t)t0 * stride + nt0 * kTileN;
-        const int cols = min(a.n - nt0 * kTileN, 2 * kTileN);
-        const bool add = a.epilogue == B200_EPI_RESIDUAL;
-        if (add) {
-          for (int idx = tid; idx < rows_here * 32; idx += kTc2DequantThreads)
-            if ((idx & 31) * 8 < cols)
-              *reinterpret_cast<uint4*>(stage_h + (size_t)idx * 8) = *reinterpret_cast<const uint4*>(a.residual + o0 + (size_t)(idx >> 5) * stride + (idx & 31) * 8);
-          asm volatile("bar.sync 1, 512;" ::: "memory");
-        }
-        if (etile < n_tiles) {
-          const int lq = warp & 3;
-          const int ch = ((tn_here / 2 + 31) / 32) * 32;
-          const int c_end = min(rows_here, (half + 1) * ch);
-          for (int c0 = half * ch; c0 < c_end; c0 += 32) {
-            uint32_t v[32];
-            ptx::tmem_ld32(tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(etile * 256 + c0), v);
-            const float rs_mine = c0 + lane < rows_here ? a.row_scale(t0 + c0 + lane) : 0.f;
-            ptx::tmem_ld_wait();
-            __nv_bfloat16* mine = stage_h + (size_t)c0 * 256 + etile * kTileN + lq * 32 + lane;
-            const int left = rows_here - c0;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float rs = __shfl_sync(0xffffffffu, rs_mine, j);
-              if (j < left) {
-                float acc = __uint_as_float(v[j]);
-                if (add) acc += __bfloat162float(mine[j * 256]);
-                else acc = activate(a.epilogue, acc);
-                mine[j * 256] = __float2bfloat16(acc * rs);
-              }
-            }
-          }
-        }
-        asm volatile("bar.sync 1, 512;" ::: "memory");
-        for (int idx = tid; idx < rows_here * 32; idx += kTc2DequantThreads)
-          if ((idx & 31) * 8 < cols)
-            *reinterpret_cast<uint4*>(a.y + o0 + (size_t)(idx >> 5) * stride + (idx & 31) * 8) = *reinterpret_cast<const uint4*>(stage_h + (size_t)idx * 8);
-      }
-    } else if (ok && etile < n_tiles) {
-      ptx::tc_fence_after_sync();
-      const int lq = warp & 3;
-      const int nt = nt0 + etile, n = nt * kTileN + lq * 32 + lane;
-      const bool direct = gridDim.y == 1 && !a.keep_f32;
-      float* wsp = a.ws + (((size_t)(nt * gridDim.z + tt) * gridDim.y + split) * tn) * kTileN + lq * 32 + lane;
-      const int ch = ((tn_here / 2 + 31) / 32) * 32;
-      const int c_end = min(rows_here, (half + 1) * ch);
-      for (int c0 = half * ch; c0 < c_end; c0 += 32) {
-        uint32_t v[32];
-        ptx::tmem_ld32(tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(etile * 256 + c0), v);
-        ptx::tmem_ld_wait();
-        tile_epilogue_store(a, v, c0, rows_here, t0, n, lane, direct, wsp, (size_t)kTileN);
-      }
-    }
+    pair_epilogue(a, smem, tmem_base, 256u, ok, rows_here, tn_here, t0, nt0, n_tiles, tt, split);
   }
   if (!ok) atomicExch(a.err, B200_ERR_DEVICE_FLAGGED);
   ptx::tc_fence_before_sync();
   __syncthreads();
   if (warp == 17) ptx::tmem_dealloc(tmem_base, kCols);
+}
+
+// ---- tile pairs with the weight operand in tensor memory: 17..128 rows --------------------------
+// Between the streams of a few rows and the tile pairs above a matmul is a weight stream that has to be dequantised on the way.  A CTA of
+// qmm_tca_kernel takes one weight tile: every tile fetches all activations again (512 KiB at 64 rows of K = 4096, against 288 KiB of
+// weights), and a grid such as gate/up's 224 tiles leaves half of the SMs with one CTA where the others have two.  Here a CTA per SM owns two
+// adjacent tiles and 16 warps dequantise them into tensor memory, so the activations are fetched half as often and every SM has the same work.
+//   * unit = two chunks (128 columns of K) of both tiles.  A stage of shared memory holds a unit's raw blocks and its two activation tiles; one
+//     warp fills it, the commit of the unit's 16 MMAs frees it and frees the slot of tensor memory at the same time (one barrier for both).
+//   * the weights of the first stages are asked for before the kernels ahead in the stream have ended: nothing writes weights after their
+//     creation, which waits for the device.
+constexpr int kTpThreads = 18 * 32;  // warps 0-15 dequantise, 16 loads, 17 issues MMAs
+constexpr int kTpMaxStages = 12;
+
+template <int MODE>
+__global__ void __launch_bounds__(kTpThreads, 1) qmm_tp_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  constexpr uint32_t BB = block_bytes(MODE);
+  static_assert(4 * BB % 1024 == 0, "the activation tiles of a stage start on swizzle atoms");
+  const int tn = a.tn, S = a.stages, Q = a.a_slots;
+  const uint32_t x_bytes = (uint32_t)tn * 128u, stage_bytes = 4 * BB + 2 * x_bytes;  // [tile][chunk] raw blocks, then [chunk] activation tiles
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)S * stage_bytes);
+  const uint32_t smem_u = ptx::smem_u32(smem), full = ptx::smem_u32(bars);  // [S] a unit has landed
+  const uint32_t done = full + 8u * S;                                      // [S] its MMAs are done
+  const uint32_t a_ready = done + 8u * S;                                   // [Q] a dequantised unit is in tensor memory
+  uint64_t* accum_ready = bars + 2 * S + Q;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum_ready + 1);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nt0 = 2 * blockIdx.x, n_tiles = min(2, a.nt - nt0), split = blockIdx.y, tt = blockIdx.z;
+  const int t0 = tt * tn, rows_here = min(tn, a.rows - t0);
+  const int kc0 = split * a.chunks_per_split, n_chunks = min(a.chunks_per_split, a.kc - kc0), n_units = (n_chunks + 1) >> 1;
+  const uint32_t acc_cols = (uint32_t)(tn + 31) / 32 * 32;
+
+  if (tid == 0) {
+    for (int s = 0; s < 2 * S; ++s) ptx::mbar_init(&bars[s], 1);
+    for (int q = 0; q < Q; ++q) ptx::mbar_init(&bars[2 * S + q], kPairThreads / 32);
+    ptx::mbar_init(accum_ready, 1);
+    ptx::mbar_fence_init();
+  }
+  __syncthreads();
+  const unsigned char* wsrc = a.blocks + ((size_t)nt0 * a.kc + kc0) * BB;
+  const size_t tile_stride = (size_t)a.kc * BB;
+  auto load_weights = [&](int p, int s) {
+    const int n_here = min(2, n_chunks - 2 * p);
+    ptx::mbar_expect_tx_addr(full + 8u * s, (uint32_t)n_here * (n_tiles * BB + x_bytes));
+    for (int tile = 0; tile < n_tiles; ++tile)
+      ptx::bulk_g2s_addr(smem_u + (uint32_t)s * stage_bytes + tile * 2 * BB, wsrc + tile * tile_stride + (size_t)p * 2 * BB, n_here * BB, full + 8u * s);
+  };
+  auto load_x = [&](int p, int s) {
+    const int n_here = min(2, n_chunks - 2 * p);
+    for (int j = 0; j < n_here; ++j)
+      ptx::tma_load_2d(smem + (size_t)s * stage_bytes + 4 * BB + j * x_bytes, &xmap, (kc0 + 2 * p + j) * kChunkK, a.x_row0 + t0, &bars[s]);
+  };
+  const int ahead = min(S, n_units);
+  if (warp == 16 && lane == 0)
+    for (int p = 0; p < ahead; ++p) load_weights(p, p);
+  wait_previous();
+  if (warp == 17) {
+    ptx::tmem_alloc(tmem_slot, 512);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot, a_col0 = tmem_base + 2 * acc_cols;
+  bool ok = true;
+
+  if (warp == 16) {
+    if (lane == 0) {
+      for (int p = 0; p < ahead; ++p) load_x(p, p);
+      int s = 0;
+      uint32_t ph = 0;
+      for (int p = ahead; p < n_units; ++p) {
+        ok = ptx::mbar_wait_addr(done + 8u * s, ph);
+        if (!ok) break;
+        load_weights(p, s);
+        load_x(p, s);
+        if (++s == S) { s = 0; ph ^= 1u; }
+      }
+    }
+  } else if (warp == 17) {
+    if (ptx::elect_one()) {
+      const uint32_t idesc = ptx::umma_idesc_bf16(kTileN, tn);
+      int s = 0, q = 0;
+      uint32_t ph = 0, qh = 0;
+      for (int p = 0; p < n_units; ++p) {
+        ok = ptx::mbar_wait_addr(full + 8u * s, ph) && ptx::mbar_wait_addr(a_ready + 8u * q, qh);
+        if (!ok) break;
+        ptx::tc_fence_after_sync();
+        const uint64_t db = ptx::umma_desc_k_sw128(smem_u + (uint32_t)s * stage_bytes + 4 * BB);
+        const int n_here = min(2, n_chunks - 2 * p);
+        for (int tile = 0; tile < n_tiles; ++tile) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            if (j < n_here) {
+#pragma unroll
+              for (int k4 = 0; k4 < 4; ++k4)
+                ptx::umma_bf16_tmem_a(tmem_base + tile * acc_cols, a_col0 + (uint32_t)(q * 128 + tile * 64 + j * 32 + k4 * 8), db + j * (x_bytes >> 4) + 2 * k4,
+                                      idesc, (p > 0 || j > 0 || k4 > 0) ? 1u : 0u);
+            }
+          }
+        }
+        ptx::umma_commit(&bars[S + s]);
+        if (++s == S) { s = 0; ph ^= 1u; }
+        if (++q == Q) { q = 0; qh ^= 1u; }
+      }
+      if (ok) ptx::umma_commit(accum_ready);
+      let_next_start();
+    }
+  } else {
+    // ---- dequantise: thread (r, plane, tile) owns one 32-column half of weight row r of a tile ----
+    const int r = tid & (kTileN - 1), plane = (tid >> 7) & 1, tile = tid >> 8;
+    const bool mine = tile < n_tiles;
+    const uint32_t my_taddr = a_col0 + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(tile * 64 + plane * 16);
+    const unsigned char* my_blk = smem + tile * 2 * BB;
+    int s = 0, q = 0, sd = 0, pending = -1;
+    uint32_t ph = 0, phd = 0;  // sd, phd: the unit that last used tensor-memory slot q
+    // The stores of a unit into tensor memory stay in flight while the next one is read and its first chunk dequantised.
+    auto announce = [&]() {
+      ptx::tmem_st_wait();
+      ptx::tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive_addr(a_ready + 8u * pending);
+    };
+    for (int p = 0; p < n_units; ++p) {
+      ok = ptx::mbar_wait_addr(full + 8u * s, ph);
+      if (!ok) break;
+      const bool two = 2 * p + 1 < n_chunks;
+      const unsigned char* blk = my_blk + (size_t)s * stage_bytes;
+      uint4 raw0 = make_uint4(0u, 0u, 0u, 0u), raw1 = raw0;
+      __nv_bfloat162 s20 = __float2bfloat162_rn(0.f), b20 = s20, s21 = s20, b21 = s20;
+      if (mine) {
+        raw0 = *reinterpret_cast<const uint4*>(blk + plane * kPlaneBytes + r * 16);
+        row_params<MODE>(blk, r, plane, s20, b20);
+        if (two) {
+          raw1 = *reinterpret_cast<const uint4*>(blk + BB + plane * kPlaneBytes + r * 16);
+          row_params<MODE>(blk + BB, r, plane, s21, b21);
+        }
+      }
+      uint32_t v[16];
+      {
+        const uint32_t words[4] = {raw0.x, raw0.y, raw0.z, raw0.w};
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const uint4 d = dequant_word<MODE>(words[w], s20, b20);
+          v[4 * w] = d.x; v[4 * w + 1] = d.y; v[4 * w + 2] = d.z; v[4 * w + 3] = d.w;
+        }
+      }
+      if (pending >= 0) announce();
+      if (p >= Q) {
+        ok = ptx::mbar_wait_addr(done + 8u * sd, phd);
+        if (!ok) { pending = -1; break; }
+        if (++sd == S) { sd = 0; phd ^= 1u; }
+      }
+      ptx::tc_fence_after_sync();
+      if (mine) ptx::tmem_st16(my_taddr + (uint32_t)(q * 128), v);
+      if (two && mine) {
+        const uint32_t words[4] = {raw1.x, raw1.y, raw1.z, raw1.w};
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const uint4 d = dequant_word<MODE>(words[w], s21, b21);
+          v[4 * w] = d.x; v[4 * w + 1] = d.y; v[4 * w + 2] = d.z; v[4 * w + 3] = d.w;
+        }
+        ptx::tmem_st16(my_taddr + (uint32_t)(q * 128 + 32), v);
+      }
+      pending = q;
+      if (++s == S) { s = 0; ph ^= 1u; }
+      if (++q == Q) q = 0;
+    }
+    if (pending >= 0) announce();
+    if (ok) ok = ptx::mbar_wait(accum_ready, 0);
+    pair_epilogue(a, smem, tmem_base, acc_cols, ok, rows_here, tn, t0, nt0, n_tiles, tt, split);
+  }
+  if (!ok) atomicExch(a.err, B200_ERR_DEVICE_FLAGGED);
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 17) ptx::tmem_dealloc(tmem_base, 512);
 }
 
 // ---- small-batch kernel: register dequantisation + mma.sync -------------------------------------
@@ -1119,7 +1312,6 @@ __device__ __forceinline__ uint32_t operand_pair(uint32_t word, int i, __nv_bflo
 
 template <int MODE, int NT8>
 __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma_kernel(QmmArgs a) {
-  after_previous();
   extern __shared__ __align__(128) unsigned char gsm[];
   const int stages = a.stages;
   constexpr int kSlotBytes = 2 * kRawStride;  // a ring slot holds the blocks of two adjacent weight tiles
@@ -1168,8 +1360,10 @@ __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma_kernel
           if (++s == stages) { s = 0; phase ^= 1u; }
         }
       }
+      let_next_start();
     }
   } else {
+    wait_previous();  // (the producer need not: it reads weights only)
     const int vec_per_row = n_chunks * (kChunkK * 2 / 16);
     for (int idx = tid; idx < TILE * vec_per_row; idx += kGemvConsumers * 32) {
       const int row = idx / vec_per_row, v = idx - row * vec_per_row;
@@ -1460,7 +1654,6 @@ __host__ __device__ constexpr int slab8_stride(int chunks) { return (chunks * kC
 
 template <int NT8>
 __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma8_kernel(QmmArgs a) {
-  after_previous();
   extern __shared__ __align__(128) unsigned char gsm[];
   const int stages = a.stages;
   constexpr int kSlotBytes = 2 * kRawStride;
@@ -1507,8 +1700,10 @@ __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma8_kerne
           if (++s == stages) { s = 0; phase ^= 1u; }
         }
       }
+      let_next_start();
     }
   } else {
+    wait_previous();  // (the producer need not: it reads weights only)
     // ---- stage the activations: 16-bit fixed point with one scale per token and 64-column group ----
     // One thread per 8 columns; the 8 threads of a group (consecutive lanes) agree on the group's scale,
     // quantise, and add up the group's integer sum.  A single pass, one barrier at the end.
@@ -1810,7 +2005,7 @@ struct MxActMaps {
 
 __global__ void __launch_bounds__(kMxThreads, 1)
     qmm_mx_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ MxActMaps amaps, QmmArgs a) {
-  after_previous();
+  wait_previous();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int tn = a.tn, P = a.stages;
@@ -1904,6 +2099,7 @@ __global__ void __launch_bounds__(kMxThreads, 1)
         ptx::umma_commit(&slot_free[s]);
       }
       if (ok) ptx::umma_commit(accum_ready);
+      let_next_start();
     }
   } else {
     // ---- scales: lane l of every warp holds rows l, 32+l, 64+l, 96+l of the tile (4 K32 blocks each) ----
@@ -2000,7 +2196,7 @@ constexpr int kMxpStageTokens = 16;
 
 __global__ void __launch_bounds__(kMxpThreads, 1)
     qmm_mxp_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ MxActMaps amaps, QmmArgs a) {
-  after_previous();
+  wait_previous();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int tn = a.tn, P = a.stages;
@@ -2136,6 +2332,7 @@ __global__ void __launch_bounds__(kMxpThreads, 1)
         }
         if (ok) ptx::umma_commit(&accum_ready[set]);
       }
+      let_next_start();
     }
   } else {
     // ---- epilogue: warps 0-3 drain tile 0, warps 6-9 tile 1 (a warp reads the tensor-memory lanes 32 * (warp % 4)) ----
@@ -2627,6 +2824,50 @@ static b200_status launch_tca(QmmArgs& a, int rows, cudaStream_t s) {
   return direct ? B200_OK : launch_finish(a, splits, s);
 }
 
+// Quantised weights, 17..128 rows: tile pairs with the weights in tensor memory.
+template <int MODE>
+static b200_status launch_tp(QmmArgs& a, int rows, cudaStream_t s) {
+  const int tn = (rows + 15) / 16 * 16;  // (one token tile: 128 rows at most)
+  a.tn = tn;
+  b200_status st = ensure_state(0);
+  if (st != B200_OK) return st;
+  static int smem_budget[3] = {0, 0, 0};
+  if (smem_budget[MODE] == 0) {
+    int dev = 0, optin = 0;
+    B200_CUDA_TRY(cudaGetDevice(&dev));
+    B200_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    cudaFuncAttributes fa;
+    B200_CUDA_TRY(cudaFuncGetAttributes(&fa, qmm_tp_kernel<MODE>));
+    const int budget = optin - (int)fa.sharedSizeBytes;
+    B200_CUDA_TRY(cudaFuncSetAttribute(qmm_tp_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
+    smem_budget[MODE] = budget;
+  }
+  // tensor memory: two accumulators of tn columns, then slots of 128 columns (a unit of both tiles)
+  a.a_slots = std::min(3, (512 - 2 * ((tn + 31) / 32 * 32)) / 128);
+  const int stage = 4 * block_bytes(MODE) + 2 * tn * 128, fixed = 1024 + 8 * (2 * kTpMaxStages + 3 + 2);
+  a.stages = std::min(kTpMaxStages, (smem_budget[MODE] - fixed) / stage);
+  if (a.stages < 2 || a.a_slots < 2) {
+    b200_set_error("qmm: %d bytes of shared memory per stage, %d available", stage, smem_budget[MODE]);
+    return B200_ERR_CAPACITY;
+  }
+  const size_t smem = (size_t)a.stages * stage + fixed;
+  const int pairs = (a.nt + 1) / 2;
+  const int splits0 = pick_splits(pairs, a.kc, g_sms, 1, 12);  // (4 instead of 12 chunks: gate/up 33.9 -> 53.6 us at 61 rows)
+  a.chunks_per_split = (a.kc + splits0 - 1) / splits0;
+  const int splits = (a.kc + a.chunks_per_split - 1) / a.chunks_per_split;
+  const bool direct = splits == 1 && !a.keep_f32;
+  st = ensure_state(direct ? 0 : (size_t)splits * tn * a.nt * kTileN * sizeof(float));
+  if (st != B200_OK) return st;
+  a.ws = g_ws[g_place]; a.err = g_err;
+  CUtensorMap xmap;
+  st = make_x_map(&xmap, a.x, rows, a.k, tn);
+  if (st != B200_OK) return st;
+  a.x_row0 = 0;
+  launch_after(qmm_tp_kernel<MODE>, dim3(pairs, splits, 1), kTpThreads, smem, s, xmap, a);
+  B200_LAUNCH_CHECK();
+  return direct ? B200_OK : launch_finish(a, splits, s);
+}
+
 // ---- block-scaled MXFP4 path: second weight layout, activation split, launch --------------------------
 unsigned char* g_mx_act = nullptr;  // [hi: rows x k][lo: rows x k][unscale: rows f32], grown on demand
 size_t g_mx_act_bytes = 0;
@@ -3093,6 +3334,11 @@ static b200_status qmm_entry(const b200_qweight* w, const void* d_x, int32_t row
       if (w->mode == B200_Q_MXFP4_G32) return launch_simt<B200_Q_MXFP4_G32>(a, rows, s);
       return launch_simt<B200_Q_BF16>(a, rows, s);
     }
+    // A matrix of more tile pairs than SMs runs in waves, and two CTAs of the kernel of single tiles hide each other's epilogues there
+    // (128256 outputs at 61 rows: 109 us against 134); up to one wave the pairs are ahead (28672 outputs: 33.9 against 38.2 us at 61 rows,
+    // 33.6 against 34.6 at 17, 37.1 against 43.6 at 120; 4096 outputs of K = 14336 20.4 against 21.0, 6144 of K = 4096 13.3 against 14.3).
+    if (path == B200_QMM_TCGEN05_TMEM_A && w->mode != B200_Q_BF16 && rows <= 128 && ensure_state(0) == B200_OK && (w->nt + 1) / 2 <= g_sms)
+      return w->mode == B200_Q_AFFINE4_G64 ? launch_tp<B200_Q_AFFINE4_G64>(a, rows, s) : launch_tp<B200_Q_MXFP4_G32>(a, rows, s);
     if (path == B200_QMM_TCGEN05_TMEM_A && w->mode != B200_Q_BF16)
       return w->mode == B200_Q_AFFINE4_G64 ? launch_tca<B200_Q_AFFINE4_G64>(a, rows, s) : launch_tca<B200_Q_MXFP4_G32>(a, rows, s);
     if (path == B200_QMM_TCGEN05_X2) {

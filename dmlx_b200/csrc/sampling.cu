@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(const T* __res
                                                                   const uint32_t* __restrict__ ctx, const int* __restrict__ ctx_off,
                                                                   float* __restrict__ scratch, uint32_t* __restrict__ tokens,
                                                                   float* __restrict__ logprobs) {
-  after_previous();
+  wait_previous();
   extern __shared__ __align__(16) unsigned char sample_dyn[];
   Shared& s = *reinterpret_cast<Shared*>(sample_dyn);
   cg::cluster_group cluster = cg::this_cluster();
