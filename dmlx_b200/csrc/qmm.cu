@@ -381,7 +381,6 @@ constexpr int kPrefetchAhead = 12;  // weight blocks requested into L2 ahead of 
 
 template <int MODE>
 __global__ void __launch_bounds__(kTcThreads, 2) qmm_tc_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
-  wait_previous();
   extern __shared__ unsigned char smem_raw[];
   // 1024-byte alignment: the 128B swizzle pattern is a function of the shared-memory address.
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -416,6 +415,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) qmm_tc_kernel(const __grid_cons
   }
   int rows_here = min(tn, a.rows - t0);
   if (a.items) {
+    wait_previous();
     if ((int)blockIdx.z >= *a.n_items) return;
     const int4 it = a.items[blockIdx.z];
     blocks += (size_t)it.x * a.expert_stride;
@@ -437,6 +437,21 @@ __global__ void __launch_bounds__(kTcThreads, 2) qmm_tc_kernel(const __grid_cons
     ptx::mbar_init(accum_ready, 1);
     ptx::mbar_fence_init();
   }
+  // dense bf16 blocks are stored in the swizzled K-major layout and land in the MMA tile directly
+  const unsigned char* wsrc = blocks + ((size_t)nt * a.kc + kc0) * BB;
+  auto load_weights = [&](int i, int s) {
+    ptx::mbar_expect_tx(&loaded[s], BB + tn * 128);
+    ptx::bulk_g2s(MODE == B200_Q_BF16 ? a_tile(s) : raw_blk(s), wsrc + (size_t)i * BB, BB, &loaded[s]);
+  };
+  const int ahead = a.items ? 0 : min(stages, n_chunks);  // weights asked for before the kernels ahead in the stream have ended
+  if (!a.items) {
+    __syncthreads();
+    if (warp == 8 && lane == 0) {
+      for (int i = 0; i < ahead; ++i) load_weights(i, i);
+      for (int i = ahead; i < min(n_chunks, kPrefetchAhead); ++i) ptx::bulk_prefetch_l2(wsrc + (size_t)i * BB, BB);
+    }
+    wait_previous();
+  }
   if (warp == 9) {
     ptx::tmem_alloc(tmem_slot, ncols);
     ptx::tmem_relinquish();
@@ -449,21 +464,20 @@ __global__ void __launch_bounds__(kTcThreads, 2) qmm_tc_kernel(const __grid_cons
 
   if (warp == 8) {
     if (lane == 0) {
+      auto load_x = [&](int i, int s) { ptx::tma_load_2d(x_tile(s), &xmap, x_col + (kc0 + i) * kChunkK, a.x_row0 + t0, &loaded[s]); };
+      for (int i = 0; i < ahead; ++i) load_x(i, i);
       // The weight blocks of this CTA are contiguous in HBM: ask for them in L2 well ahead of the
       // stage that will copy them, so that a stage's refill waits for L2, not for HBM.
-      const unsigned char* wsrc = blocks + ((size_t)nt * a.kc + kc0) * BB;
-      for (int i = 0; i < min(n_chunks, kPrefetchAhead); ++i) ptx::bulk_prefetch_l2(wsrc + (size_t)i * BB, BB);
-      int s = 0;
-      uint32_t ph = 0;  // stage cursor kept incrementally: no division by the runtime stage count
-      for (int i = 0; i < n_chunks && ok; ++i, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
+      if (a.items)
+        for (int i = 0; i < min(n_chunks, kPrefetchAhead); ++i) ptx::bulk_prefetch_l2(wsrc + (size_t)i * BB, BB);
+      int s = ahead == stages ? 0 : ahead;
+      uint32_t ph = ahead == stages ? 1 : 0;  // stage cursor kept incrementally: no division by the runtime stage count
+      for (int i = ahead; i < n_chunks && ok; ++i, ph ^= (s + 1 == stages), s = (s + 1 == stages) ? 0 : s + 1) {
         if (i + kPrefetchAhead < n_chunks) ptx::bulk_prefetch_l2(wsrc + (size_t)(i + kPrefetchAhead) * BB, BB);
         ok = ptx::mbar_wait(&mma_done[s], ph ^ 1u);
         if (!ok) break;
-        ptx::mbar_expect_tx(&loaded[s], BB + tn * 128);
-        // dense bf16 blocks are stored in the swizzled K-major layout and land in the MMA tile directly
-        ptx::bulk_g2s(MODE == B200_Q_BF16 ? a_tile(s) : raw_blk(s), blocks + ((size_t)nt * a.kc + kc0 + i) * BB, BB,
-                      &loaded[s]);
-        ptx::tma_load_2d(x_tile(s), &xmap, x_col + (kc0 + i) * kChunkK, a.x_row0 + t0, &loaded[s]);
+        load_weights(i, s);
+        load_x(i, s);
       }
     }
   } else if (warp == 9) {
@@ -923,7 +937,6 @@ __device__ __forceinline__ void pair_epilogue(const QmmArgs& a, unsigned char* s
 // dequantisation runs.  Dense bf16 blocks land in the stage's MMA tiles directly (SR = stages there).
 template <int MODE>
 __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
-  wait_previous();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   constexpr int BB = block_bytes(MODE);
@@ -948,6 +961,7 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
   int t0 = tt * tn, rows_here = min(tn, a.rows - t0);
   const unsigned char* blocks = a.blocks;
   if (a.items) {  // a work item of expert-sorted rows, loaded 64 at a time
+    wait_previous();
     if (tt >= *a.n_items) return;
     const int4 it = a.items[tt];
     blocks += (size_t)it.x * a.expert_stride;
@@ -975,6 +989,18 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
     ptx::mbar_init(accum_ready, 1);
     ptx::mbar_fence_init();
   }
+  auto load_weights = [&](int i, int s) {
+    ptx::mbar_expect_tx(&raw_full[s], n_tiles * BB);
+    for (int tile = 0; tile < n_tiles; ++tile)
+      ptx::bulk_g2s(kDense ? a_tile(s, tile) : raw_blk(s, tile), blocks + ((size_t)(nt0 + tile) * a.kc + kc0 + i) * BB, BB, &raw_full[s]);
+  };
+  const int ahead = a.items ? 0 : min(SR, n_chunks);  // weights asked for before the kernels ahead in the stream have ended
+  if (!a.items) {
+    __syncthreads();
+    if (warp == 16 && lane == 0)
+      for (int i = 0; i < ahead; ++i) load_weights(i, i);
+    wait_previous();
+  }
   if (warp == 17) {
     ptx::tmem_alloc(tmem_slot, kCols);
     ptx::tmem_relinquish();
@@ -987,16 +1013,13 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
 
   if (warp == 16) {
     if (lane == 0) {  // the weight stream
-      int s = 0;
-      uint32_t ph = 1;
-      for (int i = 0; i < n_chunks; ++i) {
+      int s = ahead == SR ? 0 : ahead;
+      uint32_t ph = ahead == SR ? 0 : 1;
+      for (int i = ahead; i < n_chunks; ++i) {
         // dense blocks go into the stage's MMA tiles, so their slot is the stage and frees with its MMAs
         ok = ptx::mbar_wait(kDense ? &mma_done[s] : &raw_free[s], ph);
         if (!ok) break;
-        ptx::mbar_expect_tx(&raw_full[s], n_tiles * BB);
-        for (int tile = 0; tile < n_tiles; ++tile)
-          ptx::bulk_g2s(kDense ? a_tile(s, tile) : raw_blk(s, tile), blocks + ((size_t)(nt0 + tile) * a.kc + kc0 + i) * BB, BB,
-                        &raw_full[s]);
+        load_weights(i, s);
         if (++s == SR) { s = 0; ph ^= 1u; }
       }
     }
@@ -1897,7 +1920,7 @@ __global__ void __launch_bounds__(256) mx_split_activations_kernel(const __nv_bf
                                                                    unsigned char* __restrict__ hi, unsigned char* __restrict__ lo,
                                                                    float* __restrict__ unscale, const int* __restrict__ gather,
                                                                    int gather_div, const int* __restrict__ rows_valid) {
-  after_previous();
+  wait_previous();  // (CTAs of the matmul that were placed while rows are still split made it slower: 24576 rows of K = 2048 335 -> 374 us)
   __shared__ float s_max[8];
   const int row = blockIdx.x;
   if (rows_valid && row >= *rows_valid) return;  // capacity beyond the rows that exist: nothing to read
@@ -1998,9 +2021,9 @@ __device__ __forceinline__ bool __syncthreads_and_epi8(bool pred) {
 // Activation tensor maps with boxes of 32, 64, 96 and 128 rows: a work item loads (and multiplies) only
 // as many token rows as it has, rounded up to 32.  The activation tiles are re-read by every CTA of
 // an item and are two thirds of the bytes a stage moves.
-struct MxActMaps {
-  CUtensorMap hi[4];
-  CUtensorMap lo[4];
+struct MxActMaps {  // boxes of 32, 64, 96 and 128 rows (none above the token tile), and of 16
+  CUtensorMap hi[5];
+  CUtensorMap lo[5];
 };
 
 __global__ void __launch_bounds__(kMxThreads, 1)
@@ -2194,6 +2217,7 @@ __global__ void __launch_bounds__(kMxThreads, 1)
 //                 the last slab has been read, before it is stored.
 constexpr int kMxpStageTokens = 16;
 
+template <bool SIDE>
 __global__ void __launch_bounds__(kMxpThreads, 1)
     qmm_mxp_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ MxActMaps amaps, QmmArgs a) {
   wait_previous();
@@ -2240,9 +2264,8 @@ __global__ void __launch_bounds__(kMxpThreads, 1)
       k.kc0 = k.split * a.chunks_per_split;
       k.n_chunks = min(a.chunks_per_split, a.kc128 - k.kc0);
     }
-    k.tn_eff = min(tn, ((k.rows_here + 31) / 32) * 32);
-    if (k.tn_eff < 16) k.tn_eff = 16;
-    k.map_idx = (k.tn_eff + 31) / 32 - 1;
+    k.tn_eff = k.rows_here <= 16 ? 16 : min(tn, ((k.rows_here + 31) / 32) * 32);
+    k.map_idx = k.tn_eff == 16 ? 4 : (k.tn_eff + 31) / 32 - 1;
     return k;
   };
 
@@ -2272,7 +2295,11 @@ __global__ void __launch_bounds__(kMxpThreads, 1)
   // slab of the epilogue: the MoE stack spent a quarter of its time there (10.7 ms -> 7.9 ms with the epilogue left
   // out, timing only).  Wider tiles keep one set of two 128-column accumulators.
   const bool dual = 4 * tn + 8 * P + 8 <= (int)kCols;
-  const uint32_t acc_stride = dual ? (uint32_t)tn : 128u, set_stride = 2u * acc_stride;
+  // Up to 48 rows (SIDE) the two halves of an activation (E4M3 code, code of 16 x the residual) are multiplied side by side, as 2 x tn columns of one
+  // MMA, and added up by the epilogue: an MMA of N <= 64 takes some 46 cycles whatever its N, and a stage is 8 of them instead of 16 (gate/up
+  // and down of 32 experts of 4096 x 2048, 24 tokens: 73 + 39 -> 66 + 35 us).
+  // (SIDE is a template parameter: as a variable it cost the wide tiles of 24576 expert rows 4 %.)
+  const uint32_t acc_stride = SIDE ? 2u * (uint32_t)tn : (dual ? (uint32_t)tn : 128u), set_stride = 2u * acc_stride;
   const uint32_t sfa_col0 = tmem_base + (dual ? 2u * set_stride : 256u), sfb_hi = sfa_col0 + 8u * (uint32_t)P, sfb_lo = sfb_hi + 4u;
   bool ok = true;
 
@@ -2294,7 +2321,7 @@ __global__ void __launch_bounds__(kMxpThreads, 1)
             ptx::bulk_g2s(sf_tile(s, tile), sf_src + ((size_t)tile * a.kc128 + kc) * 512, 512, &full[s]);
           }
           ptx::tma_load_2d(b_tile(s, 0), &amaps.hi[k.map_idx], kc * kMxK, a.x_row0 + k.t0, &full[s]);
-          ptx::tma_load_2d(b_tile(s, 1), &amaps.lo[k.map_idx], kc * kMxK, a.x_row0 + k.t0, &full[s]);
+          ptx::tma_load_2d(SIDE ? b_tile(s, 0) + k.tn_eff * 128 : b_tile(s, 1), &amaps.lo[k.map_idx], kc * kMxK, a.x_row0 + k.t0, &full[s]);
         }
       }
     }
@@ -2321,11 +2348,18 @@ __global__ void __launch_bounds__(kMxpThreads, 1)
             const uint64_t da = ptx::umma_desc_k_sw128(ptx::smem_u32(a_tile(s, tile)));
             const uint32_t sfa = sfa_col0 + (uint32_t)((s * 2 + tile) * 4);
             ptx::tmem_cp_32x128b_warpx4(sfa, ptx::umma_desc_k_noswizzle_16B(ptx::smem_u32(sf_tile(s, tile))));
+            if (SIDE) {
 #pragma unroll
-            for (int k4 = 0; k4 < 4; ++k4) {
-              const uint32_t idesc = ptx::umma_idesc_mx_e2m1_e4m3(kTileN, k.tn_eff, k4);
-              ptx::umma_mxf8f6f4(acc0 + tile * acc_stride, da + 2 * k4, dh + 2 * k4, idesc, (i > 0 || k4 > 0) ? 1u : 0u, sfa, sfb_hi);
-              ptx::umma_mxf8f6f4(acc0 + tile * acc_stride, da + 2 * k4, dl + 2 * k4, idesc, 1u, sfa, sfb_lo);
+              for (int k4 = 0; k4 < 4; ++k4)
+                ptx::umma_mxf8f6f4(acc0 + tile * acc_stride, da + 2 * k4, dh + 2 * k4, ptx::umma_idesc_mx_e2m1_e4m3(kTileN, 2 * k.tn_eff, k4),
+                                   (i > 0 || k4 > 0) ? 1u : 0u, sfa, sfb_hi);
+            } else {
+#pragma unroll
+              for (int k4 = 0; k4 < 4; ++k4) {
+                const uint32_t idesc = ptx::umma_idesc_mx_e2m1_e4m3(kTileN, k.tn_eff, k4);
+                ptx::umma_mxf8f6f4(acc0 + tile * acc_stride, da + 2 * k4, dh + 2 * k4, idesc, (i > 0 || k4 > 0) ? 1u : 0u, sfa, sfb_hi);
+                ptx::umma_mxf8f6f4(acc0 + tile * acc_stride, da + 2 * k4, dl + 2 * k4, idesc, 1u, sfa, sfb_lo);
+              }
             }
           }
           ptx::umma_commit(&slot_free[s]);
@@ -2364,8 +2398,17 @@ __global__ void __launch_bounds__(kMxpThreads, 1)
         const float us_mine = (lane < kMxpStageTokens && c0 + lane < k.rows_here) ? a.act_unscale[k.t0 + c0 + lane] : 0.f;
         if (mine) {
           uint32_t v[16];
-          ptx::tmem_ld16(acc0 + lane_base + (uint32_t)etile * acc_stride + (uint32_t)c0, v);
-          ptx::tmem_ld_wait();
+          const uint32_t from = acc0 + lane_base + (uint32_t)etile * acc_stride + (uint32_t)c0;
+          ptx::tmem_ld16(from, v);
+          if (SIDE) {
+            uint32_t low[16];
+            ptx::tmem_ld16(from + (uint32_t)k.tn_eff, low);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(fmaf(__uint_as_float(low[j]), 0.0625f, __uint_as_float(v[j])));
+          } else {
+            ptx::tmem_ld_wait();
+          }
           if (partial) {
             // [weight tile][token tile][split][tn][128] f32, summed by the finish kernel
             float* wsp = a.ws + (((size_t)((k.nt0 + etile) * tts + k.tt) * splits + k.split) * tn) * kTileN + (warp & 3) * 32 + lane;
@@ -2945,8 +2988,9 @@ static b200_status launch_mx(const b200_qweight* w, QmmArgs& a, int rows, cudaSt
   std::memset(&amaps, 0, sizeof(amaps));
   const uint64_t dims[2] = {(uint64_t)a.k, (uint64_t)rows};
   const uint64_t strides[1] = {(uint64_t)a.k};
-  for (int i = 0; i < 4 && 32 * (i + 1) <= ((tn + 31) / 32) * 32; ++i) {
-    const uint32_t box[2] = {(uint32_t)kMxK, (uint32_t)std::min(tn, 32 * (i + 1))};
+  for (int i = 0; i < 5; ++i) {
+    if (i < 4 && 32 * (i + 1) > ((tn + 31) / 32) * 32) continue;
+    const uint32_t box[2] = {(uint32_t)kMxK, (uint32_t)(i == 4 ? 16 : std::min(tn, 32 * (i + 1)))};
     st = b200_make_tensor_map(&amaps.hi[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, hi, dims, strides, box);
     if (st == B200_OK) st = b200_make_tensor_map(&amaps.lo[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, lo, dims, strides, box);
     if (st != B200_OK) return st;
@@ -2958,10 +3002,11 @@ static b200_status launch_mx(const b200_qweight* w, QmmArgs& a, int rows, cudaSt
     B200_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     cudaFuncAttributes fa, fb;
     B200_CUDA_TRY(cudaFuncGetAttributes(&fa, qmm_mx_kernel));
-    B200_CUDA_TRY(cudaFuncGetAttributes(&fb, qmm_mxp_kernel));
+    B200_CUDA_TRY(cudaFuncGetAttributes(&fb, qmm_mxp_kernel<false>));
     const int budget = optin - (int)std::max(fa.sharedSizeBytes, fb.sharedSizeBytes);
     B200_CUDA_TRY(cudaFuncSetAttribute(qmm_mx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
-    B200_CUDA_TRY(cudaFuncSetAttribute(qmm_mxp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
+    B200_CUDA_TRY(cudaFuncSetAttribute(qmm_mxp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
+    B200_CUDA_TRY(cudaFuncSetAttribute(qmm_mxp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
     smem_budget = budget;
   }
   a.err = g_err;
@@ -2995,7 +3040,8 @@ static b200_status launch_mx(const b200_qweight* w, QmmArgs& a, int rows, cudaSt
     }
     const long long n_work = a.items ? (long long)pairs * a.max_items : (long long)pairs * tts * real_splits;
     const int grid = (int)std::max<long long>(1, std::min<long long>(g_sms, n_work));
-    launch_after(qmm_mxp_kernel, grid, kMxpThreads, smem, s, *reinterpret_cast<const CUtensorMap*>(w->mx_map), amaps, a);
+    const bool side = 8 * tn + 8 * a.stages + 8 <= 512;  // both halves of an activation side by side: columns of tensor memory for two sets
+    launch_after(side ? qmm_mxp_kernel<true> : qmm_mxp_kernel<false>, grid, kMxpThreads, smem, s, *reinterpret_cast<const CUtensorMap*>(w->mx_map), amaps, a);
     B200_LAUNCH_CHECK();
     return real_splits > 1 ? launch_finish(a, real_splits, s) : B200_OK;
   }
@@ -3610,8 +3656,14 @@ extern "C" b200_status b200_qmm_error_word(int32_t* out) {
 b200_status b200_qmm_error_words_async(int32_t* h_out, void* stream) {
   h_out[0] = h_out[1] = 0;
   if (g_err) B200_CUDA_TRY(cudaMemcpyAsync(h_out, g_err, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
-  if (int* se = static_err_of_current_device())
-    B200_CUDA_TRY(cudaMemcpyAsync(h_out + 1, se, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  return b200_qmm_static_error_word_async(h_out + 1, stream);
+}
+
+const int* b200_qmm_err_word_device() { return g_err; }
+
+b200_status b200_qmm_static_error_word_async(int32_t* h_out, void* stream) {
+  *h_out = 0;
+  if (int* se = static_err_of_current_device()) B200_CUDA_TRY(cudaMemcpyAsync(h_out, se, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
   return B200_OK;
 }
 

@@ -100,3 +100,7 @@ b200_status b200_qmm_grouped_from_tokens(const b200_qweight* w, const void* d_to
 // nothing cleared): h_out[0] = the word of b200_qmm and the grouped launches, h_out[1] = the word of
 // b200_qmm_static_scratch on the current device.
 b200_status b200_qmm_error_words_async(int32_t* h_out, void* stream);
+// The first of these two words on the device; null before the first matmul.
+const int* b200_qmm_err_word_device();
+// The second one, copied as above where there is one.
+b200_status b200_qmm_static_error_word_async(int32_t* h_out, void* stream);
