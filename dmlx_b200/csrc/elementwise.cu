@@ -4,6 +4,7 @@
 
 #include "common.h"
 #include "launch.cuh"
+#include "qmm.cuh"
 
 namespace {
 
@@ -153,15 +154,20 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const 
   for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) dp[i] = sp[i];
 }
 
-// `flags` (optional) points at the pool's state words: a step whose page reservation or attention was
+// `flags` points at the pool's eight state words: a step whose page reservation or attention was
 // flagged has computed its tokens from stale pages, so the sequences keep the input token they had
 // and the step can be run again once the cause (an exhausted pool) is gone.
 __global__ void scatter_tokens_kernel(const uint32_t* __restrict__ next, const b200_pack_desc* __restrict__ desc,
                                       uint32_t* __restrict__ last_token, int n_req, const int* __restrict__ flags,
-                                      int flag_a, int flag_b) {
+                                      int flag_a, int flag_b, const int* __restrict__ qmm_err, uint32_t* __restrict__ h_next,
+                                      int* __restrict__ h_state) {
   after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (flags && (flags[flag_a] != 0 || flags[flag_b] != 0)) return;
+  // The host's copies, straight into its pinned buffers: three copies behind the kernel took 6 us each, copy and gap, of an 8-request step.
+  if (i < n_req) h_next[i] = next[i];
+  if (i < 8) h_state[i] = flags[i];
+  if (i == 8) h_state[8] = qmm_err ? *qmm_err : 0;
+  if (flags[flag_a] != 0 || flags[flag_b] != 0) return;
   if (i < n_req && desc[i].count > 0) last_token[desc[i].seq_slot] = next[i];
 }
 
@@ -175,12 +181,13 @@ b200_status b200_gather_rows(const void* d_src, const int32_t* d_idx, void* d_ds
   return B200_OK;
 }
 
-// The sampled token of request i becomes the next decode input of its sequence slot.
+// The sampled token of request i becomes the next decode input of its sequence slot.  Pinned host buffers: h_next[n_req] gets the tokens,
+// h_state[0..7] the pool's state words, h_state[8] the matmuls' error word.
 b200_status b200_scatter_tokens(const uint32_t* d_next, const b200_pack_desc* d_desc, uint32_t* d_last_token, int32_t n_req,
-                                const int* d_flags, int flag_a, int flag_b, void* stream) {
+                                const int* d_flags, int flag_a, int flag_b, uint32_t* h_next, int32_t* h_state, void* stream) {
   if (n_req <= 0) return B200_OK;
   launch_after(scatter_tokens_kernel, (n_req + 127) / 128, 128, 0, (cudaStream_t)stream, d_next, d_desc, d_last_token, n_req, d_flags,
-                                                                              flag_a, flag_b);
+               flag_a, flag_b, b200_qmm_err_word_device(), h_next, h_state);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }

@@ -9,11 +9,10 @@
 #include "qmm.cuh"
 
 b200_model::~b200_model() {
-  void* dev[] = {logits, d_desc, d_prefill, d_tokens, d_next, d_last_token, d_cu, d_pos, d_row_to_req, d_row_seq, d_row_ctx, d_logit_row,
+  void* dev[] = {logits, d_desc, d_tokens, d_next, d_last_token, d_cu, d_pos, d_row_to_req, d_row_seq, d_row_ctx, d_logit_row,
                  d_samp, d_logprobs};
   for (void* p : dev) if (p) cudaFree(p);
   if (h_desc) cudaFreeHost(h_desc);
-  if (h_prefill) cudaFreeHost(h_prefill);
   if (h_next) cudaFreeHost(h_next);
   if (h_samp) cudaFreeHost(h_samp);
   if (h_state) cudaFreeHost(h_state);
@@ -26,7 +25,7 @@ b200_status b200_model::alloc_step(int vocab_, int max_rows_, int max_reqs_, int
   const int R = max_rows, Q = max_reqs;
   auto dev = [](auto** p, size_t bytes) { return cudaMalloc((void**)p, bytes) == cudaSuccess; };
   auto pin = [](auto** p, size_t bytes) { return cudaMallocHost((void**)p, bytes) == cudaSuccess; };
-  if (!dev(&logits, (size_t)Q * vocab * (f32 ? 4 : 2)) || !dev(&d_desc, sizeof(b200_pack_desc) * Q) || !dev(&d_prefill, sizeof(uint32_t) * R) ||
+  if (!dev(&logits, (size_t)Q * vocab * (f32 ? 4 : 2)) || !dev(&d_desc, sizeof(b200_pack_desc) * Q + sizeof(uint32_t) * R) ||
       !dev(&d_tokens, sizeof(uint32_t) * R) || !dev(&d_next, sizeof(uint32_t) * Q) || !dev(&d_last_token, sizeof(uint32_t) * max_seqs) ||
       !dev(&d_cu, sizeof(int32_t) * (Q + 1)) || !dev(&d_pos, sizeof(int32_t) * R) || !dev(&d_row_to_req, sizeof(int32_t) * R) ||
       !dev(&d_row_seq, sizeof(int32_t) * R) || !dev(&d_row_ctx, sizeof(int32_t) * R) || !dev(&d_logit_row, sizeof(int32_t) * Q) ||
@@ -34,11 +33,13 @@ b200_status b200_model::alloc_step(int vocab_, int max_rows_, int max_reqs_, int
     b200_set_error("model: device allocation of the step buffers failed");
     return B200_ERR_CUDA;
   }
-  if (!pin(&h_desc, sizeof(b200_pack_desc) * Q) || !pin(&h_prefill, sizeof(uint32_t) * R) || !pin(&h_next, sizeof(uint32_t) * Q) ||
+  if (!pin(&h_desc, sizeof(b200_pack_desc) * Q + sizeof(uint32_t) * R) || !pin(&h_next, sizeof(uint32_t) * Q) ||
       !pin(&h_samp, sizeof(b200_sample_params) * Q) || !pin(&h_state, sizeof(int32_t) * 16)) {
     b200_set_error("pinned host allocation failed");
     return B200_ERR_CUDA;
   }
+  d_prefill = reinterpret_cast<uint32_t*>(d_desc + Q);  // (behind the descriptors, so that one copy brings both)
+  h_prefill = reinterpret_cast<uint32_t*>(h_desc + Q);
   B200_CUDA_TRY(cudaMemset(d_last_token, 0, sizeof(uint32_t) * max_seqs));
   return B200_OK;
 }
@@ -127,7 +128,7 @@ b200_status b200_model::eager(b200_kv* kv, const b200_pack_desc* desc, int n_req
   } else {
     MODEL_STEP(b200_argmax(logits, n_req, vocab, d_next, stream));
   }
-  MODEL_STEP(b200_scatter_tokens(d_next, desc, d_last_token, n_req, kv->dev.state, ST_ERR, ST_ATTN_ERR, stream));
+  MODEL_STEP(b200_scatter_tokens(d_next, desc, d_last_token, n_req, kv->dev.state, ST_ERR, ST_ATTN_ERR, h_next, h_state, stream));
   launches += g_b200_launch_counter - launches_before;
   return B200_OK;
 }
@@ -165,9 +166,14 @@ b200_status b200_model::step(b200_kv* kv, const b200_pack_desc* descs, int n_req
       return B200_ERR_INVALID_ARGUMENT;
     }
   if (n_prefill_tokens > 0) std::memcpy(h_prefill, h_prefill_tokens, sizeof(uint32_t) * n_prefill_tokens);
-  if (n_req > 0) B200_CUDA_TRY(cudaMemcpyAsync(d_desc, h_desc, sizeof(b200_pack_desc) * n_req, cudaMemcpyHostToDevice, s));
-  if (n_prefill_tokens > 0)
-    B200_CUDA_TRY(cudaMemcpyAsync(d_prefill, h_prefill, sizeof(uint32_t) * n_prefill_tokens, cudaMemcpyHostToDevice, s));
+  // descriptors and tokens in one copy, unless the descriptors that are not used would take longer than a second one
+  if (n_prefill_tokens > 0 && sizeof(b200_pack_desc) * max_reqs <= 65536) {
+    B200_CUDA_TRY(cudaMemcpyAsync(d_desc, h_desc, sizeof(b200_pack_desc) * max_reqs + sizeof(uint32_t) * n_prefill_tokens, cudaMemcpyHostToDevice, s));
+  } else {
+    if (n_req > 0) B200_CUDA_TRY(cudaMemcpyAsync(d_desc, h_desc, sizeof(b200_pack_desc) * n_req, cudaMemcpyHostToDevice, s));
+    if (n_prefill_tokens > 0)
+      B200_CUDA_TRY(cudaMemcpyAsync(d_prefill, h_prefill, sizeof(uint32_t) * n_prefill_tokens, cudaMemcpyHostToDevice, s));
+  }
   sampling = samp_n > 0;
   if (sampling) {
     if (samp_n != n_req) {
@@ -178,9 +184,13 @@ b200_status b200_model::step(b200_kv* kv, const b200_pack_desc* descs, int n_req
   }
   b200_status st = forward(kv, d_desc, n_req, (int)total, d_prefill, stream);
   if (st != B200_OK) return st;
-  if (n_req > 0) B200_CUDA_TRY(cudaMemcpyAsync(h_next, d_next, sizeof(uint32_t) * n_req, cudaMemcpyDeviceToHost, s));
-  B200_CUDA_TRY(cudaMemcpyAsync(h_state, kv->dev.state, sizeof(int32_t) * 8, cudaMemcpyDeviceToHost, s));
-  st = b200_qmm_error_words_async(h_state + 8, stream);
+  if (n_req > 0 && total > 0) {  // the last kernel has written tokens and words to the host
+    st = b200_qmm_static_error_word_async(h_state + 9, stream);
+  } else {
+    if (n_req > 0) B200_CUDA_TRY(cudaMemcpyAsync(h_next, d_next, sizeof(uint32_t) * n_req, cudaMemcpyDeviceToHost, s));
+    B200_CUDA_TRY(cudaMemcpyAsync(h_state, kv->dev.state, sizeof(int32_t) * 8, cudaMemcpyDeviceToHost, s));
+    st = b200_qmm_error_words_async(h_state + 8, stream);
+  }
   if (st != B200_OK) return st;
   B200_CUDA_TRY(cudaStreamSynchronize(s));
   for (int i = 0; i < n_req; ++i) h_next_tokens[i] = h_next[i];

@@ -14,7 +14,7 @@
 
 b200_status b200_gather_rows(const void* d_src, const int32_t* d_idx, void* d_dst, int32_t rows, int32_t hidden, void* stream);
 b200_status b200_scatter_tokens(const uint32_t* d_next, const b200_pack_desc* d_desc, uint32_t* d_last_token, int32_t n_req,
-                                const int* d_flags, int flag_a, int flag_b, void* stream);
+                                const int* d_flags, int flag_a, int flag_b, uint32_t* h_next, int32_t* h_state, void* stream);
 
 struct b200_model {
   int vocab = 0, max_rows = 0, max_reqs = 0, max_seqs = 0;
@@ -31,7 +31,7 @@ struct b200_model {
   // pinned staging
   b200_pack_desc* h_desc = nullptr;
   uint32_t *h_prefill = nullptr, *h_next = nullptr;
-  int32_t* h_state = nullptr;  // [8] pool state words + [2] matmul error words
+  int32_t* h_state = nullptr;  // [8] pool state words + [2] matmul error words; written by the step's last kernel, as h_next is
   std::vector<int32_t> want;   // extra logit rows of the coming step (b200_model_want_logits, used once)
   int last_logit_rows = 0;
   // per-request sampler rows of the coming step (b200_model_set_samplers, used once)
