@@ -404,7 +404,8 @@ def sample_rows(logits: torch.Tensor, rows, context: Optional[Sequence[Sequence[
     Returns (tokens int32 [R], logprobs float32 [R] or None)."""
     assert logits.dtype in (torch.bfloat16, torch.float32) and logits.is_contiguous()
     n, v = logits.shape
-    d_params = torch.from_numpy(sample_params_array(rows)).to(logits.device)
+    # (from pinned memory: a pageable upload waits for the kernels ahead of it in the stream)
+    d_params = torch.from_numpy(sample_params_array(rows)).pin_memory().to(logits.device, non_blocking=True)
     tokens = torch.empty(n, dtype=torch.int32, device=logits.device)
     lp = torch.empty(n, dtype=torch.float32, device=logits.device) if logprobs else None
     d_ctx = d_off = scratch = None
