@@ -116,29 +116,28 @@ __global__ void __launch_bounds__(1024) window_plan_kernel(const int* __restrict
     ppc = forced_ppc;
   } else {
     constexpr int kCand = Lengths::kCand;
-    long long chunks[kCand] = {}, slots[kCand] = {}, pages_sum = 0;
+    // (a thread's counts stop at 2^25, where no plan is chosen any more, so that a warp's sums are single reductions of 32 bits; as 64-bit shuffles
+    // they were half of the 19 us that 18 lengths took for 16 rows)
+    constexpr int kMost = 1 << 25;
+    int chunks[kCand] = {}, slots[kCand] = {}, pages_sum = 0;
     int longest = 0;
     for (int g = tid; g < n_groups; g += blockDim.x) {
       const int first = group_first[g], next = group_first[g + 1];
       const int pages = group_pages(row_ctx[first], row_ctx[next - 1], window, page_size);
-      pages_sum += pages;
+      pages_sum = min(pages_sum + pages, kMost);
       longest = max(longest, pages);
 #pragma unroll
       for (int k = 0; k < kCand; ++k) {
         const int c = k == kCand - 1 ? 1 : (pages + Lengths::at(k) - 1) / Lengths::at(k);
-        chunks[k] += c;
-        slots[k] += c > 1 ? c * (next - first) : 0;
+        chunks[k] = min(chunks[k] + c, kMost);
+        slots[k] = min(slots[k] + (c > 1 ? (int)min((long long)c * (next - first), (long long)kMost) : 0), kMost);
       }
     }
     __shared__ long long s_red[32][2 * kCand + 2];
 #pragma unroll
     for (int k = 0; k < 2 * kCand + 2; ++k) {
-      long long v = k < kCand ? chunks[k < kCand ? k : 0] : (k < 2 * kCand ? slots[k < 2 * kCand ? (k >= kCand ? k - kCand : 0) : 0] : (k == 2 * kCand ? pages_sum : longest));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const long long w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = k == 2 * kCand + 1 ? (v > w ? v : w) : v + w;
-      }
+      const int mine = k < kCand ? chunks[k < kCand ? k : 0] : (k < 2 * kCand ? slots[k < 2 * kCand ? (k >= kCand ? k - kCand : 0) : 0] : (k == 2 * kCand ? pages_sum : longest));
+      const int v = k == 2 * kCand + 1 ? __reduce_max_sync(0xffffffffu, mine) : __reduce_add_sync(0xffffffffu, mine);
       if ((tid & 31) == 0) s_red[tid >> 5][k] = v;
     }
     __syncthreads();
@@ -152,11 +151,12 @@ __global__ void __launch_bounds__(1024) window_plan_kernel(const int* __restrict
       s_red[0][tid] = tid == 2 * kCand + 1 ? most : sum;
     }
     __syncthreads();
-    if (tid == 0) {
+    if (tid < 32) {  // a lane per length
       const long long* tot = s_red[0];
       const float per = (float)items_per_chunk / (float)n_workers, load = (float)tot[2 * kCand] * per;
       float best = 3.4e38f;
-      for (int k = 0; k < kCand; ++k) {
+      int at = 0;
+      if (const int k = tid; k < kCand) {
         const float length = fminf(k == kCand - 1 ? 1e9f : (float)Lengths::at(k), (float)tot[2 * kCand + 1]);
         const float items = (float)tot[k] * per;
         float t;
@@ -167,11 +167,19 @@ __global__ void __launch_bounds__(1024) window_plan_kernel(const int* __restrict
           t = fmaxf(load, length) + (items > 1.f ? 0.5f * length : 0.f) + item_cost * items;
         }
         if (tot[kCand + k] > 0) t += 3.f + slot_cost * (float)tot[kCand + k] * per;
-        if (t < best) { best = t; carry_chunks = k; }
+        best = t;
+        at = k;
       }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {  // the shortest of the best
+        const float t = __shfl_xor_sync(0xffffffffu, best, o);
+        const int k = __shfl_xor_sync(0xffffffffu, at, o);
+        if (t < best || (t == best && k < at)) { best = t; at = k; }
+      }
+      if (tid == 0) carry_chunks = at;
       // Equal shares: about one more item per worker than whole groups would make.  (Not for prompts: there the workers should walk
       // neighbouring groups side by side, which read the same pages.)
-      if (kCand > 6 && items_per_chunk == 1 && n_groups <= 4 * n_workers) {
+      if (tid == 0 && kCand > 6 && items_per_chunk == 1 && n_groups <= 4 * n_workers) {
         const long long pages = tot[2 * kCand];
         const int share = max((int)((pages + n_workers - 1) / n_workers), 4);
         const float cuts = (float)pages / (float)share, items = ((float)n_groups + cuts) / (float)n_workers;
@@ -725,7 +733,9 @@ b200_status b200_attn_make_plan(b200_kv* kv, int32_t window, int32_t qt, int32_t
   }
   const int forced = b200_attn_pages_per_chunk <= 0 ? 0 : std::min(std::max(b200_attn_pages_per_chunk, 1), 1 << 20);
   auto* kernel = fine ? window_plan_kernel<FineLengths> : window_plan_kernel<CoarseLengths>;
-  launch_after(kernel, 1, 1024, 0, (cudaStream_t)stream, d_row_seq, d_row_ctx, total_rows, kv->cfg.page_size, window, qt,
+  // (a thread per row where that is enough: fewer warps for every barrier and scan)
+  const int threads = std::min(1024, std::max(64, (total_rows + 31) / 32 * 32));
+  launch_after(kernel, 1, threads, 0, (cudaStream_t)stream, d_row_seq, d_row_ctx, total_rows, kv->cfg.page_size, window, qt,
                                                           items_per_chunk, n_workers, forced, kv->max_chunks, item_cost, slot_cost,
                                                           p->buf, p->buf + R, p->buf + 2 * R, p->buf + 3 * R, p->buf + 4 * R, p->buf + 5 * R);
   B200_LAUNCH_CHECK();

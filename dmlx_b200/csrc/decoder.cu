@@ -402,10 +402,24 @@ __global__ void __launch_bounds__(256) decoder_final_kernel(const float* __restr
   after_previous();
   __shared__ float part[32];
   const float* xr = x + (size_t)max(idx[blockIdx.x], 0) * hidden;
-  float ss = 0.f;
-  for (int c = threadIdx.x; c < hidden; c += blockDim.x) ss += xr[c] * xr[c];
+  constexpr int kHeld = 8;  // columns of a thread that stay in registers, with their weights on the way during the sum
+  float ss = 0.f, v[kHeld], g[kHeld];
+#pragma unroll
+  for (int k = 0; k < kHeld; ++k) {
+    const int c = threadIdx.x + k * blockDim.x;
+    v[k] = c < hidden ? xr[c] : 0.f;
+    g[k] = c < hidden ? w[c] : 0.f;
+  }
+#pragma unroll
+  for (int k = 0; k < kHeld; ++k) ss += v[k] * v[k];
+  for (int c = threadIdx.x + kHeld * blockDim.x; c < hidden; c += blockDim.x) ss += xr[c] * xr[c];
   const float r = 1.0f / sqrtf(block_sum(ss, part) / (float)hidden + eps);
-  for (int c = threadIdx.x; c < hidden; c += blockDim.x) st(out + (size_t)blockIdx.x * out_stride + c, xr[c] * r * w[c]);
+#pragma unroll
+  for (int k = 0; k < kHeld; ++k) {
+    const int c = threadIdx.x + k * blockDim.x;
+    if (c < hidden) st(out + (size_t)blockIdx.x * out_stride + c, v[k] * r * g[k]);
+  }
+  for (int c = threadIdx.x + kHeld * blockDim.x; c < hidden; c += blockDim.x) st(out + (size_t)blockIdx.x * out_stride + c, xr[c] * r * w[c]);
 }
 
 __global__ void __launch_bounds__(256) decoder_logits_kernel(MatSrc src, float* __restrict__ logits, int vocab) {

@@ -1,10 +1,13 @@
 // Row-wise pieces of the layer stack: RMSNorm, RoPE, embedding gather, greedy argmax.
 // All activations are bf16 with f32 arithmetic; every kernel is a single pass over its rows.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include "common.h"
 #include "launch.cuh"
 #include "qmm.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -91,12 +94,15 @@ __global__ void embed_kernel(const __nv_bfloat16* __restrict__ table, const uint
 }
 
 // First strict maximum of each row (ties keep the smaller index).
+// A row belongs to a cluster of CTAs, a contiguous part each (16 rows of 32000 f32 values: ARGMAX).
 template <typename T>
 __global__ void argmax_kernel(const T* __restrict__ logits, int vocab, uint32_t* __restrict__ out) {
   after_previous();
   __shared__ float s_val[32];
   __shared__ int s_idx[32];
-  const int row = blockIdx.x;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int parts = cluster.num_blocks(), part = cluster.block_rank(), row = blockIdx.x / parts;
+  const int per = ((vocab + parts - 1) / parts + 7) / 8 * 8, lo = min(part * per, vocab), hi = min(lo + per, vocab);
   const T* lr = logits + (size_t)row * vocab;
   float best = -INFINITY;
   int bi = 0x7fffffff;
@@ -105,7 +111,7 @@ __global__ void argmax_kernel(const T* __restrict__ logits, int vocab, uint32_t*
   const bool vec = sizeof(T) == 2 && (vocab % 8 == 0) && ((reinterpret_cast<uintptr_t>(lr) & 15) == 0);
   if (vec) {
     const uint4* lv = reinterpret_cast<const uint4*>(lr);
-    for (int c = threadIdx.x; c < vocab / 8; c += blockDim.x) {
+    for (int c = lo / 8 + threadIdx.x; c < hi / 8; c += blockDim.x) {
       const uint4 q = lv[c];
       const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -116,7 +122,7 @@ __global__ void argmax_kernel(const T* __restrict__ logits, int vocab, uint32_t*
       }
     }
   } else {
-    for (int i = threadIdx.x; i < vocab; i += blockDim.x) {
+    for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
       float v = (float)lr[i];
       if (v > best || (v == best && i < bi)) { best = v; bi = i; }
     }
@@ -140,8 +146,40 @@ __global__ void argmax_kernel(const T* __restrict__ logits, int vocab, uint32_t*
       int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (better(ov, oi, best, bi)) { best = ov; bi = oi; }
     }
-    if (threadIdx.x == 0) out[row] = bi == 0x7fffffff ? 0u : (uint32_t)bi;
+    if (threadIdx.x == 0) { s_val[0] = best; s_idx[0] = bi; }
   }
+  cluster.sync();
+  if (part == 0 && threadIdx.x == 0) {
+    for (int q = 1; q < parts; ++q) {
+      const float ov = *cluster.map_shared_rank(&s_val[0], q);
+      const int oi = *cluster.map_shared_rank(&s_idx[0], q);
+      if (better(ov, oi, best, bi)) { best = ov; bi = oi; }
+    }
+    out[row] = bi == 0x7fffffff ? 0u : (uint32_t)bi;
+  }
+  cluster.sync();  // nobody leaves while its shared memory may be read
+}
+
+template <typename T>
+b200_status launch_argmax(const T* logits, int rows, int vocab, uint32_t* out, cudaStream_t s) {
+  // parts of 4096 values and more, as long as the CTAs run at once (a cluster's stay within a GPC: some 32 clusters of eight at two CTAs per SM)
+  int parts = 1;
+  while (parts < 8 && vocab >= parts * 8192 && (long long)rows * parts * 2 <= 256) parts *= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)rows * parts);
+  cfg.blockDim = dim3(parts > 1 ? 512 : 1024);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = parts;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (as launch_after)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, argmax_kernel<T>, logits, vocab, out));
+  B200_LAUNCH_CHECK();
+  return B200_OK;
 }
 
 __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ idx,
@@ -235,18 +273,14 @@ b200_status b200_argmax(const void* d_logits, int32_t rows, int32_t vocab, uint3
   b200_status st = b200_require_device();
   if (st != B200_OK) return st;
   if (rows <= 0) return B200_OK;
-  launch_after(argmax_kernel<__nv_bfloat16>, rows, 1024, 0, (cudaStream_t)stream, (const __nv_bfloat16*)d_logits, vocab, d_out);
-  B200_LAUNCH_CHECK();
-  return B200_OK;
+  return launch_argmax((const __nv_bfloat16*)d_logits, rows, vocab, d_out, (cudaStream_t)stream);
 }
 
 b200_status b200_argmax_f32(const float* d_logits, int32_t rows, int32_t vocab, uint32_t* d_out, void* stream) {
   b200_status st = b200_require_device();
   if (st != B200_OK) return st;
   if (rows <= 0) return B200_OK;
-  launch_after(argmax_kernel<float>, rows, 1024, 0, (cudaStream_t)stream, d_logits, vocab, d_out);
-  B200_LAUNCH_CHECK();
-  return B200_OK;
+  return launch_argmax(d_logits, rows, vocab, d_out, (cudaStream_t)stream);
 }
 
 }  // extern "C"

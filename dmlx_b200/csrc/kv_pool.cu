@@ -25,6 +25,7 @@
 #include "common.h"
 #include "kv_pool.cuh"
 #include "launch.cuh"
+#include "pack.cuh"
 #include "tma.cuh"
 
 static int g_device_state = -1;  // -1 unknown, 0 none, 1 ok
@@ -120,8 +121,7 @@ __device__ int4 block_exscan4(int4 v, int4* total, int4* warp_sums) {
 // One CTA.  See b200_kv_reserve in the header for the contract.  A chain of dependent loads and barriers, so up to 256 requests take a thread each
 // in a block of 256: 8 requests 9.0 -> 3.4 us, 61 requests 13.7 -> 5.2.
 template <int THREADS, int ITEMS>
-__global__ void __launch_bounds__(THREADS) reserve_kernel(KvDev d, const b200_pack_desc* desc, int n_req) {
-  after_previous();
+__device__ __forceinline__ void reserve(const KvDev& d, const b200_pack_desc* desc, int n_req) {
   __shared__ int4 warp_sums[32], s_total;  // {pages needed, pages touched, copies, rows}
   __shared__ int s_any_cow;
   const int tid = threadIdx.x;
@@ -250,6 +250,22 @@ __global__ void __launch_bounds__(THREADS) reserve_kernel(KvDev d, const b200_pa
     d.state[ST_N_TOUCH] = s_total.y;
     d.state[ST_N_COW] = s_total.z;
   }
+}
+
+template <int THREADS, int ITEMS>
+__global__ void __launch_bounds__(THREADS) reserve_kernel(KvDev d, const b200_pack_desc* desc, int n_req) {
+  after_previous();
+  reserve<THREADS, ITEMS>(d, desc, n_req);
+}
+// Small steps: one block packs the batch, another one reserves its pages (a launch each for the scan, the rows and the pages were 5 us more of an
+// 8-request step's chain).
+constexpr int kSmallStep = 256;
+__global__ void __launch_bounds__(kSmallStep) pack_reserve_kernel(KvDev d, const b200_pack_desc* __restrict__ desc, int n_req,
+                                                                  const uint32_t* __restrict__ prefill_tokens, const uint32_t* __restrict__ last_token,
+                                                                  int total_rows, PackOut out) {
+  after_previous();
+  if (blockIdx.x == 0) reserve<kSmallStep, 1>(d, desc, n_req);
+  else pack_by_block<kSmallStep>(desc, n_req, prefill_tokens, last_token, total_rows, out);
 }
 
 // Copies every queued CoW page (all layers, K and V, scales for FP8 pools).
@@ -813,6 +829,13 @@ b200_status b200_kv_filter(b200_kv* kv, const int32_t* keep, int32_t n_keep) {
   return b200_kv_release(kv, drop.data(), (int)drop.size());
 }
 
+static b200_status copy_reserved_pages(b200_kv* kv, cudaStream_t s) {
+  dim3 grid(std::min(kv->cfg.max_seqs, 256), kv->cfg.n_layers * 2);
+  launch_after(cow_copy_kernel, grid, 256, 0, s, kv->dev);
+  B200_LAUNCH_CHECK();
+  return B200_OK;
+}
+
 b200_status b200_kv_reserve(b200_kv* kv, const b200_pack_desc* d_desc, int32_t n_req, void* stream) {
   if (n_req < 0 || n_req > kReserveThreads * kReserveItems) {
     b200_set_error("reserve: %d requests in one step (limit %d)", n_req, kReserveThreads * kReserveItems);
@@ -822,11 +845,22 @@ b200_status b200_kv_reserve(b200_kv* kv, const b200_pack_desc* d_desc, int32_t n
   if (n_req <= 256) launch_after(reserve_kernel<256, 1>, 1, 256, 0, s, kv->dev, d_desc, n_req);
   else launch_after(reserve_kernel<kReserveThreads, kReserveItems>, 1, kReserveThreads, 0, s, kv->dev, d_desc, n_req);
   B200_LAUNCH_CHECK();
-  dim3 grid(std::min(kv->cfg.max_seqs, 256), kv->cfg.n_layers * 2);
-  launch_after(cow_copy_kernel, grid, 256, 0, s, kv->dev);
-  B200_LAUNCH_CHECK();
-  return B200_OK;
+  return copy_reserved_pages(kv, s);
 }
+
+}  // extern "C"
+bool b200_kv_packs(int32_t n_req, int32_t total_rows) { return n_req <= kSmallStep && total_rows <= 4 * kSmallStep; }
+
+b200_status b200_kv_pack_reserve(b200_kv* kv, const b200_pack_desc* d_desc, int32_t n_req, const uint32_t* d_prefill_tokens, const uint32_t* d_last_token,
+                                 int32_t* d_cu_seqlens, uint32_t* d_token_ids, int32_t* d_position_ids, int32_t* d_row_to_req, int32_t* d_row_seq,
+                                 int32_t* d_row_ctx, int32_t* d_last_row, int32_t total_rows, void* stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  launch_after(pack_reserve_kernel, 2, kSmallStep, 0, s, kv->dev, d_desc, n_req, d_prefill_tokens, d_last_token, total_rows,
+               PackOut{d_cu_seqlens, d_position_ids, d_row_to_req, d_row_seq, d_row_ctx, d_last_row, d_token_ids});
+  B200_LAUNCH_CHECK();
+  return copy_reserved_pages(kv, s);
+}
+extern "C" {
 
 b200_status b200_kv_append(b200_kv* kv, int32_t layer, const void* d_k_rows, const void* d_v_rows,
                            int32_t total_rows, void* stream) {

@@ -119,3 +119,9 @@ b200_status b200_paged_attn_decode_strided(b200_kv* kv, int32_t layer, const voi
 b200_status b200_paged_attn_prefill_strided(b200_kv* kv, int32_t layer, const void* d_q, int32_t q_stride,
                                             const int32_t* d_row_seq, const int32_t* d_row_ctx, int32_t total_rows,
                                             void* d_out, void* stream, int32_t reuse_plan);
+
+// b200_pack_batch and b200_kv_reserve in one launch, for the steps that b200_kv_packs says it takes.
+bool b200_kv_packs(int32_t n_req, int32_t total_rows);
+b200_status b200_kv_pack_reserve(b200_kv* kv, const b200_pack_desc* d_desc, int32_t n_req, const uint32_t* d_prefill_tokens, const uint32_t* d_last_token,
+                                 int32_t* d_cu_seqlens, uint32_t* d_token_ids, int32_t* d_position_ids, int32_t* d_row_to_req, int32_t* d_row_seq,
+                                 int32_t* d_row_ctx, int32_t* d_last_row, int32_t total_rows, void* stream);

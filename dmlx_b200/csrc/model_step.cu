@@ -114,11 +114,17 @@ b200_status b200_model::eager(b200_kv* kv, const b200_pack_desc* desc, int n_req
   if (n_req == 0 || total_rows == 0) return B200_OK;
   const long long launches_before = g_b200_launch_counter;
   cudaStream_t cs = (cudaStream_t)stream;
-  MODEL_STEP(b200_pack_batch(desc, n_req, d_prefill_tokens, d_last_token, d_cu, d_tokens, d_pos, d_row_to_req, d_row_seq, d_row_ctx,
-                             d_logit_row, total_rows, stream));
+  const bool small = b200_kv_packs(n_req, total_rows);
+  if (small) {
+    MODEL_STEP(b200_kv_pack_reserve(kv, desc, n_req, d_prefill_tokens, d_last_token, d_cu, d_tokens, d_pos, d_row_to_req, d_row_seq, d_row_ctx,
+                                    d_logit_row, total_rows, stream));
+  } else {
+    MODEL_STEP(b200_pack_batch(desc, n_req, d_prefill_tokens, d_last_token, d_cu, d_tokens, d_pos, d_row_to_req, d_row_seq, d_row_ctx,
+                               d_logit_row, total_rows, stream));
+  }
   if (!want.empty())
     B200_CUDA_TRY(cudaMemcpyAsync(d_logit_row + n_req, want.data(), sizeof(int32_t) * want.size(), cudaMemcpyHostToDevice, cs));
-  MODEL_STEP(b200_kv_reserve(kv, desc, n_req, stream));
+  if (!small) MODEL_STEP(b200_kv_reserve(kv, desc, n_req, stream));
   st = run_layers(kv, n_req, total_rows, n_logits, stream);
   if (st != B200_OK) return st;
   if (sampling) {

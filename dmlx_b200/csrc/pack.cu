@@ -3,6 +3,7 @@
 // src/batch_builder.zig:122-205 — the mask is implied by (row_seq, row_ctx).
 #include "common.h"
 #include "launch.cuh"
+#include "pack.cuh"
 
 namespace {
 
@@ -66,14 +67,7 @@ __global__ void pack_fill_kernel(const b200_pack_desc* __restrict__ desc, int n_
     int mid = (lo + hi + 1) >> 1;
     if (cu_seqlens[mid] <= row) lo = mid; else hi = mid - 1;
   }
-  b200_pack_desc d = desc[lo];
-  int j = row - cu_seqlens[lo];
-  int pos = d.base_pos + j;
-  token_ids[row] = d.src_offset >= 0 ? prefill_tokens[d.src_offset + j] : last_token[d.seq_slot];
-  position_ids[row] = pos;
-  row_to_req[row] = lo;
-  row_seq[row] = d.seq_slot;
-  row_ctx[row] = pos + 1;
+  pack_row(desc[lo], lo, cu_seqlens[lo], row, prefill_tokens, last_token, PackOut{nullptr, position_ids, row_to_req, row_seq, row_ctx, nullptr, token_ids});
 }
 
 }  // namespace

@@ -1548,8 +1548,12 @@ constexpr int kFewRows = 16, kFewWarps = 8;
 
 template <int MT, int NT>
 __global__ void __launch_bounds__(kFewWarps * 32) qmm_few_kernel(QmmArgs a) {
-  after_previous();
   constexpr int R = MT * 16, TOK = NT * 8, U = 2 / MT;
+  // While the kernels ahead in the stream end, this CTA's weights are brought into L2, R neighbouring rows of every block.
+  if (!a.items)
+    for (int c = threadIdx.x; c < a.kc; c += kFewWarps * 32)
+      ptx::bulk_prefetch_l2(a.blocks + ((size_t)(blockIdx.x * R / kTileN) * a.kc + c) * (kTileN * 128) + (size_t)(blockIdx.x * R % kTileN) * 128, R * 128);
+  after_previous();
   __shared__ float red[kFewWarps][TOK][R + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   int t0 = 0, rows_here = a.rows;
