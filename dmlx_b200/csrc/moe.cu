@@ -15,6 +15,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "common.h"
@@ -33,56 +34,56 @@ constexpr int kMaxRouterTop = 32;
 
 __device__ __forceinline__ bool beats(float va, int ia, float vb, int ib) { return va > vb || (va == vb && ia > ib); }
 
-// One warp per token.  E <= 1024 (32 experts per lane).
-template <typename LogitT>
-__global__ void route_kernel(const LogitT* __restrict__ logits, const float* __restrict__ bias, int n_tokens, int n_experts,
-                             int k, int scoring, float route_scale, uint32_t* __restrict__ out_idx,
-                             float* __restrict__ out_w, int* __restrict__ counts) {
-  after_previous();
-  const int token = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (token >= n_tokens) return;
-  constexpr int PER = kMaxExperts / 32;
+// A warp chooses a token's experts: lane j < k gets the j-th of them, in ascending (score, index), and its weight.  Up to 32 * PER experts; PER is
+// known to the compiler, so that a lane's scores stay in registers (4096 tokens, 32 experts: ROUTE).
+template <int PER, typename LogitT>
+__device__ __forceinline__ void route_token(const LogitT* __restrict__ logits, const float* __restrict__ bias, int n_experts, int k, int scoring,
+                                            float route_scale, int lane, int& expert, float& weight) {
   float sc[PER];      // unbiased scores
   float ch[PER];      // scores used for the choice
-  const int per = (n_experts + 31) / 32;
   float mx = -INFINITY;
-  for (int i = 0; i < per; ++i) {
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
     const int e = i * 32 + lane;
-    float v = -INFINITY;
-    if (e < n_experts) v = (float)logits[(size_t)token * n_experts + e];
-    sc[i] = v;
-    mx = fmaxf(mx, v);
+    sc[i] = e < n_experts ? (float)logits[e] : -INFINITY;
+    mx = fmaxf(mx, sc[i]);
   }
   if (scoring == 0) {  // softmax in f32 (deepseek_v4.zig:562-564)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     float sum = 0.f;
-    for (int i = 0; i < per; ++i) {
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
       const float e = (i * 32 + lane < n_experts) ? expf(sc[i] - mx) : 0.f;
       sc[i] = e;
       sum += e;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    for (int i = 0; i < per; ++i) sc[i] = sc[i] / sum;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) sc[i] = sc[i] / sum;
   } else if (scoring == 1) {  // sigmoid
-    for (int i = 0; i < per; ++i) sc[i] = 1.0f / (1.0f + expf(-sc[i]));
+#pragma unroll
+    for (int i = 0; i < PER; ++i) sc[i] = 1.0f / (1.0f + expf(-sc[i]));
   } else {  // sqrt(softplus)
-    for (int i = 0; i < per; ++i) sc[i] = sqrtf(log1pf(expf(sc[i])));
+#pragma unroll
+    for (int i = 0; i < PER; ++i) sc[i] = sqrtf(log1pf(expf(sc[i])));
   }
-  for (int i = 0; i < per; ++i) {
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
     const int e = i * 32 + lane;
     ch[i] = e < n_experts ? sc[i] + (bias ? bias[e] : 0.f) : -INFINITY;
   }
   // k rounds of warp arg-max under (score, index) order; results come out descending.
-  float sel_w[kMaxTopK];
-  int sel_e[kMaxTopK];
+  expert = 0;
+  weight = 0.f;
   for (int r = 0; r < k; ++r) {
     float bv = -INFINITY;
-    int be = -1, bi = -1;
-    for (int i = 0; i < per; ++i) {
+    int be = -1;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
       const int e = i * 32 + lane;
-      if (e < n_experts && beats(ch[i], e, bv, be)) { bv = ch[i]; be = e; bi = i; }
+      if (e < n_experts && beats(ch[i], e, bv, be)) { bv = ch[i]; be = e; }
     }
     float wv = bv;
     int we = be;
@@ -94,24 +95,94 @@ __global__ void route_kernel(const LogitT* __restrict__ logits, const float* __r
     }
     // the owning lane retires the winner and publishes its unbiased score
     float w_unbiased = 0.f;
-    if (we == be && bi >= 0) { w_unbiased = sc[bi]; ch[bi] = -INFINITY; }
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (we >= 0 && we == i * 32 + lane) { w_unbiased = sc[i]; ch[i] = -INFINITY; }
     w_unbiased = __shfl_sync(0xffffffffu, w_unbiased, we & 31);
-    sel_w[r] = w_unbiased;
-    sel_e[r] = we;
+    if (lane == k - 1 - r) { expert = max(we, 0); weight = w_unbiased; }  // (no score is a number: expert 0, with weight 0)
   }
-  if (lane == 0) {
-    float denom = 1.0f;
-    if (scoring != 0) {  // non-softmax scores are renormalised over the selection (deepseek_v4.zig:663-672)
-      float s = 0.f;
-      for (int r = k - 1; r >= 0; --r) s += sel_w[r];  // ascending order, as the reference sums
-      denom = s + 1e-20f;
+  if (scoring != 0) {  // non-softmax scores are renormalised over the selection (deepseek_v4.zig:663-672)
+    float s = 0.f;
+    for (int j = 0; j < k; ++j) s += __shfl_sync(0xffffffffu, weight, j);  // ascending order, as the reference sums
+    weight = weight / (s + 1e-20f);
+  }
+  weight *= route_scale;
+}
+
+// One warp per token.  E <= 1024 (32 experts per lane).
+template <typename LogitT, int PER>
+__global__ void __launch_bounds__(256) route_kernel(const LogitT* __restrict__ logits, const float* __restrict__ bias, int n_tokens, int n_experts,
+                                                    int k, int scoring, float route_scale, uint32_t* __restrict__ out_idx,
+                                                    float* __restrict__ out_w, int* __restrict__ counts) {
+  after_previous();
+  const int token = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (token >= n_tokens) return;
+  int expert;
+  float weight;
+  route_token<PER>(logits + (size_t)token * n_experts, bias, n_experts, k, scoring, route_scale, lane, expert, weight);
+  if (lane < k) {
+    out_idx[(size_t)token * k + lane] = (uint32_t)expert;
+    out_w[(size_t)token * k + lane] = weight;
+    if (counts) atomicAdd(&counts[expert], 1);
+  }
+}
+
+// Few tokens: routing, the experts' offsets and work items, the places of the assignments and the sorted rows' weights by one block.  As kernels of
+// their own, with the counters cleared ahead of them, they were five links of the chain (24 tokens: MOE_SMALL).
+constexpr int kSmallAssign = 512;  // assignments: their ranks are counted one by one
+template <int PER>
+__global__ void __launch_bounds__(1024) route_small_kernel(const __nv_bfloat16* __restrict__ logits, const float* __restrict__ bias, int n_tokens, int n_experts,
+                                                           int k, int scoring, float route_scale, int tile_rows, uint32_t* __restrict__ out_idx,
+                                                           float* __restrict__ out_w, int* __restrict__ counts, int* __restrict__ offsets,
+                                                           int4* __restrict__ items, int* __restrict__ n_items, int* __restrict__ order,
+                                                           int* __restrict__ inv_order, float* __restrict__ row_scales) {
+  after_previous();
+  __shared__ int s_expert[kSmallAssign], s_count[kMaxExperts], s_off[kMaxExperts], warp_rows[32], warp_items[32];
+  __shared__ float s_weight[kSmallAssign];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_assign = n_tokens * k;
+  s_count[tid] = 0;
+  __syncthreads();
+  for (int token = warp; token < n_tokens; token += 32) {
+    int expert;
+    float weight;
+    route_token<PER>(logits + (size_t)token * n_experts, bias, n_experts, k, scoring, route_scale, lane, expert, weight);
+    if (lane < k) {
+      const int a = token * k + lane;
+      s_expert[a] = expert;
+      s_weight[a] = weight;
+      out_idx[a] = (uint32_t)expert;
+      out_w[a] = weight;
+      atomicAdd(&s_count[expert], 1);
     }
-    for (int r = 0; r < k; ++r) {
-      const int src = k - 1 - r;  // ascending (score, index)
-      out_idx[(size_t)token * k + r] = (uint32_t)sel_e[src];
-      out_w[(size_t)token * k + r] = (scoring != 0 ? sel_w[src] / denom : sel_w[src]) * route_scale;
-      if (counts) atomicAdd(&counts[sel_e[src]], 1);
-    }
+  }
+  __syncthreads();
+  // a thread per expert
+  const int rows = s_count[tid], tiles = (rows + tile_rows - 1) / tile_rows;
+  int rows_incl = rows, tiles_incl = tiles;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, rows_incl, o), b = __shfl_up_sync(0xffffffffu, tiles_incl, o);
+    if (lane >= o) { rows_incl += a; tiles_incl += b; }
+  }
+  if (lane == 31) { warp_rows[warp] = rows_incl; warp_items[warp] = tiles_incl; }
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) { rows_incl += warp_rows[w]; tiles_incl += warp_items[w]; }
+  const int first = rows_incl - rows;
+  s_off[tid] = first;
+  if (tid < n_experts) {
+    counts[tid] = rows;
+    offsets[tid] = first;
+    for (int t = 0, i = tiles_incl - tiles; t < rows; t += tile_rows, ++i) items[i] = make_int4(tid, first + t, min(tile_rows, rows - t), 0);
+    if (tid == n_experts - 1) { offsets[n_experts] = rows_incl; *n_items = tiles_incl; }
+  }
+  __syncthreads();
+  if (tid < n_assign) {
+    const int e = s_expert[tid];
+    int at = s_off[e];
+    for (int b = 0; b < tid; ++b) at += s_expert[b] == e;
+    order[at] = tid;
+    inv_order[tid] = at;
+    row_scales[at] = s_weight[tid];
   }
 }
 
@@ -566,6 +637,16 @@ b200_status b200_moe_gather_order(const void* d_x, const int* d_order, int top, 
   return B200_OK;
 }
 
+// f(experts per lane), one of a few.
+template <typename F>
+static void by_experts(int n_experts, F f) {
+  if (n_experts <= 32) f(std::integral_constant<int, 1>{});
+  else if (n_experts <= 64) f(std::integral_constant<int, 2>{});
+  else if (n_experts <= 128) f(std::integral_constant<int, 4>{});
+  else if (n_experts <= 256) f(std::integral_constant<int, 8>{});
+  else f(std::integral_constant<int, 32>{});
+}
+
 extern "C" {
 
 b200_status b200_moe_route(const void* d_logits, int32_t logits_are_f32, const float* d_bias, int32_t n_tokens,
@@ -581,12 +662,16 @@ b200_status b200_moe_route(const void* d_logits, int32_t logits_are_f32, const f
   cudaStream_t s = (cudaStream_t)stream;
   if (d_counts) B200_CUDA_TRY(cudaMemsetAsync(d_counts, 0, sizeof(int) * n_experts, s));
   const int blocks = (n_tokens * 32 + 255) / 256;
-  if (logits_are_f32)
-    launch_after(route_kernel<float>, blocks, 256, 0, s, (const float*)d_logits, d_bias, n_tokens, n_experts, k, scoring, route_scale,
-                                               d_indices, d_weights, d_counts);
-  else
-    launch_after(route_kernel<__nv_bfloat16>, blocks, 256, 0, s, (const __nv_bfloat16*)d_logits, d_bias, n_tokens, n_experts, k, scoring,
-                                                       route_scale, d_indices, d_weights, d_counts);
+  auto launch = [&](auto per) {
+    constexpr int PER = decltype(per)::value;
+    if (logits_are_f32)
+      launch_after(route_kernel<float, PER>, blocks, 256, 0, s, (const float*)d_logits, d_bias, n_tokens, n_experts, k, scoring, route_scale,
+                   d_indices, d_weights, d_counts);
+    else
+      launch_after(route_kernel<__nv_bfloat16, PER>, blocks, 256, 0, s, (const __nv_bfloat16*)d_logits, d_bias, n_tokens, n_experts, k, scoring,
+                   route_scale, d_indices, d_weights, d_counts);
+  };
+  by_experts(n_experts, launch);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -801,16 +886,29 @@ b200_status b200_moe_forward(b200_moe* m, const void* d_x, int32_t n_tokens, voi
     STEP(b200_qmm(m->sh_down, m->sh_act, n_tokens, m->sh_out, B200_EPI_NONE, nullptr, 0.f, B200_QMM_AUTO, stream));
   }
   STEP(b200_qmm(m->gate, d_x, n_tokens, m->logits, B200_EPI_NONE, nullptr, 0.f, B200_QMM_AUTO, stream));
-  STEP(b200_moe_route(m->logits, 0, m->d_bias, n_tokens, c.n_experts, c.top_k, c.scoring, c.route_scale, m->indices,
-                      m->weights, m->counts, stream));
-  STEP(b200_moe_group(m->indices, m->counts, n_tokens, c.top_k, c.n_experts, tile_rows, m->offsets, m->order,
-                      m->inv_order, m->items, m->n_items, stream));
+  // (what b200_moe_route refuses goes there to be refused)
+  const bool small = A <= kSmallAssign && c.n_experts <= 256 && c.top_k > 0 && c.top_k <= std::min(kMaxTopK, c.n_experts) && c.scoring >= 0 && c.scoring <= 2;
+  if (small) {
+    by_experts(c.n_experts, [&](auto per) {
+      constexpr int PER = decltype(per)::value <= 8 ? decltype(per)::value : 8;
+      launch_after(route_small_kernel<PER>, 1, 1024, 0, (cudaStream_t)stream, m->logits, m->d_bias, n_tokens, c.n_experts, c.top_k, c.scoring, c.route_scale,
+                   tile_rows, m->indices, m->weights, m->counts, m->offsets, m->items, m->n_items, m->order, m->inv_order, m->row_scales);
+    });
+    B200_LAUNCH_CHECK();
+  } else {
+    STEP(b200_moe_route(m->logits, 0, m->d_bias, n_tokens, c.n_experts, c.top_k, c.scoring, c.route_scale, m->indices,
+                        m->weights, m->counts, stream));
+    STEP(b200_moe_group(m->indices, m->counts, n_tokens, c.top_k, c.n_experts, tile_rows, m->offsets, m->order,
+                        m->inv_order, m->items, m->n_items, stream));
+  }
   // gate/up with clipped SwiGLU and the routing score folded in before the down projection (:787-805)
   if (b200_qmm_grouped_takes_tokens(m->exp_gu, tile_rows)) {
     // the block-scaled path re-encodes every activation row anyway: it reads the rows from the token
     // matrix through `order`, and no expert-sorted bf16 copy is made
-    launch_after(row_scales_kernel, (A + 255) / 256, 256, 0, (cudaStream_t)stream, m->order, m->weights, A, m->row_scales, nullptr);
-    B200_LAUNCH_CHECK();
+    if (!small) {
+      launch_after(row_scales_kernel, (A + 255) / 256, 256, 0, (cudaStream_t)stream, m->order, m->weights, A, m->row_scales, nullptr);
+      B200_LAUNCH_CHECK();
+    }
     STEP(b200_qmm_grouped_from_tokens(m->exp_gu, d_x, m->order, c.top_k, A, m->act_sorted, B200_EPI_SWIGLU, m->row_scales,
                                       c.swiglu_limit, m->items, m->n_items, m->max_items, tile_rows, stream));
   } else {
