@@ -47,6 +47,12 @@
 #include "qmm.cuh"
 #include "tma.cuh"
 
+#ifndef CP_RULE
+#define CP_RULE true
+#endif
+#ifndef CP_ROWS
+#define CP_ROWS 256
+#endif
 namespace {
 
 constexpr int kTileN = 128;
@@ -1107,6 +1113,296 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
   ptx::tc_fence_before_sync();
   __syncthreads();
   if (warp == 17) ptx::tmem_dealloc(tmem_base, kCols);
+}
+
+// ---- pairs of CTAs: more than 256 rows ------------------------------------------------------------
+// In qmm_tc2_kernel an MMA of M128 x N256 reads 12 KiB of shared memory in the 128 cycles that it takes, and the stages are written at half that
+// rate again (dequantised tiles, raw blocks, activations): 140 to 180 bytes per cycle where 128 can be had, and all of tensor memory holds one
+// item's sums, so the epilogue runs with the tensor cores idle.  Here two CTAs (a cluster) share an MMA of M256 x N256: each brings 128 weight
+// rows and half of the activations, reads 8 KiB per MMA, and an item's sums are half of its tensor memory, so that the epilogue warps drain one
+// half while the next item's MMAs fill the other.  Persistent: a pair walks the items (pair of weight tiles, 256 rows), rows fastest, so that
+// weights come from memory once.
+// Warps, quantised weights: 0-15 dequantise this CTA's weight tile into the stage's MMA tile, two groups of eight in turn (a thread per row and
+// 32-column plane; one group of eight took 700 cycles per chunk, longer than the chunk's 512 of MMAs), then one each for the weights (a ring of raw
+// blocks), the MMAs of both CTAs (in the first one), the activations, and for telling the first CTA that this one's copies have landed, and four
+// that bring the sums to the output.  Dense weights land in the stage; eight warps bring out their sums.
+template <int MODE>
+struct CpShape {
+  static constexpr bool kDense = MODE == B200_Q_BF16;
+  static constexpr int kWorkers = kDense ? 0 : 16, kEpilogue = kDense ? 8 : 4, kThreads = (kWorkers + 4 + kEpilogue) * 32;
+  static constexpr int kRawSlots = kDense ? 0 : 5;
+};
+constexpr int kCpTokens = 256, kCpMaxStages = 8;
+constexpr int kCpBatch = 16, kCpPitch = 36;  // epilogue: tokens at a time, floats between them in a warp's staging tile of 32 weight rows
+
+// Eight neighbouring outputs of one token (four after SwiGLU), n..n+7 of the matrix.
+__device__ __forceinline__ void store8(const QmmArgs& a, int token, int n, const float (&v)[8], const uint4& res) {
+  const float rs = a.row_scale(token);
+  if (a.epilogue == B200_EPI_SWIGLU) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(gated(a, v[0], v[1]) * rs, gated(a, v[2], v[3]) * rs);
+    const __nv_bfloat162 hi = __floats2bfloat162_rn(gated(a, v[4], v[5]) * rs, gated(a, v[6], v[7]) * rs);
+    *reinterpret_cast<uint2*>(a.y + (size_t)token * a.out_stride(a.n / 2) + n / 2) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    return;
+  }
+  const uint32_t r[4] = {res.x, res.y, res.z, res.w};
+  uint32_t out[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float x = v[2 * q], y = v[2 * q + 1];
+    if (a.epilogue == B200_EPI_RESIDUAL) { x += ptx::bf16_lo(r[q]); y += ptx::bf16_hi(r[q]); }
+    else { x = activate(a.epilogue, x); y = activate(a.epilogue, y); }
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x * rs, y * rs);
+    out[q] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  *reinterpret_cast<uint4*>(a.y + (size_t)token * a.out_stride(a.n) + n) = make_uint4(out[0], out[1], out[2], out[3]);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(const __grid_constant__ CUtensorMap xmap, QmmArgs a) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  using Z = CpShape<MODE>;
+  constexpr bool kDense = Z::kDense;
+  constexpr uint32_t BB = block_bytes(MODE), kTile = kTileN * 128, kStage = 2 * kTile;  // [weight tile][half of the activations]
+  constexpr int SR = Z::kRawSlots, kRoles = Z::kWorkers;  // first of the warps with a role of their own
+  const int S = a.stages, kc = a.kc;
+  unsigned char* raw = smem + (size_t)S * kStage;
+  float* staging = reinterpret_cast<float*>(raw + SR * BB);  // [epilogue warp][16 tokens][32 rows]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(staging + Z::kEpilogue * kCpBatch * kCpPitch);
+  const uint32_t smem_u = ptx::smem_u32(smem), raw_u = ptx::smem_u32(raw), bars_u = ptx::smem_u32(bars);
+  const uint32_t full = bars_u;               // [S] this CTA's copies have landed
+  const uint32_t done = full + 8u * S;        // [S] the MMAs reading the stage are done
+  const uint32_t ready = done + 8u * S;       // [S] first CTA: both CTAs' stages are complete
+  const uint32_t raw_full = ready + 8u * S;   // [SR] a raw block has landed
+  const uint32_t raw_free = raw_full + 8u * SR;
+  const uint32_t acc_full = raw_free + 8u * SR;  // [2] an item's sums are complete
+  const uint32_t acc_free = acc_full + 16u;      // [2] first CTA: both CTAs' epilogues have read them
+  const uint32_t drain = acc_free + 16u;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * S + 2 * SR + 5);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = ptx::cluster_rank();
+  const int tts = (a.rows + kCpTokens - 1) / kCpTokens, n_work = (a.nt + 1) / 2 * tts, first_work = blockIdx.x / 2, step = gridDim.x / 2;
+  if (tid == 0) {
+    for (int s = 0; s < S; ++s) {
+      ptx::mbar_init(&bars[s], kDense ? 2 : 1);
+      ptx::mbar_init(&bars[S + s], 1);
+      ptx::mbar_init(&bars[2 * S + s], kDense ? 2 : 2 + 2 * 8);  // a word from each CTA, and its dequantising warps
+    }
+    for (int s = 0; s < SR; ++s) {
+      ptx::mbar_init(&bars[3 * S + s], 1);
+      ptx::mbar_init(&bars[3 * S + SR + s], 8);
+    }
+    for (int q = 0; q < 2; ++q) {
+      ptx::mbar_init(&bars[3 * S + 2 * SR + q], 1);
+      ptx::mbar_init(&bars[3 * S + 2 * SR + 2 + q], 2 * Z::kEpilogue);
+    }
+    ptx::mbar_init(&bars[3 * S + 2 * SR + 4], 1);
+    ptx::mbar_fence_init();
+  }
+  __syncthreads();
+  // chunk i of weight tile nt, as number n of this CTA's stream
+  auto load_weights = [&](int nt, int i, uint32_t slot) {
+    const uint32_t bar = (kDense ? full : raw_full) + 8u * slot;
+    const bool exists = nt < a.nt;  // (an odd tile count leaves the last pair's second CTA without one: it multiplies what lies there)
+    ptx::mbar_expect_tx_addr(bar, exists ? BB : 0u);
+    if (exists) ptx::bulk_g2s_addr(kDense ? smem_u + slot * kStage : raw_u + slot * BB, a.blocks + ((size_t)nt * kc + i) * BB, BB, bar);
+  };
+  const int slots = kDense ? S : SR;
+  const int ahead = first_work < n_work ? min(slots, kc) : 0;  // of the first item, before the kernels ahead in the stream have ended
+  if (warp == kRoles && lane == 0)
+    for (int i = 0; i < ahead; ++i) load_weights(2 * (first_work / tts) + (int)rank, i, i);
+  wait_previous();
+  ptx::cluster_sync();  // both CTAs' barriers are there
+  if (warp == kRoles + 1) {
+    ptx::tmem_alloc2(tmem_slot, 512);
+    ptx::tmem_relinquish2();
+  }
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  bool ok = true;
+
+  if (warp == kRoles) {
+    if (lane == 0) {
+      uint32_t slot = 0, ph = 1;
+      int skip = ahead;
+      for (int w = first_work; w < n_work && ok; w += step) {
+        const int nt = 2 * (w / tts) + (int)rank;
+        for (int i = 0; i < kc; ++i) {
+          if (skip > 0) {
+            --skip;
+          } else {
+            ok = kDense ? ptx::mbar_wait_addr(done + 8u * slot, ph) : ptx::mbar_wait_addr(raw_free + 8u * slot, ph);
+            if (!ok) break;
+            load_weights(nt, i, slot);
+          }
+          if (++slot == (uint32_t)slots) { slot = 0; ph ^= 1u; }
+        }
+      }
+      let_next_start();
+    }
+  } else if (warp == kRoles + 2) {
+    if (lane == 0) {
+      uint32_t s = 0, ph = 1;
+      for (int w = first_work; w < n_work && ok; w += step) {
+        const int t0 = w % tts * kCpTokens, n_here = (min(kCpTokens, a.rows - t0) + 15) / 16 * 16;
+        const int row0 = a.x_row0 + t0 + (rank ? n_here / 2 : 0);
+        for (int i = 0; i < kc; ++i) {
+          ok = ptx::mbar_wait_addr(done + 8u * s, ph);
+          if (!ok) break;
+          ptx::mbar_expect_tx_addr(full + 8u * s, kTile);
+          ptx::tma_load_2d(smem + (size_t)s * kStage + kTile, &xmap, i * kChunkK, row0, &bars[s]);
+          if (++s == (uint32_t)S) { s = 0; ph ^= 1u; }
+        }
+      }
+    }
+  } else if (warp == kRoles + 3) {
+    if (lane == 0) {
+      const uint32_t to = ptx::map_to_rank(ready, 0);
+      uint32_t s = 0, ph = 0;
+      for (int w = first_work; w < n_work && ok; w += step)
+        for (int i = 0; i < kc; ++i) {
+          ok = ptx::mbar_wait_addr(full + 8u * s, ph);
+          if (!ok) break;
+          ptx::mbar_arrive_cluster(to + 8u * s);
+          if (++s == (uint32_t)S) { s = 0; ph ^= 1u; }
+        }
+    }
+  } else if (warp == kRoles + 1) {
+    if (rank == 0 && ptx::elect_one()) {
+      uint32_t s = 0, ph = 0, n_item = 0;
+      for (int w = first_work; w < n_work && ok; w += step, ++n_item) {
+        const int t0 = w % tts * kCpTokens, n_here = (min(kCpTokens, a.rows - t0) + 15) / 16 * 16;
+        const uint32_t idesc = ptx::umma_idesc_bf16(2 * kTileN, n_here), set = n_item & 1u, acc = tmem_base + set * 256u;
+        if (n_item >= 2) ok = ptx::mbar_wait_addr(acc_free + 8u * set, ((n_item >> 1) - 1u) & 1u);
+        if (!ok) break;
+        ptx::tc_fence_after_sync();
+        for (int i = 0; i < kc; ++i) {
+          ok = ptx::mbar_wait_addr(ready + 8u * s, ph);
+          if (!ok) break;
+          ptx::tc_fence_after_sync();
+          const uint64_t da = ptx::umma_desc_k_sw128(smem_u + s * kStage), db = ptx::umma_desc_k_sw128(smem_u + s * kStage + kTile);
+#pragma unroll
+          for (int k4 = 0; k4 < 4; ++k4) ptx::umma2_bf16(acc, da + 2 * k4, db + 2 * k4, idesc, (i > 0 || k4 > 0) ? 1u : 0u);
+          ptx::umma2_commit(done + 8u * s);
+          if (++s == (uint32_t)S) { s = 0; ph ^= 1u; }
+        }
+        if (ok) ptx::umma2_commit(acc_full + 8u * set);
+      }
+      if (!ok) {  // the MMAs on the way read both CTAs' shared memory
+        ptx::umma2_commit(drain);
+        ptx::mbar_wait_addr(drain, 0);
+      }
+    }
+    __syncwarp();
+  } else if (warp < kRoles) {
+    if constexpr (!kDense) {
+      const int r = tid & (kTileN - 1), plane = (tid >> 7) & 1, group = warp >> 3;
+      const uint32_t to = ptx::map_to_rank(ready, 0);
+      const int n_chunks = first_work < n_work ? ((n_work - 1 - first_work) / step + 1) * kc : 0;
+      int s = group, sr = group;
+      uint32_t ph = 1, phr = 0;
+      for (int i = group; i < n_chunks; i += 2) {
+        ok = ptx::mbar_wait_addr(raw_full + 8u * sr, phr);
+        if (!ok) break;
+        const unsigned char* blk = raw + (size_t)sr * BB;
+        const uint4 q = *reinterpret_cast<const uint4*>(blk + plane * kPlaneBytes + r * 16);
+        __nv_bfloat162 s2, b2;
+        row_params<MODE>(blk, r, plane, s2, b2);
+        ptx::warp_loads_landed(q.x ^ q.y ^ q.z ^ q.w ^ *reinterpret_cast<const uint32_t*>(&s2) ^ *reinterpret_cast<const uint32_t*>(&b2));
+        if (lane == 0) ptx::mbar_arrive_addr(raw_free + 8u * sr);
+        uint4 d[4];
+        const uint32_t words[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) d[x] = dequant_word<MODE>(words[x], s2, b2);
+        ok = ptx::mbar_wait_addr(done + 8u * s, ph);
+        if (!ok) break;
+        unsigned char* arow = smem + (size_t)s * kStage + r * 128;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) *reinterpret_cast<uint4*>(arow + (((plane * 4 + x) ^ (r & 7)) << 4)) = d[x];
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster(to + 8u * s);
+        s += 2;
+        if (s >= S) { s -= S; ph ^= 1u; }
+        sr += 2;
+        if (sr >= SR) { sr -= SR; phr ^= 1u; }
+      }
+    }
+  } else {
+    // ---- a warp's 32 weight rows, 16 tokens at a time, through shared memory: 16-byte stores (2-byte ones straight from the accumulator layout
+    // took longer than the MMAs: 2026 rows of 16384 x 2048 with SwiGLU 161 us, CP_DENSE this way, 71 without an epilogue) ----
+    const int lq = warp & 3, part = (warp - kRoles - 4) >> 2;  // dense: two warps share a quarter, half of the tokens each
+    constexpr int kParts = Z::kEpilogue / 4;
+    float* tile = staging + (warp - kRoles - 4) * kCpBatch * kCpPitch;
+    const uint32_t to = ptx::map_to_rank(acc_free, 0);
+    const bool swiglu = a.epilogue == B200_EPI_SWIGLU, add = a.epilogue == B200_EPI_RESIDUAL;
+    const bool wide = a.keep_f32 || (a.n % 8 == 0 && (swiglu ? a.out_stride(a.n / 2) % 4 == 0 && ((uintptr_t)a.y & 7) == 0
+                                                                : a.out_stride(a.n) % 8 == 0 && (((uintptr_t)a.y | (uintptr_t)(add ? a.residual : nullptr)) & 15) == 0));
+    uint32_t n_item = 0;
+    for (int w = first_work; w < n_work; w += step, ++n_item) {
+      const int nt = 2 * (w / tts) + (int)rank, tt = w % tts, t0 = tt * kCpTokens, rows_here = min(kCpTokens, a.rows - t0);
+      const uint32_t set = n_item & 1u;
+      ok = ptx::mbar_wait_addr(acc_full + 8u * set, (n_item >> 1) & 1u);
+      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+      ptx::tc_fence_after_sync();
+      const uint32_t acc = tmem_base + ((uint32_t)(lq * 32) << 16) + set * 256u;
+      const int n0 = nt * kTileN + lq * 32;
+      float* wsp = a.ws + (size_t)(nt * tts + tt) * kCpTokens * kTileN + lq * 32;
+      const int per = (rows_here + 32 * kParts - 1) / (32 * kParts) * 32, c_end = min(rows_here, (part + 1) * per);
+      if (!wide) {
+        for (int c0 = part * per; c0 < c_end; c0 += 32) {
+          uint32_t v[32];
+          ptx::tmem_ld32(acc + (uint32_t)c0, v);
+          ptx::tmem_ld_wait();
+          if (nt < a.nt) tile_epilogue_store(a, v, c0, rows_here, t0, n0 + lane, lane, true, wsp, (size_t)kTileN);
+        }
+      } else {
+        for (int c0 = part * per; c0 < c_end; c0 += kCpBatch) {
+          uint4 res[2] = {};
+          if (add && nt < a.nt) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              const int piece = q * 32 + lane, tok = c0 + (piece >> 2), n = n0 + (piece & 3) * 8;
+              if (tok < rows_here && n < a.n) res[q] = *reinterpret_cast<const uint4*>(a.residual + (size_t)(t0 + tok) * a.out_stride(a.n) + n);
+            }
+          }
+          uint32_t v[16];
+          ptx::tmem_ld16(acc + (uint32_t)c0, v);
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int x = 0; x < 16; ++x) tile[x * kCpPitch + lane] = __uint_as_float(v[x]);
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int piece = q * 32 + lane, tok = c0 + (piece >> 2), seg = (piece & 3) * 8, n = n0 + seg;
+            const float4 f0 = *reinterpret_cast<const float4*>(tile + (piece >> 2) * kCpPitch + seg), f1 = *reinterpret_cast<const float4*>(tile + (piece >> 2) * kCpPitch + seg + 4);
+            if (tok >= rows_here || nt >= a.nt) continue;
+            if (a.keep_f32) {
+              float4* dst = reinterpret_cast<float4*>(wsp + (size_t)tok * kTileN + seg);
+              dst[0] = f0;
+              dst[1] = f1;
+            } else if (n < a.n) {
+              const float x[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+              store8(a, t0 + tok, n, x, res[q]);
+            }
+          }
+          __syncwarp();
+        }
+      }
+      // all that this warp reads of the item's sums has been read
+      ptx::tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive_cluster(to + 8u * set);
+    }
+  }
+  if (!ok) atomicExch(a.err, B200_ERR_DEVICE_FLAGGED);
+  __syncwarp();
+  ptx::tc_fence_before_sync();
+  ptx::cluster_sync();  // nobody leaves while its memory may be read or arrived on
+  if (warp == kRoles + 1) ptx::tmem_dealloc2(tmem_base, 512);
 }
 
 // ---- tile pairs with the weight operand in tensor memory: 17..128 rows --------------------------
@@ -2871,6 +3167,66 @@ static b200_status launch_tca(QmmArgs& a, int rows, cudaStream_t s) {
   return direct ? B200_OK : launch_finish(a, splits, s);
 }
 
+static bool takes_pairs(const QmmArgs& a, int rows) {
+  return rows > CP_ROWS && CP_RULE;
+}
+
+// Pairs of CTAs: as many as run at the same time (a cluster stays within a GPC).
+template <int MODE>
+static b200_status launch_cp(QmmArgs& a, int rows, cudaStream_t s) {
+  a.tn = kCpTokens;
+  const int tts = (rows + kCpTokens - 1) / kCpTokens, n_work = (a.nt + 1) / 2 * tts;
+  b200_status st = ensure_state(0);
+  if (st != B200_OK) return st;
+  constexpr int BB = block_bytes(MODE);
+  using Z = CpShape<MODE>;
+  constexpr int fixed = 1024 /*alignment slack*/ + Z::kRawSlots * BB + Z::kEpilogue * kCpBatch * kCpPitch * (int)sizeof(float) +
+                        8 * (3 * kCpMaxStages + 2 * Z::kRawSlots + 5) + 16;
+  static int smem_budget[3] = {0, 0, 0}, most_pairs[3] = {0, 0, 0};
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (as launch_after)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(Z::kThreads);
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  if (smem_budget[MODE] == 0) {
+    int dev = 0, optin = 0;
+    B200_CUDA_TRY(cudaGetDevice(&dev));
+    B200_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    cudaFuncAttributes fa;
+    B200_CUDA_TRY(cudaFuncGetAttributes(&fa, qmm_cp_kernel<MODE>));
+    const int budget = optin - (int)fa.sharedSizeBytes;
+    B200_CUDA_TRY(cudaFuncSetAttribute(qmm_cp_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
+    cudaLaunchConfig_t ask = cfg;
+    ask.gridDim = dim3(2 * (g_sms / 2));
+    ask.dynamicSmemBytes = budget;
+    ask.numAttrs = 1;
+    int pairs = 0;
+    B200_CUDA_TRY(cudaOccupancyMaxActiveClusters(&pairs, qmm_cp_kernel<MODE>, &ask));
+    if (pairs < 1) { b200_set_error("qmm: no pair of CTAs fits the device"); return B200_ERR_CAPACITY; }
+    most_pairs[MODE] = pairs;
+    smem_budget[MODE] = budget;
+  }
+  a.stages = std::min(kCpMaxStages, (smem_budget[MODE] - fixed) / (2 * kTileN * 128));
+  cfg.dynamicSmemBytes = (size_t)a.stages * 2 * kTileN * 128 + fixed;
+  cfg.gridDim = dim3(2 * std::min(most_pairs[MODE], n_work));
+  st = ensure_state(a.keep_f32 ? (size_t)tts * kCpTokens * a.nt * kTileN * sizeof(float) : 0);
+  if (st != B200_OK) return st;
+  a.ws = g_ws[g_place]; a.err = g_err;
+  CUtensorMap xmap;
+  st = make_x_map(&xmap, a.x, rows, a.k, kCpTokens / 2);
+  if (st != B200_OK) return st;
+  a.x_row0 = 0;
+  (void)cudaLaunchKernelEx(&cfg, qmm_cp_kernel<MODE>, xmap, a);
+  B200_LAUNCH_CHECK();
+  return a.keep_f32 ? launch_finish(a, 1, s) : B200_OK;
+}
+
 // Quantised weights, 17..128 rows: tile pairs with the weights in tensor memory.
 template <int MODE>
 static b200_status launch_tp(QmmArgs& a, int rows, cudaStream_t s) {
@@ -3391,6 +3747,11 @@ static b200_status qmm_entry(const b200_qweight* w, const void* d_x, int32_t row
       return w->mode == B200_Q_AFFINE4_G64 ? launch_tp<B200_Q_AFFINE4_G64>(a, rows, s) : launch_tp<B200_Q_MXFP4_G32>(a, rows, s);
     if (path == B200_QMM_TCGEN05_TMEM_A && w->mode != B200_Q_BF16)
       return w->mode == B200_Q_AFFINE4_G64 ? launch_tca<B200_Q_AFFINE4_G64>(a, rows, s) : launch_tca<B200_Q_MXFP4_G32>(a, rows, s);
+    if (path == B200_QMM_TCGEN05_X2 && takes_pairs(a, rows)) {
+      if (w->mode == B200_Q_AFFINE4_G64) return launch_cp<B200_Q_AFFINE4_G64>(a, rows, s);
+      if (w->mode == B200_Q_MXFP4_G32) return launch_cp<B200_Q_MXFP4_G32>(a, rows, s);
+      return launch_cp<B200_Q_BF16>(a, rows, s);
+    }
     if (path == B200_QMM_TCGEN05_X2) {
       if (w->mode == B200_Q_AFFINE4_G64) return launch_tc2<B200_Q_AFFINE4_G64>(a, rows, s);
       if (w->mode == B200_Q_MXFP4_G32) return launch_tc2<B200_Q_MXFP4_G32>(a, rows, s);
