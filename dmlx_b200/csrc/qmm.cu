@@ -47,12 +47,6 @@
 #include "qmm.cuh"
 #include "tma.cuh"
 
-#ifndef CP_RULE
-#define CP_RULE true
-#endif
-#ifndef CP_ROWS
-#define CP_ROWS 256
-#endif
 namespace {
 
 constexpr int kTileN = 128;
@@ -1115,13 +1109,13 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
   if (warp == 17) ptx::tmem_dealloc(tmem_base, kCols);
 }
 
-// ---- pairs of CTAs: more than 256 rows ------------------------------------------------------------
+// ---- pairs of CTAs: more than 128 rows ------------------------------------------------------------
 // In qmm_tc2_kernel an MMA of M128 x N256 reads 12 KiB of shared memory in the 128 cycles that it takes, and the stages are written at half that
 // rate again (dequantised tiles, raw blocks, activations): 140 to 180 bytes per cycle where 128 can be had, and all of tensor memory holds one
 // item's sums, so the epilogue runs with the tensor cores idle.  Here two CTAs (a cluster) share an MMA of M256 x N256: each brings 128 weight
 // rows and half of the activations, reads 8 KiB per MMA, and an item's sums are half of its tensor memory, so that the epilogue warps drain one
-// half while the next item's MMAs fill the other.  Persistent: a pair walks the items (pair of weight tiles, 256 rows), rows fastest, so that
-// weights come from memory once.
+// half while the next item's MMAs fill the other.  Persistent: a pair walks the items (pair of weight tiles, up to 256 rows, range of K), rows
+// fastest, so that weights come from memory once.
 // Warps, quantised weights: 0-15 dequantise this CTA's weight tile into the stage's MMA tile, two groups of eight in turn (a thread per row and
 // 32-column plane; one group of eight took 700 cycles per chunk, longer than the chunk's 512 of MMAs), then one each for the weights (a ring of raw
 // blocks), the MMAs of both CTAs (in the first one), the activations, and for telling the first CTA that this one's copies have landed, and four
@@ -1129,11 +1123,12 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
 template <int MODE>
 struct CpShape {
   static constexpr bool kDense = MODE == B200_Q_BF16;
-  static constexpr int kWorkers = kDense ? 0 : 16, kEpilogue = kDense ? 8 : 4, kThreads = (kWorkers + 4 + kEpilogue) * 32;
+  static constexpr int kWorkers = kDense ? 0 : 16, kEpilogue = 8, kThreads = (kWorkers + 4 + kEpilogue) * 32;
   static constexpr int kRawSlots = kDense ? 0 : 5;
+  static constexpr int kBatch = kDense ? 16 : 8;  // epilogue: tokens at a time
 };
 constexpr int kCpTokens = 256, kCpMaxStages = 8;
-constexpr int kCpBatch = 16, kCpPitch = 36;  // epilogue: tokens at a time, floats between them in a warp's staging tile of 32 weight rows
+constexpr int kCpPitch = 36;  // epilogue: floats between tokens in a warp's staging tile of 32 weight rows
 
 // Eight neighbouring outputs of one token (four after SwiGLU), n..n+7 of the matrix.
 __device__ __forceinline__ void store8(const QmmArgs& a, int token, int n, const float (&v)[8], const uint4& res) {
@@ -1168,7 +1163,7 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
   const int S = a.stages, kc = a.kc;
   unsigned char* raw = smem + (size_t)S * kStage;
   float* staging = reinterpret_cast<float*>(raw + SR * BB);  // [epilogue warp][16 tokens][32 rows]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(staging + Z::kEpilogue * kCpBatch * kCpPitch);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(staging + Z::kEpilogue * Z::kBatch * kCpPitch);
   const uint32_t smem_u = ptx::smem_u32(smem), raw_u = ptx::smem_u32(raw), bars_u = ptx::smem_u32(bars);
   const uint32_t full = bars_u;               // [S] this CTA's copies have landed
   const uint32_t done = full + 8u * S;        // [S] the MMAs reading the stage are done
@@ -1182,7 +1177,35 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = ptx::cluster_rank();
-  const int tts = (a.rows + kCpTokens - 1) / kCpTokens, n_work = (a.nt + 1) / 2 * tts, first_work = blockIdx.x / 2, step = gridDim.x / 2;
+  // Grouped: an item of expert-sorted rows {expert, first row, rows} in place of a row tile; the list is known when the kernels ahead have ended.
+  if (a.items) wait_previous();
+  const int tn = a.tn, tts = a.items ? min(*a.n_items, a.max_items) : (a.rows + tn - 1) / tn;
+  const int per_split = (a.nt + 1) / 2 * tts, n_work = per_split * a.splits, first_work = blockIdx.x / 2, step = gridDim.x / 2;
+  struct Work { int nt, tt, t0, rows, n_here, split, kc0, n_chunks; const unsigned char* blocks; };  // n_here: rows of its MMAs; no chunks: nothing to do
+  auto decode = [&](int w) {
+    Work k;
+    k.split = w / per_split;
+    const int rest = w - k.split * per_split;
+    k.blocks = a.blocks;
+    if (a.items) {  // (weight tiles fastest: an item's rows are read by neighbouring pairs of CTAs at a time)
+      const int pairs = (a.nt + 1) / 2;
+      k.tt = rest / pairs;
+      k.nt = 2 * (rest - k.tt * pairs) + (int)rank;
+      const int4 it = a.items[k.tt];
+      k.blocks += (size_t)it.x * a.expert_stride;
+      k.t0 = it.y;
+      k.rows = min(it.z, tn);
+    } else {
+      k.nt = 2 * (rest / tts) + (int)rank;
+      k.tt = rest % tts;
+      k.t0 = k.tt * tn;
+      k.rows = min(tn, a.rows - k.t0);
+    }
+    k.n_here = (k.rows + 15) / 16 * 16;
+    k.kc0 = k.split * a.chunks_per_split;
+    k.n_chunks = k.rows > 0 ? min(a.chunks_per_split, kc - k.kc0) : 0;
+    return k;
+  };
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
       ptx::mbar_init(&bars[s], kDense ? 2 : 1);
@@ -1202,17 +1225,19 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
   }
   __syncthreads();
   // chunk i of weight tile nt, as number n of this CTA's stream
-  auto load_weights = [&](int nt, int i, uint32_t slot) {
+  auto load_weights = [&](const unsigned char* blocks, int nt, int i, uint32_t slot) {
     const uint32_t bar = (kDense ? full : raw_full) + 8u * slot;
     const bool exists = nt < a.nt;  // (an odd tile count leaves the last pair's second CTA without one: it multiplies what lies there)
     ptx::mbar_expect_tx_addr(bar, exists ? BB : 0u);
-    if (exists) ptx::bulk_g2s_addr(kDense ? smem_u + slot * kStage : raw_u + slot * BB, a.blocks + ((size_t)nt * kc + i) * BB, BB, bar);
+    if (exists) ptx::bulk_g2s_addr(kDense ? smem_u + slot * kStage : raw_u + slot * BB, blocks + ((size_t)nt * kc + i) * BB, BB, bar);
   };
   const int slots = kDense ? S : SR;
-  const int ahead = first_work < n_work ? min(slots, kc) : 0;  // of the first item, before the kernels ahead in the stream have ended
-  if (warp == kRoles && lane == 0)
-    for (int i = 0; i < ahead; ++i) load_weights(2 * (first_work / tts) + (int)rank, i, i);
-  wait_previous();
+  const int ahead = !a.items && first_work < n_work ? min(slots, decode(first_work).n_chunks) : 0;  // of the first item, before the kernels ahead have ended
+  if (warp == kRoles && lane == 0 && ahead > 0) {
+    const Work k = decode(first_work);
+    for (int i = 0; i < ahead; ++i) load_weights(k.blocks, k.nt, k.kc0 + i, i);
+  }
+  if (!a.items) wait_previous();
   ptx::cluster_sync();  // both CTAs' barriers are there
   if (warp == kRoles + 1) {
     ptx::tmem_alloc2(tmem_slot, 512);
@@ -1229,14 +1254,14 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
       uint32_t slot = 0, ph = 1;
       int skip = ahead;
       for (int w = first_work; w < n_work && ok; w += step) {
-        const int nt = 2 * (w / tts) + (int)rank;
-        for (int i = 0; i < kc; ++i) {
+        const Work k = decode(w);
+        for (int i = 0; i < k.n_chunks; ++i) {
           if (skip > 0) {
             --skip;
           } else {
             ok = kDense ? ptx::mbar_wait_addr(done + 8u * slot, ph) : ptx::mbar_wait_addr(raw_free + 8u * slot, ph);
             if (!ok) break;
-            load_weights(nt, i, slot);
+            load_weights(k.blocks, k.nt, k.kc0 + i, slot);
           }
           if (++slot == (uint32_t)slots) { slot = 0; ph ^= 1u; }
         }
@@ -1247,13 +1272,13 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
     if (lane == 0) {
       uint32_t s = 0, ph = 1;
       for (int w = first_work; w < n_work && ok; w += step) {
-        const int t0 = w % tts * kCpTokens, n_here = (min(kCpTokens, a.rows - t0) + 15) / 16 * 16;
-        const int row0 = a.x_row0 + t0 + (rank ? n_here / 2 : 0);
-        for (int i = 0; i < kc; ++i) {
+        const Work k = decode(w);
+        const int row0 = a.x_row0 + k.t0 + (rank ? k.n_here / 2 : 0);
+        for (int i = 0; i < k.n_chunks; ++i) {
           ok = ptx::mbar_wait_addr(done + 8u * s, ph);
           if (!ok) break;
-          ptx::mbar_expect_tx_addr(full + 8u * s, kTile);
-          ptx::tma_load_2d(smem + (size_t)s * kStage + kTile, &xmap, i * kChunkK, row0, &bars[s]);
+          ptx::mbar_expect_tx_addr(full + 8u * s, (uint32_t)tn * 64u);
+          ptx::tma_load_2d(smem + (size_t)s * kStage + kTile, &xmap, (k.kc0 + i) * kChunkK, row0, &bars[s]);
           if (++s == (uint32_t)S) { s = 0; ph ^= 1u; }
         }
       }
@@ -1263,7 +1288,7 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
       const uint32_t to = ptx::map_to_rank(ready, 0);
       uint32_t s = 0, ph = 0;
       for (int w = first_work; w < n_work && ok; w += step)
-        for (int i = 0; i < kc; ++i) {
+        for (int i = decode(w).n_chunks; i > 0; --i) {
           ok = ptx::mbar_wait_addr(full + 8u * s, ph);
           if (!ok) break;
           ptx::mbar_arrive_cluster(to + 8u * s);
@@ -1273,13 +1298,14 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
   } else if (warp == kRoles + 1) {
     if (rank == 0 && ptx::elect_one()) {
       uint32_t s = 0, ph = 0, n_item = 0;
-      for (int w = first_work; w < n_work && ok; w += step, ++n_item) {
-        const int t0 = w % tts * kCpTokens, n_here = (min(kCpTokens, a.rows - t0) + 15) / 16 * 16;
-        const uint32_t idesc = ptx::umma_idesc_bf16(2 * kTileN, n_here), set = n_item & 1u, acc = tmem_base + set * 256u;
+      for (int w = first_work; w < n_work && ok; w += step) {
+        const Work k = decode(w);
+        if (k.n_chunks == 0) continue;
+        const uint32_t idesc = ptx::umma_idesc_bf16(2 * kTileN, k.n_here), set = n_item & 1u, acc = tmem_base + set * 256u;
         if (n_item >= 2) ok = ptx::mbar_wait_addr(acc_free + 8u * set, ((n_item >> 1) - 1u) & 1u);
         if (!ok) break;
         ptx::tc_fence_after_sync();
-        for (int i = 0; i < kc; ++i) {
+        for (int i = 0; i < k.n_chunks; ++i) {
           ok = ptx::mbar_wait_addr(ready + 8u * s, ph);
           if (!ok) break;
           ptx::tc_fence_after_sync();
@@ -1290,6 +1316,7 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
           if (++s == (uint32_t)S) { s = 0; ph ^= 1u; }
         }
         if (ok) ptx::umma2_commit(acc_full + 8u * set);
+        ++n_item;
       }
       if (!ok) {  // the MMAs on the way read both CTAs' shared memory
         ptx::umma2_commit(drain);
@@ -1301,7 +1328,8 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
     if constexpr (!kDense) {
       const int r = tid & (kTileN - 1), plane = (tid >> 7) & 1, group = warp >> 3;
       const uint32_t to = ptx::map_to_rank(ready, 0);
-      const int n_chunks = first_work < n_work ? ((n_work - 1 - first_work) / step + 1) * kc : 0;
+      int n_chunks = 0;
+      for (int w = first_work; w < n_work; w += step) n_chunks += decode(w).n_chunks;
       int s = group, sr = group;
       uint32_t ph = 1, phr = 0;
       for (int i = group; i < n_chunks; i += 2) {
@@ -1335,67 +1363,60 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
     // ---- a warp's 32 weight rows, 16 tokens at a time, through shared memory: 16-byte stores (2-byte ones straight from the accumulator layout
     // took longer than the MMAs: 2026 rows of 16384 x 2048 with SwiGLU 161 us, CP_DENSE this way, 71 without an epilogue) ----
     const int lq = warp & 3, part = (warp - kRoles - 4) >> 2;  // dense: two warps share a quarter, half of the tokens each
-    constexpr int kParts = Z::kEpilogue / 4;
-    float* tile = staging + (warp - kRoles - 4) * kCpBatch * kCpPitch;
+    constexpr int kParts = Z::kEpilogue / 4, kB = Z::kBatch, kPieces = kB / 8;  // pieces of eight outputs of a lane
+    float* tile = staging + (warp - kRoles - 4) * kB * kCpPitch;
     const uint32_t to = ptx::map_to_rank(acc_free, 0);
-    const bool swiglu = a.epilogue == B200_EPI_SWIGLU, add = a.epilogue == B200_EPI_RESIDUAL;
-    const bool wide = a.keep_f32 || (a.n % 8 == 0 && (swiglu ? a.out_stride(a.n / 2) % 4 == 0 && ((uintptr_t)a.y & 7) == 0
-                                                                : a.out_stride(a.n) % 8 == 0 && (((uintptr_t)a.y | (uintptr_t)(add ? a.residual : nullptr)) & 15) == 0));
+    const bool partial = a.keep_f32 || a.splits > 1, add = a.epilogue == B200_EPI_RESIDUAL && !partial;
     uint32_t n_item = 0;
-    for (int w = first_work; w < n_work; w += step, ++n_item) {
-      const int nt = 2 * (w / tts) + (int)rank, tt = w % tts, t0 = tt * kCpTokens, rows_here = min(kCpTokens, a.rows - t0);
+    for (int w = first_work; w < n_work; w += step) {
+      const Work k = decode(w);
+      if (k.n_chunks == 0) continue;
+      const int nt = k.nt, t0 = k.t0, rows_here = k.rows;
       const uint32_t set = n_item & 1u;
       ok = ptx::mbar_wait_addr(acc_full + 8u * set, (n_item >> 1) & 1u);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
       ptx::tc_fence_after_sync();
       const uint32_t acc = tmem_base + ((uint32_t)(lq * 32) << 16) + set * 256u;
       const int n0 = nt * kTileN + lq * 32;
-      float* wsp = a.ws + (size_t)(nt * tts + tt) * kCpTokens * kTileN + lq * 32;
+      float* wsp = a.ws + ((size_t)(nt * tts + k.tt) * a.splits + k.split) * tn * kTileN + lq * 32;
       const int per = (rows_here + 32 * kParts - 1) / (32 * kParts) * 32, c_end = min(rows_here, (part + 1) * per);
-      if (!wide) {
-        for (int c0 = part * per; c0 < c_end; c0 += 32) {
-          uint32_t v[32];
-          ptx::tmem_ld32(acc + (uint32_t)c0, v);
-          ptx::tmem_ld_wait();
-          if (nt < a.nt) tile_epilogue_store(a, v, c0, rows_here, t0, n0 + lane, lane, true, wsp, (size_t)kTileN);
-        }
-      } else {
-        for (int c0 = part * per; c0 < c_end; c0 += kCpBatch) {
-          uint4 res[2] = {};
-          if (add && nt < a.nt) {
+      for (int c0 = part * per; c0 < c_end; c0 += kB) {
+        uint4 res[kPieces] = {};
+        if (add && nt < a.nt) {
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const int piece = q * 32 + lane, tok = c0 + (piece >> 2), n = n0 + (piece & 3) * 8;
-              if (tok < rows_here && n < a.n) res[q] = *reinterpret_cast<const uint4*>(a.residual + (size_t)(t0 + tok) * a.out_stride(a.n) + n);
-            }
+          for (int q = 0; q < kPieces; ++q) {
+            const int piece = q * 32 + lane, tok = c0 + (piece >> 2), n = n0 + (piece & 3) * 8;
+            if (tok < rows_here && n < a.n) res[q] = *reinterpret_cast<const uint4*>(a.residual + (size_t)(t0 + tok) * a.out_stride(a.n) + n);
           }
-          uint32_t v[16];
-          ptx::tmem_ld16(acc + (uint32_t)c0, v);
-          ptx::tmem_ld_wait();
-#pragma unroll
-          for (int x = 0; x < 16; ++x) tile[x * kCpPitch + lane] = __uint_as_float(v[x]);
-          __syncwarp();
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int piece = q * 32 + lane, tok = c0 + (piece >> 2), seg = (piece & 3) * 8, n = n0 + seg;
-            const float4 f0 = *reinterpret_cast<const float4*>(tile + (piece >> 2) * kCpPitch + seg), f1 = *reinterpret_cast<const float4*>(tile + (piece >> 2) * kCpPitch + seg + 4);
-            if (tok >= rows_here || nt >= a.nt) continue;
-            if (a.keep_f32) {
-              float4* dst = reinterpret_cast<float4*>(wsp + (size_t)tok * kTileN + seg);
-              dst[0] = f0;
-              dst[1] = f1;
-            } else if (n < a.n) {
-              const float x[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
-              store8(a, t0 + tok, n, x, res[q]);
-            }
-          }
-          __syncwarp();
         }
+        uint32_t v[kB];
+        if constexpr (kB == 16) ptx::tmem_ld16(acc + (uint32_t)c0, v);
+        else ptx::tmem_ld8(acc + (uint32_t)c0, v);
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (int x = 0; x < kB; ++x) tile[x * kCpPitch + lane] = __uint_as_float(v[x]);
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < kPieces; ++q) {
+          const int piece = q * 32 + lane, tok = c0 + (piece >> 2), seg = (piece & 3) * 8, n = n0 + seg;
+          const float4 f0 = *reinterpret_cast<const float4*>(tile + (piece >> 2) * kCpPitch + seg), f1 = *reinterpret_cast<const float4*>(tile + (piece >> 2) * kCpPitch + seg + 4);
+          if (tok >= rows_here || nt >= a.nt) continue;
+          if (partial) {
+            float4* dst = reinterpret_cast<float4*>(wsp + (size_t)tok * kTileN + seg);
+            dst[0] = f0;
+            dst[1] = f1;
+          } else if (n < a.n) {
+            const float x[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+            store8(a, t0 + tok, n, x, res[q]);
+          }
+        }
+        __syncwarp();
       }
       // all that this warp reads of the item's sums has been read
       ptx::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive_cluster(to + 8u * set);
+      ++n_item;
     }
   }
   if (!ok) atomicExch(a.err, B200_ERR_DEVICE_FLAGGED);
@@ -3167,20 +3188,29 @@ static b200_status launch_tca(QmmArgs& a, int rows, cudaStream_t s) {
   return direct ? B200_OK : launch_finish(a, splits, s);
 }
 
+// Whether launch_finish leaves the sums to the caller's next kernel.
+static bool takes_sums(const QmmArgs& a) { return a.defer && a.epilogue == B200_EPI_NONE && !a.items && !a.row_scales && !a.norm_w; }
+
 static bool takes_pairs(const QmmArgs& a, int rows) {
-  return rows > CP_ROWS && CP_RULE;
+  if (rows <= 128) return false;
+  // The kernel stores eight outputs at a time (four after SwiGLU).
+  const bool swiglu = a.epilogue == B200_EPI_SWIGLU;
+  const int stride = a.y_stride > 0 ? a.y_stride : (swiglu ? a.n / 2 : a.n);
+  const uintptr_t places = (uintptr_t)a.y | (a.epilogue == B200_EPI_RESIDUAL ? (uintptr_t)a.residual : 0);
+  return a.keep_f32 || (a.n % 8 == 0 && (swiglu ? stride % 4 == 0 && places % 8 == 0 : stride % 8 == 0 && places % 16 == 0));
 }
 
 // Pairs of CTAs: as many as run at the same time (a cluster stays within a GPC).
 template <int MODE>
 static b200_status launch_cp(QmmArgs& a, int rows, cudaStream_t s) {
-  a.tn = kCpTokens;
-  const int tts = (rows + kCpTokens - 1) / kCpTokens, n_work = (a.nt + 1) / 2 * tts;
+  // tiles of equally many rows: what lies behind the last whole tile of 256 would cost most of one
+  const int tts = a.items ? a.max_items : (rows + kCpTokens - 1) / kCpTokens;
+  a.tn = a.items ? kCpTokens : ((rows + tts - 1) / tts + 15) / 16 * 16;
   b200_status st = ensure_state(0);
   if (st != B200_OK) return st;
   constexpr int BB = block_bytes(MODE);
   using Z = CpShape<MODE>;
-  constexpr int fixed = 1024 /*alignment slack*/ + Z::kRawSlots * BB + Z::kEpilogue * kCpBatch * kCpPitch * (int)sizeof(float) +
+  constexpr int fixed = 1024 /*alignment slack*/ + Z::kRawSlots * BB + Z::kEpilogue * Z::kBatch * kCpPitch * (int)sizeof(float) +
                         8 * (3 * kCpMaxStages + 2 * Z::kRawSlots + 5) + 16;
   static int smem_budget[3] = {0, 0, 0}, most_pairs[3] = {0, 0, 0};
   cudaLaunchAttribute attr[2]{};
@@ -3214,17 +3244,35 @@ static b200_status launch_cp(QmmArgs& a, int rows, cudaStream_t s) {
   }
   a.stages = std::min(kCpMaxStages, (smem_budget[MODE] - fixed) / (2 * kTileN * 128));
   cfg.dynamicSmemBytes = (size_t)a.stages * 2 * kTileN * 128 + fixed;
-  cfg.gridDim = dim3(2 * std::min(most_pairs[MODE], n_work));
-  st = ensure_state(a.keep_f32 ? (size_t)tts * kCpTokens * a.nt * kTileN * sizeof(float) : 0);
+  // K is split where the items would leave pairs of CTAs idle in their last round: rounds x chunks, and for partial sums a finish pass of some 16
+  // chunks and their way to memory and back, 2.5 MB in the time of a chunk
+  const int items = (a.nt + 1) / 2 * tts;
+  int splits = 1;
+  double best = 0;
+  for (int sp = 1; sp <= (a.items ? 1 : 8) && (sp == 1 || a.kc / sp >= 16); ++sp) {
+    const int cps = (a.kc + sp - 1) / sp;
+    if ((a.kc + cps - 1) / cps != sp) continue;
+    const double rounds = (items * sp + most_pairs[MODE] - 1) / most_pairs[MODE];
+    const double cost = rounds * (cps + 2) + (sp > 1 ? 16.0 + (double)rows * a.n * sp * 8.0 / 2.5e6 : 0.0);
+    if (sp == 1 || cost < best) { best = cost; splits = sp; }
+  }
+  a.splits = splits;
+  a.chunks_per_split = (a.kc + splits - 1) / splits;
+  cfg.gridDim = dim3(2 * std::min(most_pairs[MODE], items * splits));
+  // A caller that takes partial sums has had 32-bit ones wherever qmm_tc2_kernel would split K, and gets them still.
+  const int old_tn = std::min(256, (rows + 15) / 16 * 16);
+  if (splits == 1 && takes_sums(a) && pick_splits((a.nt + 1) / 2 * ((rows + old_tn - 1) / old_tn), a.kc, g_sms, 1, 2 + old_tn / 32) > 1) a.keep_f32 = 1;
+  const bool partial = splits > 1 || a.keep_f32;
+  st = ensure_state(partial ? (size_t)splits * tts * a.tn * a.nt * kTileN * sizeof(float) : 0);
   if (st != B200_OK) return st;
   a.ws = g_ws[g_place]; a.err = g_err;
   CUtensorMap xmap;
-  st = make_x_map(&xmap, a.x, rows, a.k, kCpTokens / 2);
+  st = make_x_map(&xmap, a.x, rows, a.k, a.tn / 2);
   if (st != B200_OK) return st;
   a.x_row0 = 0;
   (void)cudaLaunchKernelEx(&cfg, qmm_cp_kernel<MODE>, xmap, a);
   B200_LAUNCH_CHECK();
-  return a.keep_f32 ? launch_finish(a, 1, s) : B200_OK;
+  return partial ? launch_finish(a, splits, s) : B200_OK;
 }
 
 // Quantised weights, 17..128 rows: tile pairs with the weights in tensor memory.
@@ -3258,6 +3306,8 @@ static b200_status launch_tp(QmmArgs& a, int rows, cudaStream_t s) {
   const int splits0 = pick_splits(pairs, a.kc, g_sms, 1, 12);  // (4 instead of 12 chunks: gate/up 33.9 -> 53.6 us at 61 rows)
   a.chunks_per_split = (a.kc + splits0 - 1) / splits0;
   const int splits = (a.kc + a.chunks_per_split - 1) / a.chunks_per_split;
+  // (as in launch_cp: where qmm_tca_kernel would split K, a caller that takes partial sums gets 32-bit ones)
+  if (splits == 1 && takes_sums(a) && pick_splits(a.nt, a.kc, g_sms, 2, 12) > 1) a.keep_f32 = 1;
   const bool direct = splits == 1 && !a.keep_f32;
   st = ensure_state(direct ? 0 : (size_t)splits * tn * a.nt * kTileN * sizeof(float));
   if (st != B200_OK) return st;
@@ -3958,8 +4008,9 @@ b200_status b200_qmm_grouped(const b200_qweight* w, const void* d_x, int32_t row
   if (w->mode == B200_Q_AFFINE4_G64) return launch_tc<B200_Q_AFFINE4_G64>(a, rows, s);
   if (w->mode == B200_Q_MXFP4_G32) return launch_tc<B200_Q_MXFP4_G32>(a, rows, s);
   if (takes_few(a, tile_rows)) return launch_few(a, tile_rows, s);
-  // dense weights, items of more than 128 rows: two weight tiles share the item's rows (32 experts of 1024 x 2048 with 253 rows on average:
-  // gate/up 175 -> 99 us, down 141 -> 64)
+  // dense weights, items of more than 128 rows: pairs of CTAs (32 experts of 1024 x 2048 with 253 rows on average: gate/up 98 -> CP_EXP us, down
+  // 64 -> CP_EXPD against two weight tiles per CTA, which takes what the pairs' wide stores cannot)
+  if (tile_rows > 128 && tile_rows <= kCpTokens && takes_pairs(a, tile_rows)) return launch_cp<B200_Q_BF16>(a, rows, s);
   return tile_rows > 128 ? launch_tc2<B200_Q_BF16>(a, rows, s) : launch_tc<B200_Q_BF16>(a, rows, s);
 }
 
