@@ -897,6 +897,10 @@ extern "C" b200_status b200_kv_rope_append(b200_kv* kv, int32_t layer, void* d_q
                                      total_rows, n_q_heads, theta, stream);
 }
 
+// Blocks that share a row's heads: eight per SM altogether.  With a head per warp and row, angles and page lookups were most of a warp's work (2105
+// rows, 48 heads from partial sums: 38 us, 21 with the row's heads in one block).
+static int rope_blocks(int rows, int most) { return std::min(most, std::max(1, (8 * 148 + rows - 1) / rows)); }
+
 // RoPE + append fed from the split-K partial sums of the fused q/k/v projection (head_dim 128 = one 128-row weight
 // tile per head).  One warp per (row, head): the lane's four columns (two rotation pairs) are summed over the splits
 // in split order and rounded to bf16 as the matmul's finish pass would have done, then rotated and stored: q into the
@@ -915,6 +919,9 @@ __global__ void __launch_bounds__(256) rope_append_partials_bf16_kernel(KvDev d,
   const int page = have_page ? d.block_table[(size_t)seq * d.max_pages_per_seq + page_idx] : 0;
   const int tt = row / p.tn, tr = row - tt * p.tn;
   const size_t split_stride = (size_t)p.tn * 128;
+  float sn[2], cs[2];  // the lane's two rotations, of every head
+#pragma unroll
+  for (int j = 0; j < 2; ++j) sincosf((float)pos * exp2f(-log2_theta * (2.0f * (lane * 2 + j)) / (float)D), &sn[j], &cs[j]);
   for (int h = blockIdx.y * 8 + warp; h < hq + 2 * H; h += 8 * gridDim.y) {
     const float* base = p.d_ws + (((size_t)(h * p.tts + tt) * p.splits) * p.tn + tr) * 128;
     if (h < hq + H) {
@@ -934,11 +941,8 @@ __global__ void __launch_bounds__(256) rope_append_partials_bf16_kernel(KvDev d,
       float o1[2], o2[2];
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const int i = lane * 2 + j;
-        float sn, cs;
-        sincosf((float)pos * exp2f(-log2_theta * (2.0f * i) / (float)D), &sn, &cs);
-        o1[j] = x1[j] * cs - x2[j] * sn;
-        o2[j] = x1[j] * sn + x2[j] * cs;
+        o1[j] = x1[j] * cs[j] - x2[j] * sn[j];
+        o2[j] = x1[j] * sn[j] + x2[j] * cs[j];
       }
       if (dst) {
         *reinterpret_cast<__nv_bfloat162*>(dst + 2 * lane) = __floats2bfloat162_rn(o1[0], o1[1]);
@@ -971,7 +975,7 @@ extern "C" b200_status b200_kv_rope_append_partials(b200_kv* kv, int32_t layer, 
   }
   if (layer < 0 || layer >= c.n_layers) { b200_set_error("append: layer %d out of range", layer); return B200_ERR_INVALID_ARGUMENT; }
   if (total_rows <= 0) return B200_OK;
-  launch_after(rope_append_partials_bf16_kernel, dim3(total_rows, (n_q_heads + 2 * c.n_kv_heads + 7) / 8), 256, 0, (cudaStream_t)stream,
+  launch_after(rope_append_partials_bf16_kernel, dim3(total_rows, rope_blocks(total_rows, (n_q_heads + 2 * c.n_kv_heads + 7) / 8)), 256, 0, (cudaStream_t)stream,
       kv->dev, layer, *parts, (__nv_bfloat16*)d_q, q_stride, d_positions, d_row_seq, n_q_heads, log2f(theta));
   B200_LAUNCH_CHECK();
   return B200_OK;
@@ -991,7 +995,7 @@ b200_status b200_kv_rope_append_strided(b200_kv* kv, int32_t layer, void* d_q, c
   }
   if (layer < 0 || layer >= c.n_layers) { b200_set_error("append: layer %d out of range", layer); return B200_ERR_INVALID_ARGUMENT; }
   if (total_rows <= 0) return B200_OK;
-  launch_after(rope_append_bf16_kernel, dim3(total_rows, (n_q_heads + c.n_kv_heads + 7) / 8), 256, 0, (cudaStream_t)stream, kv->dev, layer, (__nv_bfloat16*)d_q, (const __nv_bfloat16*)d_k_rows,
+  launch_after(rope_append_bf16_kernel, dim3(total_rows, rope_blocks(total_rows, (n_q_heads + c.n_kv_heads + 7) / 8)), 256, 0, (cudaStream_t)stream, kv->dev, layer, (__nv_bfloat16*)d_q, (const __nv_bfloat16*)d_k_rows,
                                                                          (const __nv_bfloat16*)d_v_rows, q_stride, k_stride, v_stride,
                                                                          d_positions, d_row_seq, n_q_heads, log2f(theta));
   B200_LAUNCH_CHECK();

@@ -335,7 +335,7 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
 }
 // What the arrival announces is shared memory that the async proxy reads (written ahead of a fence of that proxy, or by a copy whose barrier the
 // thread has waited for) or tensor memory that has been read: no write that a wider scope would have to flush.  With .release.cluster here and
-// .acquire.cluster in the waits every chunk of a matmul took 1900 cycles instead of CP_CYCLES.
+// .acquire.cluster in the waits a chunk of a matmul took 1900 cycles instead of 950 (2048 x 8192, 512 rows, before its epilogue was changed).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t mapped_bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mapped_bar) : "memory");
 }

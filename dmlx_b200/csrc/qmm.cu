@@ -18,8 +18,12 @@
 //   * qmm_mma8_kernel (affine int4, up to 8 rows): the same on int8 mma.sync, from the raw codes.
 //   * qmm_few_kernel  (dense bf16, up to 16 rows, and experts' items of up to 16 rows): a CTA's eight
 //     warps share K of 16 or 32 weight rows, memory to mma.sync registers; no ring, no K split.
-//   * qmm_tca_kernel  (17..256 rows, quantised weights): qmm_tc_kernel with the dequantised weights in
-//     tensor memory.  qmm_mx_kernel, qmm_mxp_kernel: block-scaled MMAs on MXFP4 codes.
+//   * qmm_tp_kernel   (17..128 rows, quantised weights): two weight tiles per CTA, dequantised into tensor
+//     memory by 16 warps.  qmm_tca_kernel (matrices of more tile pairs than SMs, 129..256 rows of most
+//     shapes, grouped launches): one tile per CTA, two CTAs per SM.
+//   * qmm_mx_kernel, qmm_mxp_kernel: block-scaled MMAs on MXFP4 codes.
+//   * qmm_cp_kernel   (more than 128 rows, and dense experts' items of more than 128): an MMA of M256 over a
+//     pair of CTAs, two sets of sums, persistent.
 //   * qmm_tc_kernel   (17..128 rows per token tile, and the grouped MoE launches): "swap-AB" tcgen05
 //     GEMM.  The 128 weight rows are the MMA M dimension, the packed tokens (16..256 per tile) the N
 //     dimension, so small and large batches both map to dense tensor-core tiles.  Per 64-column
@@ -28,8 +32,8 @@
 //     tile (one row and one 32-column plane per thread); warp 9 issues 4 tcgen05.mma (M128 x N x
 //     K16) accumulating in tensor memory and commits to free the stage.  After the last chunk all
 //     eight dequantising warps read the accumulator with tcgen05.ld, 32 tokens in turn per half.
-//   * qmm_tc2_kernel  (129..256 rows per token tile, and dense experts' items of more than 128): the
-//     same with two weight tiles per CTA sharing one activation tile.
+//   * qmm_tc2_kernel  (what qmm_cp_kernel's wide stores cannot address): the same with two weight tiles per
+//     CTA sharing one activation tile.
 //   * qmm_simt_kernel : CUDA-core GEMV kept as a forced path for tests.
 // Split-K partials go to an f32 scratch; a finish kernel sums them in split order (deterministic),
 // applies the epilogue (residual add, SwiGLU) and writes bf16.  No CTA waits on another.
@@ -128,9 +132,23 @@ __device__ __forceinline__ void finish_store(const QmmArgs& a, int token, int n,
   const float rs = a.row_scale(token);
   if (a.epilogue == B200_EPI_SWIGLU) {
     const float y0 = gated(a, acc.x, acc.y) * rs, y1 = gated(a, acc.z, acc.w) * rs;
-    *reinterpret_cast<__nv_bfloat162*>(a.y + (size_t)a.row_base_out(token) * a.out_stride(a.n / 2) + n / 2) = __floats2bfloat162_rn(y0, y1);
+    __nv_bfloat16* dst = a.y + (size_t)a.row_base_out(token) * a.out_stride(a.n / 2) + n / 2;
+    if (a.n % 4 == 0 && ((uintptr_t)dst & 3) == 0) {
+      *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(y0, y1);
+    } else {
+      dst[0] = __float2bfloat16(y0);
+      if (n + 2 < a.n) dst[1] = __float2bfloat16(y1);
+    }
   } else {
     const size_t o = (size_t)a.row_base_out(token) * a.out_stride(a.n) + n;
+    if (a.n % 4 != 0 || ((uintptr_t)(a.y + o) & 7) != 0 || (a.epilogue == B200_EPI_RESIDUAL && ((uintptr_t)(a.residual + o) & 7) != 0)) {
+      // outputs that do not come in aligned fours, one by one
+      const float v[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (n + j < a.n) a.y[o + j] = __float2bfloat16((a.epilogue == B200_EPI_RESIDUAL ? v[j] + __bfloat162float(a.residual[o + j]) : activate(a.epilogue, v[j])) * rs);
+      return;
+    }
     if (a.epilogue == B200_EPI_RESIDUAL) {
       const uint2 rv = *reinterpret_cast<const uint2*>(a.residual + o);
       acc.x += ptx::bf16_lo(rv.x); acc.y += ptx::bf16_hi(rv.x); acc.z += ptx::bf16_lo(rv.y); acc.w += ptx::bf16_hi(rv.y);
@@ -1361,7 +1379,7 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
     }
   } else {
     // ---- a warp's 32 weight rows, 16 tokens at a time, through shared memory: 16-byte stores (2-byte ones straight from the accumulator layout
-    // took longer than the MMAs: 2026 rows of 16384 x 2048 with SwiGLU 161 us, CP_DENSE this way, 71 without an epilogue) ----
+    // took longer than the MMAs: 2026 rows of 16384 x 2048 with SwiGLU 161 us, 94 this way, 71 without an epilogue) ----
     const int lq = warp & 3, part = (warp - kRoles - 4) >> 2;  // dense: two warps share a quarter, half of the tokens each
     constexpr int kParts = Z::kEpilogue / 4, kB = Z::kBatch, kPieces = kB / 8;  // pieces of eight outputs of a lane
     float* tile = staging + (warp - kRoles - 4) * kB * kCpPitch;
@@ -2237,23 +2255,28 @@ __device__ __forceinline__ float2 mx_e4m3x2_to_f32x2(uint32_t codes) {
 }
 
 // x [rows, k] bf16 -> hi, lo [rows, k] E4M3 and unscale[rows].  One CTA per row; k % 8 == 0.
-__global__ void __launch_bounds__(256) mx_split_activations_kernel(const __nv_bfloat16* __restrict__ x, int k,
-                                                                   unsigned char* __restrict__ hi, unsigned char* __restrict__ lo,
-                                                                   float* __restrict__ unscale, const int* __restrict__ gather,
-                                                                   int gather_div, const int* __restrict__ rows_valid) {
-  wait_previous();  // (CTAs of the matmul that were placed while rows are still split made it slower: 24576 rows of K = 2048 335 -> 374 us)
+// A row's codes, hi and residual, by a block of 256 threads; f(first column / 8, hi of eight columns, lo of them) stores them.  Returns the factor
+// that undoes the row's scaling.  What a thread read for the row's maximum stays in registers up to K = 4096.
+template <typename F>
+__device__ __forceinline__ float split_row(const uint4* __restrict__ xr, int k8, F f) {
   __shared__ float s_max[8];
-  const int row = blockIdx.x;
-  if (rows_valid && row >= *rows_valid) return;  // capacity beyond the rows that exist: nothing to read
-  const int src_row = gather ? gather[row] / gather_div : row;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)src_row * k);
-  float amax = 0.f;
-  for (int i = threadIdx.x; i < k / 8; i += blockDim.x) {
-    const uint4 q = xr[i];
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+  constexpr int kHeld = 2;
+  uint4 held[kHeld];
+  __nv_bfloat162 top = __floats2bfloat162_rn(0.f, 0.f);
+  auto look = [&](const uint4& q) {  // (a value that is no number does not count)
+    const uint32_t w[4] = {q.x & 0x7FFF7FFFu, q.y & 0x7FFF7FFFu, q.z & 0x7FFF7FFFu, q.w & 0x7FFF7FFFu};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) amax = fmaxf(amax, fmaxf(fabsf(ptx::bf16_lo(w[j])), fabsf(ptx::bf16_hi(w[j]))));
+    for (int j = 0; j < 4; ++j) top = __hmax2(top, *reinterpret_cast<const __nv_bfloat162*>(&w[j]));
+  };
+#pragma unroll
+  for (int h = 0; h < kHeld; ++h) {
+    const int i = threadIdx.x + h * 256;
+    held[h] = i < k8 ? xr[i] : make_uint4(0u, 0u, 0u, 0u);
   }
+#pragma unroll
+  for (int h = 0; h < kHeld; ++h) look(held[h]);
+  for (int i = threadIdx.x + kHeld * 256; i < k8; i += 256) look(xr[i]);
+  float amax = fmaxf(__low2float(top), __high2float(top));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = amax;
@@ -2264,11 +2287,7 @@ __global__ void __launch_bounds__(256) mx_split_activations_kernel(const __nv_bf
   // amax = m * 2^ex with m in [1, 2): scale by 2^(7 - ex) (zero, vanishing and non-finite rows keep scale 1)
   const int ex = amax >= 1e-30f && amax < 3e38f ? (int)((__float_as_uint(amax) >> 23) & 0xFF) - 127 : 7;
   const float qs = __uint_as_float((uint32_t)(127 + 7 - ex) << 23);
-  if (threadIdx.x == 0) unscale[row] = __uint_as_float((uint32_t)(127 + ex - 7) << 23);
-  uint2* hr = reinterpret_cast<uint2*>(hi + (size_t)row * k);
-  uint2* lr = reinterpret_cast<uint2*>(lo + (size_t)row * k);
-  for (int i = threadIdx.x; i < k / 8; i += blockDim.x) {
-    const uint4 q = xr[i];
+  auto split = [&](int i, const uint4& q) {
     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
     uint32_t h[4], l[4];
 #pragma unroll
@@ -2278,9 +2297,43 @@ __global__ void __launch_bounds__(256) mx_split_activations_kernel(const __nv_bf
       const float2 back = mx_e4m3x2_to_f32x2(h[j]);
       l[j] = mx_f32x2_to_e4m3x2((a - back.x) * 16.f, (b - back.y) * 16.f);
     }
-    hr[i] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-    lr[i] = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
-  }
+    f(i, make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16)), make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16)));
+  };
+#pragma unroll
+  for (int h = 0; h < kHeld; ++h)
+    if (const int i = threadIdx.x + h * 256; i < k8) split(i, held[h]);
+  for (int i = threadIdx.x + kHeld * 256; i < k8; i += 256) split(i, xr[i]);
+  return __uint_as_float((uint32_t)(127 + ex - 7) << 23);
+}
+
+__global__ void __launch_bounds__(256) mx_split_activations_kernel(const __nv_bfloat16* __restrict__ x, int k,
+                                                                   unsigned char* __restrict__ hi, unsigned char* __restrict__ lo,
+                                                                   float* __restrict__ unscale, const int* __restrict__ gather,
+                                                                   int gather_div, const int* __restrict__ rows_valid) {
+  wait_previous();  // (CTAs of the matmul that were placed while rows are still split made it slower: 24576 rows of K = 2048 335 -> 374 us)
+  const int row = blockIdx.x;
+  if (rows_valid && row >= *rows_valid) return;  // capacity beyond the rows that exist: nothing to read
+  const int src_row = gather ? gather[row] / gather_div : row;
+  uint2 *hr = reinterpret_cast<uint2*>(hi + (size_t)row * k), *lr = reinterpret_cast<uint2*>(lo + (size_t)row * k);
+  const float us = split_row(reinterpret_cast<const uint4*>(x + (size_t)src_row * k), k / 8, [&](int i, uint2 h, uint2 l) { hr[i] = h; lr[i] = l; });
+  if (threadIdx.x == 0) unscale[row] = us;
+}
+
+// The same for tokens whose rows are wanted at `top` places each: a token is split once (4096 tokens, 6 places, K = 4096: 78 us row by row, 35 this way).
+constexpr int kMaxPlaces = 16;
+__global__ void __launch_bounds__(256) mx_split_tokens_kernel(const __nv_bfloat16* __restrict__ x, int k, unsigned char* __restrict__ hi,
+                                                              unsigned char* __restrict__ lo, float* __restrict__ unscale, const int* __restrict__ places, int top) {
+  wait_previous();
+  __shared__ int s_place[kMaxPlaces];
+  if (threadIdx.x < top) s_place[threadIdx.x] = places[(size_t)blockIdx.x * top + threadIdx.x];  // (the barrier inside split_row publishes it)
+  const float us = split_row(reinterpret_cast<const uint4*>(x + (size_t)blockIdx.x * k), k / 8, [&](int i, uint2 h, uint2 l) {
+    for (int j = 0; j < top; ++j) {
+      const size_t at = (size_t)s_place[j] * k;
+      reinterpret_cast<uint2*>(hi + at)[i] = h;
+      reinterpret_cast<uint2*>(lo + at)[i] = l;
+    }
+  });
+  if (threadIdx.x < top) unscale[s_place[threadIdx.x]] = us;
 }
 
 // Tile-major blocks -> row-major codes + scale atoms (see b200_qweight).  One thread per 32-bit word of a plane.
@@ -3392,7 +3445,10 @@ static b200_status launch_mx(const b200_qweight* w, QmmArgs& a, int rows, cudaSt
   unsigned char* hi = g_mx_act;
   unsigned char* lo = hi + (size_t)rows * a.k;
   float* unscale = reinterpret_cast<float*>(lo + (((size_t)rows * a.k + 255) / 256) * 256);
-  launch_after(mx_split_activations_kernel, rows, 256, 0, s, a.x, a.k, hi, lo, unscale, a.x_gather, a.x_gather_div, a.rows_valid);
+  if (a.x_places && a.x_gather_div <= kMaxPlaces)
+    launch_after(mx_split_tokens_kernel, rows / a.x_gather_div, 256, 0, s, a.x, a.k, hi, lo, unscale, a.x_places, a.x_gather_div);
+  else
+    launch_after(mx_split_activations_kernel, rows, 256, 0, s, a.x, a.k, hi, lo, unscale, a.x_gather, a.x_gather_div, a.rows_valid);
   B200_LAUNCH_CHECK();
   MxActMaps amaps;
   std::memset(&amaps, 0, sizeof(amaps));
@@ -3756,9 +3812,10 @@ static b200_status qmm_entry(const b200_qweight* w, const void* d_x, int32_t row
       const int tn = std::min(256, ((rows + 15) / 16) * 16), pair_ctas = ((w->nt + 1) / 2) * ((rows + tn - 1) / tn);
       if (ensure_state(0) != B200_OK) return B200_ERR_CUDA;
       const bool one_wave = pair_ctas <= g_sms && pair_ctas * 2 >= g_sms;
-      // more than one 256-row token tile (prefill chunks): the tile-pair kernel is ahead or level on
-      // every projection shape (gate/up 122 vs 158 us at 384 rows, 126 vs 172 us at 512, 317 vs 337 us
-      // at 1024; down 113 vs 121 us at 1024)
+      // more than one 256-row token tile (prefill chunks): the tile pairs are ahead or level on every projection shape (with two
+      // tiles per CTA already: gate/up 122 vs 158 us at 384 rows, 317 vs 337 at 1024; on pairs of CTAs 102 at 400 and 181 at 1024).
+      // 129..256 rows: pairs of CTAs where the grid was one wave of tile pairs (gate/up 54..59 us against 55..64) and for dense weights
+      // (16384 x 2048 at 256 rows 39 -> 25 us); elsewhere the tensor-memory kernel stays ahead (4096 x 14336 31..43 against 38..44 us)
       path = (one_wave || rows > 256 || w->mode == B200_Q_BF16) ? B200_QMM_TCGEN05_X2 : B200_QMM_TCGEN05_TMEM_A;
     } else {
       path = w->mode == B200_Q_BF16 ? B200_QMM_TCGEN05 : B200_QMM_TCGEN05_TMEM_A;
@@ -4008,8 +4065,8 @@ b200_status b200_qmm_grouped(const b200_qweight* w, const void* d_x, int32_t row
   if (w->mode == B200_Q_AFFINE4_G64) return launch_tc<B200_Q_AFFINE4_G64>(a, rows, s);
   if (w->mode == B200_Q_MXFP4_G32) return launch_tc<B200_Q_MXFP4_G32>(a, rows, s);
   if (takes_few(a, tile_rows)) return launch_few(a, tile_rows, s);
-  // dense weights, items of more than 128 rows: pairs of CTAs (32 experts of 1024 x 2048 with 253 rows on average: gate/up 98 -> CP_EXP us, down
-  // 64 -> CP_EXPD against two weight tiles per CTA, which takes what the pairs' wide stores cannot)
+  // dense weights, items of more than 128 rows: pairs of CTAs (32 experts of 1024 x 2048 with 253 rows on average: gate/up 98 -> 75 us, down
+  // 64 -> 54 against two weight tiles per CTA, which takes what the pairs' wide stores cannot)
   if (tile_rows > 128 && tile_rows <= kCpTokens && takes_pairs(a, tile_rows)) return launch_cp<B200_Q_BF16>(a, rows, s);
   return tile_rows > 128 ? launch_tc2<B200_Q_BF16>(a, rows, s) : launch_tc<B200_Q_BF16>(a, rows, s);
 }
@@ -4022,7 +4079,7 @@ int b200_qmm_grouped_takes_tokens(const b200_qweight* w, int32_t tile_rows) {
 b200_status b200_qmm_grouped_from_tokens(const b200_qweight* w, const void* d_tokens, const int* d_order, int32_t top_k,
                                          int32_t rows, void* d_y, int32_t epilogue, const float* d_row_scales,
                                          float swiglu_limit, const int4* d_items, const int* d_n_items, int32_t max_items,
-                                         int32_t tile_rows, void* stream, const int* d_rows_valid) {
+                                         int32_t tile_rows, void* stream, const int* d_rows_valid, const int* d_places) {
   b200_status st = b200_require_device();
   if (st != B200_OK) return st;
   if (rows <= 0) return B200_OK;
@@ -4032,7 +4089,7 @@ b200_status b200_qmm_grouped_from_tokens(const b200_qweight* w, const void* d_to
   a.row_scales = d_row_scales;
   a.rows = rows; a.n = w->n; a.k = w->k; a.nt = w->nt; a.kc = w->kc; a.epilogue = epilogue; a.swiglu_limit = swiglu_limit;
   a.items = d_items; a.n_items = d_n_items; a.max_items = max_items; a.tn = tile_rows;
-  a.x_gather = d_order; a.x_gather_div = top_k;
+  a.x_gather = d_order; a.x_gather_div = top_k; a.x_places = d_places;
   a.rows_valid = d_rows_valid;
   return launch_mx(w, a, rows, (cudaStream_t)stream);
 }

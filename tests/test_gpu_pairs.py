@@ -1,0 +1,152 @@
+"""Matmuls on pairs of CTAs (more than 128 rows), on pairs of weight tiles in tensor memory (17 to 128 rows), experts of few rows with both halves
+of an activation side by side, and the small kernels of a step's chain, at the sizes where each can go wrong.
+
+Tolerance of a matmul's row, as 2-norms: the result is rounded to bf16 (2^-9 of each value), a quantised weight too (2^-9 of each weight), SwiGLU
+multiplies two sums that carry the weights' part: 3 * 2^-9, and the sums' own rounding is far below that."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import ref_math
+
+pytestmark = pytest.mark.gpu
+ROW_TOL = 3 * 2.0 ** -9
+
+
+def _weight(mode, n, k, seed):
+    from dmlx_b200 import device as dev
+
+    rng = np.random.default_rng(seed)
+    if mode == "bf16":
+        w = ref_math.bf16_round(rng.normal(0, k ** -0.5, (n, k)))
+        bits = (w.astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+        return dev.QWeight(dev.Q_BF16, bits, np.zeros(1, np.uint8), None, n, k), w
+    if mode == "mxfp4":
+        packed, scales = rng.integers(0, 256, (n, k // 2), dtype=np.uint8), rng.integers(119, 123, (n, k // 32), dtype=np.uint8)
+        return dev.QWeight(dev.Q_MXFP4_G32, packed, scales, None, n, k), ref_math.dequantize_mxfp4(packed, scales)
+    packed = rng.integers(0, 2 ** 32, (n, k // 8), dtype=np.uint32)
+    s = ref_math.bf16_round(rng.uniform(0.6, 1.4, (n, k // 64)) / (4.6 * k ** 0.5)).astype(np.float32)
+    b = ref_math.bf16_round(-7.5 * s).astype(np.float32)
+    bits = lambda a: (a.view(np.uint32) >> 16).astype(np.uint16)  # noqa: E731
+    return dev.QWeight(dev.Q_AFFINE4_G64, packed, bits(s), bits(b), n, k), ref_math.dequantize_affine4(packed, s, b)
+
+
+def _rows(rows, k, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn((rows, k), generator=g, device="cuda").bfloat16()
+
+
+def _check(got, want):
+    err = (got.double() - want).norm(dim=1) / want.norm(dim=1).clamp_min(1e-30)
+    assert float(err.max()) <= ROW_TOL, float(err.max())
+
+
+def _run(mode, n, k, rows, path=None):
+    from dmlx_b200 import device as dev
+
+    w, dense = _weight(mode, n, k, n + k)
+    dense = torch.tensor(np.asarray(dense, np.float32), device="cuda").double()
+    kw = {} if path is None else {"path": getattr(dev, path)}
+    x = _rows(rows, k, rows)
+    plain = x.double() @ dense.T
+    guard = torch.full((rows + 2, n), 7.0, dtype=torch.bfloat16, device="cuda")  # the rows behind the last one stay as they are
+    _check(dev.qmm(w, x, out=guard[:rows], **kw), plain)
+    assert bool((guard[rows:] == 7.0).all())
+    residual = _rows(rows, n, rows + 1)
+    _check(dev.qmm(w, x, dev.EPI_RESIDUAL, residual=residual, **kw), plain + residual.double())
+    if n % 2 == 0:
+        _check(dev.qmm(w, x, dev.EPI_SWIGLU, **kw), torch.nn.functional.silu(plain[:, 0::2]) * plain[:, 1::2])
+    assert dev.qmm_error_word() == 0
+
+
+# one chunk of K and several, an odd number of weight tiles, outputs that end inside a tile (dense), K so long that it is split
+@pytest.mark.parametrize("mode,n,k", [("bf16", 256, 64), ("bf16", 384, 192), ("bf16", 1000, 320), ("bf16", 1004, 128), ("bf16", 256, 8192), ("affine4", 384, 64),
+                                      ("affine4", 256, 4096), ("mxfp4", 384, 192)])
+@pytest.mark.parametrize("rows", [129, 144, 255, 256, 257, 273, 512, 513, 770])
+def test_pairs_of_ctas(mode, n, k, rows):
+    _run(mode, n, k, rows, "QMM_TCGEN05_X2")
+
+
+@pytest.mark.parametrize("n", [33, 34, 129, 130])
+@pytest.mark.parametrize("rows", [65, 128, 200, 300])
+def test_outputs_that_do_not_come_in_fours(n, rows):
+    """The finish pass of split or widely tiled products stored four outputs at a time whatever the row's length."""
+    _run("bf16", n, 2048, rows)
+    _run("bf16", n, 256, rows)
+
+
+@pytest.mark.parametrize("mode,n,k", [("affine4", 384, 192), ("affine4", 256, 4096), ("mxfp4", 128, 64)])
+@pytest.mark.parametrize("rows", [17, 32, 33, 64, 65, 96, 97, 128])
+def test_pairs_of_tiles(mode, n, k, rows):
+    _run(mode, n, k, rows, "QMM_TCGEN05_TMEM_A")
+
+
+def _grouped(mode, e, n, k, sizes, tile, swiglu):
+    from dmlx_b200 import device as dev
+
+    w = dev.QWeight.random(getattr(dev, "Q_BF16" if mode == "bf16" else "Q_MXFP4_G32"), n, k, n_experts=e, seed=n)
+    x = _rows(sum(sizes), k, e)
+    items, first, want = [], 0, []
+    for i, s in enumerate(sizes):
+        items.append((i % e, first, s, 0))
+        packed, scales, _ = w.export(i % e)
+        if mode == "bf16":
+            dense = torch.tensor(packed.astype(np.int32), device="cuda").to(torch.int32).mul(65536).view(torch.float32).double().reshape(n, k)
+        else:
+            dense = torch.tensor(np.asarray(ref_math.dequantize_mxfp4(packed, scales), np.float32), device="cuda").double()
+        y = x[first:first + s].double() @ dense.T
+        want.append(torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2] if swiglu else y)
+        first += s
+    dev_items = torch.tensor(items + [(0, 0, 9, 0)], dtype=torch.int32, device="cuda")  # (one more than the list says it has)
+    count = torch.tensor([len(items)], dtype=torch.int32, device="cuda")
+    scale = torch.rand(sum(sizes), device="cuda") + 0.5
+    got = dev.moe_grouped_qmm(w, x, dev_items, count, tile, dev.EPI_SWIGLU if swiglu else dev.EPI_NONE, row_scales=scale)
+    assert dev.qmm_error_word() == 0
+    _check(got, torch.cat(want) * scale.double()[:, None])
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("sizes", [[1, 15, 16, 17, 0, 255, 256], [130, 129, 241, 256, 3, 64, 65, 66], [200] * 80])
+def test_dense_experts_on_pairs_of_ctas(sizes, swiglu):
+    _grouped("bf16", 4, 384, 192, sizes, 256, swiglu)
+
+
+@pytest.mark.parametrize("sizes,tile", [([1, 15, 16], 16), ([1, 16, 17, 31, 32], 32), ([2, 16, 17, 32, 33, 47, 48], 48), ([5] * 160, 48), ([49, 64, 3], 64)])
+def test_block_scaled_experts_of_few_rows(sizes, tile):
+    # (activations as two E4M3 codes: exact for bf16 rows whose values lie within 2^13 of the largest)
+    _grouped("mxfp4", 3, 384, 256, sizes, tile, False)
+
+
+@pytest.mark.parametrize("tokens", [1, 31, 32, 33, 85, 86, 128, 129])  # 6 choices: 510 assignments are routed by one block, 516 are not
+@pytest.mark.parametrize("experts", [8, 33, 200])
+def test_routing_by_one_block_is_the_routing_by_kernels(tokens, experts):
+    from dmlx_b200 import device as dev
+
+    h, inter, top = 256, 128, 6
+    gate = torch.eye(experts, h, device="cuda").bfloat16()  # logits are values of x, whichever kernel multiplies
+    bits = lambda t: t.cpu().view(torch.int16).numpy().view(np.uint16)  # noqa: E731
+    layer = dev.MoELayer(h, experts, inter, top, dev.QWeight(dev.Q_BF16, bits(gate), np.zeros(1, np.uint8), None, experts, h),
+                         dev.QWeight.random(dev.Q_MXFP4_G32, 2 * inter, h, n_experts=experts), dev.QWeight.random(dev.Q_MXFP4_G32, h, inter, n_experts=experts),
+                         None, None, route_scale=1.5, max_tokens=256)
+    x = _rows(256, h, tokens)
+    few, many = layer.forward(x[:tokens]).double(), layer.forward(x).double()[:tokens]
+    # another row tile adds a row's two halves up in another order; bf16 activations may then round to the other neighbour
+    assert float((few - many).norm() / many.norm()) <= 2.0 ** -8
+    assert dev.qmm_error_word() == 0
+
+
+@pytest.mark.parametrize("vocab", [7, 8191, 8192, 32000, 32001, 128256])
+@pytest.mark.parametrize("rows", [1, 16, 17, 33, 130])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_argmax_takes_the_first_maximum_wherever_the_row_is_cut(dtype, rows, vocab):
+    from dmlx_b200 import device as dev
+
+    x = torch.randn((rows, vocab), generator=torch.Generator(device="cuda").manual_seed(vocab), device="cuda").to(dtype)
+    for r in range(rows):  # the maximum twice, on both sides of a cut or at the ends
+        at = [0, vocab // 8, vocab // 4 - 1, vocab // 2, vocab - 1][r % 5]
+        x[r, max(at, 0)] = 50.0
+        x[r, vocab - 1] = 50.0
+    if rows > 1:
+        x[1] = -float("inf")
+    want = np.array([int(np.argmax(row)) for row in x.float().cpu().numpy()])
+    assert np.array_equal(dev.argmax(x).cpu().numpy(), want)
