@@ -130,7 +130,7 @@ __device__ __forceinline__ int scan(int v, int* warp_buf) {  // inclusive, over 
   if (lane == 31) warp_buf[warp] = v;
   __syncthreads();
   if (warp == 0) {
-    int w = warp_buf[lane];
+    int w = lane < (int)(blockDim.x >> 5) ? warp_buf[lane] : (MAX ? -1 : 0);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int t = __shfl_up_sync(0xffffffffu, w, o);
@@ -165,22 +165,52 @@ __global__ void __launch_bounds__(1024) prompt_plan_kernel(const int* __restrict
   if (tid == 0) { s_old = 0; s_longest = 0; s_pick = 0; }
   if (tid < 256) hist[tid] = 0;
   __syncthreads();
-  for (int base = 0; base < total_rows; base += blockDim.x) {
-    const int i = base + tid;
-    const bool valid = i < total_rows;
-    const bool joins = valid && i > 0 && row_seq[i] == row_seq[i - 1] && row_ctx[i] == row_ctx[i - 1] + 1;
-    const int run = max(scan<true>(valid && !joins ? i : -1, warp_buf), carry[0]);
-    const int head = valid && (i - run) % q_tokens == 0 ? 1 : 0;
-    const int heads_incl = scan<false>(head, warp_buf), gid = carry[1] + heads_incl - 1;
-    int old = 0;
-    if (valid) {
+  // four neighbouring rows a thread, so that one round of scans is enough for 1024 rows in 256 threads and 4096 in 1024
+  constexpr int kRows = 4;
+  for (int base = 0; base < total_rows; base += kRows * blockDim.x) {
+    const int i0 = base + kRows * tid;
+    int seq[kRows + 1], ctx[kRows + 1], run[kRows];
+#pragma unroll
+    for (int k = 0; k <= kRows; ++k) {
+      const int i = i0 + k - 1;
+      const bool there = i >= 0 && i < total_rows;
+      seq[k] = there ? row_seq[i] : -1;
+      ctx[k] = there ? row_ctx[i] : 0;
+    }
+    int last_start = -1;
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+      const int i = i0 + k;
+      const bool joins = i > 0 && seq[k + 1] == seq[k] && ctx[k + 1] == ctx[k] + 1;
+      if (i < total_rows && !joins) last_start = i;
+      run[k] = last_start;
+    }
+    const int starts = scan<true>(last_start, warp_buf);  // of this thread's rows and those before
+    int before = __shfl_up_sync(0xffffffffu, starts, 1);
+    if (lane == 0) before = tid > 0 ? warp_buf[(tid >> 5) - 1] : -1;
+    before = max(before, carry[0]);
+    int heads = 0;
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+      run[k] = max(run[k], before);
+      heads += i0 + k < total_rows && (i0 + k - run[k]) % q_tokens == 0 ? 1 : 0;
+    }
+    __syncthreads();  // (the scans share a buffer)
+    const int heads_incl = scan<false>(heads, warp_buf);
+    int gid = carry[1] + heads_incl - heads - 1, old = 0;
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+      const int i = i0 + k;
+      if (i >= total_rows) break;
+      const bool head = (i - run[k]) % q_tokens == 0;
+      gid += head ? 1 : 0;
       row_group[i] = gid;
       if (head) group_first[gid] = i;
       if (old_tokens > 0) {  // slots of this row as the limit counts them: by the context of its group's last row
-        const int last = (i - run) / old_tokens * old_tokens + old_tokens - 1 + run;
+        const int last = (i - run[k]) / old_tokens * old_tokens + old_tokens - 1 + run[k];
         int end = i;
         while (end < last && end + 1 < total_rows && row_seq[end + 1] == row_seq[end] && row_ctx[end + 1] == row_ctx[end] + 1) ++end;
-        old = ((max(row_ctx[end], 0) + page_size - 1) / page_size + 7) / 8;
+        old += ((max(row_ctx[end], 0) + page_size - 1) / page_size + 7) / 8;
       }
     }
     if (old_tokens > 0) {
@@ -188,7 +218,7 @@ __global__ void __launch_bounds__(1024) prompt_plan_kernel(const int* __restrict
       if (lane == 0) atomicAdd(&s_old, old);
     }
     __syncthreads();
-    if (tid == blockDim.x - 1) { carry[0] = run; carry[1] += heads_incl; }
+    if (tid == blockDim.x - 1) { carry[0] = max(starts, carry[0]); carry[1] += heads_incl; }
     __syncthreads();
   }
   const int n_groups = carry[1];
@@ -263,7 +293,7 @@ __global__ void __launch_bounds__(1024) prompt_plan_kernel(const int* __restrict
   if (tid < 256) hist[tid] = h_incl - h;
   __syncthreads();
   for (int g = tid; g < n_groups; g += blockDim.x) {
-    const int blocks = g < 1024 ? s_group[g].y : look(g).y, chunks = max((blocks + len - 1) / len, 1);
+    const int blocks = g < (int)blockDim.x ? s_group[g].y : look(g).y, chunks = max((blocks + len - 1) / len, 1);
     for (int c = 0; c < chunks; ++c) items[atomicAdd(&hist[bucket(min(len, blocks - c * len))], 1)] = make_int2(g, c);
   }
   if (tid == 0) {
@@ -875,7 +905,7 @@ b200_status b200_attn_prompt(b200_kv* kv, int32_t layer, const void* d_q, int32_
   a.scale_log2 = 1.4426950408889634f / sqrtf((float)c.head_dim);
   a.may_split = may_split;
   if (!reuse_plan) {
-    launch_after(prompt_plan_kernel, 1, 1024, 0, s, d_row_seq, d_row_ctx, total_rows, c.page_size, 2 * kTileRows / g, kTileRows / g, c.n_kv_heads, g_prompt_sms,
+    launch_after(prompt_plan_kernel, 1, total_rows <= 1024 ? 256 : 1024, 0, s, d_row_seq, d_row_ctx, total_rows, c.page_size, 2 * kTileRows / g, kTileRows / g, c.n_kv_heads, g_prompt_sms,
                                           may_split ? 1 : 0, kv->max_chunks, may_split ? 16 / g : 0, kv->d_chunk_start, kv->d_groups, kv->d_groups + stride,
                                           kv->d_groups + 2 * stride, reinterpret_cast<int2*>(kv->d_prompt + kHdr), kv->d_prompt, kv->dev.state + ST_ATTN_ERR);
     B200_LAUNCH_CHECK();
