@@ -31,8 +31,8 @@
 // The plan is the published one of attention on this chip: two tiles of rows, P in place of S, a warp each for loads and MMAs.
 //
 // Measured on one B200, bf16, 32/8 heads of 128, a call over 3 portions of 683 tokens over 700..8000 cached, plan included: 981 us in groups of
-// 16 rows per warp on mma.sync (paged_attn.cu), 179 us here (the kernel alone 171); a step of four 512-token portions and 57 decoding requests
-// through four layers 7.27 and 5.00 ms.
+// 16 rows per warp on mma.sync (paged_attn.cu), 167 us here (plan 8, the kernel 154); a step of four 512-token portions and 57 decoding requests
+// through four layers 7.27 and 5.00 ms with the other kernels as they were (4.4 now).
 #include <cuda_bf16.h>
 
 #include <algorithm>

@@ -378,19 +378,30 @@ __global__ void __launch_bounds__(256) gla_chunk_kernel(Gla a) {
 // o^T = S^T q^T.  A ring of stages, each a chunk's block and its slice of values (two bulk copies).
 // DELTA: the values that enter the state are u = U - W S with the state at the chunk's start, W [tokens][dk] and U [tokens][dv] made by
 // delta_chunk_kernel (delta.cu); u is f32 and enters the tensor cores as two terms.
-template <int NT, bool DELTA>  // NT: 8-channel tiles of the state a warp holds
+// Bound by the MMAs of a warp: at 128 channels 312 per chunk by the delta rule (208 without), 16 cycles each where the warp has the tensor core of
+// its quarter of an SM to itself.  Few portions of few heads (2 portions, 16 heads: 64 CTAs) leave SMs idle, and another SM can only be put to
+// work by splitting the channels: W warps share 16 columns, a part of the channels each, and add up what they have of W S and of o through
+// shared memory once a chunk; each finishes the outputs of 4 / W tiles of tokens.
+// Portions of 1013 tokens: delta rule, 16 heads of 128 x 128, one portion 103 -> 49 us (W = 4), two 104 -> 75 (W = 2); gated, 8 heads of 128 x 256,
+// two 68 -> 46 (W = 2).  Three portions of the first are 96 CTAs and stay whole.
+template <int NT, bool DELTA, int W>  // NT: 8-channel tiles of the state a warp holds
 __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
   wait_previous();
   extern __shared__ unsigned char scan_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(scan_dyn) + 127) & ~(uintptr_t)127);
-  const int req = blockIdx.x, head = blockIdx.y, slice = blockIdx.z;
+  constexpr int kStrips = kScanWarps / W, kOwn = 4 / W;  // strips of 16 columns per CTA, tiles of tokens whose outputs a warp finishes
+  const int req = blockIdx.x, head = blockIdx.y, slice = blockIdx.z / W;
   const int c0 = a.first_chunk[req], c1 = a.first_chunk[req + 1];
   if (c0 >= c1 || a.d.state[ST_ERR] != 0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int dkp = a.dkp, n_t = dkp / 8, stages = a.stages;
+  const int strip = (blockIdx.z % W) * kStrips + warp / W, part = warp % W;  // of the slice's columns; of the channels
+  if (W > 1 && slice * kScanCols + (int)(blockIdx.z % W) * kStrips * 16 >= a.dva) return;
+  const int j0 = part * NT, n0 = part * kOwn;  // first tile of channels and first tile of tokens
+  const int dkp = a.dkp, n_t = dkp / 8 - j0, stages = a.stages;  // (n_t: what is left from j0 on)
   constexpr uint32_t vbytes = (uint32_t)(DELTA ? kUSlice : kVSlice);
   const uint32_t cbytes = (uint32_t)(DELTA ? delta_chunk_size(dkp) : chunk_size(dkp)), stage_bytes = cbytes + vbytes;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)stages * stage_bytes);
+  float4* sums = reinterpret_cast<float4*>(smem + (size_t)stages * stage_bytes + 64);  // W > 1: [warp][o 0..3, w 0..3][lane]
   const int r0 = a.cu[req], slot = a.row_seq[r0];
   if (slot < 0 || slot >= a.d.max_seqs) return;
   if (tid == 0) {
@@ -408,7 +419,7 @@ __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
   if (tid == 0)
     for (int s = 0; s < stages && c0 + s < c1; ++s) load(c0 + s, s);
 
-  const int m0 = slice * kScanCols + warp * 16;  // first value column of the warp
+  const int m0 = slice * kScanCols + strip * 16;  // first value column of the warp
   float* S = a.state + (size_t)slot * a.rec_elems + (size_t)head * a.dk * a.dvs;
   float acc[NT][4];
   const bool fresh = a.pos[r0] == 0;
@@ -416,7 +427,7 @@ __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
   for (int j = 0; j < NT; ++j) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const int col = m0 + g + (e >> 1) * 8, ch = j * 8 + 2 * t + (e & 1);
+      const int col = m0 + g + (e >> 1) * 8, ch = (j0 + j) * 8 + 2 * t + (e & 1);
       acc[j][e] = !fresh && ch < a.dk && col < a.dva ? S[(size_t)ch * a.dvs + col] : 0.f;
     }
   }
@@ -454,7 +465,7 @@ __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
           uint32_t qh[2][4], ql[2][4], wh[2][4], wl[2][4];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const uint32_t at = base + (uint32_t)(((n + e) * 8 + lr) * qk_row(dkp) + kk * 64 + lm * 16);
+            const uint32_t at = base + (uint32_t)(((n + e) * 8 + lr) * qk_row(dkp) + j0 * 16 + kk * 64 + lm * 16);
             ldsm4(at + (uint32_t)off_part(dkp, 0), qh[e]);
             ldsm4(at + (uint32_t)off_part(dkp, 1), ql[e]);
             if constexpr (DELTA) {
@@ -480,10 +491,38 @@ __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
         }
       }
     }
+    float own[kOwn][4];  // the outputs that this warp finishes
+    if constexpr (W == 1) {
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) own[n][e] = o[n][e];
+    } else {
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        sums[(warp * 8 + n) * 32 + lane] = make_float4(o[n][0], o[n][1], o[n][2], o[n][3]);
+        if constexpr (DELTA) sums[(warp * 8 + 4 + n) * 32 + lane] = make_float4(w[n][0], w[n][1], w[n][2], w[n][3]);
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / W), "n"(W * 32) : "memory");
+      auto total = [&](int what, float (&to)[4]) {  // in the order of the parts, in every warp
+        to[0] = to[1] = to[2] = to[3] = 0.f;
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          const float4 x = sums[((warp / W * W + i) * 8 + what) * 32 + lane];
+          to[0] += x.x; to[1] += x.y; to[2] += x.z; to[3] += x.w;
+        }
+      };
+#pragma unroll
+      for (int n = 0; n < kOwn; ++n) total(n0 + n, own[n]);
+      if constexpr (DELTA) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n) total(4 + n, w[n]);
+      }
+    }
     // v^T as A operand: rows = value columns, k = tokens (two steps of 16)
     uint32_t va[2][4], vr[2][4];  // vr: the remainders
     if constexpr (DELTA) {
-      const float* U = reinterpret_cast<const float*>(st_ + cbytes) + (warp * 16 + g) * kUStride + 2 * t;
+      const float* U = reinterpret_cast<const float*>(st_ + cbytes) + (strip * 16 + g) * kUStride + 2 * t;
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
         const float2 x = *reinterpret_cast<const float2*>(U + n * 8), y = *reinterpret_cast<const float2*>(U + 8 * kUStride + n * 8);
@@ -494,21 +533,21 @@ __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         // the four 8 x 8 blocks of v [tokens][columns], transposed: (cols 0-7, tok 0-7), (cols 8-15, tok 0-7), (cols 0-7, tok 8-15), ...
-        const int row = u * 16 + (lm >> 1) * 8 + lr, col = warp * 16 + (lm & 1) * 8;
+        const int row = u * 16 + (lm >> 1) * 8 + lr, col = strip * 16 + (lm & 1) * 8;
         ldsm4_trans(vbase + (uint32_t)(row * kVRow + col * 2), va[u]);
       }
     }
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
+    for (int n = 0; n < kOwn; ++n) {
       uint32_t bh[4], bl[4];
-      const uint32_t at = base + (uint32_t)((n * 8 + lr) * kARow + lm * 16);
+      const uint32_t at = base + (uint32_t)(((n0 + n) * 8 + lr) * kARow + lm * 16);
       ldsm4(at + (uint32_t)off_a(dkp, 0), bh);
       ldsm4(at + (uint32_t)off_a(dkp, 1), bl);
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        mma16816(o[n], va[u], bh[2 * u], bh[2 * u + 1]);
-        mma16816(o[n], va[u], bl[2 * u], bl[2 * u + 1]);
-        if constexpr (DELTA) mma16816(o[n], vr[u], bh[2 * u], bh[2 * u + 1]);
+        mma16816(own[n], va[u], bh[2 * u], bh[2 * u + 1]);
+        mma16816(own[n], va[u], bl[2 * u], bl[2 * u + 1]);
+        if constexpr (DELTA) mma16816(own[n], vr[u], bh[2 * u], bh[2 * u + 1]);
       }
     }
     // the state moves on: decay its columns, add v^T k
@@ -518,7 +557,7 @@ __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
       if (j < n_t) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float2 d = *reinterpret_cast<const float2*>(dec + (j + e) * 8 + 2 * t);
+          const float2 d = *reinterpret_cast<const float2*>(dec + (j0 + j + e) * 8 + 2 * t);
           acc[j + e][0] *= d.x; acc[j + e][1] *= d.y; acc[j + e][2] *= d.x; acc[j + e][3] *= d.y;
         }
 #pragma unroll
@@ -528,7 +567,7 @@ __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
           for (int p = 0; p < 2; ++p) {
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const int row = u * 16 + (lm & 1) * 8 + lr, col = (j + 2 * e) * 8 + (lm >> 1) * 8;
+              const int row = u * 16 + (lm & 1) * 8 + lr, col = (j0 + j + 2 * e) * 8 + (lm >> 1) * 8;
               ldsm4_trans(base + (uint32_t)(off_part(dkp, 2 + p) + row * qk_row(dkp) + col * 2), b[p][e]);
             }
           }
@@ -545,11 +584,11 @@ __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
     }
     const int row0 = a.plan[c].x, rows = a.plan[c].y;
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
+    for (int n = 0; n < kOwn; ++n) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int tok = n * 8 + 2 * t + (e & 1), col = m0 + g + (e >> 1) * 8;
-        if (tok < rows && col < a.dva) a.o[((size_t)(row0 + tok) * a.heads + head) * a.dvs + col] = o[n][e];
+        const int tok = (n0 + n) * 8 + 2 * t + (e & 1), col = m0 + g + (e >> 1) * 8;
+        if (tok < rows && col < a.dva) a.o[((size_t)(row0 + tok) * a.heads + head) * a.dvs + col] = own[n][e];
       }
     }
     __syncthreads();  // every warp has read the stage
@@ -564,7 +603,7 @@ __global__ void __launch_bounds__(kScanWarps * 32) gla_scan_kernel(Gla a) {
   for (int j = 0; j < NT; ++j) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const int col = m0 + g + (e >> 1) * 8, ch = j * 8 + 2 * t + (e & 1);
+      const int col = m0 + g + (e >> 1) * 8, ch = (j0 + j) * 8 + 2 * t + (e & 1);
       if (ch < a.dk && col < a.dva) S[(size_t)ch * a.dvs + col] = acc[j][e];
     }
   }
@@ -723,25 +762,37 @@ __global__ void __launch_bounds__(256) memory_out_kernel(Gla a) {
   }
 }
 
-template <int NT, bool DELTA>
+template <int NT, bool DELTA, int W = 1>
 b200_status launch_scan(Gla& a, int n_req, cudaStream_t s) {
   const size_t stage = DELTA ? delta_chunk_size(a.dkp) + kUSlice : chunk_size(a.dkp) + kVSlice;
-  a.stages = (int)std::min<size_t>(4, (220 * 1024) / stage);
-  const size_t smem = a.stages * (stage + sizeof(uint64_t)) + 128;
+  constexpr size_t kSums = W > 1 ? kScanWarps * 8 * 32 * sizeof(float4) : 0;
+  a.stages = (int)std::min<size_t>(4, (220 * 1024 - kSums) / stage);
+  const size_t smem = a.stages * stage + 64 + kSums + 128;
   static bool configured = false;
   if (!configured) {
-    B200_CUDA_TRY((cudaFuncSetAttribute(gla_scan_kernel<NT, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024)));
+    B200_CUDA_TRY((cudaFuncSetAttribute(gla_scan_kernel<NT, DELTA, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024)));
     configured = true;
   }
-  launch_after(gla_scan_kernel<NT, DELTA>, dim3(n_req, a.heads, a.n_slices), kScanWarps * 32, smem, s, a);
+  launch_after(gla_scan_kernel<NT, DELTA, W>, dim3(n_req, a.heads, a.n_slices * W), kScanWarps * 32, smem, s, a);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
 
 template <bool DELTA>
 b200_status launch_scan_of(Gla& a, int n_req, cudaStream_t s) {
+  // The channels are split where that makes no more CTAs than SMs: beyond, it would make more rounds of shorter CTAs.  (Portions in chunks are
+  // longer than kGlaStepTokens; how many there are only the device knows.)
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    B200_CUDA_TRY(cudaGetDevice(&dev));
+    B200_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  }
+  const int ctas = std::min(n_req, a.total_rows / (kGlaStepTokens + 1)) * a.heads * a.n_slices;
   if (a.dkp <= 32) return launch_scan<4, DELTA>(a, n_req, s);
-  if (a.dkp <= 64) return launch_scan<8, DELTA>(a, n_req, s);
+  if (a.dkp <= 64) return 2 * ctas <= sms ? launch_scan<4, DELTA, 2>(a, n_req, s) : launch_scan<8, DELTA>(a, n_req, s);
+  if (4 * ctas <= sms && a.dkp <= 128) return launch_scan<4, DELTA, 4>(a, n_req, s);
+  if (2 * ctas <= sms) return a.dkp <= 128 ? launch_scan<8, DELTA, 2>(a, n_req, s) : launch_scan<16, DELTA, 2>(a, n_req, s);
   return a.dkp <= 128 ? launch_scan<16, DELTA>(a, n_req, s) : launch_scan<32, DELTA>(a, n_req, s);
 }
 

@@ -19,7 +19,7 @@
 //
 // Bound by the latency of its passes (loads, cluster barriers), not by bytes.  64 rows of 128256 bf16 words on one B200: greedy 20 us, top-k 50 40,
 // the whole distribution 48, a nucleus of 0.9 over all words 75, 3000 candidates 87.  One CTA per row that walked the sorted order 512
-// candidates at a time, one thread adding, took 1286 us for a mixture of these rows (800 to 1760 from call to call); this takes 104, upload of
+// candidates at a time, one thread adding, took 1286 us for a mixture of these rows (800 to 1760 from call to call); this takes 85 to 90, upload of
 // the rows' parameters included.  More than 148 rows are a CTA each; 256 rows, before and now: greedy 44 and 48 us, top-k 50
 // 149 and 59, the whole distribution 202 and 155, a nucleus of 0.9 5943 and 166, 3000 candidates 1716 and 193.
 #include <cooperative_groups.h>

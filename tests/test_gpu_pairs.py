@@ -150,3 +150,23 @@ def test_argmax_takes_the_first_maximum_wherever_the_row_is_cut(dtype, rows, voc
         x[1] = -float("inf")
     want = np.array([int(np.argmax(row)) for row in x.float().cpu().numpy()])
     assert np.array_equal(dev.argmax(x).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("rule", ["gated", "delta"])
+@pytest.mark.parametrize("dk,dv", [(33, 40), (64, 64), (96, 17), (128, 100), (160, 64), (256, 33)])
+@pytest.mark.parametrize("ctas", [24, 60, 90])
+def test_scan_of_channels_split_over_warps(ctas, dk, dv, rule):
+    """Few CTAs: four or two warps share a strip of value columns; many: one.  Portions that end inside a chunk, states handed on.
+    The factors carry 16 bits, so what is left is the rounding of the outputs: the same bound as for chunks against single tokens, three times it."""
+    from tests.test_gpu_lorulix import DeltaCase
+    from tests.test_gpu_sotavik import GlaCase, _bf16, _error
+
+    lens = (37, 5, 66)
+    heads = ctas // (3 * (-(-dv // 64)))
+    case = DeltaCase(lens, heads, heads, dk, dv, 2) if rule == "delta" else GlaCase(list(lens), heads, dk, dv)
+    first = case.step([(0, 0, 37), (1, 0, 5), (2, 0, 33)])
+    got = [first[0], first[1], np.concatenate([first[2], case.step([(2, 33, 66)])[0]])]
+    for s in range(3):
+        want, out = case.want(s), np.asarray(got[s])
+        want, out = want.reshape(len(want), -1), out.reshape(len(out), -1)
+        assert _error(out, want) <= 3 * _error(_bf16(want), want), (rule, s)
