@@ -850,7 +850,7 @@ def run_qmm(args, local):
         roof = {"bound": "tensor", "achieved": per_shape[top]["tflops"], "peak": tpeak, "unit": "TFLOP/s",
                 "frac": per_shape[top]["tflops"] / tpeak, "peak_kind": "of measured (burst cuBLAS bf16)" if peaks else "of fallback",
                 "traffic": None}
-    roof["kernel"] = f"{top}: " + ("qmm_mma_kernel" if rows <= 16 and args.path in (0, 3) else "automatic choice between qmm_tca_kernel and qmm_tc2_kernel" if args.path == 0 else f"path {args.path}")
+    roof["kernel"] = f"{top}: " + ("qmm_mma_kernel" if rows <= 16 and args.path in (0, 3) else "automatic choice among qmm_tp_kernel, qmm_tca_kernel and qmm_cp_kernel" if args.path == 0 else f"path {args.path}")
     print(json.dumps({
         "metric": "quantised matmul weight bytes per second", "value": total_w / total_us / 1e3, "unit": "GB/s", "n_gpus": 1,
         "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": total_us / 1e3, "higher_is_better": True,
