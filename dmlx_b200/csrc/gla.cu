@@ -20,6 +20,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.h"
 #include "gla_chunks.cuh"
@@ -245,8 +246,20 @@ __global__ void __launch_bounds__(1024) gla_plan_kernel(const int* __restrict__ 
 // on this route; a chunk whose decays are stronger takes the pairs one by one.
 constexpr float kMaxGrowth = 60.f;
 
+// A value of the projection, by where it is: 0 rows, 1 sums of an unsplit K, 2 of several splits.
+template <typename T, int VEC, int FROM>
+__device__ __forceinline__ Vec<VEC> value_of(const MatSrc& s, int row, int c) {
+  if constexpr (FROM == 0) return load_vec<VEC>((const T*)s.y + (size_t)row * s.y_stride + c);
+  if constexpr (FROM == 2) return mat_value<T, VEC>(s, row, c);
+  const int tt = row / s.tn;
+  return load_vec<VEC>(s.ws + ((size_t)((c >> 7) * s.tts + tt) * s.tn + (row - tt * s.tn)) * 128 + (c & 127));
+}
+
+// Bound by the latency of its phases, three or four CTAs of an SM beside one another in a single wave: loads go out kAhead at a time, a lane reads its
+// row of the decay projection in words of 16 bytes (64 chunks of 8 heads, 128 channels and 256 value columns: 43.5 -> 36.5 us).
+constexpr int kAhead = 4;
 template <typename T, int VEC>
-__global__ void __launch_bounds__(256) gla_chunk_kernel(Gla a) {
+__global__ void __launch_bounds__(256, 4) gla_chunk_kernel(Gla a) {
   after_previous();
   extern __shared__ __align__(16) float sh[];
   __shared__ int s_range;
@@ -262,18 +275,51 @@ __global__ void __launch_bounds__(256) gla_chunk_kernel(Gla a) {
     a1[i] = t < n ? mat_value<T, 1>(a.src, it.x + t, a.col_a() + r).v[0] : 0.f;
   }
   const int groups = dkp / VEC;
-  for (int i = tid; i < kC * groups; i += 256) {
-    const int t = i / groups, c = (i - t * groups) * VEC;
-    Vec<VEC> x{}, y{};
-    if (t < n && c < dk) {
-      x = mat_value<T, VEC>(a.src, it.x + t, head * dk + c);
-      y = mat_value<T, VEC>(a.src, it.x + t, a.col_k() + head * dk + c);
-    }
+  constexpr int kPer = kScanCols / VEC;
+  // FROM: what value_of reads, so that no branch or loop stands between the loads of a round
+  auto fill = [&](auto from) {
+    constexpr int FROM = decltype(from)::value;
+    for (int i0 = tid; i0 < kC * groups; i0 += 256 * kAhead) {
+      Vec<VEC> x[kAhead], y[kAhead];
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) x.v[e] *= a.q_scale;
-    store_vec<VEC>(q + t * ldr + c, x);
-    store_vec<VEC>(k + t * ldr + c, y);
-  }
+      for (int u = 0; u < kAhead; ++u) {
+        const int i = i0 + u * 256, t = i / groups, c = (i - t * groups) * VEC;
+        x[u] = y[u] = Vec<VEC>{};
+        if (t < n && c < dk) {
+          x[u] = value_of<T, VEC, FROM>(a.src, it.x + t, head * dk + c);
+          y[u] = value_of<T, VEC, FROM>(a.src, it.x + t, a.col_k() + head * dk + c);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int i = i0 + u * 256, t = i / groups, c = (i - t * groups) * VEC;
+        if (t < kC) {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) x[u].v[e] *= a.q_scale;
+          store_vec<VEC>(q + t * ldr + c, x[u]);
+          store_vec<VEC>(k + t * ldr + c, y[u]);
+        }
+      }
+    }
+    for (int i0 = tid; i0 < a.n_slices * kC * kPer; i0 += 256 * kAhead) {
+      Vec<VEC> v[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int i = i0 + u * 256, s = i / (kC * kPer), rest = i - s * kC * kPer, t = rest / kPer, col = s * kScanCols + (rest - t * kPer) * VEC;
+        v[u] = Vec<VEC>{};
+        if (t < n && col < a.dv) v[u] = value_of<T, VEC, FROM>(a.src, it.x + t, a.col_v() + head * a.dv + col);
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int i = i0 + u * 256, s = i / (kC * kPer), rest = i - s * kC * kPer, t = rest / kPer, c = (rest - t * kPer) * VEC;
+        if (s < a.n_slices)
+          store_vec<VEC>(reinterpret_cast<__nv_bfloat16*>(a.values + ((size_t)chunk * a.heads + head) * a.v_bytes + (size_t)s * kVSlice + (size_t)t * kVRow + c * 2), v[u]);
+      }
+    }
+  };
+  if (!a.src.ws) fill(std::integral_constant<int, 0>{});
+  else if (a.src.splits == 1) fill(std::integral_constant<int, 1>{});
+  else fill(std::integral_constant<int, 2>{});
   __syncthreads();
   for (int i = tid; i < 4 * dkp; i += 256) {  // eight tokens of one key channel
     const int part = i / dkp, c = i - part * dkp, t0 = part * 8;
@@ -283,10 +329,21 @@ __global__ void __launch_bounds__(256) gla_chunk_kernel(Gla a) {
     for (int t = 0; t < 8; ++t) z[t] = b;
     if (c < dk) {
       const float* w = a.a2 + (size_t)(head * dk + c) * a.rank;
-      for (int r = 0; r < a.rank; ++r) {
-        const float wr = w[r];
+      if (a.rank % 4 == 0 && reinterpret_cast<uintptr_t>(a.a2) % 16 == 0) {  // (a lane's row lies rank words from its neighbour's)
+        for (int r = 0; r < a.rank; r += 4) {
+          const float4 wr = *reinterpret_cast<const float4*>(w + r);
 #pragma unroll
-        for (int t = 0; t < 8; ++t) z[t] = fmaf(wr, a1[(t0 + t) * a.rank + r], z[t]);
+          for (int t = 0; t < 8; ++t) {
+            const float* x = a1 + (t0 + t) * a.rank + r;
+            z[t] = fmaf(wr.w, x[3], fmaf(wr.z, x[2], fmaf(wr.y, x[1], fmaf(wr.x, x[0], z[t]))));
+          }
+        }
+      } else {
+        for (int r = 0; r < a.rank; ++r) {
+          const float wr = w[r];
+#pragma unroll
+          for (int t = 0; t < 8; ++t) z[t] = fmaf(wr, a1[(t0 + t) * a.rank + r], z[t]);
+        }
       }
     }
 #pragma unroll
@@ -295,10 +352,17 @@ __global__ void __launch_bounds__(256) gla_chunk_kernel(Gla a) {
   __syncthreads();
   for (int c = tid; c < dkp; c += 256) {
     float s = 0.f, half = 0.f;
-    for (int t = 0; t < kC; ++t) {
-      if (t == 16) half = s;
-      s += L[t * ldr + c];
-      L[t * ldr + c] = s;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float l[16];
+#pragma unroll
+      for (int t = 0; t < 16; ++t) l[t] = L[(h * 16 + t) * ldr + c];
+#pragma unroll
+      for (int t = 0; t < 16; ++t) {
+        s += l[t];
+        L[(h * 16 + t) * ldr + c] = s;
+      }
+      if (h == 0) half = s;
     }
     atomicMax(&s_range, __float_as_int(fmaxf(-half, half - s)));  // (both are >= 0: their bits order like the numbers)
     reinterpret_cast<float*>(out + off_decay(dkp))[c] = expf(s);
@@ -316,14 +380,6 @@ __global__ void __launch_bounds__(256) gla_chunk_kernel(Gla a) {
     split_bf16(kt.x * expf(le.x - lt.x), kt.y * expf(le.y - lt.y), hi, lo);
     *reinterpret_cast<uint32_t*>(at + off_part(dkp, 2)) = hi;
     *reinterpret_cast<uint32_t*>(at + off_part(dkp, 3)) = lo;
-  }
-  constexpr int kPer = kScanCols / VEC;
-  for (int i = tid; i < a.n_slices * kC * kPer; i += 256) {
-    const int s = i / (kC * kPer), rest = i - s * kC * kPer, t = rest / kPer, c = (rest - t * kPer) * VEC, col = s * kScanCols + c;
-    Vec<VEC> v{};
-    if (t < n && col < a.dv) v = mat_value<T, VEC>(a.src, it.x + t, a.col_v() + head * a.dv + col);
-    unsigned char* dst = a.values + ((size_t)chunk * a.heads + head) * a.v_bytes + (size_t)s * kVSlice + (size_t)t * kVRow + c * 2;
-    store_vec<VEC>(reinterpret_cast<__nv_bfloat16*>(dst), v);
   }
   unsigned char *ahi = out + off_a(dkp, 0), *alo = out + off_a(dkp, 1);
   if (__int_as_float(s_range) >= kMaxGrowth) {
