@@ -168,6 +168,7 @@ _sig("b200_rope", i32, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp)
 _sig("b200_embed_gather", i32, vp, vp, vp, i32, i32, vp)
 _sig("b200_argmax", i32, vp, i32, i32, vp, vp)
 _sig("b200_sample_rows", i32, vp, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp)
+_sig("b200_sample_rows_host", i32, vp, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp)
 _sig("b200_prng_seed", None, u64, P(u64))
 _sig("b200_prng_next_u64", u64, P(u64))
 _sig("b200_prng_next_f32", f32, P(u64))

@@ -19,7 +19,7 @@
 //
 // Bound by the latency of its passes (loads, cluster barriers), not by bytes.  64 rows of 128256 bf16 words on one B200: greedy 20 us, top-k 50 40,
 // the whole distribution 48, a nucleus of 0.9 over all words 75, 3000 candidates 87.  One CTA per row that walked the sorted order 512
-// candidates at a time, one thread adding, took 1286 us for a mixture of these rows (800 to 1760 from call to call); this takes 85 to 90, upload of
+// candidates at a time, one thread adding, took 1286 us for a mixture of these rows (800 to 1760 from call to call); this takes 80, upload of
 // the rows' parameters included.  More than 148 rows are a CTA each; 256 rows, before and now: greedy 44 and 48 us, top-k 50
 // 149 and 59, the whole distribution 202 and 155, a nucleus of 0.9 5943 and 166, 3000 candidates 1716 and 193.
 #include <cooperative_groups.h>
@@ -703,8 +703,19 @@ struct Sampler {
   }
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(const T* __restrict__ logits, int V, const b200_sample_params* __restrict__ params,
+// The rows' parameters: in device memory, or of up to 128 rows in the arguments of the launch (4 KB at most), which spares an upload ahead of the kernel
+// (64 rows in passes behind one another: pageable upload 105 us, pinned 88, in the arguments 80; the first pass on new buffers 163, 170, 148).
+struct InMemory {
+  const b200_sample_params* p;
+  __device__ __forceinline__ const b200_sample_params& operator[](int row) const { return p[row]; }
+};
+struct InArguments {
+  b200_sample_params p[B200_SAMPLE_HOST_ROWS];
+  __device__ __forceinline__ const b200_sample_params& operator[](int row) const { return p[row]; }
+};
+
+template <typename T, typename Params>
+__global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(const T* __restrict__ logits, int V, const __grid_constant__ Params params,
                                                                   const uint32_t* __restrict__ ctx, const int* __restrict__ ctx_off,
                                                                   float* __restrict__ scratch, uint32_t* __restrict__ tokens,
                                                                   float* __restrict__ logprobs) {
@@ -744,11 +755,11 @@ __global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(const T* __res
   }
 }
 
-template <typename T>
-b200_status launch(const T* logits, int rows, int vocab, const b200_sample_params* params, const uint32_t* ctx, const int* ctx_off, float* scratch,
+template <typename T, typename Params>
+b200_status launch(const T* logits, int rows, int vocab, const Params& params, const uint32_t* ctx, const int* ctx_off, float* scratch,
                    uint32_t* tokens, float* logprobs, cudaStream_t s) {
   // (asked for at every launch: the attribute belongs to the device that the calling thread uses)
-  B200_CUDA_TRY(cudaFuncSetAttribute(sample_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared)));
+  B200_CUDA_TRY(cudaFuncSetAttribute(sample_rows_kernel<T, Params>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared)));
   // CTAs per row: 8192 words each at least (16 a thread), and no more altogether than run at the same time: two per SM, and a cluster's within one
   // GPC, which leaves room for 32 clusters of eight (37 rows, a nucleus of 0.9: 111 us in eight CTAs a row, 88 in four).
   int ranks = 1;
@@ -766,9 +777,25 @@ b200_status launch(const T* logits, int rows, int vocab, const b200_sample_param
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, sample_rows_kernel<T>, logits, vocab, params, ctx, ctx_off, scratch, tokens, logprobs));
+  B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, sample_rows_kernel<T, Params>, logits, vocab, params, ctx, ctx_off, scratch, tokens, logprobs));
   B200_LAUNCH_CHECK();
   return B200_OK;
+}
+
+template <typename Params>
+b200_status sample(const void* d_logits, int32_t logits_f32, int32_t rows, int32_t vocab, const Params& params, bool no_params, const uint32_t* d_ctx_tokens,
+                   const int32_t* d_ctx_offsets, float* d_scratch, uint32_t* d_tokens, float* d_logprobs, void* stream) {
+  if (vocab < 1 || vocab > (1 << 24) || d_logits == nullptr || no_params || d_tokens == nullptr) {
+    b200_set_error("sample_rows: vocab %d outside 1..2^24 or a null argument", vocab);
+    return B200_ERR_INVALID_ARGUMENT;
+  }
+  if ((d_ctx_offsets != nullptr) != (d_ctx_tokens != nullptr) || (d_ctx_offsets != nullptr && d_scratch == nullptr)) {
+    b200_set_error("sample_rows: context tokens, their offsets and the f32 scratch go together");
+    return B200_ERR_INVALID_ARGUMENT;
+  }
+  cudaStream_t cs = (cudaStream_t)stream;
+  return logits_f32 ? launch((const float*)d_logits, rows, vocab, params, d_ctx_tokens, d_ctx_offsets, d_scratch, d_tokens, d_logprobs, cs)
+                    : launch((const __nv_bfloat16*)d_logits, rows, vocab, params, d_ctx_tokens, d_ctx_offsets, d_scratch, d_tokens, d_logprobs, cs);
 }
 
 }  // namespace
@@ -781,17 +808,22 @@ b200_status b200_sample_rows(const void* d_logits, int32_t logits_f32, int32_t r
   b200_status st = b200_require_device();
   if (st != B200_OK) return st;
   if (rows <= 0) return B200_OK;
-  if (vocab < 1 || vocab > (1 << 24) || d_logits == nullptr || d_params == nullptr || d_tokens == nullptr) {
-    b200_set_error("sample_rows: vocab %d outside 1..2^24 or a null argument", vocab);
+  return sample(d_logits, logits_f32, rows, vocab, InMemory{d_params}, d_params == nullptr, d_ctx_tokens, d_ctx_offsets, d_scratch, d_tokens, d_logprobs, stream);
+}
+
+b200_status b200_sample_rows_host(const void* d_logits, int32_t logits_f32, int32_t rows, int32_t vocab,
+                                  const b200_sample_params* h_params, const uint32_t* d_ctx_tokens, const int32_t* d_ctx_offsets,
+                                  float* d_scratch, uint32_t* d_tokens, float* d_logprobs, void* stream) {
+  b200_status st = b200_require_device();
+  if (st != B200_OK) return st;
+  if (rows <= 0) return B200_OK;
+  if (rows > B200_SAMPLE_HOST_ROWS) {
+    b200_set_error("sample_rows_host: %d rows, %d at most", rows, B200_SAMPLE_HOST_ROWS);
     return B200_ERR_INVALID_ARGUMENT;
   }
-  if ((d_ctx_offsets != nullptr) != (d_ctx_tokens != nullptr) || (d_ctx_offsets != nullptr && d_scratch == nullptr)) {
-    b200_set_error("sample_rows: context tokens, their offsets and the f32 scratch go together");
-    return B200_ERR_INVALID_ARGUMENT;
-  }
-  cudaStream_t cs = (cudaStream_t)stream;
-  return logits_f32 ? launch((const float*)d_logits, rows, vocab, d_params, d_ctx_tokens, d_ctx_offsets, d_scratch, d_tokens, d_logprobs, cs)
-                    : launch((const __nv_bfloat16*)d_logits, rows, vocab, d_params, d_ctx_tokens, d_ctx_offsets, d_scratch, d_tokens, d_logprobs, cs);
+  InArguments params{};
+  if (h_params) std::copy_n(h_params, rows, params.p);
+  return sample(d_logits, logits_f32, rows, vocab, params, h_params == nullptr, d_ctx_tokens, d_ctx_offsets, d_scratch, d_tokens, d_logprobs, stream);
 }
 
 }  // extern "C"

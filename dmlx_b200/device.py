@@ -404,8 +404,12 @@ def sample_rows(logits: torch.Tensor, rows, context: Optional[Sequence[Sequence[
     Returns (tokens int32 [R], logprobs float32 [R] or None)."""
     assert logits.dtype in (torch.bfloat16, torch.float32) and logits.is_contiguous()
     n, v = logits.shape
-    # (from pinned memory: a pageable upload waits for the kernels ahead of it in the stream)
-    d_params = torch.from_numpy(sample_params_array(rows)).pin_memory().to(logits.device, non_blocking=True)
+    params = sample_params_array(rows)
+    if n <= 128 and len(params) >= n:  # in the arguments of the launch
+        sample, p_params = lib.b200_sample_rows_host, params.ctypes.data
+    else:  # (from pinned memory: a pageable upload waits for the kernels ahead of it in the stream)
+        d_params = torch.from_numpy(params).pin_memory().to(logits.device, non_blocking=True)
+        sample, p_params = lib.b200_sample_rows, _ptr(d_params)
     tokens = torch.empty(n, dtype=torch.int32, device=logits.device)
     lp = torch.empty(n, dtype=torch.float32, device=logits.device) if logprobs else None
     d_ctx = d_off = scratch = None
@@ -415,8 +419,8 @@ def sample_rows(logits: torch.Tensor, rows, context: Optional[Sequence[Sequence[
         d_ctx = torch.tensor(flat + [0], dtype=torch.int64).to(torch.int32).to(logits.device)
         d_off = torch.from_numpy(offs).to(logits.device)
         scratch = torch.empty((n, v), dtype=torch.float32, device=logits.device)
-    _lib.check(lib.b200_sample_rows(_ptr(logits), int(logits.dtype == torch.float32), n, v, _ptr(d_params), _ptr(d_ctx),
-                                    _ptr(d_off), _ptr(scratch), _ptr(tokens), _ptr(lp), _stream()))
+    _lib.check(sample(_ptr(logits), int(logits.dtype == torch.float32), n, v, p_params, _ptr(d_ctx), _ptr(d_off), _ptr(scratch),
+                      _ptr(tokens), _ptr(lp), _stream()))
     return tokens, lp
 
 

@@ -170,3 +170,22 @@ def test_scan_of_channels_split_over_warps(ctas, dk, dv, rule):
         want, out = case.want(s), np.asarray(got[s])
         want, out = want.reshape(len(want), -1), out.reshape(len(out), -1)
         assert _error(out, want) <= 3 * _error(_bf16(want), want), (rule, s)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("rows", [1, 64, 127, 128, 129])
+def test_sampler_parameters_in_the_launch_and_in_memory_draw_alike(rows, dtype):
+    """The same kernel reads them from either place: tokens and log probabilities are the same bits."""
+    from dmlx_b200 import device as dev
+    from dmlx_b200._lib import check, lib
+
+    rng = np.random.default_rng(rows)
+    logits = torch.tensor(rng.normal(size=(rows, 4099)) * 3, dtype=getattr(torch, dtype), device="cuda")
+    params = [(0.0 if i % 5 == 0 else 0.5 + 0.1 * (i % 7), int(rng.integers(0, 60)), float(rng.uniform(0.3, 1.0)), float(rng.uniform())) for i in range(rows)]
+    got, got_lp = dev.sample_rows(logits, params)
+    d = torch.from_numpy(dev.sample_params_array(params)).cuda()
+    want, want_lp = torch.empty(rows, dtype=torch.int32, device="cuda"), torch.empty(rows, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    check(lib.b200_sample_rows(logits.data_ptr(), int(dtype == "float32"), rows, 4099, d.data_ptr(), None, None, None, want.data_ptr(), want_lp.data_ptr(), None))
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and torch.equal(got_lp, want_lp)
