@@ -25,7 +25,7 @@
 namespace {
 
 // Angles in f64, brought into one turn before they become f32: positions far out keep their accuracy.
-__global__ void __launch_bounds__(256) rotation_table_kernel(const double* __restrict__ freq, int half, float size, const int* __restrict__ pos, int rows,
+__global__ void __launch_bounds__(256) rotation_table_kernel(const double* freq, int half, float size, const int* pos, int rows,
                                                              float2* __restrict__ out) {
   after_previous();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;

@@ -150,7 +150,7 @@ __device__ __forceinline__ int chunk_blocks(int k) { return k == 0 ? 1 << 24 : 1
 // key ranges may be cut into chunks; the length is the one with the smallest estimated time among those whose partial sums fit.
 // old_limit > 0: batches of this kind are refused (CAPACITY) where groups of old_tokens rows in chunks of 8 pages would need more partial
 // slots than that, the documented limit of the pool's scratch.
-__global__ void __launch_bounds__(1024) prompt_plan_kernel(const int* __restrict__ row_seq, const int* __restrict__ row_ctx, int total_rows, int page_size,
+__global__ void __launch_bounds__(1024) prompt_plan_kernel(const int* row_seq, const int* row_ctx, int total_rows, int page_size,
                                                            int q_tokens, int tile_tokens, int heads, int workers, int may_split, int max_slots,
                                                            int old_tokens, int* __restrict__ chunk_start, int* __restrict__ group_first,
                                                            int* __restrict__ part_base, int* __restrict__ row_group, int2* __restrict__ items,
@@ -830,7 +830,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // A warp per (row, query head): merges the chunks of rows whose key range was split.
 template <int D>
-__global__ void __launch_bounds__(256) prompt_combine_kernel(Args a, const int* __restrict__ row_group) {
+__global__ void __launch_bounds__(256) prompt_combine_kernel(Args a, const int* row_group) {
   after_previous();
   const int u = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (u >= a.total_rows * a.n_q_heads || a.hdr[4] == 0 || a.d.state[ST_ATTN_ERR] != 0) return;

@@ -81,7 +81,7 @@ struct FineLengths {
 // the uneven end of the walk, a page and a bit per item for its start and end, and, where groups are cut, the partial sums
 // and the combine pass.  It doubles until the partial slots fit the scratch (uncut groups need none), so a step always fits.
 template <typename Lengths>
-__global__ void __launch_bounds__(1024) window_plan_kernel(const int* __restrict__ row_seq, const int* __restrict__ row_ctx, int total_rows,
+__global__ void __launch_bounds__(1024) window_plan_kernel(const int* row_seq, const int* row_ctx, int total_rows,
                                                            int page_size, int window, int q_tokens, int items_per_chunk,
                                                            int n_workers, int forced_ppc, int max_slots, float item_cost, float slot_cost, int* __restrict__ group_first,
                                                            int* __restrict__ chunk_start, int* __restrict__ part_base,

@@ -397,7 +397,7 @@ b200_status launch_input_conv(const InputConvArgs& a, int rows, bool f32, cudaSt
 
 // Rows idx[r] of x, normalised, as the head's operand.
 template <typename T>
-__global__ void __launch_bounds__(256) decoder_final_kernel(const float* __restrict__ x, const int* __restrict__ idx, const float* __restrict__ w,
+__global__ void __launch_bounds__(256) decoder_final_kernel(const float* x, const int* idx, const float* w,
                                                             T* __restrict__ out, int hidden, int out_stride, float eps) {
   after_previous();
   __shared__ float part[32];

@@ -6,27 +6,15 @@
 #include "common.h"
 #include "launch.cuh"
 #include "qmm.cuh"
+#include "rows.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace {
 
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// One CTA per row; hidden % 8 == 0.
-__global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                               __nv_bfloat16* __restrict__ out, int hidden, float eps) {
-  after_previous();
+// A row by a block; nvec vectors of eight.
+__device__ __forceinline__ void rmsnorm_row(const uint4* __restrict__ xr, const uint4* __restrict__ wr, uint4* __restrict__ orow, int nvec, float eps) {
   __shared__ float s_part[32];
-  const int row = blockIdx.x;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * hidden);
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
-  uint4* orow = reinterpret_cast<uint4*>(out + (size_t)row * hidden);
-  const int nvec = hidden / 8;
   float ss = 0.f;
   for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
     uint4 v = xr[i];
@@ -43,7 +31,7 @@ __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
   if (threadIdx.x < 32) {
     float t = threadIdx.x < (blockDim.x >> 5) ? s_part[threadIdx.x] : 0.f;
     t = warp_sum(t);
-    if (threadIdx.x == 0) s_part[0] = rsqrtf(t / (float)hidden + eps);
+    if (threadIdx.x == 0) s_part[0] = rsqrtf(t / (float)(8 * nvec) + eps);
   }
   __syncthreads();
   const float r = s_part[0];
@@ -61,10 +49,17 @@ __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
   }
 }
 
+// One CTA per row; hidden % 8 == 0.
+__global__ void rmsnorm_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* out, int hidden, float eps) {
+  after_previous();
+  const size_t at = (size_t)blockIdx.x * hidden;
+  rmsnorm_row(reinterpret_cast<const uint4*>(x + at), reinterpret_cast<const uint4*>(w), reinterpret_cast<uint4*>(out + at), hidden / 8, eps);
+}
+
 // Non-traditional RoPE: pair (i, i + D/2) of every head rotates by pos * theta^(-2i/D).
 // One thread per (row, head, i); q heads first, then k heads.
-__global__ void rope_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ k,
-                            const int* __restrict__ positions, int rows, int hq, int hkv, int D, int q_stride,
+__global__ void rope_kernel(__nv_bfloat16* q, __nv_bfloat16* k,
+                            const int* positions, int rows, int hq, int hkv, int D, int q_stride,
                             int k_stride, float log2_theta) {
   after_previous();
   const int half = D / 2;
@@ -84,19 +79,19 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __rest
   base[i + half] = __float2bfloat16(x1 * s + x2 * c);
 }
 
-__global__ void embed_kernel(const __nv_bfloat16* __restrict__ table, const uint32_t* __restrict__ ids,
+__global__ void embed_kernel(const __nv_bfloat16* table, const uint32_t* ids,
                              __nv_bfloat16* __restrict__ out, int hidden) {
   after_previous();
   const int row = blockIdx.x;
   const uint4* src = reinterpret_cast<const uint4*>(table + (size_t)ids[row] * hidden);
   uint4* dst = reinterpret_cast<uint4*>(out + (size_t)row * hidden);
-  for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) dst[i] = src[i];
+  copy_vectors(dst, src, hidden / 8);
 }
 
 // First strict maximum of each row (ties keep the smaller index).
 // A row belongs to a cluster of CTAs, a contiguous part each (16 rows of 32000 f32 values: 9.9 us by a block each, 6.8 this way).
 template <typename T>
-__global__ void argmax_kernel(const T* __restrict__ logits, int vocab, uint32_t* __restrict__ out) {
+__global__ void argmax_kernel(const T* logits, int vocab, uint32_t* __restrict__ out) {
   after_previous();
   __shared__ float s_val[32];
   __shared__ int s_idx[32];
@@ -182,22 +177,22 @@ b200_status launch_argmax(const T* logits, int rows, int vocab, uint32_t* out, c
   return B200_OK;
 }
 
-__global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ idx,
+__global__ void gather_rows_kernel(const __nv_bfloat16* src, const int* idx,
                                    __nv_bfloat16* __restrict__ dst, int hidden) {
   after_previous();
   const int row = blockIdx.x;
   const int s = max(idx[row], 0);
   const uint4* sp = reinterpret_cast<const uint4*>(src + (size_t)s * hidden);
   uint4* dp = reinterpret_cast<uint4*>(dst + (size_t)row * hidden);
-  for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) dp[i] = sp[i];
+  copy_vectors(dp, sp, hidden / 8);
 }
 
 // `flags` points at the pool's eight state words: a step whose page reservation or attention was
 // flagged has computed its tokens from stale pages, so the sequences keep the input token they had
 // and the step can be run again once the cause (an exhausted pool) is gone.
-__global__ void scatter_tokens_kernel(const uint32_t* __restrict__ next, const b200_pack_desc* __restrict__ desc,
-                                      uint32_t* __restrict__ last_token, int n_req, const int* __restrict__ flags,
-                                      int flag_a, int flag_b, const int* __restrict__ qmm_err, uint32_t* __restrict__ h_next,
+__global__ void scatter_tokens_kernel(const uint32_t* next, const b200_pack_desc* desc,
+                                      uint32_t* __restrict__ last_token, int n_req, const int* flags,
+                                      int flag_a, int flag_b, const int* qmm_err, uint32_t* __restrict__ h_next,
                                       int* __restrict__ h_state) {
   after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

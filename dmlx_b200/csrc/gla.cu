@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(1024) memory_gates_kernel(GateArgs a) {
 
 // ---- chunks: plan ------------------------------------------------------------------------------------------------
 // One CTA: the chunks of every portion that goes chunk by chunk, and where each request's start.
-__global__ void __launch_bounds__(1024) gla_plan_kernel(const int* __restrict__ cu, int n_req, int max_chunks, int4* __restrict__ plan,
+__global__ void __launch_bounds__(1024) gla_plan_kernel(const int* cu, int n_req, int max_chunks, int4* __restrict__ plan,
                                                         int* __restrict__ first_chunk) {
   after_previous();
   __shared__ int sums[32];

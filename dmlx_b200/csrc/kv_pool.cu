@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(THREADS) reserve_kernel(KvDev d, const b200_pa
 // Small steps: one block packs the batch, another one reserves its pages (a launch each for the scan, the rows and the pages were 5 us more of an
 // 8-request step's chain).
 constexpr int kSmallStep = 256;
-__global__ void __launch_bounds__(kSmallStep) pack_reserve_kernel(KvDev d, const b200_pack_desc* __restrict__ desc, int n_req,
-                                                                  const uint32_t* __restrict__ prefill_tokens, const uint32_t* __restrict__ last_token,
+__global__ void __launch_bounds__(kSmallStep) pack_reserve_kernel(KvDev d, const b200_pack_desc* desc, int n_req,
+                                                                  const uint32_t* prefill_tokens, const uint32_t* last_token,
                                                                   int total_rows, PackOut out) {
   after_previous();
   if (blockIdx.x == 0) reserve<kSmallStep, 1>(d, desc, n_req);
@@ -291,8 +291,8 @@ __global__ void cow_copy_kernel(KvDev d) {
 }
 
 // bf16 append: one CTA per (page touch, kv head) copies rows into the page tile.
-__global__ void append_bf16_kernel(KvDev d, int layer, const __nv_bfloat16* __restrict__ k_rows,
-                                   const __nv_bfloat16* __restrict__ v_rows, int k_stride, int v_stride) {
+__global__ void append_bf16_kernel(KvDev d, int layer, const __nv_bfloat16* k_rows,
+                                   const __nv_bfloat16* v_rows, int k_stride, int v_stride) {
   after_previous();
   const int n_touch = d.state[ST_N_TOUCH];
   const int head = blockIdx.y, D = d.head_dim, H = d.n_kv_heads;
@@ -304,8 +304,10 @@ __global__ void append_bf16_kernel(KvDev d, int layer, const __nv_bfloat16* __re
     uint4* vd = (uint4*)((__nv_bfloat16*)d.v_pool + tile + (size_t)tc.w * D);
     for (int i = threadIdx.x; i < tc.z * vec_per_row; i += blockDim.x) {
       int r = i / vec_per_row, c = i % vec_per_row;
-      kd[r * vec_per_row + c] = ((const uint4*)(k_rows + (size_t)(tc.y + r) * k_stride + head * D))[c];
-      vd[r * vec_per_row + c] = ((const uint4*)(v_rows + (size_t)(tc.y + r) * v_stride + head * D))[c];
+      const uint4 k = ((const uint4*)(k_rows + (size_t)(tc.y + r) * k_stride + head * D))[c];
+      const uint4 v = ((const uint4*)(v_rows + (size_t)(tc.y + r) * v_stride + head * D))[c];
+      kd[r * vec_per_row + c] = k;
+      vd[r * vec_per_row + c] = v;
     }
   }
 }
@@ -315,10 +317,10 @@ __global__ void append_bf16_kernel(KvDev d, int layer, const __nv_bfloat16* __re
 // 8y..8y+7 of a packed row, one per warp; lane l the rotation pairs (2l, 2l+1) of a head (non-traditional RoPE:
 // pair (i, i + D/2) rotates by pos * theta^(-2i/D)), so sin/cos are computed once per thread.
 // The page comes from the block table that b200_kv_reserve has just grown.
-__global__ void __launch_bounds__(256) rope_append_bf16_kernel(KvDev d, int layer, __nv_bfloat16* __restrict__ q,
-                                                               const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
+__global__ void __launch_bounds__(256) rope_append_bf16_kernel(KvDev d, int layer, __nv_bfloat16* q,
+                                                               const __nv_bfloat16* k, const __nv_bfloat16* v,
                                                                int q_stride, int k_stride, int v_stride,
-                                                               const int* __restrict__ positions, const int* __restrict__ row_seq, int hq,
+                                                               const int* positions, const int* row_seq, int hq,
                                                                float log2_theta) {
   after_previous();
   const int row = blockIdx.x, D = d.head_dim, H = d.n_kv_heads, half = D / 2;
@@ -376,8 +378,8 @@ __device__ __forceinline__ float from_e4m3(unsigned char b) {
 
 // FP8 append: per (touch, head, K|V): new scale = max(old, amax(new rows)/448); when it grows the
 // rows already in the tile are re-encoded at the new scale; then the new rows are encoded.
-__global__ void append_fp8_kernel(KvDev d, int layer, const __nv_bfloat16* __restrict__ k_rows,
-                                  const __nv_bfloat16* __restrict__ v_rows, int k_stride, int v_stride) {
+__global__ void append_fp8_kernel(KvDev d, int layer, const __nv_bfloat16* k_rows,
+                                  const __nv_bfloat16* v_rows, int k_stride, int v_stride) {
   after_previous();
   __shared__ float s_red[32];
   __shared__ float s_scale[2];
@@ -906,8 +908,8 @@ static int rope_blocks(int rows, int most) { return std::min(most, std::max(1, (
 // in split order and rounded to bf16 as the matmul's finish pass would have done, then rotated and stored: q into the
 // activation buffer, k and v into the row's page.
 __global__ void __launch_bounds__(256) rope_append_partials_bf16_kernel(KvDev d, int layer, b200_qmm_partials p, __nv_bfloat16* __restrict__ q,
-                                                                        int q_stride, const int* __restrict__ positions,
-                                                                        const int* __restrict__ row_seq, int hq, float log2_theta) {
+                                                                        int q_stride, const int* positions,
+                                                                        const int* row_seq, int hq, float log2_theta) {
   after_previous();
   constexpr int D = 128, half = 64;
   const int row = blockIdx.x, H = d.n_kv_heads;
@@ -1080,8 +1082,8 @@ b200_status b200_kv_page_load(b200_kv* kv, int32_t layer, int32_t page, const vo
 // extend (src/kvcache/paged.zig:947-1109): a sequence of another pool of the same shape becomes a new
 // sequence of this one, with its own copies of the pages.  One launch copies every layer's K and V
 // page (and, for FP8 pools, the per-head scales); grid = (pages of the sequence, layers).
-__global__ void __launch_bounds__(256) copy_pages_kernel(KvDev src, KvDev dst, const int* __restrict__ src_table,
-                                                         const int* __restrict__ dst_table) {
+__global__ void __launch_bounds__(256) copy_pages_kernel(KvDev src, KvDev dst, const int* src_table,
+                                                         const int* dst_table) {
   after_previous();
   const int layer = blockIdx.y, sp = src_table[blockIdx.x], dp = dst_table[blockIdx.x];
   if (sp < 0 || sp >= src.n_pages || dp < 0 || dp >= dst.n_pages) return;

@@ -5,8 +5,14 @@
 // the kernel before has passed `let_next_start` and there is room; they set up what needs no memory and wait.
 //
 // In every kernel that is launched through `launch_after`, each thread that reads or writes global memory (weights apart, which nothing writes
-// after their creation) or allocates tensor memory runs `wait_previous` before it does, and so does some thread of every block before it ends.  So the bodies of two kernels of a stream never overlap, and as a kernel ends only after its
-// own wait did, the wait of the next one covers all that came before.
+// after their creation) or allocates tensor memory runs `wait_previous` before it does, and so does some thread of every block before it ends.
+// So the bodies of two kernels of a stream never overlap, and as a kernel ends only after its own wait did, the wait of the next one covers all
+// that came before.
+//
+// No kernel's input is `const T* __restrict__`: a kernel runs from its early start on, so what the one ahead writes changes within its lifetime, and
+// the qualifier would let the compiler load it ahead of the wait (no other pointer reaches the object, so the wait's "memory" clobber would not
+// stand in the way) or through the read-only path.  Memory that is only written may be `__restrict__`, so that loads are not held back by stores,
+// and so may the parameters of a function that is called after the wait.
 #pragma once
 #include <cuda_runtime.h>
 

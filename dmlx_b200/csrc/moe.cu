@@ -111,9 +111,9 @@ __device__ __forceinline__ void route_token(const LogitT* __restrict__ logits, c
 
 // One warp per token.  E <= 1024 (32 experts per lane).
 template <typename LogitT, int PER>
-__global__ void __launch_bounds__(256) route_kernel(const LogitT* __restrict__ logits, const float* __restrict__ bias, int n_tokens, int n_experts,
+__global__ void __launch_bounds__(256) route_kernel(const LogitT* logits, const float* bias, int n_tokens, int n_experts,
                                                     int k, int scoring, float route_scale, uint32_t* __restrict__ out_idx,
-                                                    float* __restrict__ out_w, int* __restrict__ counts) {
+                                                    float* __restrict__ out_w, int* counts) {
   after_previous();
   const int token = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (token >= n_tokens) return;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(256) route_kernel(const LogitT* __restrict__ l
 // their own, with the counters cleared ahead of them, they were five links of the chain (24 tokens: 17 us, 6.3 this way).
 constexpr int kSmallAssign = 512;  // assignments: their ranks are counted one by one
 template <int PER>
-__global__ void __launch_bounds__(1024) route_small_kernel(const __nv_bfloat16* __restrict__ logits, const float* __restrict__ bias, int n_tokens, int n_experts,
+__global__ void __launch_bounds__(1024) route_small_kernel(const __nv_bfloat16* logits, const float* bias, int n_tokens, int n_experts,
                                                            int k, int scoring, float route_scale, int tile_rows, uint32_t* __restrict__ out_idx,
                                                            float* __restrict__ out_w, int* __restrict__ counts, int* __restrict__ offsets,
                                                            int4* __restrict__ items, int* __restrict__ n_items, int* __restrict__ order,
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(1024) route_small_kernel(const __nv_bfloat16* 
 }
 
 // offsets = exclusive scan of counts; work items {expert, first row, rows} for tiles of `tile_rows`.
-__global__ void offsets_items_kernel(const int* __restrict__ counts, int n_experts, int tile_rows, int* __restrict__ offsets,
+__global__ void offsets_items_kernel(const int* counts, int n_experts, int tile_rows, int* __restrict__ offsets,
                                      int4* __restrict__ items, int* __restrict__ n_items) {
   after_previous();
   __shared__ int s_off[kMaxExperts + 1], s_item[kMaxExperts + 1];
@@ -271,8 +271,8 @@ __device__ __forceinline__ void place_assignments(const uint32_t* __restrict__ i
   }
 }
 
-__global__ void __launch_bounds__(1024) place_kernel(const uint32_t* __restrict__ indices, int n_assign,
-                                                     const int* __restrict__ offsets, int* __restrict__ order,
+__global__ void __launch_bounds__(1024) place_kernel(const uint32_t* indices, int n_assign,
+                                                     const int* offsets, int* __restrict__ order,
                                                      int* __restrict__ inv_order) {
   after_previous();
   place_assignments(indices, n_assign, offsets, order, inv_order);
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(1024) place_kernel(const uint32_t* __restrict_
 // ---- experts by token id ----------------------------------------------------------------------------------------------
 // Without a router the experts of a step's tokens are known before the first layer runs: one CTA per layer looks them up, counts
 // them and lays out the work items; one CTA per (expert, layer) then places the assignments.
-__global__ void __launch_bounds__(1024) table_route_kernel(const MoeTableLayer* __restrict__ layers, const uint32_t* __restrict__ tokens, int n_tokens,
+__global__ void __launch_bounds__(1024) table_route_kernel(const MoeTableLayer* layers, const uint32_t* tokens, int n_tokens,
                                                            int vocab, int tile_rows) {
   after_previous();
   __shared__ int s_count[kMaxExperts], s_off[kMaxExperts + 1], s_item[kMaxExperts + 1];
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(1024) table_route_kernel(const MoeTableLayer* 
   }
 }
 
-__global__ void __launch_bounds__(1024) table_place_kernel(const MoeTableLayer* __restrict__ layers, int n_tokens) {
+__global__ void __launch_bounds__(1024) table_place_kernel(const MoeTableLayer* layers, int n_tokens) {
   after_previous();
   const MoeTableLayer L = layers[blockIdx.y];
   if ((int)blockIdx.x >= L.n_experts) return;
@@ -449,18 +449,18 @@ __global__ void __launch_bounds__(1024) plan_kernel(MoeTableLayer L, int n_token
 }
 
 // Rows of x in the experts' order, 16 bytes at a time.
-__global__ void __launch_bounds__(128) gather_rows_by_order_kernel(const uint4* __restrict__ x, const int* __restrict__ order, int top, int vecs,
+__global__ void __launch_bounds__(128) gather_rows_by_order_kernel(const uint4* x, const int* order, int top, int vecs,
                                                                    uint4* __restrict__ out) {
   after_previous();
   const uint4* src = x + (size_t)(order[blockIdx.x] / top) * vecs;
   uint4* dst = out + (size_t)blockIdx.x * vecs;
-  for (int i = threadIdx.x; i < vecs; i += blockDim.x) dst[i] = src[i];
+  copy_vectors(dst, src, vecs);
 }
 
 // row_scales[p] = weights[order[p]] alone (the rows themselves are read in place by the matmul).
 // n_valid (optional, device): rows that exist when n is only the capacity.
-__global__ void row_scales_kernel(const int* __restrict__ order, const float* __restrict__ weights, int n, float* __restrict__ out,
-                                  const int* __restrict__ n_valid) {
+__global__ void row_scales_kernel(const int* order, const float* weights, int n, float* __restrict__ out,
+                                  const int* n_valid) {
   after_previous();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p < n && (!n_valid || p < *n_valid)) out[p] = weights[order[p]];
@@ -468,7 +468,7 @@ __global__ void row_scales_kernel(const int* __restrict__ order, const float* __
 
 // Expert parallelism: global expert ids -> ids among this rank's experts, everything else marked as
 // "not mine" (a value no expert matches, so the counting sort leaves those assignments out).
-__global__ void localize_kernel(const uint32_t* __restrict__ idx, int n_assign, int first_expert, int n_local,
+__global__ void localize_kernel(const uint32_t* idx, int n_assign, int first_expert, int n_local,
                                 uint32_t* __restrict__ local_idx) {
   after_previous();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -479,7 +479,7 @@ __global__ void localize_kernel(const uint32_t* __restrict__ idx, int n_assign, 
 
 // Expert parallelism: this rank's share of every token's sum over k (f32; zero where none of the
 // token's experts lives here).  inv_order[a] < 0 marks an assignment served by another rank.
-__global__ void combine_partial_kernel(const __nv_bfloat16* __restrict__ y_sorted, const int* __restrict__ inv_order, int k,
+__global__ void combine_partial_kernel(const __nv_bfloat16* y_sorted, const int* inv_order, int k,
                                        int hidden, float* __restrict__ out) {
   after_previous();
   const int t = blockIdx.x;
@@ -504,7 +504,7 @@ __global__ void combine_partial_kernel(const __nv_bfloat16* __restrict__ y_sorte
 }
 
 // Expert parallelism: out = bf16(routed sum (f32, reduced over the ranks) + shared expert).
-__global__ void add_shared_kernel(const float* __restrict__ routed, const __nv_bfloat16* __restrict__ shared_out, size_t n8,
+__global__ void add_shared_kernel(const float* routed, const __nv_bfloat16* shared_out, size_t n8,
                                   __nv_bfloat16* __restrict__ out) {
   after_previous();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -525,22 +525,22 @@ __global__ void add_shared_kernel(const float* __restrict__ routed, const __nv_b
   reinterpret_cast<uint4*>(out)[i] = o;
 }
 
-__global__ void gather_sorted_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ order,
-                                     const float* __restrict__ weights, int k, int hidden,
+__global__ void gather_sorted_kernel(const __nv_bfloat16* x, const int* order,
+                                     const float* weights, int k, int hidden,
                                      __nv_bfloat16* __restrict__ x_sorted, float* __restrict__ row_scales,
-                                     const int* __restrict__ n_valid) {
+                                     const int* n_valid) {
   after_previous();
   const int p = blockIdx.x;
   if (n_valid && p >= *n_valid) return;
   const int a = order[p];
   const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(a / k) * hidden);
   uint4* dst = reinterpret_cast<uint4*>(x_sorted + (size_t)p * hidden);
-  for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) dst[i] = src[i];
+  copy_vectors(dst, src, hidden / 8);
   if (threadIdx.x == 0 && row_scales) row_scales[p] = weights[a];
 }
 
-__global__ void combine_kernel(const __nv_bfloat16* __restrict__ y_sorted, const int* __restrict__ inv_order, int k, int hidden,
-                               const __nv_bfloat16* __restrict__ shared_out, __nv_bfloat16* __restrict__ out) {
+__global__ void combine_kernel(const __nv_bfloat16* y_sorted, const int* inv_order, int k, int hidden,
+                               const __nv_bfloat16* shared_out, __nv_bfloat16* __restrict__ out) {
   after_previous();
   const int t = blockIdx.x;
   if (hidden % 8 == 0 && k <= 16) {

@@ -10,7 +10,7 @@ namespace {
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 
-__global__ void __launch_bounds__(kScanThreads) pack_scan_kernel(const b200_pack_desc* __restrict__ desc, int n_req,
+__global__ void __launch_bounds__(kScanThreads) pack_scan_kernel(const b200_pack_desc* desc, int n_req,
                                                                  int* __restrict__ cu_seqlens, int* __restrict__ last_row) {
   after_previous();
   __shared__ int warp_sums[32];
@@ -53,8 +53,8 @@ __global__ void __launch_bounds__(kScanThreads) pack_scan_kernel(const b200_pack
   }
 }
 
-__global__ void pack_fill_kernel(const b200_pack_desc* __restrict__ desc, int n_req, const int* __restrict__ cu_seqlens,
-                                 const uint32_t* __restrict__ prefill_tokens, const uint32_t* __restrict__ last_token,
+__global__ void pack_fill_kernel(const b200_pack_desc* desc, int n_req, const int* cu_seqlens,
+                                 const uint32_t* prefill_tokens, const uint32_t* last_token,
                                  uint32_t* __restrict__ token_ids, int* __restrict__ position_ids,
                                  int* __restrict__ row_to_req, int* __restrict__ row_seq, int* __restrict__ row_ctx,
                                  int total_rows) {

@@ -67,7 +67,7 @@ __device__ __forceinline__ int attn_pages_per_chunk(const AttnArgs& a) { return 
 // partial sums and the combine pass's walk over a row's chunks cost more than the balance gains (256 requests of
 // ~47 pages: 12.8 ms per step at 8 pages per chunk against 13.1 at 16; 64 requests of ~250 pages: 0.338 ms per
 // launch at 32 against 0.377 at 8).  The choice is written to *ppc_out for the kernels that follow.
-__global__ void attn_plan_kernel(const int* __restrict__ row_ctx, int total_rows, int page_size, int pages_per_chunk,
+__global__ void attn_plan_kernel(const int* row_ctx, int total_rows, int page_size, int pages_per_chunk,
                                  int* __restrict__ chunk_start, int max_chunks, int* __restrict__ err, int* __restrict__ ppc_out) {
   after_previous();
   __shared__ int warp_sums[32];
@@ -905,7 +905,7 @@ __device__ __forceinline__ int block_scan_inclusive(int v, int* warp_buf) {
   return r;
 }
 
-__global__ void __launch_bounds__(1024) attn_plan_groups_kernel(const int* __restrict__ row_seq, const int* __restrict__ row_ctx,
+__global__ void __launch_bounds__(1024) attn_plan_groups_kernel(const int* row_seq, const int* row_ctx,
                                                                 int total_rows, int page_size, int pages_per_chunk, int q_tokens,
                                                                 int* __restrict__ chunk_start, int* __restrict__ group_first,
                                                                 int* __restrict__ part_base, int* __restrict__ row_group,

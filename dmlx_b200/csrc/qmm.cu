@@ -2306,10 +2306,10 @@ __device__ __forceinline__ float split_row(const uint4* __restrict__ xr, int k8,
   return __uint_as_float((uint32_t)(127 + ex - 7) << 23);
 }
 
-__global__ void __launch_bounds__(256) mx_split_activations_kernel(const __nv_bfloat16* __restrict__ x, int k,
+__global__ void __launch_bounds__(256) mx_split_activations_kernel(const __nv_bfloat16* x, int k,
                                                                    unsigned char* __restrict__ hi, unsigned char* __restrict__ lo,
-                                                                   float* __restrict__ unscale, const int* __restrict__ gather,
-                                                                   int gather_div, const int* __restrict__ rows_valid) {
+                                                                   float* __restrict__ unscale, const int* gather,
+                                                                   int gather_div, const int* rows_valid) {
   wait_previous();  // (CTAs of the matmul that were placed while rows are still split made it slower: 24576 rows of K = 2048 335 -> 374 us)
   const int row = blockIdx.x;
   if (rows_valid && row >= *rows_valid) return;  // capacity beyond the rows that exist: nothing to read
@@ -2321,8 +2321,8 @@ __global__ void __launch_bounds__(256) mx_split_activations_kernel(const __nv_bf
 
 // The same for tokens whose rows are wanted at `top` places each: a token is split once (4096 tokens, 6 places, K = 4096: 78 us row by row, 35 this way).
 constexpr int kMaxPlaces = 16;
-__global__ void __launch_bounds__(256) mx_split_tokens_kernel(const __nv_bfloat16* __restrict__ x, int k, unsigned char* __restrict__ hi,
-                                                              unsigned char* __restrict__ lo, float* __restrict__ unscale, const int* __restrict__ places, int top) {
+__global__ void __launch_bounds__(256) mx_split_tokens_kernel(const __nv_bfloat16* x, int k, unsigned char* __restrict__ hi,
+                                                              unsigned char* __restrict__ lo, float* __restrict__ unscale, const int* places, int top) {
   wait_previous();
   __shared__ int s_place[kMaxPlaces];
   if (threadIdx.x < top) s_place[threadIdx.x] = places[(size_t)blockIdx.x * top + threadIdx.x];  // (the barrier inside split_row publishes it)
@@ -2337,7 +2337,7 @@ __global__ void __launch_bounds__(256) mx_split_tokens_kernel(const __nv_bfloat1
 }
 
 // Tile-major blocks -> row-major codes + scale atoms (see b200_qweight).  One thread per 32-bit word of a plane.
-__global__ void mx_from_blocks_kernel(const unsigned char* __restrict__ blocks, unsigned char* __restrict__ codes,
+__global__ void mx_from_blocks_kernel(const unsigned char* blocks, unsigned char* __restrict__ codes,
                                       unsigned char* __restrict__ sf, int nt_total, int kc, int k) {
   after_previous();
   constexpr int BB = block_bytes(B200_Q_MXFP4_G32);

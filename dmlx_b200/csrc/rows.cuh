@@ -59,6 +59,11 @@ __device__ __forceinline__ void store_vec(__nv_bfloat16* p, const Vec<VEC>& x) {
   }
 }
 
+// n vectors by a block.
+__device__ __forceinline__ void copy_vectors(uint4* __restrict__ dst, const uint4* __restrict__ src, int n) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
+}
+
 // A vector as it lies in memory, for loads that are to be in flight while something else happens.
 template <typename T, int VEC>
 struct Raw;

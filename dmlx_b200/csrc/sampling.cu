@@ -715,8 +715,8 @@ struct InArguments {
 };
 
 template <typename T, typename Params>
-__global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(const T* __restrict__ logits, int V, const __grid_constant__ Params params,
-                                                                  const uint32_t* __restrict__ ctx, const int* __restrict__ ctx_off,
+__global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(const T* logits, int V, const __grid_constant__ Params params,
+                                                                  const uint32_t* ctx, const int* ctx_off,
                                                                   float* __restrict__ scratch, uint32_t* __restrict__ tokens,
                                                                   float* __restrict__ logprobs) {
   wait_previous();

@@ -1,0 +1,33 @@
+"""What the sources have to keep to so that kernels may be launched while the one ahead of them still runs (launch.cuh)."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "dmlx_b200", "csrc")
+FILES = sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")))
+
+
+def _source(path):
+    return re.sub(r"//[^\n]*|/\*.*?\*/", "", open(path).read(), flags=re.S)
+
+
+@pytest.mark.parametrize("path", FILES, ids=os.path.basename)
+def test_no_kernel_s_input_is_promised_to_stay_as_it_is(path):
+    """`const T* __restrict__` says that the object does not change while the function runs.  A kernel that starts early runs while the one ahead
+    still writes, so the compiler might load such an input ahead of the wait, or through a cache that the wait does not concern.  (Functions that
+    are called after the wait may say so.)"""
+    heads = re.findall(r"__global__[^{;]*?\b(\w+)\s*\(([^{;]*?)\)\s*\{", _source(path), re.S)
+    assert heads or "__global__" not in _source(path)
+    promised = [(name, p) for name, params in heads for p in re.findall(r"const [\w:]+\s*\*\s*__restrict__ \w+", params)]
+    assert not promised, promised
+
+
+@pytest.mark.parametrize("kernel,names", [("rope_kernel", "qk"), ("rope_append_bf16_kernel", ["q"]), ("rope_append_partials_bf16_kernel", ["positions", "row_seq"]),
+                                          ("route_kernel", ["counts"])])
+def test_neither_is_what_a_kernel_changes_in_place(kernel, names):
+    """The same of memory that a kernel reads and writes: what it reads there comes from the kernel ahead."""
+    params = re.search(r"__global__[^{;]*?\b%s\(([^{;]*?)\)\s*\{" % kernel, "\n".join(_source(f) for f in FILES), re.S).group(1)
+    for name in names:
+        assert re.search(r"\*\s*%s\b" % name, params) and not re.search(r"__restrict__ %s\b" % name, params), name
