@@ -1142,7 +1142,10 @@ template <int MODE>
 struct CpShape {
   static constexpr bool kDense = MODE == B200_Q_BF16;
   static constexpr int kWorkers = kDense ? 0 : 16, kEpilogue = 8, kThreads = (kWorkers + 4 + kEpilogue) * 32;
-  static constexpr int kRawSlots = kDense ? 0 : 5;
+  // Raw blocks: a slot's barriers alternate between two sets, so that with chunks taken in turn by two groups of warps each barrier belongs to
+  // one group.  (A wait looks at the parity of a phase.  With a barrier per slot, and five of them, a group waited for every other phase of a
+  // barrier: while the copy of the phase in between was still on its way, the one before that looked like the one waited for.)
+  static constexpr int kRawSlots = kDense ? 0 : 5, kRawBars = 2 * kRawSlots;
   static constexpr int kBatch = kDense ? 16 : 8;  // epilogue: tokens at a time
 };
 constexpr int kCpTokens = 256, kCpMaxStages = 8;
@@ -1177,7 +1180,7 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
   using Z = CpShape<MODE>;
   constexpr bool kDense = Z::kDense;
   constexpr uint32_t BB = block_bytes(MODE), kTile = kTileN * 128, kStage = 2 * kTile;  // [weight tile][half of the activations]
-  constexpr int SR = Z::kRawSlots, kRoles = Z::kWorkers;  // first of the warps with a role of their own
+  constexpr int SR = Z::kRawSlots, BR = Z::kRawBars, kRoles = Z::kWorkers;  // kRoles: first of the warps with a role of their own
   const int S = a.stages, kc = a.kc;
   unsigned char* raw = smem + (size_t)S * kStage;
   float* staging = reinterpret_cast<float*>(raw + SR * BB);  // [epilogue warp][16 tokens][32 rows]
@@ -1186,12 +1189,12 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
   const uint32_t full = bars_u;               // [S] this CTA's copies have landed
   const uint32_t done = full + 8u * S;        // [S] the MMAs reading the stage are done
   const uint32_t ready = done + 8u * S;       // [S] first CTA: both CTAs' stages are complete
-  const uint32_t raw_full = ready + 8u * S;   // [SR] a raw block has landed
-  const uint32_t raw_free = raw_full + 8u * SR;
-  const uint32_t acc_full = raw_free + 8u * SR;  // [2] an item's sums are complete
+  const uint32_t raw_full = ready + 8u * S;   // [BR] a raw block has landed: chunk n's in slot n % SR, barrier n % BR
+  const uint32_t raw_free = raw_full + 8u * BR;
+  const uint32_t acc_full = raw_free + 8u * BR;  // [2] an item's sums are complete
   const uint32_t acc_free = acc_full + 16u;      // [2] first CTA: both CTAs' epilogues have read them
   const uint32_t drain = acc_free + 16u;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * S + 2 * SR + 5);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * S + 2 * BR + 5);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = ptx::cluster_rank();
@@ -1230,21 +1233,21 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
       ptx::mbar_init(&bars[S + s], 1);
       ptx::mbar_init(&bars[2 * S + s], kDense ? 2 : 2 + 2 * 8);  // a word from each CTA, and its dequantising warps
     }
-    for (int s = 0; s < SR; ++s) {
-      ptx::mbar_init(&bars[3 * S + s], 1);
-      ptx::mbar_init(&bars[3 * S + SR + s], 8);
+    for (int b = 0; b < BR; ++b) {
+      ptx::mbar_init(&bars[3 * S + b], 1);
+      ptx::mbar_init(&bars[3 * S + BR + b], 8);
     }
     for (int q = 0; q < 2; ++q) {
-      ptx::mbar_init(&bars[3 * S + 2 * SR + q], 1);
-      ptx::mbar_init(&bars[3 * S + 2 * SR + 2 + q], 2 * Z::kEpilogue);
+      ptx::mbar_init(&bars[3 * S + 2 * BR + q], 1);
+      ptx::mbar_init(&bars[3 * S + 2 * BR + 2 + q], 2 * Z::kEpilogue);
     }
-    ptx::mbar_init(&bars[3 * S + 2 * SR + 4], 1);
+    ptx::mbar_init(&bars[3 * S + 2 * BR + 4], 1);
     ptx::mbar_fence_init();
   }
   __syncthreads();
-  // chunk i of weight tile nt, as number n of this CTA's stream
-  auto load_weights = [&](const unsigned char* blocks, int nt, int i, uint32_t slot) {
-    const uint32_t bar = (kDense ? full : raw_full) + 8u * slot;
+  // chunk i of weight tile nt
+  auto load_weights = [&](const unsigned char* blocks, int nt, int i, uint32_t slot, uint32_t b) {
+    const uint32_t bar = kDense ? full + 8u * slot : raw_full + 8u * b;
     const bool exists = nt < a.nt;  // (an odd tile count leaves the last pair's second CTA without one: it multiplies what lies there)
     ptx::mbar_expect_tx_addr(bar, exists ? BB : 0u);
     if (exists) ptx::bulk_g2s_addr(kDense ? smem_u + slot * kStage : raw_u + slot * BB, blocks + ((size_t)nt * kc + i) * BB, BB, bar);
@@ -1253,7 +1256,7 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
   const int ahead = !a.items && first_work < n_work ? min(slots, decode(first_work).n_chunks) : 0;  // of the first item, before the kernels ahead have ended
   if (warp == kRoles && lane == 0 && ahead > 0) {
     const Work k = decode(first_work);
-    for (int i = 0; i < ahead; ++i) load_weights(k.blocks, k.nt, k.kc0 + i, i);
+    for (int i = 0; i < ahead; ++i) load_weights(k.blocks, k.nt, k.kc0 + i, i, i);
   }
   if (!a.items) wait_previous();
   ptx::cluster_sync();  // both CTAs' barriers are there
@@ -1269,7 +1272,7 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
 
   if (warp == kRoles) {
     if (lane == 0) {
-      uint32_t slot = 0, ph = 1;
+      uint32_t slot = 0, b = 0, ph = 1;  // b: barrier of the chunk; its slot is free when the chunk of barrier b +- SR has been read
       int skip = ahead;
       for (int w = first_work; w < n_work && ok; w += step) {
         const Work k = decode(w);
@@ -1277,11 +1280,15 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
           if (skip > 0) {
             --skip;
           } else {
-            ok = kDense ? ptx::mbar_wait_addr(done + 8u * slot, ph) : ptx::mbar_wait_addr(raw_free + 8u * slot, ph);
+            ok = kDense ? ptx::mbar_wait_addr(done + 8u * slot, ph) : ptx::mbar_wait_addr(raw_free + 8u * (b < (uint32_t)SR ? b + SR : b - SR), ph);
             if (!ok) break;
-            load_weights(k.blocks, k.nt, k.kc0 + i, slot);
+            load_weights(k.blocks, k.nt, k.kc0 + i, slot, b);
           }
-          if (++slot == (uint32_t)slots) { slot = 0; ph ^= 1u; }
+          if (++slot == (uint32_t)slots) {
+            slot = 0;
+            if (kDense || b < (uint32_t)SR) ph ^= 1u;  // (the other set's barriers are in the same phase as this one's were)
+          }
+          if (++b == (uint32_t)BR) b = 0;
         }
       }
       let_next_start();
@@ -1348,17 +1355,17 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
       const uint32_t to = ptx::map_to_rank(ready, 0);
       int n_chunks = 0;
       for (int w = first_work; w < n_work; w += step) n_chunks += decode(w).n_chunks;
-      int s = group, sr = group;
+      int s = group, sr = group, b = group;
       uint32_t ph = 1, phr = 0;
       for (int i = group; i < n_chunks; i += 2) {
-        ok = ptx::mbar_wait_addr(raw_full + 8u * sr, phr);
+        ok = ptx::mbar_wait_addr(raw_full + 8u * b, phr);
         if (!ok) break;
         const unsigned char* blk = raw + (size_t)sr * BB;
         const uint4 q = *reinterpret_cast<const uint4*>(blk + plane * kPlaneBytes + r * 16);
         __nv_bfloat162 s2, b2;
         row_params<MODE>(blk, r, plane, s2, b2);
         ptx::warp_loads_landed(q.x ^ q.y ^ q.z ^ q.w ^ *reinterpret_cast<const uint32_t*>(&s2) ^ *reinterpret_cast<const uint32_t*>(&b2));
-        if (lane == 0) ptx::mbar_arrive_addr(raw_free + 8u * sr);
+        if (lane == 0) ptx::mbar_arrive_addr(raw_free + 8u * b);
         uint4 d[4];
         const uint32_t words[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -1374,7 +1381,9 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
         s += 2;
         if (s >= S) { s -= S; ph ^= 1u; }
         sr += 2;
-        if (sr >= SR) { sr -= SR; phr ^= 1u; }
+        if (sr >= SR) sr -= SR;
+        b += 2;
+        if (b >= BR) { b -= BR; phr ^= 1u; }
       }
     }
   } else {
@@ -3264,7 +3273,7 @@ static b200_status launch_cp(QmmArgs& a, int rows, cudaStream_t s) {
   constexpr int BB = block_bytes(MODE);
   using Z = CpShape<MODE>;
   constexpr int fixed = 1024 /*alignment slack*/ + Z::kRawSlots * BB + Z::kEpilogue * Z::kBatch * kCpPitch * (int)sizeof(float) +
-                        8 * (3 * kCpMaxStages + 2 * Z::kRawSlots + 5) + 16;
+                        8 * (3 * kCpMaxStages + 2 * Z::kRawBars + 5) + 16;
   static int smem_budget[3] = {0, 0, 0}, most_pairs[3] = {0, 0, 0};
   cudaLaunchAttribute attr[2]{};
   attr[0].id = cudaLaunchAttributeClusterDimension;

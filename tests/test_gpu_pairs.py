@@ -67,6 +67,23 @@ def test_pairs_of_ctas(mode, n, k, rows):
     _run(mode, n, k, rows, "QMM_TCGEN05_X2")
 
 
+# Items enough that the rings of raw blocks, of stages and of sums wrap many times in every pair of CTAs; a last pair of weight tiles with and without
+# a second one; chunks enough for several ranges of K.
+@pytest.mark.parametrize("mode", ["affine4", "mxfp4", "bf16"])
+@pytest.mark.parametrize("n,k,rows", [(33 * 128, 1024, 2500), (34 * 128, 1024, 2500), (256, 4096, 4096)])
+def test_pairs_of_ctas_repeat_themselves(mode, n, k, rows):
+    """A block or a stage that is read before it is complete would differ from run to run."""
+    from dmlx_b200 import device as dev
+
+    w = dev.QWeight.random({"affine4": dev.Q_AFFINE4_G64, "mxfp4": dev.Q_MXFP4_G32, "bf16": dev.Q_BF16}[mode], n, k, seed=9)
+    x = _rows(rows, k, 1)
+    for epilogue in (dev.EPI_NONE, dev.EPI_SWIGLU):
+        first = dev.qmm(w, x, epilogue, path=dev.QMM_TCGEN05_X2)
+        for _ in range(40):
+            assert torch.equal(dev.qmm(w, x, epilogue, path=dev.QMM_TCGEN05_X2), first)
+    assert dev.qmm_error_word() == 0
+
+
 @pytest.mark.parametrize("n", [33, 34, 129, 130])
 @pytest.mark.parametrize("rows", [65, 128, 200, 300])
 def test_outputs_that_do_not_come_in_fours(n, rows):
