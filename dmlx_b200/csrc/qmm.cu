@@ -1712,13 +1712,14 @@ __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma_kernel
   // activations (they meet on named barrier 1, which the producer warp is not part of).
   if (warp == kGemvConsumers) {
     if (lane == 0) {
-      int s = 0;
+      int s = 0, ahead = stages;  // slots that are filled before the kernels ahead have ended
       uint32_t phase = 1;
       for (int item = 0; item < n_items && ok; ++item) {
         const int nt0 = 2 * (grp + item * groups);
         const int tiles = min(2, a.nt - nt0);
         const unsigned char* src = a.blocks + ((size_t)nt0 * a.kc + kc0) * BB;
         for (int i = 0; i < n_chunks; ++i) {
+          if (ahead-- == 0) wait_previous();  // (a slot comes free when they have ended: their time is not part of the bounded wait)
           ok = ptx::mbar_wait(&raw_free[s], phase);
           if (!ok) break;
           ptx::mbar_expect_tx(&raw_full[s], tiles * BB);
@@ -1730,7 +1731,7 @@ __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma_kernel
       let_next_start();
     }
   } else {
-    wait_previous();  // (the producer need not: it reads weights only)
+    wait_previous();
     const int vec_per_row = n_chunks * (kChunkK * 2 / 16);
     for (int idx = tid; idx < TILE * vec_per_row; idx += kGemvConsumers * 32) {
       const int row = idx / vec_per_row, v = idx - row * vec_per_row;
@@ -2056,13 +2057,14 @@ __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma8_kerne
   bool ok = true;
   if (warp == kGemvConsumers) {
     if (lane == 0) {
-      int s = 0;
+      int s = 0, ahead = stages;  // slots that are filled before the kernels ahead have ended
       uint32_t phase = 1;
       for (int item = 0; item < n_items && ok; ++item) {
         const int nt0 = 2 * (grp + item * groups);
         const int tiles = min(2, a.nt - nt0);
         const unsigned char* src = a.blocks + ((size_t)nt0 * a.kc + kc0) * BB;
         for (int i = 0; i < n_chunks; ++i) {
+          if (ahead-- == 0) wait_previous();  // (a slot comes free when they have ended: their time is not part of the bounded wait)
           ok = ptx::mbar_wait(&raw_free[s], phase);
           if (!ok) break;
           ptx::mbar_expect_tx(&raw_full[s], tiles * BB);
@@ -2074,7 +2076,7 @@ __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma8_kerne
       let_next_start();
     }
   } else {
-    wait_previous();  // (the producer need not: it reads weights only)
+    wait_previous();
     // ---- stage the activations: 16-bit fixed point with one scale per token and 64-column group ----
     // One thread per 8 columns; the 8 threads of a group (consecutive lanes) agree on the group's scale,
     // quantise, and add up the group's integer sum.  A single pass, one barrier at the end.

@@ -31,3 +31,18 @@ def test_neither_is_what_a_kernel_changes_in_place(kernel, names):
     params = re.search(r"__global__[^{;]*?\b%s\(([^{;]*?)\)\s*\{" % kernel, "\n".join(_source(f) for f in FILES), re.S).group(1)
     for name in names:
         assert re.search(r"\*\s*%s\b" % name, params) and not re.search(r"__restrict__ %s\b" % name, params), name
+
+
+KERNELS = [(os.path.basename(f), m.group(1), m.start(), f) for f in FILES for m in re.finditer(r"__global__[^{;]*?\b(\w+_kernel)\s*\([^{;]*?\)\s*\{", _source(f), re.S)]
+
+
+@pytest.mark.parametrize("file,name,start,path", KERNELS, ids=[k[1] for k in KERNELS])
+def test_a_kernel_waits_for_those_ahead_before_its_bounded_waits_begin(file, name, start, path):
+    """A wait that gives up after so many polls, or a word written to memory, belongs behind the wait for the kernels ahead: their time would count."""
+    body = _source(path)[start:]
+    body = body[:body.index("\n}\n")]
+    wait = re.search(r"\b(after|wait)_previous\(\)", body)
+    if wait is None:
+        pytest.skip("launched plainly")
+    early = re.search(r"\bmbar_wait\w*\(|\batomic\w+\(", body[:wait.start()])
+    assert early is None, early.group(0)
