@@ -2990,6 +2990,8 @@ extern "C" b200_status b200_qweight_create(int32_t mode, int32_t n_experts, int3
   cudaError_t e = cudaMalloc((void**)&w->d_blocks, total);
   if (e != cudaSuccess) { b200_set_error("cudaMalloc(%zu) failed: %s", total, cudaGetErrorString(e)); delete w; return B200_ERR_CUDA; }
   e = cudaMemcpy(w->d_blocks, host.data(), total, cudaMemcpyHostToDevice);
+  // (a copy from pageable memory returns when it has been staged; kernels on other streams fetch weights before they wait for anything)
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
   if (e != cudaSuccess) { b200_set_error("weight upload failed: %s", cudaGetErrorString(e)); cudaFree(w->d_blocks); delete w; return B200_ERR_CUDA; }
   *out = w;
   return B200_OK;

@@ -46,3 +46,14 @@ def test_a_kernel_waits_for_those_ahead_before_its_bounded_waits_begin(file, nam
         pytest.skip("launched plainly")
     early = re.search(r"\bmbar_wait\w*\(|\batomic\w+\(", body[:wait.start()])
     assert early is None, early.group(0)
+
+
+def test_weights_are_on_the_device_when_they_are_handed_out():
+    """Kernels fetch weights before they wait for anything ahead of them, so a weight object may not leave its constructor while its blocks are on
+    their way.  (A copy from pageable memory returns when it has been staged.)"""
+    source = _source(os.path.join(CSRC, "qmm.cu"))
+    makers = re.findall(r"b200_status (b200_qweight_\w+)\([^{;]*\*\* ?out\) \{(.*?)\n\}\n", source, re.S)
+    assert {name for name, _ in makers} == {"b200_qweight_create", "b200_qweight_random"}
+    for name, body in makers:
+        filled = max(body.rfind("cudaMemcpy("), body.rfind("<<<"))
+        assert 0 < filled < body.index("Synchronize(", filled) < body.rindex("*out = w"), name
