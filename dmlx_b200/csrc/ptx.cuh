@@ -333,11 +333,37 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-// What the arrival announces is shared memory that the async proxy reads (written ahead of a fence of that proxy, or by a copy whose barrier the
-// thread has waited for) or tensor memory that has been read: no write that a wider scope would have to flush.  With .release.cluster here and
-// .acquire.cluster in the waits a chunk of a matmul took 1900 cycles instead of 950 (2048 x 8192, 512 rows, before its epilogue was changed).
+// Arrives on a barrier of the pair and releases to both CTAs what lies in this CTA's shared memory: stores ahead of a fence of the async proxy that
+// this thread has made or has seen made, and copies whose barrier it has waited for.  The other side waits in mbar_wait_cluster.  (The fences are
+// those for shared memory alone: an arrival with .release.cluster waits for the SM's stores to memory too, 1900 cycles a chunk of a matmul
+// instead of 950.)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t mapped_bar) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mapped_bar) : "memory");
+  asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapped_bar) : "memory");
+}
+// The same for tensor memory that has been read: tcgen05.fence::before_thread_sync ahead of it and after_thread_sync behind the wait order that, and
+// there are no writes to release.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t mapped_bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapped_bar) : "memory");
+}
+// mbar_wait_addr for arrivals of both CTAs.
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
+  for (uint32_t i = 0; i < kSpinLimit; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) {
+      asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+      return true;
+    }
+    if (i > 64) __nanosleep(64);
+  }
+  return false;
 }
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

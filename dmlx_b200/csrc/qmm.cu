@@ -1136,8 +1136,10 @@ __global__ void __launch_bounds__(kTc2Threads, 1) qmm_tc2_kernel(const __grid_co
 // fastest, so that weights come from memory once.
 // Warps, quantised weights: 0-15 dequantise this CTA's weight tile into the stage's MMA tile, two groups of eight in turn (a thread per row and
 // 32-column plane; one group of eight took 700 cycles per chunk, longer than the chunk's 512 of MMAs), then one each for the weights (a ring of raw
-// blocks), the MMAs of both CTAs (in the first one), the activations, and for telling the first CTA that this one's copies have landed, and four
-// that bring the sums to the output.  Dense weights land in the stage; eight warps bring out their sums.
+// blocks), the MMAs of both CTAs (in the first one), the activations, and for telling the first CTA that this one's half of a stage is complete, and
+// eight that bring the sums to the output.  Dense weights land in the stage, so none dequantise.
+// The MMAs of the pair read both CTAs' shared memory, so the word to the first CTA has the scope of the cluster.  One thread per CTA sends it, for
+// what it has seen complete on a barrier of its own CTA: a fence by each of the warps that dequantise made a mixed step 3 % longer.
 template <int MODE>
 struct CpShape {
   static constexpr bool kDense = MODE == B200_Q_BF16;
@@ -1186,7 +1188,7 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
   float* staging = reinterpret_cast<float*>(raw + SR * BB);  // [epilogue warp][16 tokens][32 rows]
   uint64_t* bars = reinterpret_cast<uint64_t*>(staging + Z::kEpilogue * Z::kBatch * kCpPitch);
   const uint32_t smem_u = ptx::smem_u32(smem), raw_u = ptx::smem_u32(raw), bars_u = ptx::smem_u32(bars);
-  const uint32_t full = bars_u;               // [S] this CTA's copies have landed
+  const uint32_t full = bars_u;               // [S] this CTA's half of the stage is complete
   const uint32_t done = full + 8u * S;        // [S] the MMAs reading the stage are done
   const uint32_t ready = done + 8u * S;       // [S] first CTA: both CTAs' stages are complete
   const uint32_t raw_full = ready + 8u * S;   // [BR] a raw block has landed: chunk n's in slot n % SR, barrier n % BR
@@ -1229,9 +1231,9 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
   };
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      ptx::mbar_init(&bars[s], kDense ? 2 : 1);
+      ptx::mbar_init(&bars[s], kDense ? 2 : 1 + 8);  // both copies; or the activations' and the eight warps that dequantise the chunk
       ptx::mbar_init(&bars[S + s], 1);
-      ptx::mbar_init(&bars[2 * S + s], kDense ? 2 : 2 + 2 * 8);  // a word from each CTA, and its dequantising warps
+      ptx::mbar_init(&bars[2 * S + s], 2);  // a word from each CTA
     }
     for (int b = 0; b < BR; ++b) {
       ptx::mbar_init(&bars[3 * S + b], 1);
@@ -1327,11 +1329,11 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
         const Work k = decode(w);
         if (k.n_chunks == 0) continue;
         const uint32_t idesc = ptx::umma_idesc_bf16(2 * kTileN, k.n_here), set = n_item & 1u, acc = tmem_base + set * 256u;
-        if (n_item >= 2) ok = ptx::mbar_wait_addr(acc_free + 8u * set, ((n_item >> 1) - 1u) & 1u);
+        if (n_item >= 2) ok = ptx::mbar_wait_cluster(acc_free + 8u * set, ((n_item >> 1) - 1u) & 1u);
         if (!ok) break;
         ptx::tc_fence_after_sync();
         for (int i = 0; i < k.n_chunks; ++i) {
-          ok = ptx::mbar_wait_addr(ready + 8u * s, ph);
+          ok = ptx::mbar_wait_cluster(ready + 8u * s, ph);
           if (!ok) break;
           ptx::tc_fence_after_sync();
           const uint64_t da = ptx::umma_desc_k_sw128(smem_u + s * kStage), db = ptx::umma_desc_k_sw128(smem_u + s * kStage + kTile);
@@ -1352,7 +1354,6 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
   } else if (warp < kRoles) {
     if constexpr (!kDense) {
       const int r = tid & (kTileN - 1), plane = (tid >> 7) & 1, group = warp >> 3;
-      const uint32_t to = ptx::map_to_rank(ready, 0);
       int n_chunks = 0;
       for (int w = first_work; w < n_work; w += step) n_chunks += decode(w).n_chunks;
       int s = group, sr = group, b = group;
@@ -1377,7 +1378,7 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
         for (int x = 0; x < 4; ++x) *reinterpret_cast<uint4*>(arow + (((plane * 4 + x) ^ (r & 7)) << 4)) = d[x];
         ptx::fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive_cluster(to + 8u * s);
+        if (lane == 0) ptx::mbar_arrive_addr(full + 8u * s);
         s += 2;
         if (s >= S) { s -= S; ph ^= 1u; }
         sr += 2;
@@ -1442,7 +1443,7 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
       // all that this warp reads of the item's sums has been read
       ptx::tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive_cluster(to + 8u * set);
+      if (lane == 0) ptx::mbar_arrive_cluster_relaxed(to + 8u * set);
       ++n_item;
     }
   }

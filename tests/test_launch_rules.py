@@ -57,3 +57,13 @@ def test_weights_are_on_the_device_when_they_are_handed_out():
     for name, body in makers:
         filled = max(body.rfind("cudaMemcpy("), body.rfind("<<<"))
         assert 0 < filled < body.index("Synchronize(", filled) < body.rindex("*out = w"), name
+
+
+def test_words_between_ctas_have_the_scope_of_the_cluster():
+    """A word that one CTA sends to another stands for shared memory that the other's MMAs read: an arrival without a scope releases to its own CTA."""
+    source = "\n".join(_source(f) for f in FILES)
+    sent = re.findall(r'"mbarrier\.arrive[^"]*shared::cluster[^"]*"', source)
+    assert sent and all(".release.cluster." in a or ".relaxed.cluster." in a for a in sent), sent
+    ahead = source[:source.index("mbarrier.arrive.relaxed.cluster")]
+    assert ahead.rstrip().endswith('asm volatile("') and "fence.release.sync_restrict::shared::cta.cluster" in ahead[-160:]
+    assert re.search(r"mbar_wait_cluster\(ready", source) and not re.search(r"mbar_wait_addr\((ready|acc_free)", source)
