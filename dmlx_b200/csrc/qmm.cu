@@ -166,8 +166,11 @@ __device__ __forceinline__ void finish_store(const QmmArgs& a, int token, int n,
 // ---- split-K finish: sums the partial tiles in split order (deterministic), applies the epilogue,
 // writes bf16.  One thread per 4 consecutive output columns of one row, so the whole GPU takes
 // part and every thread has `splits` independent 16-byte loads in flight.
+// The next kernel, more often than not another stream of weights, is let start when the sums have arrived, behind SwiGLU's arithmetic at the end.  Let
+// start at once, its loads came in between: MXFP4 28672 x 4096, 8 rows, 39.1 us (32.9 with plain launches), 29.3 this way; 160 shapes of up to
+// 16 rows 2 % less altogether.
 __global__ void qmm_finish_kernel(QmmArgs a, int splits) {
-  after_previous();
+  wait_previous();
   const int n4 = a.nt * (kTileN / 4);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)a.rows * n4) return;
@@ -201,6 +204,7 @@ __global__ void qmm_finish_kernel(QmmArgs a, int splits) {
     const float4 v = p[(size_t)s * split_stride];
     acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
   }
+  if (a.epilogue != B200_EPI_SWIGLU) let_next_start();
   finish_store(a, token, n, acc);
 }
 
