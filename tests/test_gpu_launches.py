@@ -1,0 +1,71 @@
+"""Steps whose kernels are launched while the one ahead still runs (launch.cuh) give the bits of the same steps run kernel by kernel.
+
+CUDA_LAUNCH_BLOCKING makes every launch wait until its kernel has ended, so no kernel starts early; it is read when a process starts, so each
+side is a process of its own.  Graphs are off: their kernels are not launched one by one (that they change nothing is tested model by model)."""
+import os
+import subprocess
+import sys
+import tempfile
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+MODELS = ["llama", "llama int4", "tafuvik", "sotavik", "dovorax", "lorulix"]
+
+
+def _loaded(name, path):
+    from dmlx_b200.models import Limits, load_model
+    from tests import test_gpu_decoder, test_gpu_dovorax, test_gpu_lorulix, test_gpu_models, test_gpu_sotavik
+
+    if name.startswith("llama"):
+        test_gpu_models._folder(os.path.join(path, "m"), name.endswith("int4"))
+        return load_model(os.path.join(path, "m"), "bfloat16", Limits(1024, 4, 4)), 512
+    module, case = {"tafuvik": (test_gpu_decoder, "wide_head"), "sotavik": (test_gpu_sotavik, "wide"), "dovorax": (test_gpu_dovorax, "wide"),
+                    "lorulix": (test_gpu_lorulix, "wide")}[name]
+    cfg = module.CASES[case]
+    return module._load(path, cfg, 31, "bfloat16", max_rows=1024)[0], cfg["vocab"]
+
+
+def _logits(name):
+    """Prompts of three requests in one step, the next portion of one beside two that decode, and steps of one row each."""
+    from dmlx_b200.serving import TokenFeeder
+
+    with tempfile.TemporaryDirectory() as path:
+        loaded, vocab = _loaded(name, path)
+        loaded.model.enable_graphs(False)
+        tokens = [np.random.default_rng(i).integers(0, vocab, 500).tolist() for i in range(3)]
+        at, out = [0, 0, 0], []
+        feeder = TokenFeeder(loaded, 64)
+        for portions in [(290, 33, 150)] + [(140, 1, 1)] + [(1, 1, 1)] * 12:
+            out.append(feeder.step([(i, tokens[i][at[i]:at[i] + n], [n - 1]) for i, n in enumerate(portions)]))
+            at = [a + n for a, n in zip(at, portions)]
+        return np.stack(out)
+
+
+@pytest.fixture(scope="module")
+def runs(tmp_path_factory):
+    out = []
+    for blocking in ("1", "0"):
+        path = str(tmp_path_factory.mktemp("launches") / "logits.npz")
+        subprocess.run([sys.executable, "-m", "tests.test_gpu_launches", path], check=True, cwd=ROOT, timeout=600, env={**os.environ, "CUDA_LAUNCH_BLOCKING": blocking})
+        out.append(np.load(path))
+    return out
+
+
+@pytest.mark.parametrize("name", MODELS)
+def test_steps_of_early_kernels_equal_steps_kernel_by_kernel(runs, name):
+    one_by_one, early = runs
+    assert np.isfinite(one_by_one[name]).all()
+    for again in (f"{name} 0", f"{name} 1"):
+        np.testing.assert_array_equal(early[again], one_by_one[name])
+
+
+if __name__ == "__main__":
+    results = {}
+    for model in MODELS:
+        results[model] = results[f"{model} 0"] = _logits(model)
+        results[f"{model} 1"] = _logits(model)
+    np.savez(sys.argv[1], **results)

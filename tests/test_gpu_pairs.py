@@ -98,6 +98,15 @@ def test_pairs_of_tiles(mode, n, k, rows):
     _run(mode, n, k, rows, "QMM_TCGEN05_TMEM_A")
 
 
+@pytest.mark.parametrize("mode,k", [("affine4", 128), ("affine4", 192), ("mxfp4", 128)])
+@pytest.mark.parametrize("more", [0, 1])
+@pytest.mark.parametrize("rows", [17, 64, 65, 128])
+def test_matrices_around_one_wave_of_tile_pairs(mode, k, more, rows):
+    """Up to one pair of weight tiles per SM the pairs take a matrix, beyond it the kernel of single tiles, two CTAs an SM."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    _run(mode, (2 * sms + more) * 128, k, rows)
+
+
 def _grouped(mode, e, n, k, sizes, tile, swiglu):
     from dmlx_b200 import device as dev
 
