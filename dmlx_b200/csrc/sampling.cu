@@ -26,6 +26,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.h"
 #include "launch.cuh"
@@ -728,10 +729,11 @@ __global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(const T* logit
   const T* x = logits + (size_t)row * V;
   float* lp = logprobs ? logprobs + row : nullptr;
   const int ctx_lo = ctx_off ? ctx_off[row] : 0, ctx_n = ctx_off ? ctx_off[row + 1] - ctx_lo : 0;
-  if (p.repetition_penalty > 1.0f && ctx_n > 0 && scratch != nullptr) {
+  const bool penalised = p.repetition_penalty > 1.0f && ctx_n > 0 && scratch != nullptr;
+  float* y = penalised ? scratch + (size_t)row * V : nullptr;
+  if (penalised) {
     // applyRepetitionPenalty (src/sampling.zig:328-354): every occurrence of a token divides a positive
     // logit by the penalty or multiplies a non-positive one; occurrences commute, so they may race.
-    float* y = scratch + (size_t)row * V;
     for (int i = rank * kThreads + threadIdx.x; i < V; i += ranks * kThreads) y[i] = to_f32(x[i]);
     __threadfence();
     cluster.sync();
@@ -749,10 +751,16 @@ __global__ void __launch_bounds__(kThreads, 2) sample_rows_kernel(const T* logit
     }
     __threadfence();
     cluster.sync();
-    Sampler<float>(s, Row<float>{y, V, V % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0}).run(p, tokens + row, lp);
-  } else {
-    Sampler<T>(s, Row<T>{x, V, V % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0}).run(p, tokens + row, lp);
   }
+  auto sampled = [&](auto* from) {
+    using U = std::remove_const_t<std::remove_pointer_t<decltype(from)>>;
+    Sampler<U>(s, Row<U>{from, V, V % 8 == 0 && (reinterpret_cast<uintptr_t>(from) & 15) == 0}).run(p, tokens + row, lp);
+  };
+  // (One call for f32 rows: with one for each source the compiler kept the sampler as a function, its row's
+  // parameters in local memory, where these come in the arguments: 64 rows of 128256 words 101 us, 70 now; from device memory 78 and 70.)
+  if constexpr (sizeof(T) == 4) sampled(penalised ? y : x);
+  else if (penalised) sampled(y);
+  else sampled(x);
 }
 
 template <typename T, typename Params>
