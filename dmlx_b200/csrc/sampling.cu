@@ -704,14 +704,16 @@ struct Sampler {
   }
 };
 
-// The rows' parameters: in device memory, or of up to 128 rows in the arguments of the launch (4 KB at most), which spares an upload ahead of the kernel
-// (64 rows in passes behind one another: pageable upload 105 us, pinned 88, in the arguments 80; the first pass on new buffers 163, 170, 148).
+// The rows' parameters: in device memory, or of up to 1024 rows in the arguments of the launch (24 KB; 128 rows 3 KB), which spares an upload ahead of
+// the kernel (64 rows in passes behind one another: pageable upload 105 us, pinned 88, in the arguments 80; the first pass on new buffers 163, 170,
+// 148.  256 rows of 128256 bf16 words in passes behind one another 182, 177, 167, waited for one by one 265, 264, 253; 1024 rows 461, 457, 447).
 struct InMemory {
   const b200_sample_params* p;
   __device__ __forceinline__ const b200_sample_params& operator[](int row) const { return p[row]; }
 };
+template <int ROWS>
 struct InArguments {
-  b200_sample_params p[B200_SAMPLE_HOST_ROWS];
+  b200_sample_params p[ROWS];
   __device__ __forceinline__ const b200_sample_params& operator[](int row) const { return p[row]; }
 };
 
@@ -829,9 +831,11 @@ b200_status b200_sample_rows_host(const void* d_logits, int32_t logits_f32, int3
     b200_set_error("sample_rows_host: %d rows, %d at most", rows, B200_SAMPLE_HOST_ROWS);
     return B200_ERR_INVALID_ARGUMENT;
   }
-  InArguments params{};
-  if (h_params) std::copy_n(h_params, rows, params.p);
-  return sample(d_logits, logits_f32, rows, vocab, params, h_params == nullptr, d_ctx_tokens, d_ctx_offsets, d_scratch, d_tokens, d_logprobs, stream);
+  auto run = [&](auto params) {
+    if (h_params) std::copy_n(h_params, rows, params.p);
+    return sample(d_logits, logits_f32, rows, vocab, params, h_params == nullptr, d_ctx_tokens, d_ctx_offsets, d_scratch, d_tokens, d_logprobs, stream);
+  };
+  return rows <= 128 ? run(InArguments<128>{}) : run(InArguments<B200_SAMPLE_HOST_ROWS>{});
 }
 
 }  // extern "C"

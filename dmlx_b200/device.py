@@ -405,11 +405,6 @@ def sample_rows(logits: torch.Tensor, rows, context: Optional[Sequence[Sequence[
     assert logits.dtype in (torch.bfloat16, torch.float32) and logits.is_contiguous()
     n, v = logits.shape
     params = sample_params_array(rows)
-    if n <= 128 and len(params) >= n:  # in the arguments of the launch
-        sample, p_params = lib.b200_sample_rows_host, params.ctypes.data
-    else:  # (from pinned memory: a pageable upload waits for the kernels ahead of it in the stream)
-        d_params = torch.from_numpy(params).pin_memory().to(logits.device, non_blocking=True)
-        sample, p_params = lib.b200_sample_rows, _ptr(d_params)
     tokens = torch.empty(n, dtype=torch.int32, device=logits.device)
     lp = torch.empty(n, dtype=torch.float32, device=logits.device) if logprobs else None
     d_ctx = d_off = scratch = None
@@ -419,6 +414,11 @@ def sample_rows(logits: torch.Tensor, rows, context: Optional[Sequence[Sequence[
         d_ctx = torch.tensor(flat + [0], dtype=torch.int64).to(torch.int32).to(logits.device)
         d_off = torch.from_numpy(offs).to(logits.device)
         scratch = torch.empty((n, v), dtype=torch.float32, device=logits.device)
+    if len(params) >= n and n <= 1024:  # B200_SAMPLE_HOST_ROWS: in the arguments of the launch
+        sample, p_params = lib.b200_sample_rows_host, params.ctypes.data
+    else:  # (one launch with an upload ahead of it: 1500 rows of 128256 words 948 us, 1018 as two launches without)
+        d_params = torch.from_numpy(params).to(logits.device)
+        sample, p_params = lib.b200_sample_rows, _ptr(d_params)
     _lib.check(sample(_ptr(logits), int(logits.dtype == torch.float32), n, v, p_params, _ptr(d_ctx), _ptr(d_off), _ptr(scratch),
                       _ptr(tokens), _ptr(lp), _stream()))
     return tokens, lp

@@ -401,7 +401,7 @@ b200_status b200_sample_rows(const void* d_logits, int32_t logits_f32, int32_t r
                              const int32_t* d_ctx_offsets, float* d_scratch, uint32_t* d_tokens,
                              float* d_logprobs, void* stream);
 /* The same with the rows' parameters in host memory, which may be reused when the call returns; up to B200_SAMPLE_HOST_ROWS rows. */
-#define B200_SAMPLE_HOST_ROWS 128
+#define B200_SAMPLE_HOST_ROWS 1024
 b200_status b200_sample_rows_host(const void* d_logits, int32_t logits_f32, int32_t rows, int32_t vocab,
                                   const b200_sample_params* h_params, const uint32_t* d_ctx_tokens,
                                   const int32_t* d_ctx_offsets, float* d_scratch, uint32_t* d_tokens,

@@ -394,3 +394,34 @@ def test_f32_rows_take_no_longer_with_the_parameters_in_the_arguments(rows, voca
     both = [(time(_lib.lib.b200_sample_rows, d_params.data_ptr()), time(_lib.lib.b200_sample_rows_host, params.ctypes.data)) for _ in range(12)]
     in_memory, in_arguments = (min(t) for t in zip(*both))
     assert in_arguments <= 1.1 * in_memory, (in_memory, in_arguments)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [128, 129, 1024, 1025])
+def test_parameters_travel_with_the_launch(rows):
+    """The same tokens as with the parameters in device memory, and up to 1024 rows no copy ahead of the kernel."""
+    import torch
+
+    from dmlx_b200 import _lib
+    from dmlx_b200 import device as dev
+
+    v, rng = 700, np.random.default_rng(rows)
+    logits = torch.tensor(rng.normal(0, 3, (rows, v)), dtype=torch.float32, device="cuda")
+    kinds = [(0.0, 50, 1.0), (0.8, 50, 1.0), (0.8, 50, 0.9), (0.9, 0, 1.0), (0.8, 0, 0.9)]
+    params = [(*kinds[i % 5], float(u), 1.0 + 0.2 * (i % 3)) for i, u in enumerate(rng.random(rows))]
+    history = [rng.integers(0, v, i % 4).tolist() for i in range(rows)]
+    for context in (None, history):
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as seen:
+            tokens, lp = dev.sample_rows(logits, params, context)
+            torch.cuda.synchronize()
+        names = [e.key for e in seen.key_averages()]
+        assert any("sample_rows_kernel" in n for n in names)
+        assert context is not None or rows > 1024 or not any("HtoD" in n for n in names), names
+        d_params = torch.from_numpy(dev.sample_params_array(params)).cuda()
+        offsets = torch.tensor(np.cumsum([0] + [len(c) for c in context]), dtype=torch.int32, device="cuda") if context else None
+        words = torch.tensor([t for c in context for t in c], dtype=torch.int32, device="cuda") if context else None
+        want, want_lp, scratch = torch.empty_like(tokens), torch.empty_like(lp), torch.empty_like(logits)
+        ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+        _lib.check(_lib.lib.b200_sample_rows(ptr(logits), 1, rows, v, ptr(d_params), ptr(words), ptr(offsets), ptr(scratch), ptr(want), ptr(want_lp),
+                                             torch.cuda.current_stream().cuda_stream))
+        assert torch.equal(tokens, want) and torch.equal(lp, want_lp)
