@@ -34,4 +34,6 @@ extern long long g_b200_launch_counter;
 b200_status b200_require_device();
 // The same without binding the process to a device (entry points that keep per-device state).
 b200_status b200_require_any_device();
+// SMs of the process's device, asked for once.
+int b200_sm_count();
 #endif

@@ -157,9 +157,10 @@ __global__ void argmax_kernel(const T* logits, int vocab, uint32_t* __restrict__
 
 template <typename T>
 b200_status launch_argmax(const T* logits, int rows, int vocab, uint32_t* out, cudaStream_t s) {
-  // parts of 4096 values and more, as long as the CTAs run at once (a cluster's stay within a GPC: some 32 clusters of eight at two CTAs per SM)
+  // parts of 4096 values and more, as long as the CTAs run at once, two per SM
+  static const int most = ctas_in_clusters(argmax_kernel<T>, 8, 2, b200_sm_count(), 512, 0);
   int parts = 1;
-  while (parts < 8 && vocab >= parts * 8192 && (long long)rows * parts * 2 <= 256) parts *= 2;
+  while (parts < 8 && vocab >= parts * 8192 && (long long)rows * parts * 2 <= most) parts *= 2;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)rows * parts);
   cfg.blockDim = dim3(parts > 1 ? 512 : 1024);

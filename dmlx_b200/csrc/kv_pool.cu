@@ -62,6 +62,16 @@ b200_status b200_require_device() {
   return B200_OK;
 }
 
+int b200_sm_count() {
+  static int sms = 0;
+  int dev = 0;
+  if (sms == 0 && (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)) {
+    cudaGetLastError();
+    return 1;
+  }
+  return sms;
+}
+
 extern "C" int32_t b200_device_available(void) { return b200_require_any_device() == B200_OK; }
 
 // ---------------------------------------------------------------------------------------------
@@ -901,7 +911,7 @@ extern "C" b200_status b200_kv_rope_append(b200_kv* kv, int32_t layer, void* d_q
 
 // Blocks that share a row's heads: eight per SM altogether.  With a head per warp and row, angles and page lookups were most of a warp's work (2105
 // rows, 48 heads from partial sums: 38 us, 21 with the row's heads in one block).
-static int rope_blocks(int rows, int most) { return std::min(most, std::max(1, (8 * 148 + rows - 1) / rows)); }
+static int rope_blocks(int rows, int most) { return std::min(most, std::max(1, (8 * b200_sm_count() + rows - 1) / rows)); }
 
 // RoPE + append fed from the split-K partial sums of the fused q/k/v projection (head_dim 128 = one 128-row weight
 // tile per head).  One warp per (row, head): the lane's four columns (two rotation pairs) are summed over the splits
@@ -1054,7 +1064,7 @@ b200_status b200_kv_gather(b200_kv* kv, int32_t layer, int32_t seq, void* d_k_ou
     b200_set_error("gather: layer/slot out of range");
     return B200_ERR_INVALID_BATCH_INDEX;
   }
-  launch_after(gather_kernel, 296, 256, 0, (cudaStream_t)stream, kv->dev, layer, seq, d_k_out, d_v_out, cap_rows);
+  launch_after(gather_kernel, 2 * b200_sm_count(), 256, 0, (cudaStream_t)stream, kv->dev, layer, seq, d_k_out, d_v_out, cap_rows);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }

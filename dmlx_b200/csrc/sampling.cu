@@ -770,10 +770,11 @@ b200_status launch(const T* logits, int rows, int vocab, const Params& params, c
                    uint32_t* tokens, float* logprobs, cudaStream_t s) {
   // (asked for at every launch: the attribute belongs to the device that the calling thread uses)
   B200_CUDA_TRY(cudaFuncSetAttribute(sample_rows_kernel<T, Params>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared)));
-  // CTAs per row: 8192 words each at least (16 a thread), and no more altogether than run at the same time: two per SM, and a cluster's within one
-  // GPC, which leaves room for 32 clusters of eight (37 rows, a nucleus of 0.9: 111 us in eight CTAs a row, 88 in four).
+  // CTAs per row: 8192 words each at least (16 a thread), and no more altogether than run at the same time (37 rows, a nucleus of 0.9: 111 us in eight
+  // CTAs a row, 88 in four).
+  static const int most = ctas_in_clusters(sample_rows_kernel<T, Params>, kMaxCluster, 2, b200_sm_count(), kThreads, sizeof(Shared));
   int ranks = 1;
-  while (ranks < kMaxCluster && vocab > ranks * 8192 && (long long)rows * ranks * 2 <= 256) ranks *= 2;
+  while (ranks < kMaxCluster && vocab > ranks * 8192 && (long long)rows * ranks * 2 <= most) ranks *= 2;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)rows * ranks);
   cfg.blockDim = dim3(kThreads);

@@ -67,3 +67,10 @@ def test_words_between_ctas_have_the_scope_of_the_cluster():
     ahead = source[:source.index("mbarrier.arrive.relaxed.cluster")]
     assert ahead.rstrip().endswith('asm volatile("') and "fence.release.sync_restrict::shared::cta.cluster" in ahead[-160:]
     assert re.search(r"mbar_wait_cluster\(ready", source) and not re.search(r"mbar_wait_addr\((ready|acc_free)", source)
+
+
+@pytest.mark.parametrize("path", FILES, ids=os.path.basename)
+def test_grids_are_sized_by_the_device(path):
+    """How many SMs there are, and how many CTAs run on them at once, is asked of the device."""
+    assert not re.findall(r"[^\n]*\b(?:148|296)\b[^\n]*", _source(path))
+    assert not re.findall(r"rows \* (?:parts|ranks) \* 2 <= \d+", _source(path))
