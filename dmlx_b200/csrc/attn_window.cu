@@ -586,7 +586,7 @@ struct SimtArgs {
 // weighted sum; query and output row in shared memory.
 template <typename T>
 __global__ void __launch_bounds__(128) attn_simt_kernel(SimtArgs a) {
-  after_previous();
+  wait_previous();  // (and alone: its last, longest rows share the issue slots with all that wait)
   extern __shared__ float sh[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kd = a.L.key_dim, vd = a.L.value_dim;
   float* q = sh + warp * (kd + vd);
@@ -640,6 +640,7 @@ __global__ void __launch_bounds__(128) attn_simt_kernel(SimtArgs a) {
     }
     __syncwarp();
   }
+  let_next_start();
   float f = 1.f;
   if (a.sinks_log2) {
     const float sk = a.sinks_log2[qh], mm = fmaxf(m, sk);
@@ -793,7 +794,8 @@ b200_status b200_window_attn_run(b200_kv* kv, const WindowAttnCall& c, const int
     const unsigned grid = (unsigned)(((long long)total_rows * c.n_q_heads + 3) / 4);
     auto* kernel = kv->dev.elem_bytes == 4 ? attn_simt_kernel<float> : attn_simt_kernel<__nv_bfloat16>;
     if (smem > 48 * 1024) B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_after(kernel, grid, 128, smem, s, a);
+    if (total_rows > 64) launch_apart(kernel, grid, 128, smem, s, a);
+    else launch_after(kernel, grid, 128, smem, s, a);
     B200_LAUNCH_CHECK();
     return B200_OK;
   }

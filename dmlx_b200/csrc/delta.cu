@@ -137,12 +137,13 @@ struct Delta {
 // stays in memory.
 template <typename T, int VEC, int KEEP>
 __global__ void __launch_bounds__(256, KEEP == 32 ? 1 : 2) delta_step_kernel(Delta a) {
-  after_previous();
+  wait_previous();
   extern __shared__ float sh[];
   __shared__ float part[32];
   const int req = blockIdx.x, head = blockIdx.y, dk = a.g.dk, dv = a.g.dv;
   const int r0 = a.g.cu[req], count = a.g.cu[req + 1] - r0;
   if (count <= 0 || (a.g.chunked && count > kGlaStepTokens) || a.g.d.state[ST_ERR] != 0) return;
+  if (count <= kGlaStepTokens) let_next_start();  // (as in gla_step_kernel)
   const int groups = a.g.groups, cols = a.g.cols;
   float *red_k = sh, *red_q = red_k + groups * cols * VEC, *q = red_q + groups * cols * VEC, *k = q + dk, *out = k + dk;  // out [dv]
   const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, tx = tid % cols, ty = tid / cols;
@@ -567,7 +568,9 @@ b200_status b200_delta_run(b200_kv* kv, const GlaScratch& g, const DeltaCall& c,
     if (smem > 200 * 1024) { b200_set_error("delta rule: head widths %d / %d are too large", c.dk, c.dv); return B200_ERR_UNSUPPORTED; }
     auto run = [&](auto* kernel) -> b200_status {
       if (smem > 48 * 1024) B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      launch_after(kernel, dim3(n_req, c.heads), (z.cols * z.groups + 31) / 32 * 32, smem, s, a);
+      const bool brief = z.chunked || total_rows <= kGlaStepTokens * n_req;
+      if (brief) launch_after(kernel, dim3(n_req, c.heads), (z.cols * z.groups + 31) / 32 * 32, smem, s, a);
+      else launch_apart(kernel, dim3(n_req, c.heads), (z.cols * z.groups + 31) / 32 * 32, smem, s, a);
       B200_LAUNCH_CHECK();
       return B200_OK;
     };

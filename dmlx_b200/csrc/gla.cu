@@ -43,12 +43,13 @@ __device__ __forceinline__ Vec<VEC> memory_value(const Gla& a, int row, int head
 // ---- token by token ------------------------------------------------------------------------------------------
 template <typename T, int VEC, bool MEM>
 __global__ void __launch_bounds__(256, 3) gla_step_kernel(Gla a) {
-  after_previous();
+  wait_previous();
   extern __shared__ float sh[];
   __shared__ float part[32];
   const int req = blockIdx.x, head = blockIdx.y, dk = a.dk, dv = a.dv, dvs = MEM ? a.dvs : dv, dva = MEM && VEC == 1 ? a.dva : dvs;
   const int r0 = a.cu[req], count = a.cu[req + 1] - r0;
   if (count <= 0 || (a.chunked && count > kGlaStepTokens) || a.d.state[ST_ERR] != 0) return;
+  if (count <= kGlaStepTokens) let_next_start();  // (a longer walk is left alone: the next kernel's waiting warps would share its issue slots)
   float *q = sh, *k = q + dk, *al = k + dk, *a1 = al + dk, *red = a1 + (MEM ? 0 : a.rank);  // red [groups][dvs]
   const int tid = threadIdx.x, nthr = blockDim.x, groups = a.groups, tx = tid % a.cols, ty = tid / a.cols;
   const int slot = a.row_seq[r0];
@@ -952,7 +953,9 @@ b200_status b200_gla_run(b200_kv* kv, const GlaScratch& g, const GlaCall& c, con
     if (mem) kernel = f32 ? (v4 ? gla_step_kernel<float, 4, true> : gla_step_kernel<float, 1, true>)
                           : (v4 ? gla_step_kernel<__nv_bfloat16, 4, true> : gla_step_kernel<__nv_bfloat16, 1, true>);
     if (smem > 48 * 1024) B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_after(kernel, dim3(n_req, c.heads), (a.cols * a.groups + 31) / 32 * 32, smem, s, a);
+    const bool brief = a.chunked || total_rows <= kGlaStepTokens * n_req;  // (no long walk, or few)
+    if (brief) launch_after(kernel, dim3(n_req, c.heads), (a.cols * a.groups + 31) / 32 * 32, smem, s, a);
+    else launch_apart(kernel, dim3(n_req, c.heads), (a.cols * a.groups + 31) / 32 * 32, smem, s, a);
     B200_LAUNCH_CHECK();
   }
   if (!a.chunked || total_rows <= n_req) return B200_OK;

@@ -48,6 +48,13 @@ inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(std::forward<A>(args))...);
 }
 
+// The same without the overlap, for long kernels of about as many blocks as there are SMs: scheduled while the one ahead still fills most of them,
+// their blocks would come to lie two and three on the SMs that have room, and the others stay idle.
+template <class... P, class... A>
+inline void launch_apart(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  kernel<<<grid, block, smem, s>>>(static_cast<P>(std::forward<A>(args))...);
+}
+
 // CTAs of `kernel` that run at the same time in clusters of `size`, no more than `per_sm` on an SM of `sms`: a cluster's CTAs stay within a GPC, so
 // some SMs are left over (33 clusters of eight at two CTAs on each of 148 SMs).  Rounded down to 64: the last clusters find a place late (samplers, 33
 // rows of 128256 words, a nucleus of 0.9: 81 us as 33 clusters of eight, 76 as clusters of four).

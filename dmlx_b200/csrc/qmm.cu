@@ -3911,7 +3911,7 @@ struct F32Args {
 };
 
 __global__ void __launch_bounds__(256) qmm_f32_kernel(F32Args a) {
-  after_previous();
+  wait_previous();  // (and alone: eight working warps of an SM share its issue slots with all that wait)
   __shared__ float xs[kF32K][kF32Rows + 4];
   __shared__ float ws[kF32K][kTileN + 4];
   const int nt = blockIdx.x, tid = threadIdx.x, kc = a.kc, n_valid = a.n_valid, y_stride = a.y_stride;
@@ -3969,6 +3969,7 @@ __global__ void __launch_bounds__(256) qmm_f32_kernel(F32Args a) {
       __syncthreads();
     }
   }
+  let_next_start();
   const int n = nt * kTileN + tc;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -3988,6 +3989,13 @@ __global__ void __launch_bounds__(256) qmm_f32_kernel(F32Args a) {
     }
   }
 }
+
+// Beyond a tile of rows the kernel is long and its grid mostly small (15 matmuls of 900 rows, up to 7 weight tiles each: 1355 us scheduled early and with
+// the next kernel's blocks beside it, 728 with plain launches and now).
+void launch_f32(dim3 grid, int rows, const F32Args& a, cudaStream_t s) {
+  if (rows > kF32Rows) launch_apart(qmm_f32_kernel, grid, 256, 0, s, a);
+  else launch_after(qmm_f32_kernel, grid, 256, 0, s, a);
+}
 }  // namespace
 
 b200_status b200_qmm_f32_shaped(const b200_qweight* w, const float* d_x, int32_t rows, float* d_y, int32_t y_stride, int32_t n_valid,
@@ -4005,7 +4013,7 @@ b200_status b200_qmm_f32_shaped(const b200_qweight* w, const float* d_x, int32_t
   a.blocks = w->d_blocks; a.x = d_x; a.y = d_y; a.rows = rows; a.kc = w->kc; a.x_stride = w->k; a.y_stride = y_stride; a.n_valid = n_valid;
   a.epilogue = epilogue;
   a.shape = shape;
-  launch_after(qmm_f32_kernel, dim3(w->nt, (rows + kF32Rows - 1) / kF32Rows), 256, 0, (cudaStream_t)stream, a);
+  launch_f32(dim3(w->nt, (rows + kF32Rows - 1) / kF32Rows), rows, a, (cudaStream_t)stream);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -4024,7 +4032,7 @@ b200_status b200_qmm_f32_blocks(const b200_qweight* w, const float* d_x, int32_t
   F32Args a{};
   a.blocks = w->d_blocks; a.x = d_x; a.y = d_y; a.rows = rows; a.kc = w->kc; a.x_stride = x_stride; a.y_stride = y_stride; a.n_valid = w->n;
   a.expert_stride = (size_t)w->nt * w->kc * w->block_bytes; a.x_group = x_group; a.y_group = y_group;
-  launch_after(qmm_f32_kernel, dim3(w->nt, (rows + kF32Rows - 1) / kF32Rows, w->n_experts), 256, 0, (cudaStream_t)stream, a);
+  launch_f32(dim3(w->nt, (rows + kF32Rows - 1) / kF32Rows, w->n_experts), rows, a, (cudaStream_t)stream);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -4040,7 +4048,7 @@ b200_status b200_qmm_f32_grouped(const b200_qweight* w, const float* d_x, const 
   a.blocks = w->d_blocks; a.x = d_x; a.y = d_y; a.kc = w->kc; a.x_stride = w->k; a.y_stride = y_stride; a.n_valid = swiglu ? w->n / 2 : w->n;
   a.epilogue = epilogue; a.expert_stride = (size_t)w->nt * w->kc * w->block_bytes;
   a.items = d_items; a.n_items = d_n_items; a.order = d_order; a.order_div = order_div > 0 ? order_div : 1;
-  launch_after(qmm_f32_kernel, dim3(w->nt, max_items), 256, 0, (cudaStream_t)stream, a);
+  launch_f32(dim3(w->nt, max_items), max_items, a, (cudaStream_t)stream);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }

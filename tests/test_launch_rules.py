@@ -74,3 +74,15 @@ def test_grids_are_sized_by_the_device(path):
     """How many SMs there are, and how many CTAs run on them at once, is asked of the device."""
     assert not re.findall(r"[^\n]*\b(?:148|296)\b[^\n]*", _source(path))
     assert not re.findall(r"rows \* (?:parts|ranks) \* 2 <= \d+", _source(path))
+
+
+@pytest.mark.parametrize("kernel", ["qmm_f32_kernel", "attn_simt_kernel", "gla_step_kernel", "delta_step_kernel"])
+def test_long_kernels_do_not_share_their_sms(kernel):
+    """Warps that wait take issue slots from those that work, and blocks that are scheduled before the kernel ahead has ended lie on few SMs: a kernel that
+    may take long lets the next one start when its main loop is done, and has a launch of its own for that."""
+    bodies = [(_source(path)[start:], path) for file, name, start, path in KERNELS if name == kernel]
+    assert len(bodies) == 1
+    body, source = bodies[0][0], _source(bodies[0][1])
+    body = body[:body.index("\n}\n")]
+    assert "after_previous()" not in body and "wait_previous()" in body and "let_next_start()" in body
+    assert re.search(r"launch_apart\((?:kernel|%s)\b" % kernel, source)
