@@ -48,8 +48,12 @@ inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(std::forward<A>(args))...);
 }
 
-// The same without the overlap, for long kernels of about as many blocks as there are SMs: scheduled while the one ahead still fills most of them,
-// their blocks would come to lie two and three on the SMs that have room, and the others stay idle.
+// The same without the overlap, for two kinds of kernels:
+//   * long ones of about as many blocks as there are SMs: scheduled while the one ahead still fills most of them, its blocks would come to lie two
+//     and three on the SMs that have room, and the others stay idle;
+//   * many blocks of next to no work, kManyBlocks and more: each waits for the kernels ahead by itself, 0.4 ns a block of the whole chip's time.
+//     These neither wait nor let the next kernel start.
+constexpr int kManyBlocks = 2048;
 template <class... P, class... A>
 inline void launch_apart(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   kernel<<<grid, block, smem, s>>>(static_cast<P>(std::forward<A>(args))...);

@@ -525,11 +525,12 @@ __global__ void add_shared_kernel(const float* routed, const __nv_bfloat16* shar
   reinterpret_cast<uint4*>(out)[i] = o;
 }
 
+template <bool EARLY>
 __global__ void gather_sorted_kernel(const __nv_bfloat16* x, const int* order,
                                      const float* weights, int k, int hidden,
                                      __nv_bfloat16* __restrict__ x_sorted, float* __restrict__ row_scales,
                                      const int* n_valid) {
-  after_previous();
+  if constexpr (EARLY) after_previous();
   const int p = blockIdx.x;
   if (n_valid && p >= *n_valid) return;
   const int a = order[p];
@@ -537,6 +538,12 @@ __global__ void gather_sorted_kernel(const __nv_bfloat16* x, const int* order,
   uint4* dst = reinterpret_cast<uint4*>(x_sorted + (size_t)p * hidden);
   copy_vectors(dst, src, hidden / 8);
   if (threadIdx.x == 0 && row_scales) row_scales[p] = weights[a];
+}
+// As a rule of launches, so few blocks that their own waits cost less than the overlap gives (launch.cuh).
+template <class... A>
+void launch_gather(int rows, cudaStream_t s, A... args) {
+  if (rows <= kManyBlocks) launch_after(gather_sorted_kernel<true>, rows, 128, 0, s, args...);
+  else launch_apart(gather_sorted_kernel<false>, rows, 128, 0, s, args...);
 }
 
 __global__ void combine_kernel(const __nv_bfloat16* y_sorted, const int* inv_order, int k, int hidden,
@@ -697,8 +704,8 @@ b200_status b200_moe_gather(const void* d_x, const int32_t* d_order, const float
   if (st != B200_OK) return st;
   if (hidden % 8) { b200_set_error("gather: hidden must be a multiple of 8"); return B200_ERR_INVALID_ARGUMENT; }
   if (n_assign <= 0) return B200_OK;
-  launch_after(gather_sorted_kernel, n_assign, 128, 0, (cudaStream_t)stream, (const __nv_bfloat16*)d_x, d_order, d_weights, k, hidden,
-                                                                  (__nv_bfloat16*)d_x_sorted, d_row_scales, nullptr);
+  launch_gather(n_assign, (cudaStream_t)stream, (const __nv_bfloat16*)d_x, d_order, d_weights, k, hidden, (__nv_bfloat16*)d_x_sorted, d_row_scales,
+                (const int*)nullptr);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -968,7 +975,8 @@ b200_status b200_moe_forward_ep(b200_moe* m, b200_ep* ep, const void* d_x, int32
     STEP(b200_qmm_grouped_from_tokens(m->exp_gu, m->x_all, m->order, c.top_k, A, m->act_sorted, B200_EPI_SWIGLU, m->row_scales,
                                       c.swiglu_limit, m->items, m->n_items, m->max_items, c.tile_rows, stream, rows_valid));
   } else {
-    launch_after(gather_sorted_kernel, A, 128, 0, s, m->x_all, m->order, m->weights, c.top_k, c.hidden, m->x_sorted, nullptr, rows_valid);
+    launch_gather(A, s, (const __nv_bfloat16*)m->x_all, (const int*)m->order, (const float*)m->weights, c.top_k, c.hidden, (__nv_bfloat16*)m->x_sorted,
+                  (float*)nullptr, rows_valid);
     B200_LAUNCH_CHECK();
     STEP(b200_qmm_grouped(m->exp_gu, m->x_sorted, A, m->act_sorted, B200_EPI_SWIGLU, m->row_scales, c.swiglu_limit, m->items,
                           m->n_items, m->max_items, c.tile_rows, stream));

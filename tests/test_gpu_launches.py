@@ -63,6 +63,45 @@ def test_steps_of_early_kernels_equal_steps_kernel_by_kernel(runs, name):
         np.testing.assert_array_equal(early[again], one_by_one[name])
 
 
+@pytest.mark.parametrize("pages", ["bf16", "fp8"])
+@pytest.mark.parametrize("heads,rows", [(16, 127), (16, 128), (16, 129), (8, 257), (1, 2500)])
+def test_appends_in_few_blocks_and_in_many(pages, heads, rows):
+    """Up to 2048 blocks are launched early, more are not.  Rows come out as they went in; of FP8 pages within half a step of the code (2^-4 of its
+    magnitude, or 2^-10 of the scale, which is no more than the largest magnitude / 448) and the rounding of what is read back to bf16."""
+    import torch
+
+    from dmlx_b200 import device as dev
+
+    kv = dev.PagedKVCache(1, heads, 64, 200, 4, 100, 4 * heads, kv_dtype=dev.KV_FP8_E4M3 if pages == "fp8" else dev.KV_BF16)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    k, v = (torch.randn((rows, heads, 64), generator=g, device="cuda").bfloat16() for _ in range(2))
+    first = rows // 3
+    kv.reserve(dev.pack_desc_array([(0, first, 0, 0), (1, rows - first, 0, first)]).cuda())
+    kv.append(0, k, v)
+    for seq, a, b in ((0, 0, first), (1, first, rows)):
+        for got, want in zip(kv.gather(0, seq), (k, v)):
+            got, want = got.float(), want[a:b].float()
+            if pages == "bf16":
+                assert torch.equal(got, want)
+            else:
+                assert bool(((got - want).abs() <= want.abs() * (2.0 ** -4 + 2.0 ** -8) + want.abs().max() / 448 * 2.0 ** -9).all())
+    assert kv.error_word() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 2047, 2048, 2049, 5000])
+def test_rows_sorted_for_experts_by_few_blocks_and_by_many(rows):
+    import torch
+
+    from dmlx_b200 import device as dev
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    top = 1 if rows % 2 else 2
+    x, weights = torch.randn((rows // top, 264), generator=g, device="cuda").bfloat16(), torch.rand(rows, generator=g, device="cuda")
+    order = torch.randperm(rows, generator=g, device="cuda").int()
+    xs, scales = dev.moe_gather(x, order, weights, top)
+    assert torch.equal(xs, x[order.long() // top]) and torch.equal(scales, weights[order.long()])
+
+
 if __name__ == "__main__":
     results = {}
     for model in MODELS:
