@@ -90,13 +90,13 @@ __global__ void embed_kernel(const __nv_bfloat16* table, const uint32_t* ids,
 
 // First strict maximum of each row (ties keep the smaller index).
 // A row belongs to a cluster of CTAs, a contiguous part each (16 rows of 32000 f32 values: 9.9 us by a block each, 6.8 this way).
-template <typename T>
+template <typename T, bool WHOLE>  // WHOLE: a block has a row by itself
 __global__ void argmax_kernel(const T* logits, int vocab, uint32_t* __restrict__ out) {
   after_previous();
   __shared__ float s_val[32];
   __shared__ int s_idx[32];
   cg::cluster_group cluster = cg::this_cluster();
-  const int parts = cluster.num_blocks(), part = cluster.block_rank(), row = blockIdx.x / parts;
+  const int parts = WHOLE ? 1 : cluster.num_blocks(), part = WHOLE ? 0 : cluster.block_rank(), row = blockIdx.x / parts;
   const int per = ((vocab + parts - 1) / parts + 7) / 8 * 8, lo = min(part * per, vocab), hi = min(lo + per, vocab);
   const T* lr = logits + (size_t)row * vocab;
   float best = -INFINITY;
@@ -141,8 +141,10 @@ __global__ void argmax_kernel(const T* logits, int vocab, uint32_t* __restrict__
       int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (better(ov, oi, best, bi)) { best = ov; bi = oi; }
     }
-    if (threadIdx.x == 0) { s_val[0] = best; s_idx[0] = bi; }
+    if (WHOLE && threadIdx.x == 0) out[row] = bi == 0x7fffffff ? 0u : (uint32_t)bi;
+    if (!WHOLE && threadIdx.x == 0) { s_val[0] = best; s_idx[0] = bi; }
   }
+  if (WHOLE) return;
   cluster.sync();
   if (part == 0 && threadIdx.x == 0) {
     for (int q = 1; q < parts; ++q) {
@@ -158,12 +160,18 @@ __global__ void argmax_kernel(const T* logits, int vocab, uint32_t* __restrict__
 template <typename T>
 b200_status launch_argmax(const T* logits, int rows, int vocab, uint32_t* out, cudaStream_t s) {
   // parts of 4096 values and more, as long as the CTAs run at once, two per SM
-  static const int most = ctas_in_clusters(argmax_kernel<T>, 8, 2, b200_sm_count(), 512, 0);
+  static const int most = ctas_in_clusters(argmax_kernel<T, false>, 8, 2, b200_sm_count(), 512, 0);
   int parts = 1;
   while (parts < 8 && vocab >= parts * 8192 && (long long)rows * parts * 2 <= most) parts *= 2;
+  if (parts == 1) {  // (as clusters of one 1000 rows of 4097 values took 15.8 us, 9.9 so; 150 rows of 128256 f32 values, scheduled early 45, apart 34)
+    if (vocab < 32768) launch_after(argmax_kernel<T, true>, rows, 1024, 0, s, logits, vocab, out);
+    else launch_apart(argmax_kernel<T, true>, rows, 1024, 0, s, logits, vocab, out);
+    B200_LAUNCH_CHECK();
+    return B200_OK;
+  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)rows * parts);
-  cfg.blockDim = dim3(parts > 1 ? 512 : 1024);
+  cfg.blockDim = dim3(512);
   cfg.stream = s;
   cudaLaunchAttribute attr[2]{};
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -173,7 +181,7 @@ b200_status launch_argmax(const T* logits, int rows, int vocab, uint32_t* out, c
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, argmax_kernel<T>, logits, vocab, out));
+  B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, argmax_kernel<T, false>, logits, vocab, out));
   B200_LAUNCH_CHECK();
   return B200_OK;
 }

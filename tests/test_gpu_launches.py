@@ -102,6 +102,20 @@ def test_rows_sorted_for_experts_by_few_blocks_and_by_many(rows):
     assert torch.equal(xs, x[order.long() // top]) and torch.equal(scales, weights[order.long()])
 
 
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("rows", [128, 129, 150, 1000])
+@pytest.mark.parametrize("vocab", [1, 4097, 32760, 32768, 50257])
+def test_first_maximum_of_rows_by_blocks_and_by_clusters(dtype, rows, vocab):
+    import torch
+
+    from dmlx_b200 import device as dev
+
+    g = torch.Generator(device="cuda").manual_seed(rows + vocab)
+    x = torch.randint(-40, 41, (rows, vocab), generator=g, device="cuda").to(getattr(torch, dtype))  # (ties in every row)
+    first = torch.where(x == x.amax(1, keepdim=True), torch.arange(vocab, device="cuda"), vocab).amin(1)
+    assert torch.equal(dev.argmax(x).long(), first)
+
+
 if __name__ == "__main__":
     results = {}
     for model in MODELS:
