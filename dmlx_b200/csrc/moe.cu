@@ -651,6 +651,8 @@ static void by_experts(int n_experts, F f) {
   else if (n_experts <= 64) f(std::integral_constant<int, 2>{});
   else if (n_experts <= 128) f(std::integral_constant<int, 4>{});
   else if (n_experts <= 256) f(std::integral_constant<int, 8>{});
+  else if (n_experts <= 384) f(std::integral_constant<int, 12>{});
+  else if (n_experts <= 512) f(std::integral_constant<int, 16>{});
   else f(std::integral_constant<int, 32>{});
 }
 

@@ -116,6 +116,28 @@ def test_first_maximum_of_rows_by_blocks_and_by_clusters(dtype, rows, vocab):
     assert torch.equal(dev.argmax(x).long(), first)
 
 
+@pytest.mark.parametrize("experts,top", [(256, 8), (257, 8), (384, 8), (385, 3), (512, 10), (513, 10), (1024, 16)])
+@pytest.mark.parametrize("scoring", [0, 1, 2])
+def test_routes_at_the_edges_of_what_a_lane_holds(experts, top, scoring):
+    """The chosen experts in ascending score, and their weights: f32 arithmetic of a few dozen operations, 2^-18 of the weight."""
+    import torch
+
+    from dmlx_b200 import device as dev
+
+    g = torch.Generator(device="cuda").manual_seed(experts)
+    logits = torch.stack([torch.randperm(experts, generator=g, device="cuda") for _ in range(40)]).float() * (16.0 / experts) - 8.0  # (no two alike)
+    index, weight, counts = dev.moe_route(logits, top, scoring=scoring)
+    x = logits.double()
+    score = (torch.softmax(x, 1), torch.sigmoid(x), torch.nn.functional.softplus(x).sqrt())[scoring]
+    want, place = score.topk(top, dim=1)
+    want, place = want.flip(1), place.flip(1)
+    if scoring:
+        want = want / want.sum(1, keepdim=True)
+    assert torch.equal(index.long(), place)
+    assert bool(((weight.double() - want).abs() <= 2.0 ** -18 * want).all())
+    assert torch.equal(counts.long(), torch.bincount(place.flatten(), minlength=experts))
+
+
 if __name__ == "__main__":
     results = {}
     for model in MODELS:
