@@ -160,7 +160,7 @@ __global__ void argmax_kernel(const T* logits, int vocab, uint32_t* __restrict__
 template <typename T>
 b200_status launch_argmax(const T* logits, int rows, int vocab, uint32_t* out, cudaStream_t s) {
   // parts of 4096 values and more, as long as the CTAs run at once, two per SM
-  static const int most = ctas_in_clusters(argmax_kernel<T, false>, 8, 2, b200_sm_count(), 512, 0);
+  static const int most = ctas_in_clusters(argmax_kernel<T, false>, 8, 2, b200_sm_count(), 512, 0) / 64 * 64;
   int parts = 1;
   while (parts < 8 && vocab >= parts * 8192 && (long long)rows * parts * 2 <= most) parts *= 2;
   if (parts == 1) {  // (as clusters of one 1000 rows of 4097 values took 15.8 us, 9.9 so; 150 rows of 128256 f32 values, scheduled early 45, apart 34)

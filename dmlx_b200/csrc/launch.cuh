@@ -60,8 +60,7 @@ inline void launch_apart(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
 }
 
 // CTAs of `kernel` that run at the same time in clusters of `size`, no more than `per_sm` on an SM of `sms`: a cluster's CTAs stay within a GPC, so
-// some SMs are left over (33 clusters of eight at two CTAs on each of 148 SMs).  Rounded down to 64: the last clusters find a place late (samplers, 33
-// rows of 128256 words, a nucleus of 0.9: 81 us as 33 clusters of eight, 76 as clusters of four).
+// some SMs are left over (33 clusters of eight, 71 of four and 148 of two at two CTAs on each of 148 SMs).
 template <class... P>
 inline int ctas_in_clusters(void (*kernel)(P...), int size, int per_sm, int sms, int threads, size_t smem) {
   cudaLaunchAttribute attr{};
@@ -80,6 +79,6 @@ inline int ctas_in_clusters(void (*kernel)(P...), int size, int per_sm, int sms,
     cudaGetLastError();
     return 0;
   }
-  return (int)((long long)clusters * size * std::min(per_sm, fit) / fit) / 64 * 64;
+  return (int)((long long)clusters * size * std::min(per_sm, fit) / fit);
 }
 #endif

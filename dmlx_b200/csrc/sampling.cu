@@ -772,9 +772,13 @@ b200_status launch(const T* logits, int rows, int vocab, const Params& params, c
   B200_CUDA_TRY(cudaFuncSetAttribute(sample_rows_kernel<T, Params>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared)));
   // CTAs per row: 8192 words each at least (16 a thread), and no more altogether than run at the same time (37 rows, a nucleus of 0.9: 111 us in eight
   // CTAs a row, 88 in four).
-  static const int most = ctas_in_clusters(sample_rows_kernel<T, Params>, kMaxCluster, 2, b200_sm_count(), kThreads, sizeof(Shared));
+  // Of eights less the last few, which find a place late: 33 rows of 128256 words, a nucleus of 0.9, 81 us as eights and 76 as fours; 129 rows take
+  // 150 us in a CTA each, 107 in pairs, 65 rows 94 us in pairs and 80 as fours.
+  auto at_once = [](int size) { return ctas_in_clusters(sample_rows_kernel<T, Params>, size, 2, b200_sm_count(), kThreads, sizeof(Shared)); };
+  static_assert(kMaxCluster == 8);
+  static const int most[] = {at_once(2), at_once(4), at_once(8) / 64 * 64};
   int ranks = 1;
-  while (ranks < kMaxCluster && vocab > ranks * 8192 && (long long)rows * ranks * 2 <= most) ranks *= 2;
+  for (int i = 0; i < 3 && vocab > ranks * 8192 && (long long)rows * ranks * 2 <= most[i]; ++i) ranks *= 2;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)rows * ranks);
   cfg.blockDim = dim3(kThreads);

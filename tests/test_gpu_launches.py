@@ -138,6 +138,23 @@ def test_routes_at_the_edges_of_what_a_lane_holds(experts, top, scoring):
     assert torch.equal(counts.long(), torch.bincount(place.flatten(), minlength=experts))
 
 
+@pytest.mark.parametrize("rows", [32, 33, 64, 71, 72, 128, 148, 149])
+def test_samplers_of_rows_in_clusters_of_every_size(rows):
+    """A row's token and log-probability do not depend on how many CTAs share it."""
+    import torch
+
+    from dmlx_b200 import device as dev
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    logits = (3 * torch.randn((rows, 70000), generator=g, device="cuda")).bfloat16()
+    kinds = [(0.0, 50, 1.0), (0.8, 50, 1.0), (0.8, 50, 0.9), (0.9, 0, 1.0), (0.8, 0, 0.9)]
+    params = [(*kinds[i % 5], (i + 0.5) / rows) for i in range(rows)]
+    tokens, lp = dev.sample_rows(logits, params)
+    for i in range(0, rows, 7):
+        alone, lp_alone = dev.sample_rows(logits[i:i + 1].contiguous(), params[i:i + 1])
+        assert int(alone) == int(tokens[i]) and float(lp_alone) == float(lp[i])
+
+
 if __name__ == "__main__":
     results = {}
     for model in MODELS:
