@@ -166,9 +166,9 @@ __device__ __forceinline__ void finish_store(const QmmArgs& a, int token, int n,
 // ---- split-K finish: sums the partial tiles in split order (deterministic), applies the epilogue,
 // writes bf16.  One thread per 4 consecutive output columns of one row, so the whole GPU takes
 // part and every thread has `splits` independent 16-byte loads in flight.
-// The next kernel, more often than not another stream of weights, is let start when the sums have arrived, behind SwiGLU's arithmetic at the end.  Let
-// start at once, its loads came in between: MXFP4 28672 x 4096, 8 rows, 39.1 us (32.9 with plain launches), 29.3 this way; 160 shapes of up to
-// 16 rows 2 % less altogether.
+// The next kernel, more often than not another stream of weights, is let start when all that is read here has arrived: the sums, or with an epilogue at
+// the end.  Let start at once, its loads came in between: MXFP4 28672 x 4096, 8 rows, 39.1 us (32.9 with plain launches), 29.3 this way; with a
+// residual 38.6, let start ahead of its loads, and 29.4; 160 shapes of up to 16 rows 2 % less altogether.
 __global__ void qmm_finish_kernel(QmmArgs a, int splits) {
   wait_previous();
   const int n4 = a.nt * (kTileN / 4);
@@ -204,7 +204,7 @@ __global__ void qmm_finish_kernel(QmmArgs a, int splits) {
     const float4 v = p[(size_t)s * split_stride];
     acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
   }
-  if (a.epilogue != B200_EPI_SWIGLU) let_next_start();
+  if (a.epilogue == B200_EPI_NONE) let_next_start();
   finish_store(a, token, n, acc);
 }
 
@@ -3316,7 +3316,7 @@ static b200_status launch_cp(QmmArgs& a, int rows, cudaStream_t s) {
   a.stages = std::min(kCpMaxStages, (smem_budget[MODE] - fixed) / (2 * kTileN * 128));
   cfg.dynamicSmemBytes = (size_t)a.stages * 2 * kTileN * 128 + fixed;
   // K is split where the items would leave pairs of CTAs idle in their last round: rounds x chunks, and for partial sums a finish pass of some 16
-  // chunks and their way to memory and back, 2.5 MB in the time of a chunk
+  // chunks and their way to memory and back, 2.5 MB in the time of a chunk.
   const int items = (a.nt + 1) / 2 * tts;
   int splits = 1;
   double best = 0;
