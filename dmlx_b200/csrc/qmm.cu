@@ -3316,7 +3316,9 @@ static b200_status launch_cp(QmmArgs& a, int rows, cudaStream_t s) {
   a.stages = std::min(kCpMaxStages, (smem_budget[MODE] - fixed) / (2 * kTileN * 128));
   cfg.dynamicSmemBytes = (size_t)a.stages * 2 * kTileN * 128 + fixed;
   // K is split where the items would leave pairs of CTAs idle in their last round: rounds x chunks, and for partial sums a finish pass of some 16
-  // chunks and their way to memory and back, 2.5 MB in the time of a chunk.
+  // chunks and their way to memory and back, 2.5 MB in the time of a chunk.  SwiGLU's arithmetic on the last item is not hidden behind another one's
+  // MMAs, a finish pass has the whole chip for it (dense 1024 x 2048, 256 rows: 21.2 us unsplit, 16.8 in two ranges; 17.0 on two tiles per CTA before)
+  const double tail = a.epilogue == B200_EPI_SWIGLU ? a.tn / 32 : 0;
   const int items = (a.nt + 1) / 2 * tts;
   int splits = 1;
   double best = 0;
@@ -3324,7 +3326,7 @@ static b200_status launch_cp(QmmArgs& a, int rows, cudaStream_t s) {
     const int cps = (a.kc + sp - 1) / sp;
     if ((a.kc + cps - 1) / cps != sp) continue;
     const double rounds = (items * sp + most_pairs[MODE] - 1) / most_pairs[MODE];
-    const double cost = rounds * (cps + 2) + (sp > 1 ? 16.0 + (double)rows * a.n * sp * 8.0 / 2.5e6 : 0.0);
+    const double cost = rounds * (cps + 2) + (sp > 1 ? 16.0 + (double)rows * a.n * sp * 8.0 / 2.5e6 : tail);
     if (sp == 1 || cost < best) { best = cost; splits = sp; }
   }
   a.splits = splits;

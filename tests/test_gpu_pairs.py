@@ -84,6 +84,13 @@ def test_pairs_of_ctas_repeat_themselves(mode, n, k, rows):
     assert dev.qmm_error_word() == 0
 
 
+# K in one range and in two, where SwiGLU decides
+@pytest.mark.parametrize("mode", ["bf16", "affine4", "mxfp4"])
+@pytest.mark.parametrize("n,k,rows", [(1024, 2048, 256), (1024, 2048, 400), (1024, 1024, 300), (512, 3072, 700)])
+def test_pairs_of_ctas_of_small_matrices(mode, n, k, rows):
+    _run(mode, n, k, rows, "QMM_TCGEN05_X2")
+
+
 @pytest.mark.parametrize("n", [33, 34, 129, 130])
 @pytest.mark.parametrize("rows", [65, 128, 200, 300])
 def test_outputs_that_do_not_come_in_fours(n, rows):
