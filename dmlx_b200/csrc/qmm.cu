@@ -1189,7 +1189,7 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
   constexpr int SR = Z::kRawSlots, BR = Z::kRawBars, kRoles = Z::kWorkers;  // kRoles: first of the warps with a role of their own
   const int S = a.stages, kc = a.kc;
   unsigned char* raw = smem + (size_t)S * kStage;
-  float* staging = reinterpret_cast<float*>(raw + SR * BB);  // [epilogue warp][16 tokens][32 rows]
+  float* staging = reinterpret_cast<float*>(raw + SR * BB);  // [epilogue warp][kBatch tokens][32 rows]
   uint64_t* bars = reinterpret_cast<uint64_t*>(staging + Z::kEpilogue * Z::kBatch * kCpPitch);
   const uint32_t smem_u = ptx::smem_u32(smem), raw_u = ptx::smem_u32(raw), bars_u = ptx::smem_u32(bars);
   const uint32_t full = bars_u;               // [S] this CTA's half of the stage is complete
@@ -1392,9 +1392,9 @@ __global__ void __launch_bounds__(CpShape<MODE>::kThreads, 1) qmm_cp_kernel(cons
       }
     }
   } else {
-    // ---- a warp's 32 weight rows, 16 tokens at a time, through shared memory: 16-byte stores (2-byte ones straight from the accumulator layout
+    // ---- a warp's 32 weight rows, kBatch tokens at a time, through shared memory: 16-byte stores (2-byte ones straight from the accumulator layout
     // took longer than the MMAs: 2026 rows of 16384 x 2048 with SwiGLU 161 us, 94 this way, 71 without an epilogue) ----
-    const int lq = warp & 3, part = (warp - kRoles - 4) >> 2;  // dense: two warps share a quarter, half of the tokens each
+    const int lq = warp & 3, part = (warp - kRoles - 4) >> 2;  // two warps share a quarter, half of the tokens each
     constexpr int kParts = Z::kEpilogue / 4, kB = Z::kBatch, kPieces = kB / 8;  // pieces of eight outputs of a lane
     float* tile = staging + (warp - kRoles - 4) * kB * kCpPitch;
     const uint32_t to = ptx::map_to_rank(acc_free, 0);
@@ -2270,7 +2270,6 @@ __device__ __forceinline__ float2 mx_e4m3x2_to_f32x2(uint32_t codes) {
   return __half22float2(*reinterpret_cast<const __half2*>(&h));
 }
 
-// x [rows, k] bf16 -> hi, lo [rows, k] E4M3 and unscale[rows].  One CTA per row; k % 8 == 0.
 // A row's codes, hi and residual, by a block of 256 threads; f(first column / 8, hi of eight columns, lo of them) stores them.  Returns the factor
 // that undoes the row's scaling.  What a thread read for the row's maximum stays in registers up to K = 4096.
 template <typename F>
@@ -2322,6 +2321,7 @@ __device__ __forceinline__ float split_row(const uint4* __restrict__ xr, int k8,
   return __uint_as_float((uint32_t)(127 + ex - 7) << 23);
 }
 
+// x [rows, k] bf16 -> hi, lo [rows, k] E4M3 and unscale[rows].  One CTA per row; k % 8 == 0.
 __global__ void __launch_bounds__(256) mx_split_activations_kernel(const __nv_bfloat16* x, int k,
                                                                    unsigned char* __restrict__ hi, unsigned char* __restrict__ lo,
                                                                    float* __restrict__ unscale, const int* gather,
