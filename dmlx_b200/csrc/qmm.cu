@@ -163,14 +163,19 @@ __device__ __forceinline__ void finish_store(const QmmArgs& a, int token, int n,
   }
 }
 
+constexpr int kFewRows = 16;  // rows of the kernels that are streams of weights
+constexpr int kNarrow = 64;   // weight tiles whose finish pass is short
 // ---- split-K finish: sums the partial tiles in split order (deterministic), applies the epilogue,
 // writes bf16.  One thread per 4 consecutive output columns of one row, so the whole GPU takes
 // part and every thread has `splits` independent 16-byte loads in flight.
-// The next kernel, more often than not another stream of weights, is let start when all that is read here has arrived: the sums, or with an epilogue at
-// the end.  Let start at once, its loads came in between: MXFP4 28672 x 4096, 8 rows, 39.1 us (32.9 with plain launches), 29.3 this way; with a
-// residual 38.6, let start ahead of its loads, and 29.4; 160 shapes of up to 16 rows 2 % less altogether.
+// Of up to 16 rows and more than 64 weight tiles the next kernel, more often than not another stream of weights that fills the memory's queues, is let
+// start when all that is read here has arrived: the sums, or with an epilogue at the end.  Let start at once, its loads came in between: MXFP4
+// 28672 x 4096, 8 rows, 38.6 us (32.9 with plain launches), 28.8 this way, with a residual 38.6 and 29.4.  Elsewhere it is let start at once: 24
+// tokens of 32 experts 139.8 us, 144.7 with the wait (8 tokens 110.1 and 112.0).
 __global__ void qmm_finish_kernel(QmmArgs a, int splits) {
   wait_previous();
+  const bool late = a.rows <= kFewRows && a.nt > kNarrow;
+  if (!late) let_next_start();
   const int n4 = a.nt * (kTileN / 4);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)a.rows * n4) return;
@@ -204,7 +209,7 @@ __global__ void qmm_finish_kernel(QmmArgs a, int splits) {
     const float4 v = p[(size_t)s * split_stride];
     acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
   }
-  if (a.epilogue == B200_EPI_NONE) let_next_start();
+  if (late && a.epilogue == B200_EPI_NONE) let_next_start();
   finish_store(a, token, n, acc);
 }
 
@@ -1894,7 +1899,7 @@ __global__ void __launch_bounds__(kGemvThreads, NT8 >= 4 ? 1 : 2) qmm_mma_kernel
 // the activations are read in the same pieces).  Many light CTAs, 32 to 64 KB of weights in flight per SM and CTA-wide set-up of nothing,
 // against a tensor-memory allocation, barriers, a ring and a finish pass per launch in qmm_tc_kernel: with 8 rows, 1536 x 512 outputs x K took
 // 5.3 + 2.2 us there and 2.5 here, 2816 x 512 2.9; experts of a step of 16 rows 56 -> 45 us (gate/up) and 37 -> 25 (down).
-constexpr int kFewRows = 16, kFewWarps = 8;
+constexpr int kFewWarps = 8;
 
 template <int MT, int NT>
 __global__ void __launch_bounds__(kFewWarps * 32) qmm_few_kernel(QmmArgs a) {

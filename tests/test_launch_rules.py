@@ -88,8 +88,9 @@ def test_long_kernels_do_not_share_their_sms(kernel):
     assert re.search(r"launch_apart\((?:kernel|%s)\b" % kernel, source)
 
 
-def test_the_finish_pass_lets_the_next_kernel_start_when_all_it_reads_has_arrived():
+def test_the_finish_pass_of_few_rows_and_many_outputs_lets_the_next_kernel_start_when_all_it_reads_has_arrived():
     """An epilogue's own loads and arithmetic come behind the sums: only without one may the next stream of weights begin there."""
     body = next(_source(path)[start:] for file, name, start, path in KERNELS if name == "qmm_finish_kernel")
     body = body[:body.index("\n}\n")]
-    assert re.findall(r"[^\n]*let_next_start\(\);", body) == ["  if (a.epilogue == B200_EPI_NONE) let_next_start();"]
+    assert re.findall(r"[^\n]*let_next_start\(\);", body) == ["  if (!late) let_next_start();", "  if (late && a.epilogue == B200_EPI_NONE) let_next_start();"]
+    assert body.index("if (!late)") < body.index("v0 = p[") < body.index("if (late")
